@@ -88,6 +88,7 @@ class AllReduceParams(Structure):
 
 
 _lib = None
+_native = None
 
 
 def load() -> ctypes.CDLL:
@@ -149,6 +150,20 @@ def load() -> ctypes.CDLL:
         lib.kb_debug_pdl(0)  # launch every kernel with plain stream ordering (A/B measurements)
     _lib = lib
     return lib
+
+
+def native():
+    """The CPython module `_host_ops` (csrc/host_ops.cpp): the op front-ends' direct path from tensors to
+    the C ABI. Each of its functions returns None when the operands need the front-end's general path."""
+    global _native
+    if _native is None:
+        load()
+        try:
+            from kernl_b200 import _host_ops
+        except ImportError as e:
+            raise RuntimeError(f"kernl_b200/_host_ops.so cannot be loaded ({e}): build it with `python -m kernl_b200.build`") from e
+        _native = _host_ops
+    return _native
 
 
 def status_str(status: int) -> str:

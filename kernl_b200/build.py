@@ -1,12 +1,15 @@
-"""Builds the CUDA library of kernl_b200 in-tree with nvcc for sm_100a.
+"""Builds the CUDA library of kernl_b200 in-tree with nvcc for sm_100a, and the CPython module that
+calls it from tensors.
 
-`python -m kernl_b200.build` writes kernl_b200/libkernl_b200.so next to this file. nvcc
-cross-compiles without a GPU, so this runs on any box that has the CUDA toolkit.
+`python -m kernl_b200.build` writes kernl_b200/libkernl_b200.so and kernl_b200/_host_ops.so next to
+this file. nvcc cross-compiles without a GPU, so this runs on any box that has the CUDA toolkit.
 """
+import hashlib
 import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
@@ -28,47 +31,81 @@ def _nvcc() -> str:
 
 
 HASH_PATH = LIB_PATH + ".srchash"
+PUBLIC_HEADERS = [os.path.join(HERE, "..", "include", h) for h in ("kernl_b200.h", "kernl_b200_debug.h")]
+HOST_PATH = os.path.join(HERE, "_host_ops.so")
+HOST_SOURCE = os.path.join(CSRC, "host_ops.cpp")
+HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared"]
 
 
-def _source_hash() -> str:
-    """Hash of everything the library is built from (sources, headers, flags)."""
-    import hashlib
-
-    h = hashlib.sha256(" ".join(NVCC_FLAGS).encode())
-    deps = [os.path.join(CSRC, f) for f in SOURCES + HEADERS]
-    deps += [os.path.join(HERE, "..", "include", "kernl_b200.h"), os.path.join(HERE, "..", "include", "kernl_b200_debug.h")]
+def _hash(deps, *words) -> str:
+    h = hashlib.sha256(" ".join(words).encode())
     for d in deps:
         with open(d, "rb") as f:
             h.update(f.read())
     return h.hexdigest()
 
 
-def is_stale() -> bool:
-    """The library is rebuilt when it is missing or was built from other sources. By content, not by
+def _source_hash() -> str:
+    """Hash of everything the library is built from (sources, headers, flags)."""
+    return _hash([os.path.join(CSRC, f) for f in SOURCES + HEADERS] + PUBLIC_HEADERS, *NVCC_FLAGS)
+
+
+def _host_hash() -> str:
+    """The same for the CPython module, which is also bound to this torch and this Python."""
+    import torch
+
+    return _hash([HOST_SOURCE] + PUBLIC_HEADERS, *HOST_FLAGS, torch.__version__, sys.version)
+
+
+def _differs(path, current_hash) -> bool:
+    """A binary is rebuilt when it is missing or was built from other sources. By content, not by
     modification time: a copy of the tree to another machine keeps the contents, not the times."""
-    if not os.path.exists(LIB_PATH) or not os.path.exists(HASH_PATH):
+    if not os.path.exists(path) or not os.path.exists(path + ".srchash"):
         return True
     try:
-        return open(HASH_PATH).read().strip() != _source_hash()
+        with open(path + ".srchash") as f:
+            return f.read().strip() != current_hash
     except OSError:
         return True
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile csrc/*.cu into libkernl_b200.so (skipped when up to date). Returns the path."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += ["-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
+def is_stale() -> bool:
+    return _differs(LIB_PATH, _source_hash()) or _differs(HOST_PATH, _host_hash())
+
+
+def _compile(cmd, path, source_hash, verbose=False) -> None:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
+        raise RuntimeError(f"{os.path.basename(cmd[0])} failed:\n" + proc.stdout + proc.stderr)
     if verbose:
         print(proc.stderr)
-    with open(HASH_PATH, "w") as f:
-        f.write(_source_hash() + "\n")
+    with open(path + ".srchash", "w") as f:
+        f.write(source_hash + "\n")
+
+
+def _build_host() -> None:
+    import torch
+
+    root = os.path.dirname(torch.__file__)
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")]
+    libs = ["torch_python", "torch_cuda", "torch_cpu", "torch", "c10_cuda", "c10"]
+    cmd = [shutil.which("g++") or "g++", *HOST_FLAGS, *(f"-I{i}" for i in include), "-o", HOST_PATH, HOST_SOURCE,
+           f"-L{HERE}", "-l:" + os.path.basename(LIB_PATH), "-L" + os.path.join(root, "lib"), *(f"-l{x}" for x in libs), "-Wl,-rpath,$ORIGIN"]
+    _compile(cmd, HOST_PATH, _host_hash())
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compile csrc/*.cu into libkernl_b200.so and csrc/host_ops.cpp into _host_ops.so (each skipped
+    when up to date). Returns the library's path."""
+    if force or _differs(LIB_PATH, _source_hash()):
+        cmd = [_nvcc(), *NVCC_FLAGS]
+        if verbose:
+            cmd += ["-Xptxas", "-v"]
+        cmd += ["-o", LIB_PATH] + [os.path.join(CSRC, s) for s in SOURCES]
+        _compile(cmd, LIB_PATH, _source_hash(), verbose)
+    if force or _differs(HOST_PATH, _host_hash()):
+        _build_host()
     return LIB_PATH
 
 

@@ -128,6 +128,9 @@ def attention_forward(
     columns; the tensor maps end at the real head dimension and TMA fills the rest with zeros). Beyond the reference:
     k/v may carry fewer heads than q (grouped-query attention, see `kv_group_of`).
     """
+    done = _lib.native().attention(q, k, v, output, sm_scale, is_causal, attention_mask)
+    if done is not None:
+        return done
     q, k, v, output, attention_mask = cast_if_autocast(q, k, v, output, attention_mask)
     assert q.shape[-1] == k.shape[-1]
     assert (

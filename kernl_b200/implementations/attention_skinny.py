@@ -29,6 +29,9 @@ def skinny_attention_forward(
     loaded nor scored, and because the kernel reads the count, a captured graph follows a growing
     cache (the `start_position` of experimental/llama-v2/kernel/fused_kernel_attention.py:30,63,76).
     """
+    done = _lib.native().decode_attention(q, k, v, output, sm_scale, is_causal, attention_mask, kv_len)
+    if done is not None:
+        return done
     q, k, v, output, attention_mask = cast_if_autocast(q, k, v, output, attention_mask)
     assert q.shape[-1] == k.shape[-1]
     assert (

@@ -52,6 +52,9 @@ def layer_norm(
     return the pair (y, x + residual). `out` (an extension as well): a caller-provided result tensor
     shaped like x, written instead of a new one.
     """
+    done = _lib.native().layer_norm(x, weight, bias, eps, use_rms_norm, residual, out)
+    if done is not None:
+        return done
     x, weight, bias, residual = cast_if_autocast(x, weight, bias, residual)
     assert x.dtype == weight.dtype, f"input and weight bias must have the same dtype: {x.dtype}, {weight.dtype}"
     if bias is not None:

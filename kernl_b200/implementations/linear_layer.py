@@ -25,6 +25,7 @@ def _workspace(device: torch.device) -> torch.Tensor:
         with torch.inference_mode(False):  # an ordinary tensor: it is zeroed in place again after an expired wait
             ws = torch.zeros(_WORKSPACE_BYTES // 4, dtype=torch.float32, device=device)
         _workspaces[key] = ws
+        _lib.native().register_workspace(*key, ws.data_ptr(), ws.numel() * 4)
     return ws
 
 
@@ -79,6 +80,9 @@ def linear_layer(
     signature) lets the caller provide the [M, N] result buffer (unit column stride, any row stride),
     e.g. a peer-mapped one or a column slice of a wider tensor.
     """
+    done = _lib.native().linear(x, weight, bias, _lib.ACTIVATIONS[activation], act_inputs, out) if activation in _lib.ACTIVATIONS else None
+    if done is not None:
+        return done
     x, weight, bias = cast_if_autocast(x, weight, bias)
     x_ = x if x.ndim == 2 else x.flatten(0, 1)
     assert x.dtype == weight.dtype, f"Input and weight must have the same dtype, got {x.dtype} and {weight.dtype}"

@@ -12,6 +12,9 @@ def rope_kv_write(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     k_cache / v_cache: [batch, H, max_seq, D] contiguous; cos / sin: fp32 [max_seq, D/2];
     pos: start position (int, or a 1-element int64 device tensor for captured decode steps).
     Returns q rotated, [batch, seq, H, D]; k (rotated) and v are written into the caches."""
+    done = _lib.native().rope_kv_write(qkv, k_cache, v_cache, cos, sin, pos, batch, seq)
+    if done is not None:
+        return done
     B, H, max_seq, D = k_cache.shape
     assert B == batch and v_cache.shape == k_cache.shape and k_cache.is_contiguous() and v_cache.is_contiguous()
     assert qkv.is_contiguous() and qkv.shape == (batch * seq, 3 * H * D) and qkv.dtype == k_cache.dtype
