@@ -1,10 +1,9 @@
-// Decode-shape ("skinny") attention for sm_100a: few query rows against many keys.
-// With one query row the tensor cores are pointless (M=1) and the op is bound by streaming K and V
-// from HBM once, so this is a CUDA-core split-KV kernel:
-//   part 1  grid (splits, M, B*H): each CTA scores a chunk of keys for one query row (one key per
-//           thread, 128-bit loads), runs the online softmax over the chunk in blocks of 128 keys and
-//           accumulates exp(S-m)·V; it writes (m, l, acc[D]) fp32 to scratch
-//   part 2  grid (M, B*H): merges the chunks with the online-softmax recurrence and writes O
+// Decode-shape ("skinny") attention for sm_100a: few query rows against many keys, bound by streaming
+// K and V from HBM once.
+//   attn_decode_group_kernel  the common layout: one CTA per K/V head and key share, the query heads of
+//                             a group as the rows of mma.sync, shares merged inside a cluster
+//   attn_decode_part1/2       any strides and head dimensions: one key per thread, partial results of
+//                             chunks (m, l, acc[D]) in fp32 scratch, merged by the second kernel
 // Same maths as src/kernl/implementations/attention_skinny.py:58-366 of the reference (which keeps
 // its partial outputs in fp16; fp32 here). Additive masks and the causal flag are honoured in-kernel.
 #pragma once
@@ -162,180 +161,280 @@ attn_decode_part1_kernel(const DecDev p) {
     }
 }
 
-// Coalesced variant of part 1 for the common layout (unit stride on the head dimension, rows 16-byte
-// aligned, D = 8 * LPK with LPK lanes per key in {8, 16, 32}): the lanes of a warp cover 32/LPK whole
-// keys per step with one 128-bit load each, so every load instruction of a warp reads 512 contiguous
-// bytes of K (or V) and each byte is requested exactly once. Scores are reduced over the LPK lanes
-// with shuffles; for P·V each lane accumulates its 8 output dimensions over the keys it sees and the
-// 128/LPK key groups of the CTA are summed through shared memory at the end.
-template <typename T, int LPK>
-__global__ void __launch_bounds__(kDecThreads)
-attn_decode_part1_vec_kernel(const DecDev p) {
+// Split-KV kernel for the common layout (unit stride on the head dimension, 16-byte aligned rows,
+// D = 64, 128 or 256). Bound: streaming K and V from HBM once.
+//   * One CTA of four warps takes one K/V head of one sequence, one query row, and one contiguous
+//     share of the keys. The query heads of a group (grouped-query attention) are the ROWS of the
+//     tensor-core operand, so a group reads its K/V once; with one CTA per query head a group of four
+//     read them four times (batch 16, 32 heads over 8, 3000 keys, D = 128: 137 us; the K/V alone
+//     take 30 us at the copy bandwidth).
+//   * The warps never meet inside the key loop. A warp owns every fourth piece of 16 (D = 64: 32) keys,
+//     stages it with asynchronous 16-byte copies in a ring of its own, and keeps its own running
+//     maximum, sum and accumulator; no barrier, only its own copy groups. Two CTAs of three stages
+//     keep up to 128 KB in flight per SM (D = 128), which is what the copy bandwidth needs here.
+//   * q·kᵀ and P·V are mma.sync.m16n8k16: K rows [key][d] are the "col" operand as they lie, V goes
+//     through ldmatrix.trans. mma.sync on purpose: at most 16 rows exist and the kernel is bound by
+//     memory; what counts is that a byte costs few instructions (130 per warp and 8 KB of K/V).
+//   * The key shares of one problem form a cluster (up to eight CTAs) and meet in distributed
+//     shared memory: every CTA adds up its slice of the output over the cluster. No scratch, no
+//     second launch (which alone was 3-9 us). The share is computed from the live key count on the device, so
+//     a half-filled cache is spread over all CTAs as evenly as a full one.
+template <int D>
+struct DecTile {
+    static constexpr int kKeys = D == 64 ? 32 : 16;   // keys per piece
+    static constexpr int kStages = 3;
+    static constexpr int kRowChunks = D / 8;          // 16-byte chunks per row
+    static constexpr int kTileBytes = kKeys * D * 2;  // K or V of one piece
+    static constexpr int kWarpBytes = kStages * 2 * kTileBytes;
+    static constexpr int kSmemBytes = (kDecThreads / 32) * kWarpBytes;
+    // partial results of the CTA's warps [warp][row][D] and of the CTA [row][D], in the ring's memory
+    static_assert(((kDecThreads / 32) + 1) * 16 * D * 4 <= kSmemBytes, "the partial results do not fit the ring");
+};
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t own_addr, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+
+// Grid: x = key share (the cluster dimension), y = query row, z = (sequence, K/V head, group of up to
+// ROWS of its query heads). ROWS = 8: rows 8..15 of the operand are zero and never looked at.
+template <typename T, int D, int ROWS>
+__global__ void __launch_bounds__(kDecThreads, D == 256 ? 1 : 2)
+attn_decode_group_kernel(const DecDev p, const int head_groups) {
+    using Tile = DecTile<D>;
+    constexpr int KEYS = Tile::kKeys, NT = KEYS / 8, WARPS = kDecThreads / 32, RH = ROWS / 8;
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int D = LPK * 8;
-    constexpr int KPW = 32 / LPK;                 // keys per warp per step
-    constexpr int KPS = KPW * (kDecThreads / 32);  // keys per CTA per step
-    constexpr int GROUPS = kDecThreads / LPK;      // key groups in the CTA
-    __shared__ float sc_s[kDecThreads];
-    __shared__ float red_s[kDecThreads / 32];
-    __shared__ float acc_s[GROUPS][D + 4];
-    // K and V tiles of 128 keys, staged with asynchronous 16-byte copies: a thread issues all of its
-    // 2 x 16 copies for a tile up front and holds no registers for them, so a CTA has its whole
-    // tile (64 KB at D = 128) in flight and three CTAs share an SM. With plain loads into registers
-    // the kernel was bound by memory latency (ncu: 42 % of the warps resident, 22 long-scoreboard
-    // stall cycles per issued instruction, 3.7 TB/s). Chunk j (16 bytes) of row r sits at
-    // r * LPK + (j ^ ((r & 1) << 2)), which makes both read patterns below bank-conflict free.
-    extern __shared__ uint4 kv_tiles[];
-    uint4* k_tile = kv_tiles;
-    uint4* v_tile = kv_tiles + kDecThreads * LPK;
-    const int split = blockIdx.x, row = blockIdx.y, bh = blockIdx.z;
-    const int b = bh / p.H, h = bh % p.H;
+    extern __shared__ __align__(128) uint8_t dec_smem[];
+    __shared__ float2 ml_warp[WARPS][16];  // (maximum, sum) of a warp
+    __shared__ float2 ml_cta[16];          // ... of the CTA, read by the whole cluster
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int dl = lane % LPK;    // which 8-wide slice of the head dimension
-    const int group = tid / LPK;  // == warp * KPW + sub
+    const int g = lane >> 2, c = lane & 3;
+    const int row = blockIdx.y;
+    const int hg = (int)blockIdx.z % head_groups, bk = (int)blockIdx.z / head_groups;
+    const int kv_heads = p.H / p.kv_group;
+    const int b = bk / kv_heads, hk = bk % kv_heads;
+    const int h0 = hk * p.kv_group + hg * ROWS;
+    const int rows = min(ROWS, p.kv_group - hg * ROWS);
 
-    // Scores on the tensor core: one mma.sync.m16n8k16 chain per group of 8 keys, q in row 0 of the A
-    // operand (rows 1..15 are zero), the 8 keys as the columns of B. K is [key][d] with d contiguous,
-    // which is exactly the "col" layout of B; every thread feeds the 16 bytes it loads (8 consecutive
-    // d of one key) into two MMAs, with the same permutation of d inside an MMA for q and K. One
-    // load and two MMAs per 16 bytes instead of one load, 8 conversions, 8 FMAs and log2(LPK)
-    // shuffles: the scalar version spent ~45 instructions per 32 bytes of K/V and ran out of issue slots
-    // at two thirds of the HBM bandwidth.
-    const int g8 = lane >> 2, c4 = lane & 3;
-    uint4 qf[D / 32];
-    {
-        const T* qp = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_strides[0] + (int64_t)h * p.q_strides[1] +
+    // this CTA's keys: an equal share of the live ones, in whole rounds of the four warps
+    const int live = decode_live_keys(p);
+    const int round = WARPS * KEYS;
+    const int share = ((live + p.num_splits - 1) / p.num_splits + round - 1) / round * round;
+    const int key_begin = min(live, (int)blockIdx.x * share);
+    const int key_end = min(live, key_begin + share);
+    const int pieces = (key_end - key_begin + KEYS - 1) / KEYS;
+    const int mine = pieces > warp ? (pieces - warp + WARPS - 1) / WARPS : 0;
+
+    const T* kbase = reinterpret_cast<const T*>(p.k) + (int64_t)b * p.k_strides[0] + (int64_t)hk * p.k_strides[1];
+    const T* vbase = reinterpret_cast<const T*>(p.v) + (int64_t)b * p.v_strides[0] + (int64_t)hk * p.v_strides[1];
+    const uint32_t ring = smem_u32(dec_smem) + (uint32_t)(warp * Tile::kWarpBytes);
+    // chunk j (16 bytes) of row r sits at r * kRowChunks + (j ^ (r & 7)): eight rows of one chunk column lie
+    // in eight different bank groups, for the copies as for ldmatrix
+    auto stage = [&](int i) {  // piece i of this warp -> ring slot i % kStages
+        const int k0 = key_begin + (warp + i * WARPS) * KEYS;
+        const uint32_t dst0 = ring + (uint32_t)((i % Tile::kStages) * 2 * Tile::kTileBytes);
+#pragma unroll
+        for (int it = 0; it < KEYS * Tile::kRowChunks / 32; ++it) {
+            const int idx = it * 32 + lane;
+            const int r = idx / Tile::kRowChunks, j = idx % Tile::kRowChunks;
+            const bool in = k0 + r < key_end;
+            const int key = in ? k0 + r : k0;
+            const uint32_t dst = dst0 + (uint32_t)((r * Tile::kRowChunks + (j ^ (r & 7))) * 16);
+            const int n = in ? 16 : 0;  // beyond the share: zero fill, nothing is read
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(kbase + (int64_t)key * p.k_strides[2] + j * 8), "r"(n) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + Tile::kTileBytes), "l"(vbase + (int64_t)key * p.v_strides[2] + j * 8), "r"(n) : "memory");
+        }
+    };
+#pragma unroll
+    for (int i = 0; i < Tile::kStages - 1; ++i) {
+        if (i < mine) stage(i);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+
+    // q: rows of the A operand, (row g, k 2c..) / (row g, k 2c + 8..) and the same of row g + 8
+    uint32_t qf[D / 16][2 * RH];
+#pragma unroll
+    for (int hh = 0; hh < RH; ++hh) {
+        const bool ok = g + 8 * hh < rows;
+        const T* qp = reinterpret_cast<const T*>(p.q) + (int64_t)b * p.q_strides[0] + (int64_t)(h0 + (ok ? g + 8 * hh : 0)) * p.q_strides[1] +
                       (int64_t)row * p.q_strides[2];
 #pragma unroll
-        for (int i = 0; i < D / 32; ++i)
-            qf[i] = (g8 == 0) ? __ldg(reinterpret_cast<const uint4*>(qp + 32 * i + 8 * c4)) : make_uint4(0u, 0u, 0u, 0u);
+        for (int ks = 0; ks < D / 16; ++ks)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                qf[ks][e * RH + hh] = ok ? __ldg(reinterpret_cast<const uint32_t*>(qp + ks * 16 + e * 8 + 2 * c)) : 0u;
     }
-    const int hk = h / p.kv_group;
-    const T* kbase0 = reinterpret_cast<const T*>(p.k) + (int64_t)b * p.k_strides[0] + (int64_t)hk * p.k_strides[1];
-    const T* vbase0 = reinterpret_cast<const T*>(p.v) + (int64_t)b * p.v_strides[0] + (int64_t)hk * p.v_strides[1];
-    auto stage_tile = [&](uint4* tile, const T* base, int64_t row_stride, int k0, int key_end) {
-#pragma unroll 4
-        for (int it = 0; it < LPK; ++it) {
-            const int idx = it * kDecThreads + tid;
-            const int r = idx / LPK, j = idx % LPK;
-            const int key = k0 + r;
-            const bool live = key < key_end;
-            const T* src = base + (int64_t)(live ? key : k0) * row_stride + j * 8;
-            const uint32_t dst = smem_u32(tile + r * LPK + (j ^ ((r & 1) << 2)));
-            // src-size 0 for rows beyond the chunk: the 16 bytes are zero-filled, nothing is read
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
     const float mlow = mask_lowest(p.mask_dtype);
-    const int64_t mask_off = p.mask ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] +
-                                          (int64_t)row * p.mask_strides[2]
-                                    : 0;
-    float m_run = -INFINITY, l_run = 0.f;
-    float acc[8];
+    int64_t mask_off[RH];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
+    for (int hh = 0; hh < RH; ++hh)
+        mask_off[hh] = p.mask == nullptr ? 0 : (int64_t)b * p.mask_strides[0] + (int64_t)(h0 + min(g + 8 * hh, rows - 1)) * p.mask_strides[1] +
+                                                 (int64_t)row * p.mask_strides[2];
 
-    const int key_begin = split * p.chunk;
-    const int key_end = min(decode_live_keys(p), key_begin + p.chunk);  // a chunk beyond the live keys scores nothing: (m, l) = (-inf, 0)
-    for (int k0 = key_begin; k0 < key_end; k0 += kDecThreads) {
-        stage_tile(k_tile, kbase0, p.k_strides[2], k0, key_end);
-        stage_tile(v_tile, vbase0, p.v_strides[2], k0, key_end);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // this thread's K copies have landed
-        __syncthreads();                                       // ... and everybody else's
-        // ---- scores of the block's 128 keys: step s, warp w, group row g8 -> tile row 32 s + 8 w + g8
+    float o[D / 8][4];
 #pragma unroll
-        for (int s = 0; s < kDecThreads / 32; ++s) {
-            const int r = s * 32 + warp * 8 + g8;
-            uint4 kf[D / 32];
+    for (int nt = 0; nt < D / 8; ++nt)
 #pragma unroll
-            for (int i = 0; i < D / 32; ++i) kf[i] = k_tile[r * LPK + ((4 * i + c4) ^ ((r & 1) << 2))];
-            float cacc[4] = {0.f, 0.f, 0.f, 0.f};
-            // mma.sync.aligned needs the whole warp converged; the lanes that stored the previous
-            // group's scores (g8 == 0, below) may still be apart from the others. Without this
-            // barrier the kernel produced garbage for some CTAs whenever the GPU was busy.
-            __syncwarp();
+        for (int e = 0; e < 4; ++e) o[nt][e] = 0.f;
+    float m_run[RH], l_run[RH];
 #pragma unroll
-            for (int i = 0; i < D / 32; ++i) {
-                mma_16816<T>(cacc, qf[i].x, 0u, qf[i].y, 0u, kf[i].x, kf[i].y);
-                mma_16816<T>(cacc, qf[i].z, 0u, qf[i].w, 0u, kf[i].z, kf[i].w);
+    for (int hh = 0; hh < RH; ++hh) { m_run[hh] = -INFINITY; l_run[hh] = 0.f; }
+
+    for (int i = 0; i < mine; ++i) {
+        __syncwarp();  // the slot that is refilled next has been read by all lanes
+        if (i + Tile::kStages - 1 < mine) stage(i + Tile::kStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int k0 = key_begin + (warp + i * WARPS) * KEYS;
+        float mv[RH][NT][2];
+        if (p.mask != nullptr) {  // requested before the wait for the piece
+#pragma unroll
+            for (int hh = 0; hh < RH; ++hh)
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const int key = k0 + nt * 8 + 2 * c + e;
+                        mv[hh][nt][e] = (key < key_end && g + 8 * hh < rows) ? mask_load(p.mask, mask_off[hh] + (int64_t)key * p.mask_strides[3], p.mask_dtype) : 0.f;
+                    }
+        }
+        asm volatile("cp.async.wait_group %0;" ::"n"(Tile::kStages - 1) : "memory");
+        __syncwarp();
+        const uint32_t kt = ring + (uint32_t)((i % Tile::kStages) * 2 * Tile::kTileBytes), vt = kt + Tile::kTileBytes;
+        // ---- scores: column tile nt = keys k0 + 8 nt ..
+        float s[NT][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) s[nt][e] = 0.f;
+            const int r = nt * 8 + (lane & 7);
+#pragma unroll
+            for (int ks = 0; ks < D / 16; ks += 2) {
+                uint32_t kf[4];  // d 16 ks + 8 (lane / 8) ..
+                ldmatrix_x4(kt + (uint32_t)((r * Tile::kRowChunks + ((ks * 2 + (lane >> 3)) ^ (r & 7))) * 16), kf);
+                mma_16816<T>(s[nt], qf[ks][0], RH == 2 ? qf[ks][1] : 0u, qf[ks][RH], RH == 2 ? qf[ks][2 * RH - 1] : 0u, kf[0], kf[1]);
+                mma_16816<T>(s[nt], qf[ks + 1][0], RH == 2 ? qf[ks + 1][1] : 0u, qf[ks + 1][RH], RH == 2 ? qf[ks + 1][2 * RH - 1] : 0u, kf[2], kf[3]);
             }
-            if (g8 == 0) {  // row 0 of the accumulator: lane c4 holds the scores of keys 2 c4 and 2 c4 + 1 of the group
+        }
+        // ---- online softmax of the warp's own keys (a row is spread over four lanes)
+        uint32_t pf[NT][RH];
+        float alpha[RH];
+        bool moved = false;
+#pragma unroll
+        for (int hh = 0; hh < RH; ++hh) {
+            float mx = -INFINITY;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
-                    const int kk = s * 32 + warp * 8 + 2 * c4 + e;
-                    const int key2 = k0 + kk;
-                    float sc = -INFINITY;
-                    if (key2 < key_end && !(p.is_causal && key2 > row)) {
-                        sc = cacc[e] * p.scale_log2;
-                        if (p.mask) {
-                            const float mv = mask_load(p.mask, mask_off + (int64_t)key2 * p.mask_strides[3], p.mask_dtype);
-                            sc = fmaf(fmaxf(mv, mlow), kLog2e, sc);
-                        }
-                    }
-                    sc_s[kk] = sc;
+                    const int key = k0 + nt * 8 + 2 * c + e;
+                    float x = s[nt][hh * 2 + e] * p.scale_log2;
+                    if (p.mask != nullptr) x = fmaf(fmaxf(mv[hh][nt][e], mlow), kLog2e, x);
+                    if (key >= key_end || (p.is_causal && key > row)) x = -INFINITY;
+                    s[nt][hh * 2 + e] = x;
+                    mx = fmaxf(mx, x);
                 }
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+            mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+            float m_new = fmaxf(m_run[hh], mx);
+            if (m_new == -INFINITY) m_new = 0.f;
+            alpha[hh] = m_run[hh] == -INFINITY ? 0.f : fast_exp2(m_run[hh] - m_new);
+            moved |= m_new != m_run[hh];
+            m_run[hh] = m_new;
+            float sum = 0.f;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const float e0 = fast_exp2(s[nt][hh * 2] - m_new), e1 = fast_exp2(s[nt][hh * 2 + 1] - m_new);
+                sum += e0 + e1;
+                pf[nt][hh] = Elem<T>::pack2(e0, e1);  // rounded to the input type, as the reference does (attention_skinny.py:262)
+            }
+            l_run[hh] = l_run[hh] * alpha[hh] + sum;
+        }
+        if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+            for (int nt = 0; nt < D / 8; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2 * RH; ++e) o[nt][e] *= alpha[e >> 1];
+        }
+        // ---- O += P · V: the score fragments are the A operand of the next product
+#pragma unroll
+        for (int kb = 0; kb < KEYS / 16; ++kb) {
+            const int r = kb * 16 + (lane & 15);
+#pragma unroll
+            for (int nt = 0; nt < D / 8; nt += 2) {
+                uint32_t vf[4];  // keys 0-7, 8-15 of the columns of nt, then of nt + 1
+                ldmatrix_x4_trans(vt + (uint32_t)((r * Tile::kRowChunks + ((nt + (lane >> 4)) ^ (r & 7))) * 16), vf);
+                const uint32_t a1 = RH == 2 ? pf[2 * kb][RH - 1] : 0u, a3 = RH == 2 ? pf[2 * kb + 1][RH - 1] : 0u;
+                mma_16816<T>(o[nt], pf[2 * kb][0], a1, pf[2 * kb + 1][0], a3, vf[0], vf[1]);
+                mma_16816<T>(o[nt + 1], pf[2 * kb][0], a1, pf[2 * kb + 1][0], a3, vf[2], vf[3]);
             }
         }
-        __syncthreads();
-        // ---- block maximum and exponentials (one key per thread)
-        const float sv = sc_s[tid];
-        float mx = sv;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-        if (lane == 0) red_s[warp] = mx;
-        __syncthreads();
-        mx = fmaxf(fmaxf(red_s[0], red_s[1]), fmaxf(red_s[2], red_s[3]));
-        float m_new = fmaxf(m_run, mx);
-        if (m_new == -INFINITY) m_new = 0.f;
-        const float alpha = (m_run == -INFINITY) ? 0.f : fast_exp2(m_run - m_new);
-        const float pe = fast_exp2(sv - m_new);
-        __syncthreads();  // everyone has read sc_s and red_s
-        // P is rounded to the input dtype before P·V, as the reference does (attention_skinny.py:262)
-        sc_s[tid] = Elem<T>::to_f32(Elem<T>::from_f32(pe));
-        float ps = pe;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ps += __shfl_xor_sync(0xffffffffu, ps, o);
-        if (lane == 0) red_s[warp] = ps;
-        __syncthreads();
-        asm volatile("cp.async.wait_group 0;" ::: "memory");  // this thread's V copies have landed
-        l_run = l_run * alpha + (red_s[0] + red_s[1] + red_s[2] + red_s[3]);
-        m_run = m_new;
-        __syncthreads();  // every thread's V copies are visible
-        // ---- P·V with the same key-to-lane mapping
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc[i] *= alpha;
-#pragma unroll 4
-        for (int s = 0; s < kDecThreads / KPS; ++s) {
-            const int kk = s * KPS + group;
-            const int key = k0 + kk;
-            if (key < key_end) {
-                const float pk = sc_s[kk];
-                const uint4 w = v_tile[kk * LPK + (dl ^ ((kk & 1) << 2))];
-                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float2 f = Elem<T>::unpack2(ww[i]);
-                    acc[2 * i] = fmaf(pk, f.x, acc[2 * i]);
-                    acc[2 * i + 1] = fmaf(pk, f.y, acc[2 * i + 1]);
-                }
-            }
-        }
-        __syncthreads();  // sc_s and both tiles are rewritten by the next block
     }
-    // ---- sum the key groups and write (m, l, acc[D])
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+
+    // ---- merge the four warps, then the cluster
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc_s[group][dl * 8 + i] = acc[i];
+    for (int hh = 0; hh < RH; ++hh) {
+        l_run[hh] += __shfl_xor_sync(0xffffffffu, l_run[hh], 1);
+        l_run[hh] += __shfl_xor_sync(0xffffffffu, l_run[hh], 2);
+        // a warp that saw no key it may attend to (sum zero) must not set the scale
+        if (c == 0) ml_warp[warp][g + 8 * hh] = make_float2(l_run[hh] > 0.f ? m_run[hh] : -INFINITY, l_run[hh]);
+    }
+    __syncthreads();  // every warp is done with its ring: the partial results go there
+    float* part = reinterpret_cast<float*>(dec_smem);       // [warp][row][D]
+    float* cta = part + WARPS * ROWS * D;                   // [row][D]
+#pragma unroll
+    for (int hh = 0; hh < RH; ++hh)
+        if (g + 8 * hh < rows)
+#pragma unroll
+            for (int nt = 0; nt < D / 8; ++nt)
+                *reinterpret_cast<float2*>(part + (warp * ROWS + g + 8 * hh) * D + nt * 8 + 2 * c) = make_float2(o[nt][2 * hh], o[nt][2 * hh + 1]);
     __syncthreads();
-    float* out = p.scratch + (((int64_t)bh * p.M + row) * p.num_splits + split) * (D + 2);
-    if (tid == 0) { out[0] = m_run; out[1] = l_run; }
-    for (int d = tid; d < D; d += kDecThreads) {
-        float a = 0.f;
+    const int n_out = rows * D;
+    for (int e = tid; e < n_out; e += kDecThreads) {
+        const int r = e / D;
+        float m = -INFINITY;
 #pragma unroll
-        for (int g = 0; g < GROUPS; ++g) a += acc_s[g][d];
-        out[2 + d] = a;
+        for (int w = 0; w < WARPS; ++w) m = fmaxf(m, ml_warp[w][r].x);
+        const float ref = m == -INFINITY ? 0.f : m;
+        float acc = 0.f, l = 0.f;
+#pragma unroll
+        for (int w = 0; w < WARPS; ++w) {
+            const float sc = fast_exp2(ml_warp[w][r].x - ref);
+            l = fmaf(ml_warp[w][r].y, sc, l);
+            acc = fmaf(part[(w * ROWS + r) * D + e % D], sc, acc);
+        }
+        cta[e] = acc;
+        if (e % D == 0) ml_cta[r] = make_float2(m, l);
     }
+    cluster_sync_all();  // (a cluster of one: a CTA barrier)
+    const uint32_t ml_addr = smem_u32(ml_cta), cta_addr = smem_u32(cta);
+    for (int e = (int)blockIdx.x * kDecThreads + tid; e < n_out; e += p.num_splits * kDecThreads) {
+        const int r = e / D, d = e % D;
+        float m = -INFINITY;
+        for (int q = 0; q < p.num_splits; ++q) m = fmaxf(m, ld_cluster_f32(ml_addr + 8u * r, q));
+        const float ref = m == -INFINITY ? 0.f : m;
+        float acc = 0.f, l = 0.f;
+        for (int q = 0; q < p.num_splits; ++q) {
+            const float sc = fast_exp2(ld_cluster_f32(ml_addr + 8u * r, q) - ref);
+            l = fmaf(ld_cluster_f32(ml_addr + 8u * r + 4u, q), sc, l);
+            acc = fmaf(ld_cluster_f32(cta_addr + 4u * e, q), sc, acc);
+        }
+        T* op = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)(h0 + r) * p.o_strides[1] + (int64_t)row * p.o_strides[2];
+        op[(int64_t)d * p.o_strides[3]] = Elem<T>::from_f32(acc / l);
+    }
+    cluster_sync_all();  // nobody leaves while its shared memory may still be read
 }
 
 template <typename T>
@@ -366,22 +465,63 @@ attn_decode_part2_kernel(const DecDev p) {
     }
 }
 
-template <typename T, int LPK>
-static void launch_decode_vec(dim3 grid, cudaStream_t stream, const DecDev& d) {
-    constexpr size_t smem = 2 * (size_t)kDecThreads * LPK * sizeof(uint4);  // K tile + V tile
-    static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) {
-        cudaFuncSetAttribute(attn_decode_part1_vec_kernel<T, LPK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Key shares per problem (the cluster size, at most the portable eight). A wave of CTAs costs the bytes
+// of one share plus a fixed part — first copies from DRAM, q, the merge: about 2.5 us, which at a
+// slot's part of the copy bandwidth is 56 KB — so shares are cut until one wave is full and no further.
+template <int D>
+static int decode_shares(int64_t units, int64_t N) {
+    const int64_t slots = (int64_t)sm_count() * (D == 256 ? 1 : 2);
+    const int64_t round = (kDecThreads / 32) * DecTile<D>::kKeys;
+    int best = 1;
+    double best_cost = 1e300;
+    for (int s = 1; s <= 8 && (s - 1) * round < N; ++s) {
+        const int64_t share = ((N + s - 1) / s + round - 1) / round * round;
+        const double cost = (double)((units * s + slots - 1) / slots) * ((double)share * D * 4.0 + 56.0 * 1024.0);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = s;
+        }
     }
-    launch_pdl(attn_decode_part1_vec_kernel<T, LPK>, grid, kDecThreads, smem, stream, d);
+    return best;
+}
+
+template <typename T, int D, int ROWS>
+static int launch_decode_group_r(DecDev d, cudaStream_t stream) {
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time() &&
+        cudaFuncSetAttribute(attn_decode_group_kernel<T, D, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecTile<D>::kSmemBytes) != cudaSuccess)
+        return KB_ERR_LAUNCH;
+    const int head_groups = (d.kv_group + ROWS - 1) / ROWS;
+    const int64_t units = (int64_t)d.B * (d.H / d.kv_group) * head_groups * d.M;
+    d.num_splits = decode_shares<D>(units, d.N);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)d.num_splits, (unsigned)d.M, (unsigned)(d.B * (d.H / d.kv_group) * head_groups));
+    cfg.blockDim = dim3(kDecThreads);
+    cfg.dynamicSmemBytes = DecTile<D>::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)d.num_splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 2u : 1u;
+    return cudaLaunchKernelEx(&cfg, attn_decode_group_kernel<T, D, ROWS>, (const DecDev)d, (const int)head_groups) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+}
+
+template <typename T>
+static int launch_decode_group(const DecDev& d, cudaStream_t stream) {
+    const bool wide = d.kv_group > 8;  // sixteen operand rows only where a group fills more than eight
+    if (d.D == 64) return wide ? launch_decode_group_r<T, 64, 16>(d, stream) : launch_decode_group_r<T, 64, 8>(d, stream);
+    if (d.D == 128) return wide ? launch_decode_group_r<T, 128, 16>(d, stream) : launch_decode_group_r<T, 128, 8>(d, stream);
+    return wide ? launch_decode_group_r<T, 256, 16>(d, stream) : launch_decode_group_r<T, 256, 8>(d, stream);
 }
 
 static int launch_attention_decode(const kb_attn_params& p, void* scratch, int64_t scratch_bytes, cudaStream_t stream) {
     if (p.N <= 0 || p.D > kDecMaxD) return KB_ERR_UNSUPPORTED;
     if (p.M > 65535 || p.B * p.H > 65535) return KB_ERR_UNSUPPORTED;
-    if (scratch == nullptr) return KB_ERR_BAD_ARG;
-    const int64_t need = decode_scratch_bytes(p.B, p.H, p.M, p.N, p.D);
-    if (scratch_bytes < need) return KB_ERR_BAD_ARG;
     DecDev d;
     d.q = p.q; d.k = p.k; d.v = p.v; d.o = p.o; d.mask = p.mask;
     for (int i = 0; i < 4; ++i) {
@@ -392,30 +532,27 @@ static int launch_attention_decode(const kb_attn_params& p, void* scratch, int64
     d.scale_log2 = p.sm_scale * kLog2e;
     d.is_causal = p.is_causal ? 1 : 0;
     d.mask_dtype = p.mask ? p.mask_dtype : KB_F32;
-    decode_split(p.N, p.B * p.H * p.M, &d.num_splits, &d.chunk);
     d.kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % d.kv_group != 0) return KB_ERR_BAD_ARG;
     d.kv_len_dev = reinterpret_cast<const long long*>(p.kv_len_dev);
-    d.scratch = reinterpret_cast<float*>(scratch);
-    const dim3 g1((unsigned)d.num_splits, (unsigned)p.M, (unsigned)(p.B * p.H));
-    const dim3 g2((unsigned)p.M, (unsigned)(p.B * p.H));
     const bool vec_ok = (p.D == 64 || p.D == 128 || p.D == 256) && p.q_strides[3] == 1 && p.k_strides[3] == 1 &&
                         p.v_strides[3] == 1 && (p.k_strides[2] % 8) == 0 && (p.v_strides[2] % 8) == 0 &&
                         (p.k_strides[1] % 8) == 0 && (p.v_strides[1] % 8) == 0 && (p.k_strides[0] % 8) == 0 &&
                         (p.v_strides[0] % 8) == 0 && (((uintptr_t)p.k) & 15) == 0 && (((uintptr_t)p.v) & 15) == 0 &&
                         (((uintptr_t)p.q) & 15) == 0 && (p.q_strides[0] % 8) == 0 && (p.q_strides[1] % 8) == 0 &&
                         (p.q_strides[2] % 8) == 0;
+    if (vec_ok) return p.dtype == KB_F16 ? launch_decode_group<__half>(d, stream) : launch_decode_group<__nv_bfloat16>(d, stream);
+    // any other layout: chunks through scratch and a second kernel
+    if (scratch == nullptr || scratch_bytes < decode_scratch_bytes(p.B, p.H, p.M, p.N, p.D)) return KB_ERR_BAD_ARG;
+    d.scratch = reinterpret_cast<float*>(scratch);
+    decode_split(p.N, p.B * p.H * p.M, &d.num_splits, &d.chunk);
+    const dim3 g1((unsigned)d.num_splits, (unsigned)p.M, (unsigned)(p.B * p.H));
+    const dim3 g2((unsigned)p.M, (unsigned)(p.B * p.H));
     if (p.dtype == KB_F16) {
-        if (vec_ok && p.D == 64) launch_decode_vec<__half, 8>(g1, stream, d);
-        else if (vec_ok && p.D == 128) launch_decode_vec<__half, 16>(g1, stream, d);
-        else if (vec_ok && p.D == 256) launch_decode_vec<__half, 32>(g1, stream, d);
-        else launch_pdl(attn_decode_part1_kernel<__half>, g1, kDecThreads, 0, stream, d);
+        launch_pdl(attn_decode_part1_kernel<__half>, g1, kDecThreads, 0, stream, d);
         launch_pdl(attn_decode_part2_kernel<__half>, g2, kDecThreads, 0, stream, d);
     } else {
-        if (vec_ok && p.D == 64) launch_decode_vec<__nv_bfloat16, 8>(g1, stream, d);
-        else if (vec_ok && p.D == 128) launch_decode_vec<__nv_bfloat16, 16>(g1, stream, d);
-        else if (vec_ok && p.D == 256) launch_decode_vec<__nv_bfloat16, 32>(g1, stream, d);
-        else launch_pdl(attn_decode_part1_kernel<__nv_bfloat16>, g1, kDecThreads, 0, stream, d);
+        launch_pdl(attn_decode_part1_kernel<__nv_bfloat16>, g1, kDecThreads, 0, stream, d);
         launch_pdl(attn_decode_part2_kernel<__nv_bfloat16>, g2, kDecThreads, 0, stream, d);
     }
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;

@@ -291,10 +291,9 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (len == nullptr || len->scalar_type() != at::kLong || len->numel() != 1 || len->device() != q->device()) Py_RETURN_NONE;
         p.kv_len_dev = len->data_ptr<int64_t>();
     }
-    const int64_t bytes = kb_attention_decode_scratch_bytes(p.B, p.H, p.M, p.N, p.D);
     const c10::cuda::CUDAGuard guard(q->device());
-    at::Tensor scratch = at::detail::empty_cuda({bytes > 16 ? bytes : 16}, at::kByte, q->device(), c10::nullopt);
-    const int st = kb_attention_decode_fwd(&p, scratch.data_ptr(), scratch.numel(), stream_of(*q));
+    const int st = kb_attention_decode_fwd(&p, nullptr, 0, stream_of(*q));
+    if (st == KB_ERR_BAD_ARG) Py_RETURN_NONE;  // a layout that needs scratch, which the general path allocates
     if (st != KB_OK) return failed("skinny_attention_forward", st);
     Py_INCREF(a[3]);
     return a[3];

@@ -104,7 +104,7 @@ def linear_layer(
     n_out = N // 2 if gated else N
     # The TMA path wants unit K stride and 16-byte aligned rows; anything else is copied once.
     if x_.stride(1) != 1 or x_.stride(0) % 8 != 0 or x_.data_ptr() % 16 != 0:
-        x_ = x_.contiguous()
+        x_ = _aligned(x_.contiguous())
     if K % 8 != 0:
         # K is padded with zeros to the next multiple of 8 (16-byte rows for TMA); zeros add nothing.
         pad = 8 - K % 8
