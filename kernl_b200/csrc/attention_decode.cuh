@@ -191,14 +191,6 @@ struct DecTile {
     static_assert(((kDecThreads / 32) + 1) * 16 * D * 4 <= kSmemBytes, "the partial results do not fit the ring");
 };
 
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
-    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
-}
 __device__ __forceinline__ float ld_cluster_f32(uint32_t own_addr, uint32_t rank) {
     uint32_t a;
     float v;
@@ -508,7 +500,7 @@ static int launch_decode_group_r(DecDev d, cudaStream_t stream) {
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_use_pdl ? 2u : 1u;
-    return cudaLaunchKernelEx(&cfg, attn_decode_group_kernel<T, D, ROWS>, (const DecDev)d, (const int)head_groups) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&cfg, attn_decode_group_kernel<T, D, ROWS>, d, head_groups) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
 
 template <typename T>

@@ -124,16 +124,18 @@ struct PerDeviceOnce {
 };
 
 // ---------------------------------------------------------------------------------------------
-// Warp-level mma.sync (m16n8k16, fp32 accumulate) and streaming loads for the HBM-bound kernels that
+// Warp-level mma.sync (m16n8k16, fp32 accumulate) and its operand loads for the HBM-bound kernels that
 // have only a few rows of A (few-row linear, decode attention): there the tensor-core generation
 // does not matter, the instruction count per loaded byte does.
 // ---------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint4 ld_stream_nc_16B(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
+// Four 8 x 8 matrices of 16-bit elements; lanes 8 i .. 8 i + 7 give the row addresses of matrix i.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
 }
 
 template <typename T>

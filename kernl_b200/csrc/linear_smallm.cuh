@@ -1,164 +1,297 @@
-// Linear layer for very few rows (M <= 16): y = act(x · Wᵀ + bias), the decode-step shape.
+// Linear layer for few rows (M <= 32): y = act(x · Wᵀ + bias), the decode-step shape.
 //
 // With a handful of rows the op is a single pass over W from HBM (2·N·K bytes; x is a few dozen KB and
-// lives in L1/L2), so what matters is how many bytes every SM keeps in flight and how little
-// fixed cost a launch carries — not the tensor-core generation. The tcgen05 GEMM pays for a tensor
-// map, a TMEM allocation, a 128-row tile of which 8 rows are real, and a second kernel to finish its
-// split-K sums: about 6 µs of fixed cost on a 14 µs stream. This kernel has none of that:
-//   * one CTA of 8 warps per 16 output columns; the warps split K in interleaved 64-byte pieces,
-//     so the 8 warps together read 512 contiguous bytes of each weight row per round;
-//   * every thread loads 16 bytes (8 consecutive k) of one weight row per 8-column group with
-//     streaming loads, four rounds ahead, and feeds them as the B fragments of two
-//     mma.sync.m16n8k16 (the k order inside an MMA is permuted consistently for A and B, which a dot
-//     product does not notice); x rows are the A fragments, read through L1;
-//   * launched with programmatic dependent launch: its set-up overlaps the tail of the kernel that
-//     produces x;
-//   * the 8 partial 16x16 tiles meet in shared memory, 256 threads add them and apply bias and
-//     activation. No workspace, no atomics, no second launch.
+// lives in L2), so what matters is how many bytes every SM keeps in flight, without a break, and how
+// little fixed cost a launch carries — not the tensor-core generation. The tcgen05 GEMM pays for tensor
+// maps, a TMEM allocation, a 128-row tile of which 8 rows are real, and a second kernel to finish its
+// split-K sums. Here:
+//   * W is the row operand of mma.sync.m16n8k16 (16 weight rows x 8 rows of x): up to eight rows of x
+//     cost one instruction per 16 x 16 block of W;
+//   * every CTA (two per SM) takes an equal share of the rows of W, whatever their number: 11008 rows
+//     are 37 or 38 for each of 296 CTAs. It walks them in tiles of at most 48 rows. With tiles of a fixed
+//     16 rows the same matrix was 2.3 rounds, run as 3;
+//   * the four warps of a CTA split K in interleaved pieces of 64 elements. Each warp stages its pieces
+//     — W rows and the same columns of x — with asynchronous 16-byte copies in a ring of its own: no
+//     barrier in the main loop, no register holds a byte in flight, and the ring runs on into the next
+//     tile while the four partial tiles meet in shared memory;
+//   * before it waits for the kernel that produces x, a CTA asks for its first pieces of W in L2 only
+//     (W itself may be that kernel's output, so nothing of it is read before the wait).
+// Dividing tiles between CTAs to even out the rounds (partial sums through the workspace, the last CTA
+// finishes) was tried: the fence, the counter and the second read cost 3 us at the end of every launch.
+// The kernel before this one held 8 loads per thread in registers and drained them once per
+// 1024 columns, in rounds of one 16-row tile per CTA: [16, 4096] x [11008, 4096] took 23.4 us (3.9 TB/s).
 // Same contract as the reference's linear_layer (src/kernl/implementations/linear_layer.py:213-282).
 #pragma once
 #include "linear.cuh"
 
 namespace kb {
 
-constexpr int kSmallMThreads = 256;
-constexpr int kSmallMCols = 16;    // output columns per CTA
-constexpr int kSmallMRounds = 4;   // 32-element k pieces in flight per warp
+constexpr int kStreamThreads = 128;
+constexpr int kStreamWarps = kStreamThreads / 32;
+constexpr int kStreamK = 64;  // elements of K per piece: 128-byte rows in shared memory
+constexpr int kStreamMaxM = 32;
+constexpr int kStreamSmemBytes = 112 * 1024;  // rings and partial tiles of a CTA: two CTAs per SM
 
-// HI: rows 8..15 exist (M > 8); otherwise their A fragments are zero and are not loaded.
-// Up to eight rows (HI = false) the kernel fits three CTAs per SM (80 registers): more weight bytes in
-// flight per SM. Decode step of the 7B shape: 8 layers 1.76 -> 1.69 ms, 32 layers 5.43 -> 5.40 ms;
-// four CTAs per SM (64 registers) measured no better than three.
-template <typename T, bool HI>
-__global__ void __launch_bounds__(kSmallMThreads, HI ? 2 : 3)
-linear_smallm_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
-                     T* __restrict__ act_inputs, int M, int N, int K, int64_t x_row_stride, int64_t y_row_stride,
-                     int activation) {
-    __shared__ float red[kSmallMThreads / 32][16][kSmallMCols + 1];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+constexpr int stream_red_bytes(int rmax, int nx) { return kStreamWarps * nx * 8 * (rmax + 1) * 4; }
+
+// RMAX: most rows of W per tile (a multiple of 8), NX: 8-row tiles of x.
+template <int RMAX, int NX>
+struct StreamCfg {
+    static constexpr int kTiles16 = (RMAX + 15) / 16;  // 16-row operand tiles; rows beyond the tile's hold anything
+    static constexpr int kWBytes = RMAX * kStreamK * 2;
+    static constexpr int kStageBytes = kWBytes + NX * 8 * kStreamK * 2;
+    static constexpr int kRedRow = RMAX + 1;  // partial tile of a warp: [x row][W row], rows padded
+    static constexpr int kFit = (kStreamSmemBytes - stream_red_bytes(RMAX, NX)) / (kStreamWarps * kStageBytes);
+    static constexpr int kStages = kFit > 10 ? 10 : kFit;
+    static constexpr int kSmemBytes = kStreamWarps * kStages * kStageBytes + stream_red_bytes(RMAX, NX);
+    static_assert(kStages >= 3, "a warp needs two pieces in flight");
+};
+
+// `lines`: what is shared out among the CTAs — rows of W, or pairs of a gate and an up row (gated
+// epilogue: pair o is rows 16 (o / 8) + o % 8 and eight further). `tiles`: tiles per CTA.
+template <typename T, int RMAX, int NX>
+__global__ void __launch_bounds__(kStreamThreads, 2)
+linear_stream_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
+                     T* __restrict__ act_inputs, int M, int lines, int K, int64_t x_row_stride, int64_t y_row_stride,
+                     int activation, int tiles) {
+    using Cfg = StreamCfg<RMAX, NX>;
+    constexpr int STAGES = Cfg::kStages, MT = Cfg::kTiles16;
+    extern __shared__ __align__(128) uint8_t stream_smem[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, c = lane & 3;
-    const int n0 = blockIdx.x * kSmallMCols;
+    const uint32_t ring = smem_u32(stream_smem) + (uint32_t)(warp * STAGES * Cfg::kStageBytes);
+    float* red = reinterpret_cast<float*>(stream_smem + kStreamWarps * STAGES * Cfg::kStageBytes);
+    const bool gated = activation == KB_ACT_SWIGLU;
 
-    // rows of W this thread reads (one per 8-column group) and rows of x (g and g + 8)
-    const T* wrow[2];
-    bool wlive[2];
-#pragma unroll
-    for (int grp = 0; grp < 2; ++grp) {
-        const int n = n0 + grp * 8 + g;
-        wlive[grp] = n < N;
-        wrow[grp] = w + (int64_t)(wlive[grp] ? n : 0) * K;
-    }
-    const bool lo_live = g < M, hi_live = HI && (g + 8 < M);
-    const T* xlo = x + (int64_t)(lo_live ? g : 0) * x_row_stride;
-    const T* xhi = x + (int64_t)(hi_live ? g + 8 : 0) * x_row_stride;
-
-    float acc[2][4];
-#pragma unroll
-    for (int grp = 0; grp < 2; ++grp)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[grp][i] = 0.f;
-
-    // piece p covers k in [32p, 32p + 32); warp `warp` takes pieces warp, warp + 8, ...; inside a piece
-    // this thread owns the 8 elements at 32p + 8c.
-    const int pieces = (K + 31) / 32;
-    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-    uint4 bw[kSmallMRounds][2];
-    auto load_w = [&](int p0) {
-#pragma unroll
-        for (int r = 0; r < kSmallMRounds; ++r) {
-            const int k = (p0 + r * 8) * 32 + c * 8;
-#pragma unroll
-            for (int grp = 0; grp < 2; ++grp) bw[r][grp] = (k < K && wlive[grp]) ? ld_stream_nc_16B(wrow[grp] + k) : zero4;
-        }
+    const int pieces = (K + kStreamK - 1) / kStreamK;
+    const int mine = pieces > warp ? (pieces - warp + kStreamWarps - 1) / kStreamWarps : 0;  // this warp's pieces of a tile
+    // every CTA starts elsewhere in K, so that the CTAs do not walk the memory channels in step (1-4 %)
+    const int start = mine > 0 ? (int)(blockIdx.x * 5u) % mine : 0;
+    const int cta_begin = (int)((int64_t)blockIdx.x * lines / gridDim.x);
+    const int cta_lines = (int)((int64_t)(blockIdx.x + 1) * lines / gridDim.x) - cta_begin;
+    auto tile_begin = [&](int t) { return cta_begin + t * cta_lines / tiles; };
+    // row r of the tile that covers lines [l0, l0 + n): the gate rows of its pairs, then their up rows
+    auto w_row = [&](int l0, int n, int r) {
+        if (!gated) return l0 + r;
+        const int o = l0 + (r < n ? r : r - n);
+        return (o >> 3) * 16 + (o & 7) + (r < n ? 0 : 8);
     };
-    pdl_wait();  // (W could in principle have been written by the previous kernel, e.g. a dtype conversion)
+
+    if (mine > 0) {
+        const int l0 = tile_begin(0), n = tile_begin(1) - l0, rows = gated ? 2 * n : n;
+        for (int i = lane; i < rows * min(mine, STAGES - 1); i += 32)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(w + (int64_t)w_row(l0, n, i % rows) * K + (warp + (start + i / rows) % mine * kStreamWarps) * kStreamK));
+    }
+    pdl_wait();
     pdl_launch_dependents();
-    load_w(warp);
-    for (int p0 = warp; p0 < pieces; p0 += 8 * kSmallMRounds) {
-        uint4 alo[kSmallMRounds], ahi[kSmallMRounds];
+
+    // a 16-byte chunk j of row r sits at r * 128 + (j ^ (r & 7)) * 16: conflict-free for ldmatrix. A lane copies
+    // chunk lj of every fourth row; its row pointers change only with the tile, so that a piece costs two
+    // instructions per copy (a warp has some 700 cycles per piece before it falls behind the memory).
+    const int lr = lane >> 3, lj = lane & 7;
+    const T* wp[RMAX / 4];
+    const T* xp[NX * 2];
+    int in_tile = 0, in_piece = 0, in_slot = 0, in_rows = 0;
+    auto enter_tile = [&]() {
+        const int l0 = tile_begin(in_tile), n = tile_begin(in_tile + 1) - l0;
+        in_rows = gated ? 2 * n : n;
 #pragma unroll
-        for (int r = 0; r < kSmallMRounds; ++r) {
-            const int k = (p0 + r * 8) * 32 + c * 8;
-            const bool kin = k < K;  // K is a multiple of 8, so a thread's 8 elements are in or out as a whole
-            alo[r] = (kin && lo_live) ? __ldg(reinterpret_cast<const uint4*>(xlo + k)) : zero4;
-            if (HI) ahi[r] = (kin && hi_live) ? __ldg(reinterpret_cast<const uint4*>(xhi + k)) : zero4;
-            else ahi[r] = zero4;
-        }
+        for (int it = 0; it < RMAX / 4; ++it) wp[it] = w + (int64_t)w_row(l0, n, it * 4 + lr) * K + lj * 8;
+    };
 #pragma unroll
-        for (int r = 0; r < kSmallMRounds; ++r) {
+    for (int it = 0; it < NX * 2; ++it) xp[it] = x + (int64_t)(it * 4 + lr) * x_row_stride + lj * 8;
+    if (mine > 0) enter_tile();
+    auto issue = [&]() {
+        if (mine > 0 && in_tile < tiles) {
+            const int turn = in_piece + start, k = (warp + (turn < mine ? turn : turn - mine) * kStreamWarps) * kStreamK;
+            const int n_copy = k + lj * 8 < K ? 16 : 0;  // K is a multiple of 8; nothing is read beyond it
+            const int ks = n_copy ? k : -lj * 8;
+            const uint32_t dst = ring + (uint32_t)(in_slot * Cfg::kStageBytes);
 #pragma unroll
-            for (int grp = 0; grp < 2; ++grp) {
-                mma_16816<T>(acc[grp], alo[r].x, ahi[r].x, alo[r].y, ahi[r].y, bw[r][grp].x, bw[r][grp].y);
-                mma_16816<T>(acc[grp], alo[r].z, ahi[r].z, alo[r].w, ahi[r].w, bw[r][grp].z, bw[r][grp].w);
+            for (int it = 0; it < RMAX / 4; ++it) {
+                const int r = it * 4 + lr;  // rows beyond the tile are not copied: their results are not used
+                if (r < in_rows)
+                    asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(r * 128 + ((lj ^ (r & 7)) * 16))),
+                                 "l"(wp[it] + ks), "r"(n_copy) : "memory");
+            }
+#pragma unroll
+            for (int it = 0; it < NX * 2; ++it) {
+                const int r = it * 4 + lr;
+                if (r < M)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(Cfg::kWBytes + r * 128 + ((lj ^ (r & 7)) * 16))),
+                                 "l"(xp[it] + ks), "r"(n_copy) : "memory");
+            }
+            if (++in_slot == STAGES) in_slot = 0;
+            if (++in_piece == mine) {
+                in_piece = 0;
+                if (++in_tile < tiles) enter_tile();
             }
         }
-        if (p0 + 8 * kSmallMRounds < pieces) load_w(p0 + 8 * kSmallMRounds);
-    }
-    // accumulator fragment: c0,c1 -> (row g, cols 2c, 2c+1); c2,c3 -> (row g+8, same cols)
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int i = 0; i < STAGES - 1; ++i) issue();
+
+    int slot = 0;
+    for (int tile = 0; tile < tiles; ++tile) {
+        float acc[2][MT][NX][4];  // two chains: a product waits for the one before the last
 #pragma unroll
-    for (int grp = 0; grp < 2; ++grp) {
-        red[warp][g][grp * 8 + 2 * c] = acc[grp][0];
-        red[warp][g][grp * 8 + 2 * c + 1] = acc[grp][1];
-        red[warp][g + 8][grp * 8 + 2 * c] = acc[grp][2];
-        red[warp][g + 8][grp * 8 + 2 * c + 1] = acc[grp][3];
-    }
-    __syncthreads();
-    const int m = threadIdx.x >> 4, nn = threadIdx.x & 15;
-    const int n = n0 + nn;
-    if (activation == KB_ACT_SWIGLU) {
-        // the CTA's first eight columns are a gate block, the other eight the matching up block
-        // (rows of W interleaved in blocks of eight): eight outputs at columns n0 / 2 ...
-        if (m < M && nn < 8 && n < N) {
-            float zg = 0.f, zu = 0.f;
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-            for (int wi = 0; wi < kSmallMThreads / 32; ++wi) {
-                zg += red[wi][m][nn];
-                zu += red[wi][m][nn + 8];
+            for (int nx = 0; nx < NX; ++nx)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[0][mt][nx][e] = acc[1][mt][nx][e] = 0.f;
+        for (int i = 0; i < mine; ++i) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+            __syncwarp();  // every lane's copies of this piece are visible, and the slot before it has been read
+            const uint32_t st = ring + (uint32_t)(slot * Cfg::kStageBytes), sx = st + Cfg::kWBytes;
+            if (++slot == STAGES) slot = 0;
+            uint32_t xf[NX][8], wf[kStreamK / 16][MT][4];
+#pragma unroll
+            for (int nx = 0; nx < NX; ++nx) {
+                const int r = nx * 8 + (lane & 7);
+                uint32_t f[4];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    ldmatrix_x4(sx + (uint32_t)(r * 128 + (((h * 4 + (lane >> 3)) ^ (r & 7)) * 16)), f);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) xf[nx][h * 4 + e] = f[e];
+                }
             }
-            if (bias != nullptr) {
-                zg += Elem<T>::to_f32(bias[n]);
-                zu += Elem<T>::to_f32(bias[n + 8]);
-            }
-            y[(int64_t)m * y_row_stride + (n0 >> 1) + nn] = Elem<T>::from_f32(act_silu(zg) * zu);
-        }
-        return;
-    }
-    if (m < M && n < N) {
-        float z = 0.f;
 #pragma unroll
-        for (int wi = 0; wi < kSmallMThreads / 32; ++wi) z += red[wi][m][nn];
-        if (bias != nullptr) z += Elem<T>::to_f32(bias[n]);
-        if (act_inputs != nullptr) act_inputs[(int64_t)m * y_row_stride + n] = Elem<T>::from_f32(z);
-        float v = z;
-        switch (activation) {
-            case KB_ACT_TANH: v = act_tanh(v); break;
-            case KB_ACT_GELU: v = act_gelu(v); break;
-            case KB_ACT_FAST_GELU: v = act_fast_gelu(v); break;
-            case KB_ACT_RELU: v = fmaxf(v, 0.f); break;
-            case KB_ACT_SILU: v = act_silu(v); break;
-            default: break;
+            for (int ks = 0; ks < kStreamK / 16; ++ks)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    const int r = mt * 16 + (lane & 15);
+                    ldmatrix_x4(st + (uint32_t)(r * 128 + (((ks * 2 + (lane >> 4)) ^ (r & 7)) * 16)), wf[ks][mt]);
+                }
+            issue();  // while the fragments arrive
+#pragma unroll
+            for (int ks = 0; ks < kStreamK / 16; ++ks)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int nx = 0; nx < NX; ++nx)
+                        mma_16816<T>(acc[ks & 1][mt][nx], wf[ks][mt][0], wf[ks][mt][1], wf[ks][mt][2], wf[ks][mt][3], xf[nx][ks * 2], xf[nx][ks * 2 + 1]);
         }
-        y[(int64_t)m * y_row_stride + n] = Elem<T>::from_f32(v);
+        // c0, c1 -> (W row g, x rows 2c, 2c + 1); c2, c3 -> (W row g + 8, same)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int nx = 0; nx < NX; ++nx)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const int r = mt * 16 + g + 8 * (e >> 1);
+                    if (r < RMAX) red[(warp * NX * 8 + nx * 8 + 2 * c + (e & 1)) * Cfg::kRedRow + r] = acc[0][mt][nx][e] + acc[1][mt][nx][e];
+                }
+        __syncthreads();
+        const int l0 = tile_begin(tile), n_lines = tile_begin(tile + 1) - l0;
+        auto sum = [&](int m, int r) {
+            float z = 0.f;
+#pragma unroll
+            for (int wi = 0; wi < kStreamWarps; ++wi) z += red[(wi * NX * 8 + m) * Cfg::kRedRow + r];
+            return z;
+        };
+        for (int i = tid; i < M * n_lines; i += kStreamThreads) {
+            const int m = i / n_lines, r = i % n_lines;
+            const int64_t out = (int64_t)m * y_row_stride + l0 + r;
+            float z = sum(m, r);
+            if (bias != nullptr) z += Elem<T>::to_f32(bias[w_row(l0, n_lines, r)]);
+            if (gated) {
+                float up = sum(m, n_lines + r);
+                if (bias != nullptr) up += Elem<T>::to_f32(bias[w_row(l0, n_lines, n_lines + r)]);
+                y[out] = Elem<T>::from_f32(act_silu(z) * up);
+                continue;
+            }
+            if (act_inputs != nullptr) act_inputs[out] = Elem<T>::from_f32(z);
+            switch (activation) {
+                case KB_ACT_TANH: z = act_tanh(z); break;
+                case KB_ACT_GELU: z = act_gelu(z); break;
+                case KB_ACT_FAST_GELU: z = act_fast_gelu(z); break;
+                case KB_ACT_RELU: z = fmaxf(z, 0.f); break;
+                case KB_ACT_SILU: z = act_silu(z); break;
+                default: break;
+            }
+            y[out] = Elem<T>::from_f32(z);
+        }
+        __syncthreads();  // the partial tiles are rewritten by the next round
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 static bool smallm_applicable(const kb_linear_params& p) {
-    return p.M >= 1 && p.M <= 16 && p.K % 8 == 0 && p.x_row_stride % 8 == 0 && (((uintptr_t)p.x) & 15) == 0 &&
-           (((uintptr_t)p.w) & 15) == 0 && p.N <= (int64_t)0x7fffffff / 2 && p.K <= 0x7fffffff;
+    return p.M >= 1 && p.M <= kStreamMaxM && p.K % 8 == 0 && p.x_row_stride % 8 == 0 && (((uintptr_t)p.x) & 15) == 0 &&
+           (((uintptr_t)p.w) & 15) == 0 && p.N <= (int64_t)0x7fffffff / 2 && p.K <= 0x7fffffff &&
+           // above 16 rows x weighs twice as much as W on the way from L2; a large W goes to the tcgen05 kernel
+           (p.M <= 16 || p.N * p.K <= (int64_t)20 << 20);
+}
+
+template <typename T, int RMAX, int NX>
+static int launch_linear_stream(const kb_linear_params& p, cudaStream_t stream, int64_t lines, int64_t ctas, int tiles) {
+    using Cfg = StreamCfg<RMAX, NX>;
+    static PerDeviceOnce attr_once;
+    if (attr_once.first_time() &&
+        cudaFuncSetAttribute(linear_stream_kernel<T, RMAX, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+        return KB_ERR_LAUNCH;
+    launch_pdl(linear_stream_kernel<T, RMAX, NX>, (unsigned)ctas, kStreamThreads, Cfg::kSmemBytes, stream, (const T*)p.x, (const T*)p.w,
+               (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)lines, (int)p.K, p.x_row_stride, p.y_row_stride, p.activation, tiles);
+    return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+}
+
+// Rows of W that a CTA keeps in flight with tiles of r rows: all stages but the one being read.
+template <int NX>
+static int stream_rows_in_flight(int r) {
+    if (r <= 8) return (StreamCfg<8, NX>::kStages - 1) * r;
+    if (r <= 16) return (StreamCfg<16, NX>::kStages - 1) * r;
+    if (r <= 24) return (StreamCfg<24, NX>::kStages - 1) * r;
+    if constexpr (NX < 4) {
+        if (r <= 32) return (StreamCfg<32, NX>::kStages - 1) * r;
+        if (r <= 40) return (StreamCfg<40, NX>::kStages - 1) * r;
+        return (StreamCfg<48, NX>::kStages - 1) * r;
+    }
+    return 0;
+}
+
+template <typename T, int NX>
+static int launch_linear_stream_n(const kb_linear_params& p, cudaStream_t stream) {
+    const bool gated = p.activation == KB_ACT_SWIGLU;
+    const int per_line = gated ? 2 : 1;
+    const int64_t lines = p.N / per_line;
+    // two CTAs per SM; fewer where that would leave a CTA less than eight rows (a whole mma.sync operand half)
+    int64_t ctas = 2 * (int64_t)sm_count();
+    if (lines * per_line < ctas * 8) ctas = (lines * per_line + 7) / 8;
+    const int64_t share = (lines + ctas - 1) / ctas * per_line;  // most rows of a CTA
+    // Tiles per CTA: the fewer the better (a tile costs a cross-warp sum, about as long as four pieces of a
+    // warp), as long as the tile's rows keep the ring full: below about 112 rows in flight per CTA the
+    // copies are bound by latency.
+    int best_tiles = 1, best_rows = 0;
+    double best_cost = 1e300;
+    const int max_rows = NX == 4 ? 24 : 48;
+    for (int64_t t = (share + max_rows - 1) / max_rows; t <= share && t <= (share + 7) / 8 + 1; ++t) {
+        const int rows = (int)((share / per_line + t - 1) / t) * per_line;
+        if (rows > max_rows) continue;
+        const double fill = stream_rows_in_flight<NX>(rows) / 112.0;
+        const double cost = (double)share * p.K / (fill < 1.0 ? fill : 1.0) + (double)t * 16 * kStreamK * rows;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best_tiles = (int)t;
+            best_rows = rows;
+        }
+    }
+    if (best_rows <= 8) return launch_linear_stream<T, 8, NX>(p, stream, lines, ctas, best_tiles);
+    if (best_rows <= 16) return launch_linear_stream<T, 16, NX>(p, stream, lines, ctas, best_tiles);
+    if constexpr (NX < 4) {
+        if (best_rows > 40) return launch_linear_stream<T, 48, NX>(p, stream, lines, ctas, best_tiles);
+        if (best_rows > 32) return launch_linear_stream<T, 40, NX>(p, stream, lines, ctas, best_tiles);
+        if (best_rows > 24) return launch_linear_stream<T, 32, NX>(p, stream, lines, ctas, best_tiles);
+    }
+    return launch_linear_stream<T, 24, NX>(p, stream, lines, ctas, best_tiles);
 }
 
 template <typename T>
 static int launch_linear_smallm_t(const kb_linear_params& p, cudaStream_t stream) {
-    const unsigned grid = (unsigned)((p.N + kSmallMCols - 1) / kSmallMCols);
-    if (p.M > 8)
-        launch_pdl(linear_smallm_kernel<T, true>, grid, kSmallMThreads, 0, stream, (const T*)p.x, (const T*)p.w,
-                   (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.x_row_stride,
-                   p.y_row_stride, p.activation);
-    else
-        launch_pdl(linear_smallm_kernel<T, false>, grid, kSmallMThreads, 0, stream, (const T*)p.x, (const T*)p.w,
-                   (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.x_row_stride,
-                   p.y_row_stride, p.activation);
-    return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+    if (p.M <= 8) return launch_linear_stream_n<T, 1>(p, stream);
+    if (p.M <= 16) return launch_linear_stream_n<T, 2>(p, stream);
+    return launch_linear_stream_n<T, 4>(p, stream);
 }
 
 static int launch_linear_smallm(const kb_linear_params& p, cudaStream_t stream) {
