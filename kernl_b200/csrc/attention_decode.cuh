@@ -15,6 +15,7 @@ namespace kb {
 constexpr int kDecThreads = 128;
 constexpr int kDecMaxSplits = 256;
 constexpr int kDecMaxD = 256;
+constexpr int kDecMaxShares = 16;  // the largest cluster (above eight with the non-portable size allowed)
 
 struct DecDev {
     const void* q; const void* k; const void* v; void* o; const void* mask;
@@ -52,7 +53,7 @@ static int64_t decode_scratch_bytes(int64_t B, int64_t H, int64_t M, int64_t N, 
 // Keys that exist: all N, or the device-side count of a partly filled cache.
 __device__ __forceinline__ int decode_live_keys(const DecDev& p) {
     if (p.kv_len_dev == nullptr) return p.N;
-    const long long n = *p.kv_len_dev;
+    const long long n = *reinterpret_cast<const volatile long long*>(p.kv_len_dev);
     return n < 0 ? 0 : (n < (long long)p.N ? (int)n : p.N);
 }
 
@@ -175,7 +176,7 @@ attn_decode_part1_kernel(const DecDev p) {
 //   * q·kᵀ and P·V are mma.sync.m16n8k16: K rows [key][d] are the "col" operand as they lie, V goes
 //     through ldmatrix.trans. mma.sync on purpose: at most 16 rows exist and the kernel is bound by
 //     memory; what counts is that a byte costs few instructions (130 per warp and 8 KB of K/V).
-//   * The key shares of one problem form a cluster (up to eight CTAs) and meet in distributed
+//   * The key shares of one problem form a cluster (up to sixteen CTAs) and meet in distributed
 //     shared memory: every CTA adds up its slice of the output over the cluster. No scratch, no
 //     second launch (which alone was 3-9 us). The share is computed from the live key count on the device, so
 //     a half-filled cache is spread over all CTAs as evenly as a full one.
@@ -206,8 +207,6 @@ __global__ void __launch_bounds__(kDecThreads, D == 256 ? 1 : 2)
 attn_decode_group_kernel(const DecDev p, const int head_groups) {
     using Tile = DecTile<D>;
     constexpr int KEYS = Tile::kKeys, NT = KEYS / 8, WARPS = kDecThreads / 32, RH = ROWS / 8;
-    pdl_wait();
-    pdl_launch_dependents();
     extern __shared__ __align__(128) uint8_t dec_smem[];
     __shared__ float2 ml_warp[WARPS][16];  // (maximum, sum) of a warp
     __shared__ float2 ml_cta[16];          // ... of the CTA, read by the whole cluster
@@ -219,18 +218,36 @@ attn_decode_group_kernel(const DecDev p, const int head_groups) {
     const int b = bk / kv_heads, hk = bk % kv_heads;
     const int h0 = hk * p.kv_group + hg * ROWS;
     const int rows = min(ROWS, p.kv_group - hg * ROWS);
-
-    // this CTA's keys: an equal share of the live ones, in whole rounds of the four warps
-    const int live = decode_live_keys(p);
-    const int round = WARPS * KEYS;
-    const int share = ((live + p.num_splits - 1) / p.num_splits + round - 1) / round * round;
-    const int key_begin = min(live, (int)blockIdx.x * share);
-    const int key_end = min(live, key_begin + share);
-    const int pieces = (key_end - key_begin + KEYS - 1) / KEYS;
-    const int mine = pieces > warp ? (pieces - warp + WARPS - 1) / WARPS : 0;
-
     const T* kbase = reinterpret_cast<const T*>(p.k) + (int64_t)b * p.k_strides[0] + (int64_t)hk * p.k_strides[1];
     const T* vbase = reinterpret_cast<const T*>(p.v) + (int64_t)b * p.v_strides[0] + (int64_t)hk * p.v_strides[1];
+
+    // this CTA's keys: an equal share of the live ones, in whole rounds of the four warps
+    int key_begin, key_end;
+    auto take_share = [&]() {
+        const int live = decode_live_keys(p);
+        const int round = WARPS * KEYS;
+        const int share = ((live + p.num_splits - 1) / p.num_splits + round - 1) / round * round;
+        key_begin = min(live, (int)blockIdx.x * share);
+        key_end = min(live, key_begin + share);
+    };
+    // Before the wait for the kernel ahead (which may have written q, the newest key and the count) nothing
+    // is read, but the first pieces are asked for in L2: by the count as it is now, which is a hint.
+    take_share();
+    {
+        constexpr int LINES = D * 2 / 128;  // 128-byte lines of a key
+        for (int i = tid; i < (Tile::kStages - 1) * WARPS * KEYS * LINES; i += kDecThreads) {
+            const int key = key_begin + i / LINES;
+            if (key < key_end) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(kbase + (int64_t)key * p.k_strides[2] + (i % LINES) * 64));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(vbase + (int64_t)key * p.v_strides[2] + (i % LINES) * 64));
+            }
+        }
+    }
+    pdl_wait();
+    pdl_launch_dependents();
+    take_share();
+    const int pieces = (key_end - key_begin + KEYS - 1) / KEYS;
+    const int mine = pieces > warp ? (pieces - warp + WARPS - 1) / WARPS : 0;
     const uint32_t ring = smem_u32(dec_smem) + (uint32_t)(warp * Tile::kWarpBytes);
     // chunk j (16 bytes) of row r sits at r * kRowChunks + (j ^ (r & 7)): eight rows of one chunk column lie
     // in eight different bank groups, for the copies as for ldmatrix
@@ -284,13 +301,14 @@ attn_decode_group_kernel(const DecDev p, const int head_groups) {
 #pragma unroll
     for (int hh = 0; hh < RH; ++hh) { m_run[hh] = -INFINITY; l_run[hh] = 0.f; }
 
-    for (int i = 0; i < mine; ++i) {
-        __syncwarp();  // the slot that is refilled next has been read by all lanes
-        if (i + Tile::kStages - 1 < mine) stage(i + Tile::kStages - 1);
-        asm volatile("cp.async.commit_group;" ::: "memory");
+    // Mask values of a piece, as raw bits, one piece ahead: no load is waited for where it is issued. (Fetched and
+    // converted one after the other for the piece at hand, they were the critical path of a masked call: 115 us
+    // instead of 101 before this kernel at [8, 12, 7075, 128] with a bias.)
+    uint32_t mask_next[RH][NT][2];
+    auto fetch_mask = [&](int i) {
+        if (p.mask == nullptr) return;
         const int k0 = key_begin + (warp + i * WARPS) * KEYS;
-        float mv[RH][NT][2];
-        if (p.mask != nullptr) {  // requested before the wait for the piece
+        auto fetch = [&](const auto* base) {
 #pragma unroll
             for (int hh = 0; hh < RH; ++hh)
 #pragma unroll
@@ -298,9 +316,31 @@ attn_decode_group_kernel(const DecDev p, const int head_groups) {
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
                         const int key = k0 + nt * 8 + 2 * c + e;
-                        mv[hh][nt][e] = (key < key_end && g + 8 * hh < rows) ? mask_load(p.mask, mask_off[hh] + (int64_t)key * p.mask_strides[3], p.mask_dtype) : 0.f;
+                        mask_next[hh][nt][e] = (key < key_end && g + 8 * hh < rows) ? __ldg(base + mask_off[hh] + (int64_t)key * p.mask_strides[3]) : 0u;
                     }
-        }
+        };
+        if (p.mask_dtype == KB_F32) fetch(reinterpret_cast<const uint32_t*>(p.mask));
+        else fetch(reinterpret_cast<const uint16_t*>(p.mask));
+    };
+    auto mask_value = [&](uint32_t bits) {
+        if (p.mask_dtype == KB_F32) return __uint_as_float(bits);
+        const uint16_t h = (uint16_t)bits;
+        return p.mask_dtype == KB_F16 ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
+    };
+    if (mine > 0) fetch_mask(0);
+    for (int i = 0; i < mine; ++i) {
+        __syncwarp();  // the slot that is refilled next has been read by all lanes
+        if (i + Tile::kStages - 1 < mine) stage(i + Tile::kStages - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        const int k0 = key_begin + (warp + i * WARPS) * KEYS;
+        uint32_t mv[RH][NT][2];
+#pragma unroll
+        for (int hh = 0; hh < RH; ++hh)
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) mv[hh][nt][e] = mask_next[hh][nt][e];
+        if (i + 1 < mine) fetch_mask(i + 1);
         asm volatile("cp.async.wait_group %0;" ::"n"(Tile::kStages - 1) : "memory");
         __syncwarp();
         const uint32_t kt = ring + (uint32_t)((i % Tile::kStages) * 2 * Tile::kTileBytes), vt = kt + Tile::kTileBytes;
@@ -332,7 +372,7 @@ attn_decode_group_kernel(const DecDev p, const int head_groups) {
                 for (int e = 0; e < 2; ++e) {
                     const int key = k0 + nt * 8 + 2 * c + e;
                     float x = s[nt][hh * 2 + e] * p.scale_log2;
-                    if (p.mask != nullptr) x = fmaf(fmaxf(mv[hh][nt][e], mlow), kLog2e, x);
+                    if (p.mask != nullptr) x = fmaf(fmaxf(mask_value(mv[hh][nt][e]), mlow), kLog2e, x);
                     if (key >= key_end || (p.is_causal && key > row)) x = -INFINITY;
                     s[nt][hh * 2 + e] = x;
                     mx = fmaxf(mx, x);
@@ -457,50 +497,66 @@ attn_decode_part2_kernel(const DecDev p) {
     }
 }
 
-// Key shares per problem (the cluster size, at most the portable eight). A wave of CTAs costs the bytes
-// of one share plus a fixed part — first copies from DRAM, q, the merge: about 2.5 us, which at a
-// slot's part of the copy bandwidth is 56 KB — so shares are cut until one wave is full and no further.
-template <int D>
-static int decode_shares(int64_t units, int64_t N) {
-    const int64_t slots = (int64_t)sm_count() * (D == 256 ? 1 : 2);
-    const int64_t round = (kDecThreads / 32) * DecTile<D>::kKeys;
-    int best = 1;
-    double best_cost = 1e300;
-    for (int s = 1; s <= 8 && (s - 1) * round < N; ++s) {
-        const int64_t share = ((N + s - 1) / s + round - 1) / round * round;
-        const double cost = (double)((units * s + slots - 1) / slots) * ((double)share * D * 4.0 + 56.0 * 1024.0);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = s;
-        }
-    }
-    return best;
-}
-
 template <typename T, int D, int ROWS>
 static int launch_decode_group_r(DecDev d, cudaStream_t stream) {
-    static PerDeviceOnce attr_once;
-    if (attr_once.first_time() &&
-        cudaFuncSetAttribute(attn_decode_group_kernel<T, D, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize, DecTile<D>::kSmemBytes) != cudaSuccess)
-        return KB_ERR_LAUNCH;
+    auto* kernel = attn_decode_group_kernel<T, D, ROWS>;
     const int head_groups = (d.kv_group + ROWS - 1) / ROWS;
-    const int64_t units = (int64_t)d.B * (d.H / d.kv_group) * head_groups * d.M;
-    d.num_splits = decode_shares<D>(units, d.N);
+    const unsigned problems = (unsigned)(d.B * (d.H / d.kv_group) * head_groups);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)d.num_splits, (unsigned)d.M, (unsigned)(d.B * (d.H / d.kv_group) * head_groups));
     cfg.blockDim = dim3(kDecThreads);
     cfg.dynamicSmemBytes = DecTile<D>::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)d.num_splits;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
+    // Clusters that are resident at once, by size: a cluster stays inside one GPC, so that sizes which do not
+    // divide a GPC's CTA slots leave some of them empty (asked once per device).
+    static std::mutex mu;
+    static int resident[64][kDecMaxShares + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return KB_ERR_NO_DEVICE;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (resident[dev][1] == 0) {
+            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DecTile<D>::kSmemBytes) != cudaSuccess ||
+                cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+                return KB_ERR_LAUNCH;
+            cfg.numAttrs = 1;
+            for (int s = kDecMaxShares; s >= 1; --s) {
+                int n = 0;
+                cfg.gridDim = dim3((unsigned)s);
+                attr[0].val.clusterDim.x = (unsigned)s;
+                if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+                    cudaGetLastError();
+                    n = s > 8 ? 0 : 1;  // (not every device takes the large ones)
+                }
+                resident[dev][s] = n;
+            }
+        }
+    }
+    // Key shares per problem (the cluster size). A wave of clusters costs the bytes of one share plus a fixed
+    // part — first copies from DRAM, q, the merge: about 2.5 us, which at a CTA slot's part of the copy
+    // bandwidth is 56 KB — so shares are cut until one wave is full and no further.
+    const int64_t units = (int64_t)problems * d.M, round = (kDecThreads / 32) * DecTile<D>::kKeys;
+    double best_cost = 1e300;
+    d.num_splits = 1;
+    for (int s = 1; s <= kDecMaxShares && (s - 1) * round < d.N; ++s) {
+        if (resident[dev][s] == 0) continue;
+        const int64_t share = ((d.N + s - 1) / s + round - 1) / round * round;
+        const double cost = (double)((units + resident[dev][s] - 1) / resident[dev][s]) * ((double)share * D * 4.0 + 56.0 * 1024.0);
+        if (cost < best_cost) {
+            best_cost = cost;
+            d.num_splits = s;
+        }
+    }
+    cfg.gridDim = dim3((unsigned)d.num_splits, (unsigned)d.M, problems);
+    attr[0].val.clusterDim.x = (unsigned)d.num_splits;
     cfg.numAttrs = g_use_pdl ? 2u : 1u;
-    return cudaLaunchKernelEx(&cfg, attn_decode_group_kernel<T, D, ROWS>, d, head_groups) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+    return cudaLaunchKernelEx(&cfg, kernel, d, head_groups) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
 
 template <typename T>
