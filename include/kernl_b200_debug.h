@@ -23,6 +23,9 @@ void kb_debug_split_tiles(int tiles);
  * tiles from a device-side queue, 2 = the same without the longest-batch-first tile order,
  * 0 = one CTA per query tile, -1 = dispatcher's choice. */
 void kb_debug_attention_persistent(int mode);
+/* Fused attention for short key ranges on mma.sync: 1 = wherever the layout allows it, 0 = never,
+ * -1 = dispatcher's choice. */
+void kb_debug_attention_short(int mode);
 /* 0 = large GEMMs stay on the one-CTA-per-tile kernel instead of CTA pairs on 256-row tiles;
  * 192 / 256 = CTA pairs with that tile width whatever the cost model says; 1 = dispatcher's choice. */
 void kb_debug_linear_pair(int mode);

@@ -53,6 +53,7 @@ struct AttnDev {
     int is_causal;
     int mask_dtype;
     int mask_vec;   // mask rows can be read with aligned 128-bit loads
+    int mask_async; // MODE 2, head dimension 64: mask tiles are staged in shared memory (16-bit values, unit column stride)
     int num_pairs;  // ceil(ceil(M/128)/2)
     int head_group; // heads whose CTAs are interleaved (see attn_work_item)
     int kv_group;   // query heads per K/V head (grouped-query attention), >= 1
@@ -134,6 +135,58 @@ __device__ __forceinline__ float mask_load(const void* base, int64_t off, int ma
     if (mask_dtype == KB_F16) return __half2float(reinterpret_cast<const __half*>(base)[off]);
     if (mask_dtype == KB_BF16) return __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(base)[off]);
     return reinterpret_cast<const float*>(base)[off];
+}
+
+// NV consecutive values of one mask row from `off` on, of which the first `n` exist (the rest read as 0). The
+// type is looked at once and every load is issued before the first value is used: with the type looked
+// at per value, each of a row's loads waited for the one before it (one 64-key block of a mask with odd
+// row strides: 3.3 us).
+template <typename MT, int NV>
+__device__ __forceinline__ void mask_values_t(const MT* __restrict__ row, int64_t stride, int n, float (&out)[NV]) {
+    MT raw[NV];
+    if (stride == 1 && n >= NV) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) raw[i] = __ldg(row + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < NV; ++i) raw[i] = i < n ? __ldg(row + (int64_t)i * stride) : MT(0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < NV; ++i) out[i] = (float)raw[i];
+}
+template <int NV>
+__device__ __forceinline__ void mask_values(const AttnDev& p, int64_t row_off, int col, float (&out)[NV]) {
+    static_assert(NV % 8 == 0, "whole 128-bit loads");
+    const int64_t off = row_off + (int64_t)col * p.mask_strides[3];
+    if (p.mask_vec && col + NV <= p.N) {
+        if (p.mask_dtype == KB_F32) {
+            const float4* mp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.mask) + off);
+#pragma unroll
+            for (int v4 = 0; v4 < NV / 4; ++v4) {
+                const float4 f = __ldg(mp + v4);
+                out[v4 * 4 + 0] = f.x; out[v4 * 4 + 1] = f.y; out[v4 * 4 + 2] = f.z; out[v4 * 4 + 3] = f.w;
+            }
+        } else {
+            const uint4* mp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.mask) + off);
+#pragma unroll
+            for (int v4 = 0; v4 < NV / 8; ++v4) {
+                const uint4 w = __ldg(mp + v4);
+                const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float2 f = (p.mask_dtype == KB_F16) ? Elem<__half>::unpack2(ww[i]) : Elem<__nv_bfloat16>::unpack2(ww[i]);
+                    out[v4 * 8 + 2 * i] = f.x;
+                    out[v4 * 8 + 2 * i + 1] = f.y;
+                }
+            }
+        }
+    } else if (p.mask_dtype == KB_F16) {
+        mask_values_t(reinterpret_cast<const __half*>(p.mask) + off, p.mask_strides[3], p.N - col, out);
+    } else if (p.mask_dtype == KB_BF16) {
+        mask_values_t(reinterpret_cast<const __nv_bfloat16*>(p.mask) + off, p.mask_strides[3], p.N - col, out);
+    } else {
+        mask_values_t(reinterpret_cast<const float*>(p.mask) + off, p.mask_strides[3], p.N - col, out);
+    }
 }
 
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
@@ -459,36 +512,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         for (int hc = 0; hc < 8; ++hc) {
                             const int colc = col0 + hc * 16;
                             float mvals[16];
-                            if (p.mask_vec && colc + 16 <= p.N) {
-                                // 16 consecutive mask values of this row as 128-bit loads
-                                if (p.mask_dtype == KB_F32) {
-                                    const float4* mp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 4; ++v4) {
-                                        const float4 f = __ldg(mp + v4);
-                                        mvals[v4 * 4 + 0] = f.x; mvals[v4 * 4 + 1] = f.y; mvals[v4 * 4 + 2] = f.z; mvals[v4 * 4 + 3] = f.w;
-                                    }
-                                } else {
-                                    const uint4* mp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 2; ++v4) {
-                                        const uint4 w = __ldg(mp + v4);
-                                        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                                        for (int i = 0; i < 4; ++i) {
-                                            const float2 f = (p.mask_dtype == KB_F16) ? Elem<__half>::unpack2(ww[i]) : Elem<__nv_bfloat16>::unpack2(ww[i]);
-                                            mvals[v4 * 8 + 2 * i] = f.x;
-                                            mvals[v4 * 8 + 2 * i + 1] = f.y;
-                                        }
-                                    }
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) {
-                                    const int col = colc + i;
-                                    mvals[i] = (col < p.N) ? mask_load(p.mask, mask_row_off + (int64_t)col * p.mask_strides[3], p.mask_dtype) : 0.f;
-                                }
-                            }
+                            mask_values(p, mask_row_off, colc, mvals);
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
                                 uint32_t& sv = sr[hc >> 1][(hc & 1) * 16 + i];

@@ -729,35 +729,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                         for (int hc = 0; hc < 2; ++hc) {
                             const int colc = col0 + hc * 16;
                             float mvals[16];
-                            if (p.mask_vec && colc + 16 <= p.N) {
-                                if (p.mask_dtype == KB_F32) {
-                                    const float4* mp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 4; ++v4) {
-                                        const float4 f = __ldg(mp + v4);
-                                        mvals[v4 * 4 + 0] = f.x; mvals[v4 * 4 + 1] = f.y; mvals[v4 * 4 + 2] = f.z; mvals[v4 * 4 + 3] = f.w;
-                                    }
-                                } else {
-                                    const uint4* mp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 2; ++v4) {
-                                        const uint4 w = __ldg(mp + v4);
-                                        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                                        for (int i = 0; i < 4; ++i) {
-                                            const float2 f = (p.mask_dtype == KB_F16) ? Elem<__half>::unpack2(ww[i]) : Elem<__nv_bfloat16>::unpack2(ww[i]);
-                                            mvals[v4 * 8 + 2 * i] = f.x;
-                                            mvals[v4 * 8 + 2 * i + 1] = f.y;
-                                        }
-                                    }
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) {
-                                    const int col = colc + i;
-                                    mvals[i] = (col < p.N) ? mask_load(p.mask, mask_row_off + (int64_t)col * p.mask_strides[3], p.mask_dtype) : 0.f;
-                                }
-                            }
+                            mask_values(p, mask_row_off, colc, mvals);
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
                                 uint32_t& sv = sr[hc * 16 + i];
@@ -908,7 +880,7 @@ static int attention_persist_mask_cols(int64_t N) {  // one staged mask row: who
 
 static bool attention_persist_applicable(const kb_attn_params& p, int mode) {
     const int64_t tiles = ((p.M + kAttnBlock - 1) / kAttnBlock) * p.B * p.H;
-    if (g_attn_persistent == 0) return false;
+    if (g_attn_persistent == 0 || mode == 2) return false;  // per-row masks: attention_split.cuh stages them by tile
     if (mode == 1 && (p.N > 8192 || attention_persist_mask_cols(p.N) > AttnPersistCfg::kMaskMaxCols)) return false;
     if (tiles > 0x3fffffff) return false;
     if (g_attn_persistent == 1) return true;

@@ -114,12 +114,17 @@ __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c
                  : "memory");
 }
 
-template <int TILES>
+template <int TILES, int MODE = 0>
 struct AttnSplitCfgT {
-    static constexpr int D = 64;
-    static constexpr int kKvStages = TILES == 2 ? 8 : 4;
-    static constexpr int kQTileBytes = kAttnBlock * D * 2;
-    static constexpr int kKvBytes = kBlkN * D * 2;
+    // MODE 2, one tile: mask tiles of 128 rows x 64 keys through two slots of shared memory, for which the
+    // K/V ring gives up a stage (two CTAs per SM). A row is staged as the nine 16-byte chunks that hold its
+    // 128 bytes wherever they start.
+    static constexpr bool kMaskRing = MODE == 2 && TILES == 1;
+    static constexpr int kMaskRowBytes = 9 * 16;
+    static constexpr int kMaskSlotBytes = kMaskRing ? kAttnBlock * kMaskRowBytes : 0;
+    static constexpr int kKvStages = TILES == 2 ? 8 : kMaskRing ? 3 : 4;
+    static constexpr int kQTileBytes = kAttnBlock * 64 * 2;
+    static constexpr int kKvBytes = kBlkN * 64 * 2;
     static constexpr int kTilesBytes = TILES * kQTileBytes + 2 * kKvStages * kKvBytes;
     static constexpr int kBarBytes = 1024;
     static constexpr int kXchBytes = 2 * 2 * kAttnBlock * 8;  // [tile][half][row] (m, l)
@@ -127,17 +132,58 @@ struct AttnSplitCfgT {
     // log2 domain, staged by all threads during set-up; longer rows take the general path (MODE 2)
     static constexpr int kMaskMaxN = 8192;
     static constexpr int kMaskLoads = (kMaskMaxN + SplitShape<TILES>::kThreads - 1) / SplitShape<TILES>::kThreads;  // per thread
-    static constexpr int kSmemBase = kTilesBytes + kBarBytes + kXchBytes + 1024;
-    static constexpr int kSmemMax = kSmemBase + kMaskMaxN * 4;
+    static constexpr int kSmemBase = kTilesBytes + kBarBytes + kXchBytes + 2 * kMaskSlotBytes + 1024;
+    static constexpr int kSmemMax = kSmemBase + (MODE == 1 ? kMaskMaxN * 4 : 0);
+    static_assert(!kMaskRing || 2 * (kSmemMax + 1024) <= 227 * 1024, "two CTAs per SM");
 };
 
 using AttnSplitCfg = AttnSplitCfgT<2>;
+
+// Adds sixteen mask values of a staged row to scores, in score units: s += max(mask, lowest) * inv_scale, two
+// values per instruction. `src` is the 16-byte chunk in which the row's 32 bytes begin, `shift` (0..7
+// elements) where in it: rows of a mask whose length is no multiple of eight all start differently.
+// (Read ahead of the wait for the scores instead, the sixteen words cost more in spilled registers than
+// their latency: 12.6 -> 16.1 us at [3, 12, 333, 64].)
+__device__ __forceinline__ void add_staged_mask(const AttnDev& p, const uint8_t* src, int shift, float inv_scale, uint32_t* sr) {
+    uint32_t w[12];
+    const uint4* v = reinterpret_cast<const uint4*>(src);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        if (i == 2 && p.mask_vec) break;
+        const uint4 q = v[i];
+        w[4 * i] = q.x; w[4 * i + 1] = q.y; w[4 * i + 2] = q.z; w[4 * i + 3] = q.w;
+    }
+    if (!p.mask_vec) {
+#pragma unroll
+        for (int i = 0; i < 10; ++i) w[i] = (shift & 4) ? w[i + 2] : w[i];
+#pragma unroll
+        for (int i = 0; i < 9; ++i) w[i] = (shift & 2) ? w[i + 1] : w[i];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], (uint32_t)(shift & 1) * 16u);
+    }
+    const float2 inv2 = make_float2(inv_scale, inv_scale);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        float2 f;
+        uint32_t m;
+        if (p.mask_dtype == KB_F16) {
+            asm("max.f16x2 %0, %1, %2;" : "=r"(m) : "r"(w[i]), "r"(0xfbfffbffu));  // the lowest finite value, twice
+            f = Elem<__half>::unpack2(m);
+        } else {
+            asm("max.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(w[i]), "r"(0xff7fff7fu));
+            f = Elem<__nv_bfloat16>::unpack2(m);
+        }
+        const float2 x = __ffma2_rn(f, inv2, make_float2(__uint_as_float(sr[2 * i]), __uint_as_float(sr[2 * i + 1])));
+        sr[2 * i] = __float_as_uint(x.x);
+        sr[2 * i + 1] = __float_as_uint(x.y);
+    }
+}
 
 template <typename T, int MODE, int TILES>
 __global__ void __launch_bounds__(SplitShape<TILES>::kThreads, TILES == 2 ? 1 : 2)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, const AttnDev p) {
-    using Cfg = AttnSplitCfgT<TILES>;
+    using Cfg = AttnSplitCfgT<TILES, MODE>;
     using Shape = SplitShape<TILES>;
     constexpr int kThreads = Shape::kThreads;
     constexpr int W0 = Shape::kAuxWarp;
@@ -168,13 +214,17 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     auto k_empty = [&](int s) { return bar_base + 8u * (kKvBar + KVS + s); };
     auto v_full = [&](int s) { return bar_base + 8u * (kKvBar + 2 * KVS + s); };
     auto v_empty = [&](int s) { return bar_base + 8u * (kKvBar + 3 * KVS + s); };
-    constexpr int kNumBars = kKvBar + 4 * KVS;
+    auto m_full = [&](int sl) { return bar_base + 8u * (kKvBar + 4 * KVS + sl); };
+    auto m_empty = [&](int sl) { return bar_base + 8u * (kKvBar + 4 * KVS + 2 + sl); };
+    constexpr int kNumBars = kKvBar + 4 * KVS + 4;
     static_assert(kNumBars * 8 + 32 <= Cfg::kBarBytes, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     uint32_t* act_bits = tmem_slot + 4;  // MODE 1: which key blocks have at least one unmasked key
     float2* xch = reinterpret_cast<float2*>(smem + Cfg::kTilesBytes + Cfg::kBarBytes);
-    float* mask_smem = reinterpret_cast<float*>(smem + Cfg::kTilesBytes + Cfg::kBarBytes + Cfg::kXchBytes);  // [N rounded up to 64]
+    float* mask_smem = reinterpret_cast<float*>(smem + Cfg::kTilesBytes + Cfg::kBarBytes + Cfg::kXchBytes);  // MODE 1: [N rounded up to 64]
+    uint8_t* mask_ring = reinterpret_cast<uint8_t*>(mask_smem);  // MODE 2: two slots of kMaskSlotBytes
+    const bool mask_async = Cfg::kMaskRing && p.mask_async;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     {
@@ -257,6 +307,10 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             mbar_init(pv_done(lane >> 1, lane & 1), 1);
         }
         if (lane < 8) mbar_init(ep_bar(lane >> 2, lane & 3), 2);
+        if (Cfg::kMaskRing && lane < 2) {
+            mbar_init(m_full(lane), 64);  // the threads of the two loader warps
+            mbar_init(m_empty(lane), 8);
+        }
         if (lane == 0) *abort_flag = 0;
         fence_mbar_init();
     } else if (warp == W0 + 1) {
@@ -411,6 +465,34 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 }
             }
         }
+      } else if (Cfg::kMaskRing && mask_async && warp >= W0 + 2) {
+        // ------------------------------------------------------------------ mask loaders (two warps)
+        // Eight threads in a row read neighbouring chunks of one mask row. (Every softmax thread fetching its own
+        // row touched 32 cache lines per instruction: a block with a mask took twice as long as one without.)
+        // Thread (r0, ch) of 7 x 9 takes chunk ch of rows r0, r0 + 7, ...: pointers advance by a constant.
+        const int lt = (int)threadIdx.x - (W0 + 2) * 32;
+        const int r0 = lt / 9, ch = lt % 9;
+        const int rows = lt < 63 ? min(kAttnBlock, p.M - mt[0] * kAttnBlock) : 0;
+        const int64_t step = 14 * p.mask_strides[2];
+        const uint8_t* base = reinterpret_cast<const uint8_t*>(p.mask) +
+                              2 * ((int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)(mt[0] * kAttnBlock + r0) * p.mask_strides[2]);
+        const uint32_t dst0 = smem_u32(mask_ring) + (uint32_t)(r0 * Cfg::kMaskRowBytes + ch * 16);
+        for (int j = 0; j < n_tile[0]; ++j) {
+            if (!mbar_wait(m_empty(j & 1), (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag, 640)) break;
+            const uint32_t dst = dst0 + (uint32_t)((j & 1) * Cfg::kMaskSlotBytes);
+            const uint8_t* first = base + j * (kBlkN * 2);
+            const int bytes = 2 * min(kBlkN, p.N - j * kBlkN) - ch * 16;  // of the row, from chunk ch of an aligned row on
+#pragma unroll
+            for (int it = 0; it < (kAttnBlock + 6) / 7; ++it) {
+                const uint32_t lead = (uint32_t)(uintptr_t)first & 15u;
+                // a chunk is fetched if it holds a value of the row; what else it holds is not looked at
+                if (it * 7 + r0 < rows && (int)(0u - lead) < bytes)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(it * 7 * Cfg::kMaskRowBytes)), "l"(first - lead + ch * 16) : "memory");
+                first += step;
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(m_full(j & 1)) : "memory");
+        }
+        asm volatile("cp.async.wait_all;" ::: "memory");
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape::kRegsHigh));
@@ -430,7 +512,11 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 (MODE == 2 && p.mask != nullptr)
                     ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)min(row, p.M - 1) * p.mask_strides[2]
                     : 0;
-            const float unit = (MODE == 0) ? c : 1.0f;
+            // where this row starts in its staged chunks, in elements
+            const int mask_shift = (int)(((uintptr_t)p.mask + 2 * (uintptr_t)mask_row_off) >> 1) & 7;
+            // MODE 0 and staged masks: scores stay in their own units, the exponent is (s - m) * c; else log2 domain
+            const float unit = (MODE == 0 || mask_async) ? c : 1.0f;
+            const float inv_scale = kLog2e / c;
             float m_ref = -INFINITY;
             float l = 0.f;
             bool ok = true;
@@ -457,7 +543,14 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         sr[v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 3]), c, a.w));
                     }
                 } else if (MODE == 2) {
-                    if (p.mask == nullptr) {
+                    if (mask_async) {
+                        if (!mbar_wait(m_full(bf), ph, abort_flag, 641)) { ok = false; break; }
+                        const uint8_t* src = mask_ring + bf * Cfg::kMaskSlotBytes + r_in_tile * Cfg::kMaskRowBytes + hf * 64;
+                        add_staged_mask(p, src, mask_shift, inv_scale, sr);
+                        add_staged_mask(p, src + 32, mask_shift, inv_scale, sr + 16);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(m_empty(bf));
+                    } else if (p.mask == nullptr) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) sr[i] = __float_as_uint(__uint_as_float(sr[i]) * c);
                     } else {
@@ -465,35 +558,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         for (int hc = 0; hc < 2; ++hc) {
                             const int colc = col0 + hc * 16;
                             float mvals[16];
-                            if (p.mask_vec && colc + 16 <= p.N) {
-                                if (p.mask_dtype == KB_F32) {
-                                    const float4* mp = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 4; ++v4) {
-                                        const float4 f = __ldg(mp + v4);
-                                        mvals[v4 * 4 + 0] = f.x; mvals[v4 * 4 + 1] = f.y; mvals[v4 * 4 + 2] = f.z; mvals[v4 * 4 + 3] = f.w;
-                                    }
-                                } else {
-                                    const uint4* mp = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(p.mask) + mask_row_off + colc);
-#pragma unroll
-                                    for (int v4 = 0; v4 < 2; ++v4) {
-                                        const uint4 w = __ldg(mp + v4);
-                                        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-                                        for (int i = 0; i < 4; ++i) {
-                                            const float2 f = (p.mask_dtype == KB_F16) ? Elem<__half>::unpack2(ww[i]) : Elem<__nv_bfloat16>::unpack2(ww[i]);
-                                            mvals[v4 * 8 + 2 * i] = f.x;
-                                            mvals[v4 * 8 + 2 * i + 1] = f.y;
-                                        }
-                                    }
-                                }
-                            } else {
-#pragma unroll
-                                for (int i = 0; i < 16; ++i) {
-                                    const int col = colc + i;
-                                    mvals[i] = (col < p.N) ? mask_load(p.mask, mask_row_off + (int64_t)col * p.mask_strides[3], p.mask_dtype) : 0.f;
-                                }
-                            }
+                            mask_values(p, mask_row_off, colc, mvals);
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
                                 uint32_t& sv = sr[hc * 16 + i];
@@ -620,9 +685,8 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
 template <typename T, int MODE, int TILES>
 static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stream) {
-    using Cfg = AttnSplitCfgT<TILES>;
+    using Cfg = AttnSplitCfgT<TILES, MODE>;
     using Shape = SplitShape<TILES>;
-    constexpr int D = 64;
     CUtensorMap tq, tk, tv;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;
@@ -658,6 +722,7 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
         const int64_t per16 = (p.mask_dtype == KB_F32) ? 4 : 8;
         d.mask_vec = (p.mask_strides[0] % per16 == 0 && p.mask_strides[1] % per16 == 0 && p.mask_strides[2] % per16 == 0) ? 1 : 0;
     }
+    d.mask_async = p.mask != nullptr && p.mask_dtype != KB_F32 && p.mask_strides[3] == 1 && p.sm_scale > 0.f ? 1 : 0;
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
     d.num_pairs = (num_m_tiles + TILES - 1) / TILES;  // work items per (batch, head): tile pairs, or tiles
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
@@ -709,8 +774,7 @@ static int launch_attention_split_t(const kb_attn_params& p, cudaStream_t stream
                      : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg::kMaskMaxN) ? 1 : 2;
     if (g_split_tiles == 0 && attention_persist_applicable(p, mode)) {
         if (mode == 0) return launch_attention_persist_tm<T, 0>(p, stream);
-        if (mode == 1) return launch_attention_persist_tm<T, 1>(p, stream);
-        return launch_attention_persist_tm<T, 2>(p, stream);
+        return launch_attention_persist_tm<T, 1>(p, stream);
     }
     if (mode == 0) return launch_attention_split_tm<T, 0>(p, stream);
     if (mode == 1) return launch_attention_split_tm<T, 1>(p, stream);
@@ -722,16 +786,6 @@ static int launch_attention_split(const kb_attn_params& p, cudaStream_t stream) 
     if (p.dtype == KB_F16) return launch_attention_split_t<__half>(p, stream);
     if (p.dtype == KB_BF16) return launch_attention_split_t<__nv_bfloat16>(p, stream);
     return KB_ERR_UNSUPPORTED;
-}
-
-// The fused-attention entry: head dimensions up to 64 -> the split-row kernels above, up to 128 ->
-// attention.cuh (multiples of 8; the kernels compute on 64 / 128 columns, the missing ones are zeros).
-static int launch_attention(const kb_attn_params& p, cudaStream_t stream) {
-    if (p.N <= 0) return KB_ERR_UNSUPPORTED;
-    if (p.M > 0x7fffffff || p.N > 0x7fffffff || p.B * p.H > 0x7fffffff) return KB_ERR_UNSUPPORTED;
-    if (p.D % 8 != 0 || p.D > 128) return KB_ERR_UNSUPPORTED;
-    if (p.D <= 64) return launch_attention_split(p, stream);
-    return launch_attention128(p, stream);
 }
 
 }  // namespace kb

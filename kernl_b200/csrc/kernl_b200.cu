@@ -14,6 +14,7 @@
 #include "attention.cuh"
 #include "attention_split.cuh"
 #include "attention_persist.cuh"
+#include "attention_short.cuh"
 #include "attention_decode.cuh"
 #include "allreduce.cuh"
 #include "rope.cuh"
@@ -167,6 +168,7 @@ void kb_debug_attention_persistent(int mode) {
     g_attn_persistent = mode == 2 ? 1 : mode;
     g_attn_sort_batches = mode == 2 ? 0 : 1;
 }
+void kb_debug_attention_short(int mode) { g_attn_short = mode; }
 void kb_debug_pdl(int on) { g_use_pdl = on ? 1 : 0; }
 void kb_debug_linear_pair(int mode) { g_linear_pair = (mode == 192 || mode == 256) ? mode : (mode ? 1 : 0); }
 void kb_debug_force_splits(int splits) { g_forced_splits = splits; }
