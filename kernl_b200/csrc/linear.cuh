@@ -625,20 +625,9 @@ static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream, cons
     const int64_t items = num_tiles * plan.splits;
     const int grid = (int)(items < gemm_sms() ? items : gemm_sms());
     float* ws = reinterpret_cast<float*>(p.workspace);
-    // Programmatic launch for the few-row problems of latency-bound graphs only: there the kernel
-    // before is small as well. Behind a kernel of thousands of CTAs, 148 early-resident GEMM CTAs
-    // (all of an SM's shared memory, most of its registers) would take the room its later waves need.
-    cudaError_t le;
-    if (p.M <= 1024)
-        le = launch_pdl(linear_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, tmap_x,
-                        tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.y_row_stride,
-                        p.activation, plan.splits, plan.kps, ws);
-    else {
-        linear_tc_kernel<T, BN><<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(
-            tmap_x, tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.y_row_stride,
-            p.activation, plan.splits, plan.kps, ws);
-        le = cudaSuccess;
-    }
+    const cudaError_t le = launch_pdl(linear_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, tmap_x,
+                                      tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.y_row_stride,
+                                      p.activation, plan.splits, plan.kps, ws);
     if (le != cudaSuccess) return KB_ERR_LAUNCH;
     if (cudaGetLastError() != cudaSuccess) return KB_ERR_LAUNCH;
     if (plan.splits > 1) {

@@ -206,6 +206,10 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         tc_fence_after();
     }
     const uint32_t tmem_base = (skip == 0) ? *tmem_slot : 0u;
+    // Launched with programmatic dependent launch: barriers, tensor memory and descriptors are set up while the
+    // kernel ahead drains (a 30 us GEMM of an encoder spent 2-3 us of it on them). Nothing of global memory
+    // but the status word has been touched so far.
+    pdl_wait();
 
     const int num_m = (M + 2 * kGemmBM - 1) / (2 * kGemmBM);  // 256-row tiles
     const int num_n = (N + BN - 1) / BN;
@@ -234,6 +238,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
                 }
             }
+            pdl_launch_dependents();  // every load is on its way: what is left are the last tile's products and its epilogue
             if (!ok) {
                 for (int i = 0; i < 64; ++i) __nanosleep(2000);  // let copies in flight land
             }
@@ -465,7 +470,9 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = kPairSmemBytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
@@ -491,6 +498,7 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     int pairs = (int)(tiles < max_pairs[dev] ? tiles : max_pairs[dev]);
     if (pairs > gemm_sms() / 2) pairs = gemm_sms() / 2;  // a caller-set limit leaves SMs to a concurrent collective
     cfg.gridDim = dim3(2 * (unsigned)pairs);
+    cfg.numAttrs = g_use_pdl ? 2u : 1u;
     if (cudaLaunchKernelEx(&cfg, linear_pair_kernel<T, BN>, tmap_x, tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M,
                            (int)p.N, (int)p.K, p.y_row_stride, p.activation) != cudaSuccess)
         return KB_ERR_LAUNCH;
