@@ -57,8 +57,8 @@ extern "C" {
  * (eps = max(eps, 1.6e-5), layer_norm.py:295-296) is the CALLER's job: eps is used as given.
  * mean / rstd are optional fp32 [rows] side outputs (NULL to skip).
  * residual / sum_out (an addition over the reference, for pre-norm decoders): the kernel first forms
- * s = x + residual, stores s to sum_out and normalises s. Needs unit column strides, cols % 8 == 0,
- * cols <= 6144.
+ * s = x + residual, stores s to sum_out (unless that is NULL) and normalises s. Needs unit column
+ * strides, cols % 8 == 0, cols <= 16384.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
     const void* x;          /* [rows, cols], strides x_row_stride / x_col_stride          */
@@ -74,7 +74,7 @@ typedef struct {
     int32_t     is_rms;
     int32_t     dtype;      /* KB_F16 / KB_BF16 (x, y, gamma, beta share it)              */
     const void* residual;   /* optional [rows, cols] contiguous: normalise x + residual   */
-    void*       sum_out;    /* required with residual: receives x + residual (contiguous) */
+    void*       sum_out;    /* with residual: receives x + residual (contiguous), or NULL   */
 } kb_norm_params;
 
 int kb_norm_fwd(const kb_norm_params* p, void* stream);

@@ -144,15 +144,16 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// layer_norm(x, weight, bias, eps, use_rms_norm, residual, out) -> result, (result, sum) or None
+// layer_norm(x, weight, bias, eps, use_rms_norm, residual, out, with_sum) -> result, (result, sum) or None;
+// with_sum false: the sum of x and the residual is normalised but not stored, and only the result is returned
 PyObject* layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (!arity(n, 7, "layer_norm")) return nullptr;
+    if (!arity(n, 8, "layer_norm")) return nullptr;
     const at::Tensor *x = cuda_tensor(a[0]), *w = cuda_tensor(a[1]);
     const double eps = PyFloat_AsDouble(a[3]);
     if (eps == -1.0 && PyErr_Occurred()) return nullptr;
-    const int rms = PyObject_IsTrue(a[4]);
-    if (rms < 0) return nullptr;
+    const int rms = PyObject_IsTrue(a[4]), with_sum = PyObject_IsTrue(a[7]);
+    if (rms < 0 || with_sum < 0) return nullptr;
     if (x == nullptr || w == nullptr || autocast_on() || x->dim() == 0) Py_RETURN_NONE;
     const int64_t dim = x->dim(), cols = x->size(dim - 1);
     if (!is_16bit(x->scalar_type()) || !like(*w, *x) || w->numel() != cols || w->dim() != 1 || !w->is_contiguous() || !aligned16(*w) ||
@@ -177,7 +178,7 @@ PyObject* layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     const c10::cuda::CUDAGuard guard(x->device());
     if (!y.defined()) y = empty(x->sizes(), *x);
-    if (residual != nullptr) sum = empty(x->sizes(), *x);
+    if (residual != nullptr && with_sum) sum = empty(x->sizes(), *x);
     kb_norm_params p{};
     p.x = x->data_ptr();
     p.y = y.data_ptr();
@@ -191,10 +192,10 @@ PyObject* layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.is_rms = rms;
     p.dtype = dtype_code(x->scalar_type());
     p.residual = residual != nullptr ? residual->data_ptr() : nullptr;
-    p.sum_out = residual != nullptr ? sum.data_ptr() : nullptr;
+    p.sum_out = sum.defined() ? sum.data_ptr() : nullptr;
     const int st = kb_norm_fwd(&p, stream_of(*x));
     if (st != KB_OK) return failed("layer_norm", st);
-    if (residual == nullptr) return THPVariable_Wrap(std::move(y));
+    if (!sum.defined()) return THPVariable_Wrap(std::move(y));
     PyObject* pair = PyTuple_New(2);
     if (pair == nullptr) return nullptr;
     PyTuple_SET_ITEM(pair, 0, THPVariable_Wrap(std::move(y)));

@@ -151,7 +151,6 @@ int kb_device_status_read(int32_t* status_out) {
 int kb_norm_fwd(const kb_norm_params* p, void* stream) {
     if (p == nullptr || p->x == nullptr || p->y == nullptr || p->gamma == nullptr) return KB_ERR_BAD_ARG;
     if (p->rows < 0 || p->cols <= 0) return KB_ERR_BAD_ARG;
-    if (p->residual != nullptr && p->sum_out == nullptr) return KB_ERR_BAD_ARG;
     if (p->residual != nullptr && ((((uintptr_t)p->residual) | ((uintptr_t)p->sum_out)) & 15)) return KB_ERR_UNSUPPORTED;
     if (p->rows == 0) return KB_OK;
     int st = check_device();

@@ -1,6 +1,6 @@
 // LayerNorm / RMSNorm forward for sm_100a. HBM-bound: x is read once and y written once.
 //
-// Fast path: one warp per row, the whole row held in registers as 128-bit vectors (8 elements of
+// Fast path: one, four or eight warps per row, the whole row held in registers as 128-bit vectors (8 elements of
 // a 16-bit type per load), statistics by warp shuffles in fp32 in one sweep over the registers
 // (shifted sums, no second trip to memory). Algorithmic traffic per row is 2*cols*2 bytes.
 // Generic path: arbitrary strides / column counts, one warp per row, re-reads the row (served by
@@ -30,12 +30,16 @@ __device__ __forceinline__ void st_stream_16B(void* p, uint4 v) {
                  : "memory");
 }
 
-// WPR warps share one row (1: a warp per row, for many rows; 4: the whole CTA on one row, for the
-// few rows of a decode step, where a single warp walking 4096 columns is a 19 µs chain of dependent
-// loads). CHUNKS = ceil(cols / (256 * WPR)): each lane owns CHUNKS vectors of 8 elements; vector c of
-// lane l of warp w covers columns ((c*WPR + w)*32 + l)*8 .. +8. cols must be a multiple of 8.
+constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
+
+// WPR warps share one row: 1 for many short rows, 4 (the whole CTA) for rows of more than 1024 columns and for
+// few rows, 8 above 4096 columns. A lane owns CHUNKS = ceil(cols / (256 WPR)) vectors of 8 elements, at most four
+// on every path that matters: with one warp per row a row of 4096 columns took 150 registers per thread
+// and left twelve warps on an SM, all of them loading, then all computing, then all storing:
+// [16384, 4096] bf16 add + RMSNorm 120.9 us (4.4 TB/s), with four warps per row 89.2 us (6.0 TB/s).
+// Vector c of lane l of warp w covers columns ((c*WPR + w)*32 + l)*8 .. +8. cols must be a multiple of 8.
 template <typename T, int CHUNKS, bool RMS, int WPR = 1>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
 norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ gamma,
                         const T* __restrict__ beta, float* __restrict__ mean_out,
                         float* __restrict__ rstd_out, int64_t rows, int cols, int64_t x_row_stride,
@@ -43,10 +47,10 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
                         T* __restrict__ sum_out) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float red_s[2][4];
+    __shared__ float red_s[2][8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wir = warp % WPR;  // this warp's position inside its row
-    const int64_t row = (int64_t)blockIdx.x * (4 / WPR) + warp / WPR;
+    const int64_t row = WPR == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
     if (row >= rows) return;  // (WPR > 1: the whole CTA leaves together)
     const T* xr = x + row * x_row_stride;
     T* yr = y + row * y_row_stride;
@@ -61,7 +65,9 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
     }
     // Short rows: fetch gamma/beta now, next to the row itself, instead of after the statistics, where
     // their (L1/L2) latency would sit at the end of a warp that has nothing left to overlap it with.
-    constexpr bool kEarlyAffine = CHUNKS <= 4;
+    // Not for a LayerNorm of several warps per row: gamma and beta then cost 32 registers a thread and a third of
+    // the warps on an SM ([16384, 4096] with a residual: 109.7 us early, 86.7 us late).
+    constexpr bool kEarlyAffine = CHUNKS <= 4 && (RMS || WPR == 1);
     uint4 gv[kEarlyAffine ? CHUNKS : 1], bv[kEarlyAffine ? CHUNKS : 1];
     if (kEarlyAffine) {
 #pragma unroll
@@ -77,7 +83,7 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
     }
     if (residual != nullptr) {
         // pre-norm residual stream: s = x + residual (rounded to the 16-bit type, as a separate add
-        // kernel would store it), written out once and normalised from the registers
+        // kernel would store it), written out once if it is asked for, and normalised from the registers
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
             const int col = KB_NORM_COL(c);
@@ -92,7 +98,7 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
                     sw[i] = Elem<T>::pack2(a.x + b.x, a.y + b.y);
                 }
                 v[c] = make_uint4(sw[0], sw[1], sw[2], sw[3]);
-                st_stream_16B(sum_out + row * (int64_t)cols + col, v[c]);
+                if (sum_out != nullptr) st_stream_16B(sum_out + row * (int64_t)cols + col, v[c]);
             }
         }
     }
@@ -101,19 +107,14 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
     float mean = 0.f, rstd;
     {
         // One sweep over the registers. LayerNorm accumulates sum(x-K) and sum((x-K)^2) with K = the
-        // row's first element: shifting by a value of the row itself keeps the subtraction
+        // warp's first element: shifting by a value of the row itself keeps the subtraction
         // E[(x-K)^2] - E[x-K]^2 well conditioned even when |mean| >> std (rows like -20 +- 0.5).
         float shift = 0.f;
-        if (!RMS) {
-            if (WPR == 1) {
-                shift = __shfl_sync(0xffffffffu, Elem<T>::unpack2(v[0].x).x, 0);
-            } else {  // every thread reads the row's first element itself (the sum, when a residual is added)
-                float x0 = Elem<T>::to_f32(xr[0]);
-                if (residual != nullptr) x0 = Elem<T>::to_f32(Elem<T>::from_f32(x0 + Elem<T>::to_f32(residual[row * (int64_t)cols])));
-                shift = x0;
-            }
-        }
-        float s1 = 0.f, s2 = 0.f;
+        if (!RMS) shift = __shfl_sync(0xffffffffu, Elem<T>::unpack2(v[0].x).x, 0);
+        // (two values per instruction: at 4096 columns a third of the issue slots went into this sweep and the
+        // last one, and a LayerNorm row took a quarter longer than an RMSNorm row)
+        float2 p1 = make_float2(0.f, 0.f), p2 = make_float2(0.f, 0.f);
+        const float2 neg_shift = make_float2(-shift, -shift);
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
             const int col = KB_NORM_COL(c);
@@ -121,29 +122,55 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
                 const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const float2 f = Elem<T>::unpack2(w[i]);
-                    const float a = f.x - shift, b = f.y - shift;
-                    if (!RMS) s1 += a + b;
-                    s2 = fmaf(a, a, fmaf(b, b, s2));
+                    float2 f = Elem<T>::unpack2(w[i]);
+                    if (!RMS) {
+                        f = __fadd2_rn(f, neg_shift);
+                        p1 = __fadd2_rn(p1, f);
+                    }
+                    p2 = __ffma2_rn(f, f, p2);
                 }
             }
         }
+        float s1 = p1.x + p1.y, s2 = p2.x + p2.y;
         s2 = warp_sum(s2);
         if (!RMS) s1 = warp_sum(s1);
-        if (WPR > 1) {  // WPR == 4: the CTA is one row
+        if (WPR > 1) {
+            // the warps of a row meet: their sums, or (LayerNorm) their means and squared deviations, whose
+            // combination needs no common shift
+            auto columns_of = [&](int w) {
+                int n = 0;
+#pragma unroll
+                for (int c = 0; c < CHUNKS; ++c) n += min(256, max(0, cols - (c * WPR + w) * 256));
+                return (float)n;
+            };
             if (lane == 0) {
-                red_s[0][warp] = s1;
-                red_s[1][warp] = s2;
+                const float n = columns_of(warp), d = n > 0.f ? s1 / n : 0.f;
+                red_s[0][warp] = shift + d;
+                red_s[1][warp] = RMS ? s2 : fmaxf(s2 - s1 * d, 0.f);
             }
             __syncthreads();
-            s1 = (red_s[0][0] + red_s[0][1]) + (red_s[0][2] + red_s[0][3]);
-            s2 = (red_s[1][0] + red_s[1][1]) + (red_s[1][2] + red_s[1][3]);
-        }
-        s2 *= inv_n;
-        if (!RMS) {
-            const float d = s1 * inv_n;
-            mean = shift + d;
-            s2 = fmaxf(s2 - d * d, 0.f);
+            float total = 0.f, m2 = 0.f;
+            if (!RMS) {
+#pragma unroll
+                for (int w = 0; w < WPR; ++w) total = fmaf(columns_of(w), red_s[0][w], total);
+                mean = total * inv_n;
+            }
+#pragma unroll
+            for (int w = 0; w < WPR; ++w) {
+                m2 += red_s[1][w];
+                if (!RMS) {
+                    const float d = red_s[0][w] - mean;
+                    m2 = fmaf(columns_of(w) * d, d, m2);
+                }
+            }
+            s2 = m2 * inv_n;
+        } else {
+            s2 *= inv_n;
+            if (!RMS) {
+                const float d = s1 * inv_n;
+                mean = shift + d;
+                s2 = fmaxf(s2 - d * d, 0.f);
+            }
         }
         rstd = rsqrtf(s2 + eps);
     }
@@ -152,6 +179,7 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
         if (rstd_out) rstd_out[row] = rstd;
     }
 
+    const float2 rstd2 = make_float2(rstd, rstd), neg_mean = make_float2(-mean, -mean);
 #pragma unroll
     for (int c = 0; c < CHUNKS; ++c) {
         const int col = KB_NORM_COL(c);
@@ -172,10 +200,9 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
             for (int i = 0; i < 4; ++i) {
                 const float2 xf = Elem<T>::unpack2(xw[i]);
                 const float2 gf = Elem<T>::unpack2(gw[i]);
-                const float2 bf = Elem<T>::unpack2(bw[i]);
-                const float o0 = (xf.x - mean) * rstd * gf.x + bf.x;
-                const float o1 = (xf.y - mean) * rstd * gf.y + bf.y;
-                ow[i] = Elem<T>::pack2(o0, o1);
+                float2 o = RMS ? __fmul2_rn(xf, rstd2) : __fmul2_rn(__fadd2_rn(xf, neg_mean), rstd2);
+                o = RMS ? __fmul2_rn(o, gf) : __ffma2_rn(o, gf, Elem<T>::unpack2(bw[i]));
+                ow[i] = Elem<T>::pack2(o.x, o.y);
             }
             st_stream_16B(yr + col, make_uint4(ow[0], ow[1], ow[2], ow[3]));
         }
@@ -234,45 +261,29 @@ static int launch_norm_t(const kb_norm_params& p, cudaStream_t stream) {
                         (p.x_row_stride % 8) == 0 && (p.y_row_stride % 8) == 0 &&
                         ((uintptr_t)p.x % 16) == 0 && ((uintptr_t)p.y % 16) == 0 &&
                         ((uintptr_t)p.gamma % 16) == 0 &&
-                        (p.beta == nullptr || ((uintptr_t)p.beta % 16) == 0) && p.cols <= 6144;
-    if (vec_ok && p.rows <= 1024) {
-        // few rows (a decode step, BERT at batch 1): one CTA per row, so that every row is read by 128
-        // threads at once instead of one warp walking it
-        const int chunks4 = (int)((p.cols + 1023) / 1024);
-        const unsigned grid4 = (unsigned)p.rows;
-#define KB_NORM_CASE4(C)                                                                         \
-    if (chunks4 <= C) {                                                                          \
-        return launch_pdl(norm_fwd_rowwarp_kernel<T, C, RMS, 4>, grid4, kWarps * 32, 0, stream,  \
-                   x, y, g, b, p.mean, p.rstd, p.rows, (int)p.cols, p.x_row_stride,              \
-                   p.y_row_stride, p.eps, (const T*)p.residual, (T*)p.sum_out) == cudaSuccess    \
-                   ? KB_OK : KB_ERR_LAUNCH;                                                      \
+                        (p.beta == nullptr || ((uintptr_t)p.beta % 16) == 0) && p.cols <= kNormMaxCols;
+#define KB_NORM_LAUNCH(C, W)                                                                      \
+    return launch_pdl(norm_fwd_rowwarp_kernel<T, C, RMS, W>, W == 1 ? grid : (unsigned)p.rows, W == 8 ? 256 : 128, 0, stream, \
+                      x, y, g, b, p.mean, p.rstd, p.rows, (int)p.cols, p.x_row_stride, p.y_row_stride, p.eps,                  \
+                      (const T*)p.residual, (T*)p.sum_out) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH
+    if (vec_ok && p.cols > 4096) {
+        if (p.cols <= 3 * 2048) KB_NORM_LAUNCH(3, 8);
+        if (p.cols <= 4 * 2048) KB_NORM_LAUNCH(4, 8);
+        KB_NORM_LAUNCH(8, 8);
     }
-        KB_NORM_CASE4(1)
-        KB_NORM_CASE4(2)
-        KB_NORM_CASE4(4)
-        KB_NORM_CASE4(6)
-#undef KB_NORM_CASE4
+    if (vec_ok && (p.cols > 1024 || p.rows <= 1024)) {
+        if (p.cols <= 1024) KB_NORM_LAUNCH(1, 4);
+        if (p.cols <= 2 * 1024) KB_NORM_LAUNCH(2, 4);
+        if (p.cols <= 3 * 1024) KB_NORM_LAUNCH(3, 4);
+        KB_NORM_LAUNCH(4, 4);
     }
     if (vec_ok) {
-        const int chunks = (int)((p.cols + 255) / 256);
-#define KB_NORM_CASE(C)                                                                          \
-    if (chunks <= C) {                                                                           \
-        return launch_pdl(norm_fwd_rowwarp_kernel<T, C, RMS>, grid, kWarps * 32, 0, stream,      \
-                   x, y, g, b, p.mean, p.rstd, p.rows, (int)p.cols, p.x_row_stride,              \
-                   p.y_row_stride, p.eps, (const T*)p.residual, (T*)p.sum_out) == cudaSuccess    \
-                   ? KB_OK : KB_ERR_LAUNCH;                                                      \
+        if (p.cols <= 256) KB_NORM_LAUNCH(1, 1);
+        if (p.cols <= 2 * 256) KB_NORM_LAUNCH(2, 1);
+        if (p.cols <= 3 * 256) KB_NORM_LAUNCH(3, 1);
+        KB_NORM_LAUNCH(4, 1);
     }
-        KB_NORM_CASE(1)
-        KB_NORM_CASE(2)
-        KB_NORM_CASE(3)
-        KB_NORM_CASE(4)
-        KB_NORM_CASE(6)
-        KB_NORM_CASE(8)
-        KB_NORM_CASE(12)
-        KB_NORM_CASE(16)
-        KB_NORM_CASE(24)
-#undef KB_NORM_CASE
-    }
+#undef KB_NORM_LAUNCH
     if (p.residual != nullptr) return KB_ERR_UNSUPPORTED;  // the fused add needs the vector layout
     return launch_pdl(norm_fwd_generic_kernel<T, RMS>, grid, kWarps * 32, 0, stream, x, y, g, b, p.mean, p.rstd, p.rows,
                       p.cols, p.x_row_stride, p.x_col_stride, p.y_row_stride, p.y_col_stride, p.eps) == cudaSuccess

@@ -41,6 +41,7 @@ def layer_norm(
     use_rms_norm: bool = False,
     residual: Optional[torch.Tensor] = None,
     out: Optional[torch.Tensor] = None,
+    with_sum: bool = True,
 ):
     """y = LayerNorm(x) or RMSNorm(x) over the last dimension on the sm_100a kernel.
 
@@ -49,10 +50,10 @@ def layer_norm(
     tensor shaped like x is returned. `implementation` selected one of several Triton kernels in
     the reference; there is a single CUDA implementation here, so it is accepted and ignored.
     `residual` (an extension for pre-norm decoders): normalise x + residual in the same kernel and
-    return the pair (y, x + residual). `out` (an extension as well): a caller-provided result tensor
+    return the pair (y, x + residual), or y alone, without storing the sum, with `with_sum=False`. `out` (an extension as well): a caller-provided result tensor
     shaped like x, written instead of a new one.
     """
-    done = _lib.native().layer_norm(x, weight, bias, eps, use_rms_norm, residual, out)
+    done = _lib.native().layer_norm(x, weight, bias, eps, use_rms_norm, residual, out, with_sum)
     if done is not None:
         return done
     x, weight, bias, residual = cast_if_autocast(x, weight, bias, residual)
@@ -82,9 +83,9 @@ def layer_norm(
         assert residual.shape == x.shape and residual.dtype == x.dtype
         x2 = x2.contiguous()
         residual = _aligned(residual.contiguous())
-        sum_out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
+        sum_out = torch.empty(x.shape, dtype=x.dtype, device=x.device) if with_sum else None
     if rows == 0:
-        return out if residual is None else (out, sum_out)
+        return out if sum_out is None else (out, sum_out)
     p = _lib.NormParams(
         x=x2.data_ptr(), y=out2.data_ptr(), gamma=weight.data_ptr(),
         beta=bias.data_ptr() if bias is not None else None, mean=None, rstd=None,
@@ -97,4 +98,4 @@ def layer_norm(
     )
     with torch.cuda.device(x.device):
         _lib.check(_lib.load().kb_norm_fwd(p, _lib.current_stream(x.device)), "layer_norm")
-    return out if residual is None else (out, sum_out)
+    return out if sum_out is None else (out, sum_out)

@@ -67,8 +67,10 @@ def layer_norm_residual_wrapper(a: torch.Tensor, b: torch.Tensor, layernorm: tor
         layernorm.weight.data = layernorm.weight.data.half()
     if layernorm.bias is not None and layernorm.bias.dtype == torch.float32:
         layernorm.bias.data = layernorm.bias.data.half()
-    if a.shape != b.shape or a.dtype != b.dtype or a.shape[-1] % 8 != 0 or a.shape[-1] > 6144:
+    if a.shape != b.shape or a.dtype != b.dtype or a.shape[-1] % 8 != 0 or a.shape[-1] > 16384:
         return layer_norm(a + b, layernorm.weight, layernorm.bias, layernorm.eps)
+    if a.is_cuda:  # nobody reads the sum: it is not stored
+        return layer_norm(a, layernorm.weight, layernorm.bias, layernorm.eps, residual=b, with_sum=False)
     y, _ = layer_norm(a, layernorm.weight, layernorm.bias, layernorm.eps, residual=b)
     return y
 
@@ -80,7 +82,7 @@ def layer_norm_residual_sum_wrapper(a: torch.Tensor, b: torch.Tensor, layernorm:
     if layernorm.bias is not None and layernorm.bias.dtype == torch.float32:
         layernorm.bias.data = layernorm.bias.data.half()
     fits = (a.shape == b.shape and a.dtype == b.dtype and a.dtype in (torch.float16, torch.bfloat16)
-            and a.shape[-1] % 8 == 0 and a.shape[-1] <= 6144)
+            and a.shape[-1] % 8 == 0 and a.shape[-1] <= 16384)
     if not fits:
         total = a + b
         return layer_norm(total, layernorm.weight, layernorm.bias, layernorm.eps), total
@@ -228,7 +230,7 @@ def layer_norm_rms_residual_wrapper(a: torch.Tensor, b: torch.Tensor, weight: to
     if weight.dtype == torch.float32 and a.dtype == torch.float16:
         weight.data = weight.data.half()
     fits = (a.shape == b.shape and a.dtype == b.dtype and a.dtype in (torch.float16, torch.bfloat16)
-            and a.shape[-1] % 8 == 0 and a.shape[-1] <= 6144)
+            and a.shape[-1] % 8 == 0 and a.shape[-1] <= 16384)
     if not fits:
         total = a + b
         return layer_norm(total, weight, None, eps, use_rms_norm=True), total
