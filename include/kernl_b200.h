@@ -86,11 +86,10 @@ int kb_norm_fwd(const kb_norm_params* p, void* stream);
  * stride and a row stride that is a multiple of 8 elements; K must be a multiple of 8.
  * act_inputs (optional, [M,N], row stride = y_row_stride) receives the pre-activation values
  * (linear_layer.py:193-195).
- * workspace: when the problem has fewer output tiles than SMs (few rows), K is split across work
- * items that accumulate fp32 partial sums into `workspace`. The workspace must be ALL ZERO before
- * the first call that uses it and is left all zero by every call (kb_linear_workspace_bytes gives
- * the size a problem needs); without a workspace, or with one that is too small, the same result
- * is computed unsplit. The reference fixes SPLIT_K = 1 (linear_layer.py:121-122).
+ * workspace: not used. Where a problem has fewer output tiles than SMs, K is divided among the CTAs
+ * of a cluster, which add their partial sums through distributed shared memory in a fixed order. The
+ * fields stay for callers that fill them (kb_linear_workspace_bytes is 0 for every problem). The
+ * reference fixes SPLIT_K = 1 (linear_layer.py:121-122).
  * ------------------------------------------------------------------------------------- */
 typedef struct {
     const void* x;          /* [M,K]                                                       */
@@ -103,8 +102,8 @@ typedef struct {
     int64_t     y_row_stride;
     int32_t     activation; /* KB_ACT_*                                                    */
     int32_t     dtype;      /* KB_F16 / KB_BF16                                            */
-    void*       workspace;  /* optional scratch for split-K, 16-byte aligned, or NULL      */
-    int64_t     workspace_bytes; /* split-K needs >= kb_linear_workspace_bytes(M, N)       */
+    void*       workspace;  /* not used                                                    */
+    int64_t     workspace_bytes; /* not used                                               */
 } kb_linear_params;
 
 int kb_linear_fwd(const kb_linear_params* p, void* stream);

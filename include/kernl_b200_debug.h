@@ -15,7 +15,7 @@ extern "C" {
 
 /* Force the column-tile width of the tcgen05 GEMM (32/64/128/256; 0 = cost model). */
 void kb_debug_force_bn(int bn);
-/* Force the number of K splits of the GEMM (0 = heuristic; needs a workspace). */
+/* Force the number of CTAs that divide K (0 = heuristic, at most 16). */
 void kb_debug_force_splits(int splits);
 /* Query tiles per CTA of the head-dimension-64 attention kernel (0 = dispatcher's choice, 1, 2). */
 void kb_debug_split_tiles(int tiles);

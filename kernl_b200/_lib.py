@@ -189,15 +189,6 @@ def current_stream(device: torch.device) -> int:
     return torch.cuda.current_stream(device).cuda_stream
 
 
-_expiry_hooks = []
-
-
-def on_wait_expired(hook) -> None:
-    """Register a callable that `device_status` runs when it finds that a bounded wait expired
-    (front-ends use it to put scratch that a cut-short kernel may have left dirty back in order)."""
-    _expiry_hooks.append(hook)
-
-
 def device_status() -> list:
     """Synchronise the device and return (and clear) the kernels' status word; raises when a
     bounded device-side wait expired. Kernels launched between the expiry and this call did no
@@ -207,7 +198,5 @@ def device_status() -> list:
     st = load().kb_device_status_read(out)
     vals = list(out)
     if st != KB_OK:
-        for hook in _expiry_hooks:
-            hook()
         raise RuntimeError(f"kernl_b200 device status: {status_str(st)}; word = {vals}")
     return vals

@@ -11,8 +11,6 @@
 // Measured (128 x 768 LayerNorm called back to back): 16.2 us per call through ctypes before.
 #include <Python.h>
 
-#include <vector>
-
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/EmptyTensor.h>
@@ -24,14 +22,6 @@
 #include "../../include/kernl_b200.h"
 
 namespace {
-
-struct Workspace {
-    int device;
-    cudaStream_t stream;
-    void* ptr;
-    int64_t bytes;
-};
-std::vector<Workspace> g_workspaces;  // split-K scratch registered by the Python side (guarded by the GIL)
 
 bool is_none(PyObject* o) { return o == Py_None; }
 
@@ -63,16 +53,6 @@ bool arity(Py_ssize_t got, Py_ssize_t want, const char* name) {
     if (got == want) return true;
     PyErr_Format(PyExc_TypeError, "%s takes %zd arguments, got %zd", name, want, got);
     return false;
-}
-
-// register_workspace(device_index, stream, ptr, bytes)
-PyObject* register_workspace(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (!arity(n, 4, "register_workspace")) return nullptr;
-    const Workspace w{(int)PyLong_AsLong(a[0]), reinterpret_cast<cudaStream_t>(PyLong_AsUnsignedLongLong(a[1])),
-                      reinterpret_cast<void*>(PyLong_AsUnsignedLongLong(a[2])), (int64_t)PyLong_AsLongLong(a[3])};
-    if (PyErr_Occurred()) return nullptr;
-    g_workspaces.push_back(w);
-    Py_RETURN_NONE;
 }
 
 // linear(x, weight, bias, activation_code, act_inputs, out) -> result or None
@@ -115,15 +95,6 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
     }
     void* const stream = stream_of(*x);
     kb_linear_params p{};
-    if (kb_linear_workspace_bytes(M, N) <= ((int64_t)32 << 20)) {  // (the size of the registered buffers)
-        for (const Workspace& s : g_workspaces)
-            if (s.stream == stream && s.device == x->device().index()) {
-                p.workspace = s.ptr;
-                p.workspace_bytes = s.bytes;
-                break;
-            }
-        if (p.workspace == nullptr) Py_RETURN_NONE;  // first call on this stream: the Python side allocates it
-    }
     const c10::cuda::CUDAGuard guard(x->device());
     if (!y.defined()) y = dim == 2 ? empty({M, n_out}, *x) : empty({x->size(0), x->size(1), n_out}, *x);
     p.x = x->data_ptr();
@@ -348,7 +319,7 @@ PyObject* rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
 }
 
 #define KB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {KB_METHOD(register_workspace), KB_METHOD(linear), KB_METHOD(layer_norm), KB_METHOD(attention),
+PyMethodDef methods[] = {KB_METHOD(linear), KB_METHOD(layer_norm), KB_METHOD(attention),
                          KB_METHOD(decode_attention), KB_METHOD(rope_kv_write), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -11,6 +11,7 @@
 #include "linear.cuh"
 #include "linear_pair.cuh"
 #include "linear_smallm.cuh"
+#include "linear_cluster.cuh"
 #include "attention.cuh"
 #include "attention_split.cuh"
 #include "attention_persist.cuh"
@@ -211,15 +212,13 @@ int kb_linear_fwd(const kb_linear_params* p, void* stream) {
     if (p->M > 0x7fffffff || p->N > 0x7fffffff || p->K > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     int st = check_device();
     if (st != KB_OK) return st;
-    // a handful of rows: one pass over W, no tensor map / TMEM / split-K finish (unless a test forces
-    // a tile shape or a split count of the GEMM kernel)
-    if (g_forced_bn == 0 && g_forced_splits == 0 && smallm_applicable(*p)) return launch_linear_smallm(*p, (cudaStream_t)stream);
     return launch_linear(*p, (cudaStream_t)stream, g_forced_bn, g_forced_splits);
 }
 
 int64_t kb_linear_workspace_bytes(int64_t M, int64_t N) {
-    if (M <= 0 || N <= 0) return 0;
-    return splitk_workspace_bytes(M, N);
+    (void)M;
+    (void)N;
+    return 0;  // no kernel needs one: K is divided inside a cluster
 }
 
 int kb_silu_mul(const void* gu, void* y, int64_t M, int64_t N, int32_t dtype, void* stream) {

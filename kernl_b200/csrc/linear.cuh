@@ -8,12 +8,7 @@
 //   warps 2..9  epilogue (two warps per TMEM lane quadrant, each taking half of the tile's columns):
 //               tcgen05.ld of the accumulator (one row per thread), + bias, activation in fp32,
 //               convert, store
-// Split-K: when a problem has fewer output tiles than SMs (few rows: the weight matrix is then
-// streamed from HBM by too few SMs), the K range of every tile is cut into `splits` work items; the
-// items add their fp32 partial tiles into a caller-provided, zero-initialised workspace with vector
-// atomics, and a small second kernel applies bias + activation, converts, and writes the zeros back.
-// (Letting the last-arriving epilogue warp finish its slice inside the GEMM kernel was tried and was
-// slower: the finishing warps serialise on L2 round trips that a separate, fully parallel pass hides.)
+// Problems with fewer output tiles than SMs and a long K go to linear_cluster.cuh, which divides K.
 // Both operands are K-major (x is [M,K], W is [N,K]) which is exactly what tcgen05 wants, so
 // no transposes are needed. Ragged M / N / K edges rely on TMA zero fill for loads and on
 // predicated stores.
@@ -268,8 +263,7 @@ template <typename T, int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                  const T* __restrict__ bias, T* __restrict__ y, T* __restrict__ act_inputs, int M,
-                 int N, int K, int64_t y_row_stride, int activation, int splits, int kps,
-                 float* __restrict__ ws) {
+                 int N, int K, int64_t y_row_stride, int activation) {
     using Cfg = GemmCfg<BN>;
     constexpr int STAGES = Cfg::kStages;
     extern __shared__ uint8_t smem_raw[];
@@ -328,20 +322,15 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int num_n = (N + BN - 1) / BN;
     const int num_tiles = num_m * num_n;
     const int num_k = (K + kGemmBK - 1) / kGemmBK;
-    // work item w -> (tile = w % num_tiles, split = w / num_tiles); split s covers k-blocks
-    // [s*kps, min(num_k, (s+1)*kps)), never empty by construction of `splits`
-    const int num_items = num_tiles * splits;
-
     if (warp == 0) {
         if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
+            for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
                 int m_idx, n_idx;
-                tile_coords(w % num_tiles, num_m, num_n, m_idx, n_idx);
-                const int kb0 = (w / num_tiles) * kps, kb1 = min(num_k, kb0 + kps);
-                for (int kb = kb0; kb < kb1; ++kb) {
+                tile_coords(w, num_m, num_n, m_idx, n_idx);
+                for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag, 100)) { ok = false; break; }
                     mbar_arrive_expect_tx(full_bar(stage), Cfg::kStageBytes);
                     const uint32_t a_dst = smem_base + stage * Cfg::kStageBytes;
@@ -365,12 +354,11 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             int acc = 0;
             uint32_t acc_phase = 0;
             bool ok = true;
-            for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
+            for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
                 if (!mbar_wait(tempty_bar(acc), acc_phase ^ 1, abort_flag, 200)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BN);
-                const int kb0 = (w / num_tiles) * kps, kb1 = min(num_k, kb0 + kps);
-                for (int kb = kb0; kb < kb1; ++kb) {
+                for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag, 201)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_base + stage * Cfg::kStageBytes;
@@ -380,7 +368,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                     for (int k = 0; k < kGemmBK / 16; ++k) {
                         // +32 bytes along K inside the 128-byte swizzle row = +2 in the address field
                         tc_mma_ss(d_tmem, a_desc + 2 * k, b_desc + 2 * k, idesc,
-                                  (kb > kb0 || k > 0) ? 1u : 0u);
+                                  (kb > 0 || k > 0) ? 1u : 0u);
                     }
                     tc_commit(empty_bar(stage));
                     if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -400,9 +388,9 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
-        for (int w = blockIdx.x; w < num_items && ok; w += gridDim.x) {
+        for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
             int m_idx, n_idx;
-            tile_coords(w % num_tiles, num_m, num_n, m_idx, n_idx);
+            tile_coords(w, num_m, num_n, m_idx, n_idx);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 300)) { ok = false; break; }
             tc_fence_after();
             const int row = m_idx * kGemmBM + q * 32 + lane;
@@ -416,25 +404,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + c0), r);
                 tmem_ld_wait();
                 const int col0 = n0 + c0;
-                const bool full_chunk = (col0 + 32 <= N);
-                if (splits > 1) {
-                    // partial tile: fp32 vector atomics into the workspace [M, N]
-                    if (row < M) {
-                        float* wrow = ws + (int64_t)row * N + col0;
-                        if (full_chunk && ((((uintptr_t)wrow) & 15) == 0)) {
-#pragma unroll
-                            for (int v = 0; v < 8; ++v) {
-                                atomicAdd(reinterpret_cast<float4*>(wrow) + v,
-                                          make_float4(__uint_as_float(r[v * 4 + 0]), __uint_as_float(r[v * 4 + 1]),
-                                                      __uint_as_float(r[v * 4 + 2]), __uint_as_float(r[v * 4 + 3])));
-                            }
-                        } else {
-                            for (int j = 0; j < 32; ++j)
-                                if (col0 + j < N) atomicAdd(wrow + j, __uint_as_float(r[j]));
-                        }
-                    }
-                    continue;
-                }
                 float accv[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) accv[j] = __uint_as_float(r[j]);
@@ -460,143 +429,26 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
 }
 
-// Second pass of a split-K launch: y = act(workspace + bias), four columns per thread; the sums are
-// replaced by zeros as they are read, so the workspace is clean again for the next call.
-template <typename T>
-__global__ void __launch_bounds__(256)
-linear_splitk_finish_kernel(float* __restrict__ ws, const T* __restrict__ bias, T* __restrict__ y,
-                            T* __restrict__ act_inputs, int M, int N, int64_t y_row_stride, int activation) {
-    // (no early trigger: what follows is often another GEMM, whose CTAs would sit on the SMs with all
-    // their registers and shared memory while this kernel's CTAs still look for room)
-    pdl_wait();
-    const int nq = (N + 3) / 4;
-    const int64_t total = (int64_t)M * nq;
-    const bool vec4 = (N % 4) == 0;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int row = (int)(i / nq), c0 = (int)(i % nq) * 4;
-        float z[4] = {0.f, 0.f, 0.f, 0.f};
-        float* wp = ws + (int64_t)row * N + c0;
-        if (vec4) {
-            const float4 f = __ldcg(reinterpret_cast<const float4*>(wp));
-            __stcg(reinterpret_cast<float4*>(wp), make_float4(0.f, 0.f, 0.f, 0.f));
-            z[0] = f.x; z[1] = f.y; z[2] = f.z; z[3] = f.w;
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c0 + j < N) { z[j] = __ldcg(wp + j); __stcg(wp + j, 0.f); }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (bias != nullptr && c0 + j < N) z[j] += Elem<T>::to_f32(bias[c0 + j]);
-        if (act_inputs) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (c0 + j < N) act_inputs[(int64_t)row * y_row_stride + c0 + j] = Elem<T>::from_f32(z[j]);
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float v = z[j];
-            switch (activation) {
-                case KB_ACT_TANH: v = act_tanh(v); break;
-                case KB_ACT_GELU: v = act_gelu(v); break;
-                case KB_ACT_FAST_GELU: v = act_fast_gelu(v); break;
-                case KB_ACT_RELU: v = fmaxf(v, 0.f); break;
-                case KB_ACT_SILU: v = act_silu(v); break;
-                default: break;
-            }
-            if (c0 + j < N) y[(int64_t)row * y_row_stride + c0 + j] = Elem<T>::from_f32(v);
-        }
-    }
-}
-
-// Second pass of a split-K launch with the gated epilogue (KB_ACT_SWIGLU): four output columns per
-// thread, read from the gate block and the up block eight columns further (see epilogue_chunk_swiglu).
-template <typename T>
-__global__ void __launch_bounds__(256)
-linear_splitk_finish_swiglu_kernel(float* __restrict__ ws, const T* __restrict__ bias, T* __restrict__ y, int M,
-                                   int N, int64_t y_row_stride) {
-    pdl_wait();
-    const int nq = N / 8;  // N / 2 output columns, four per thread
-    const int64_t total = (int64_t)M * nq;
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-        const int row = (int)(i / nq), oc0 = (int)(i % nq) * 4;
-        const int gc = (oc0 >> 3) * 16 + (oc0 & 7);  // gate column; the up column is gc + 8
-        float* wp = ws + (int64_t)row * N + gc;
-        const float4 g4 = __ldcg(reinterpret_cast<const float4*>(wp));
-        const float4 u4 = __ldcg(reinterpret_cast<const float4*>(wp + 8));
-        __stcg(reinterpret_cast<float4*>(wp), zero);
-        __stcg(reinterpret_cast<float4*>(wp + 8), zero);
-        float g[4] = {g4.x, g4.y, g4.z, g4.w}, u[4] = {u4.x, u4.y, u4.z, u4.w};
-        if (bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                g[j] += Elem<T>::to_f32(bias[gc + j]);
-                u[j] += Elem<T>::to_f32(bias[gc + 8 + j]);
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) y[(int64_t)row * y_row_stride + oc0 + j] = Elem<T>::from_f32(act_silu(g[j]) * u[j]);
-    }
-}
-
-// Split-K workspace: fp32 partial sums [M, N]. It must be all zero before the first call that uses
-// it; every call leaves it zero again (the finishing kernel writes the zeros back as it reads).
-static int64_t splitk_workspace_bytes(int64_t M, int64_t N) { return ((M * N * (int64_t)sizeof(float)) + 15) / 16 * 16; }
-// Splitting pays only while the extra pass over the output is small next to streaming W once:
-// few row tiles and a bounded output.
-static bool splitk_allowed(int64_t M, int64_t N) { return M <= 1024 && M * N <= (int64_t)4 << 20; }
-
-struct LinearPlan {
-    int bn;      // column-tile width
-    int splits;  // K splits per tile (1 = none)
-    int kps;     // k-blocks per split
-};
-
-// Cost model, in units of "bytes staged per SM": waves of work items x k-blocks per item (+2 for the
-// fixed per-item cost) x bytes per k-block. Wide tiles re-stream x less often; splitting K fills the
-// SMs when there are few tiles (few rows: the op is then bound by streaming W from HBM once, and
-// what counts is how many SMs pull on it and how many bytes each keeps in flight).
-static LinearPlan plan_linear(int64_t M, int64_t N, int64_t K, bool has_ws, int forced_bn, int forced_splits) {
-    const int sms = gemm_sms();
-    const int64_t num_m = (M + kGemmBM - 1) / kGemmBM;
-    const int num_k = (int)((K + kGemmBK - 1) / kGemmBK);
-    LinearPlan best{32, 1, num_k};
+// Column-tile width: waves of tiles x (k-blocks + 2 for the fixed cost of a tile) x bytes staged per k-block.
+// Wide tiles re-stream x less often, narrow ones give every SM something to do.
+static int plan_linear_bn(int64_t M, int64_t N, int64_t K, int forced_bn) {
+    const int64_t num_m = (M + kGemmBM - 1) / kGemmBM, num_k = (K + kGemmBK - 1) / kGemmBK;
+    int best = 32;
     double best_cost = 1e300;
     for (int bn : {256, 128, 64, 32}) {
         if (forced_bn != 0 && bn != forced_bn) continue;
         const int64_t tiles = num_m * ((N + bn - 1) / bn);
-        const int max_splits = has_ws ? (num_k / 2 < 1 ? 1 : (num_k / 2 > 32 ? 32 : num_k / 2)) : 1;
-        for (int s = 1; s <= max_splits; ++s) {
-            if (forced_splits != 0 && s != forced_splits && !(forced_splits > max_splits && s == max_splits)) continue;
-            const int kps = (num_k + s - 1) / s;
-            const int eff = (num_k + kps - 1) / kps;  // splits that are not empty
-            if (eff != s) continue;
-            const int64_t waves = (tiles * s + sms - 1) / sms;
-            double cost = (double)waves * ((double)kps + 2.0) * (double)(kGemmBM + bn);
-            if (s > 1) {
-                // Splitting K is not free: every split adds its tile into the fp32 workspace with
-                // atomics (8 bytes of traffic per output element and split) and a second kernel reads
-                // the sums back, applies the epilogue and clears the workspace. Measured on B200: about
-                // 2.6 µs for the extra launch plus the traffic at ~2 TB/s, against ~0.13 µs per k-block of
-                // a 128x32 tile (0.0008 µs per cost unit). With the earlier, far smaller penalty the
-                // heuristic split [512,768]x[3072,768] (25 µs instead of 10) and [128,4096]x[11008,4096]
-                // (33 µs instead of 21).
-                const double mn = (double)M * (double)N;
-                const double extra_us = 2.6 + (double)s * mn * 8.0 / 2.0e6 + mn * 6.0 / 3.0e6;
-                cost += extra_us / 0.0008;
-            }
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = LinearPlan{bn, s, kps};
-            }
+        const double cost = (double)((tiles + gemm_sms() - 1) / gemm_sms()) * ((double)num_k + 2.0) * (double)(kGemmBM + bn);
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = bn;
         }
     }
     return best;
 }
 
 template <typename T, int BN>
-static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream, const LinearPlan& plan) {
+static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream) {
     using Cfg = GemmCfg<BN>;
     CUtensorMap tmap_x, tmap_w;
     {
@@ -622,27 +474,12 @@ static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream, cons
         if (e != cudaSuccess) return KB_ERR_LAUNCH;
     }
     const int64_t num_tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + BN - 1) / BN);
-    const int64_t items = num_tiles * plan.splits;
-    const int grid = (int)(items < gemm_sms() ? items : gemm_sms());
-    float* ws = reinterpret_cast<float*>(p.workspace);
+    const int grid = (int)(num_tiles < gemm_sms() ? num_tiles : gemm_sms());
     const cudaError_t le = launch_pdl(linear_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, tmap_x,
                                       tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N, (int)p.K, p.y_row_stride,
-                                      p.activation, plan.splits, plan.kps, ws);
+                                      p.activation);
     if (le != cudaSuccess) return KB_ERR_LAUNCH;
     if (cudaGetLastError() != cudaSuccess) return KB_ERR_LAUNCH;
-    if (plan.splits > 1) {
-        const bool gated = p.activation == KB_ACT_SWIGLU;
-        const int64_t total = gated ? p.M * (p.N / 8) : p.M * ((p.N + 3) / 4);
-        int64_t blocks = (total + 255) / 256;
-        if (blocks > (int64_t)sm_count() * 8) blocks = (int64_t)sm_count() * 8;
-        if (gated)
-            launch_pdl(linear_splitk_finish_swiglu_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, stream, ws, (const T*)p.bias,
-                       (T*)p.y, (int)p.M, (int)p.N, p.y_row_stride);
-        else
-            launch_pdl(linear_splitk_finish_kernel<T>, dim3((unsigned)blocks), dim3(256), 0, stream, ws, (const T*)p.bias, (T*)p.y,
-                       (T*)p.act_inputs, (int)p.M, (int)p.N, p.y_row_stride, p.activation);
-        if (cudaGetLastError() != cudaSuccess) return KB_ERR_LAUNCH;
-    }
     return KB_OK;
 }
 
@@ -652,23 +489,13 @@ template <typename T>
 static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream);
 
 template <typename T>
-static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
-    if (forced_bn == 0 && forced_splits == 0 && linear_pair_applicable(p)) return launch_linear_pair_t<T>(p, stream);
-    const bool has_ws = p.workspace != nullptr && p.workspace_bytes >= splitk_workspace_bytes(p.M, p.N) &&
-                        (((uintptr_t)p.workspace) & 15) == 0 && (splitk_allowed(p.M, p.N) || forced_splits > 1);
-    const LinearPlan plan = plan_linear(p.M, p.N, p.K, has_ws, forced_bn, forced_splits);
-    switch (plan.bn) {
-        case 256: return launch_linear_bn<T, 256>(p, stream, plan);
-        case 128: return launch_linear_bn<T, 128>(p, stream, plan);
-        case 64: return launch_linear_bn<T, 64>(p, stream, plan);
-        default: return launch_linear_bn<T, 32>(p, stream, plan);
+static int launch_linear_single(const kb_linear_params& p, cudaStream_t stream, int forced_bn) {
+    switch (plan_linear_bn(p.M, p.N, p.K, forced_bn)) {
+        case 256: return launch_linear_bn<T, 256>(p, stream);
+        case 128: return launch_linear_bn<T, 128>(p, stream);
+        case 64: return launch_linear_bn<T, 64>(p, stream);
+        default: return launch_linear_bn<T, 32>(p, stream);
     }
-}
-
-static int launch_linear(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
-    if (p.dtype == KB_F16) return launch_linear_t<__half>(p, stream, forced_bn, forced_splits);
-    if (p.dtype == KB_BF16) return launch_linear_t<__nv_bfloat16>(p, stream, forced_bn, forced_splits);
-    return KB_ERR_UNSUPPORTED;
 }
 
 // y = silu(g) * u with gu = [g | u] along columns.

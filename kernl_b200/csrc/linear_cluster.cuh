@@ -1,0 +1,349 @@
+// Linear layer for up to about a thousand rows: one output tile per cluster, its K range divided among the
+// cluster's CTAs. y = act(x · Wᵀ + bias).
+//
+// Bound: latency (a projection of BERT-base over 128 tokens moves 1-5 MB and takes 0.1 us of tensor time)
+// and, for a large W, HBM. What such a launch pays for is the bytes each SM has to pull through its own
+// port to L2 (a 128 x 32 tile over K = 768 pulled 245 KB, 2 us, on 24 of 148 SMs) and the passes around the
+// products. So:
+//   * W is the M = 128 operand of tcgen05.mma, x the N = 32, 64 or 128 one: a few rows waste no tensor
+//     memory or shared memory on absent ones, and a tile of 128 x 128 reads the least per product;
+//   * the K range of a tile goes to `splits` CTAs (one cluster, up to sixteen), so that every SM takes part
+//     and each pulls little. The fp32 partial tiles meet in distributed shared memory: every CTA adds up
+//     its share of the tile over the cluster, applies bias and activation and stores it. No workspace, no
+//     atomics, no second launch (the split-K this replaces took 2.6 us for its finishing kernel alone and
+//     added in no fixed order);
+//   * two CTAs share an SM; barriers, tensor memory and descriptors are set up, and the first W tiles asked
+//     for in L2, while the kernel ahead drains (programmatic dependent launch).
+// Warps: 0 TMA producer, 1 tcgen05 issuer, 2..5 tensor memory -> shared memory; all six add and store.
+#pragma once
+#include "linear.cuh"
+#include "linear_pair.cuh"
+#include "linear_smallm.cuh"
+
+namespace kb {
+
+constexpr int kClThreads = 192;
+constexpr int kClMaxSplits = 16;
+
+template <int NB>
+struct ClCfg {  // NB: rows of x per tile
+    static constexpr int kWBytes = 128 * kGemmBK * 2;
+    static constexpr int kStageBytes = kWBytes + NB * kGemmBK * 2;
+    static constexpr int kStages = NB == 128 ? 3 : NB == 64 ? 4 : 5;
+    static constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
+    static_assert(NB * 128 * 4 <= kStages * kStageBytes, "the partial tile reuses the stages");
+    static_assert(2 * (kSmemBytes + 1024) <= 227 * 1024, "two CTAs per SM");
+};
+
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* map, int x, int y) {
+    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t own_addr, uint32_t rank) {
+    uint32_t a;
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+
+template <typename T, int NB>
+__global__ void __launch_bounds__(kClThreads, 2)
+linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const T* __restrict__ bias,
+                      T* __restrict__ y, T* __restrict__ act_inputs, int M, int N, int K, int64_t y_row_stride, int activation, int splits) {
+    using Cfg = ClCfg<NB>;
+    constexpr int STAGES = Cfg::kStages;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * Cfg::kStageBytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+    const uint32_t smem_base = smem_u32(smem), bar_base = smem_u32(bars);
+    auto full_bar = [&](int s) { return bar_base + 8u * s; };
+    auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
+    const uint32_t done_bar = bar_base + 8u * (2 * STAGES);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)blockIdx.x % splits, tile = (int)blockIdx.x / splits;
+    const int num_m = (M + NB - 1) / NB;
+    const int m0 = (tile % num_m) * NB, n0 = (tile / num_m) * 128;  // the row tiles of one W tile are neighbours
+    const int num_k = (K + kGemmBK - 1) / kGemmBK;
+    const int kb0 = rank * num_k / splits, kb1 = (rank + 1) * num_k / splits;  // never empty: splits <= num_k
+
+    if (threadIdx.x == 0) {
+        tma_prefetch_desc(&tmap_w);
+        tma_prefetch_desc(&tmap_x);
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(full_bar(s), 1);
+            mbar_init(empty_bar(s), 1);
+        }
+        mbar_init(done_bar, 1);
+        *abort_flag = 0;
+        fence_mbar_init();
+        // only a hint to L2: W may be the output of the kernel ahead, so nothing of it is read before the wait
+        for (int kb = kb0; kb < min(kb1, kb0 + STAGES); ++kb) tma_prefetch_l2_2d(&tmap_w, kb * kGemmBK, n0);
+    }
+    if (warp == 1) {
+        tmem_alloc(smem_u32(tmem_slot), NB);
+        tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    pdl_launch_dependents();
+    // set by a wait that expired in an earlier launch: nothing is stored then (looked at in the end, so that the
+    // CTAs of a cluster, which may read it at different times, take the same way through its barriers)
+    const int skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+
+    if (warp == 0) {
+        if (elect_one()) {
+            bool ok = true;
+            for (int kb = kb0; kb < kb1 && ok; ++kb) {
+                const int i = kb - kb0, s = i % STAGES;
+                if (!mbar_wait(empty_bar(s), (uint32_t)((i / STAGES) & 1) ^ 1u, abort_flag, 130)) { ok = false; break; }
+                mbar_arrive_expect_tx(full_bar(s), Cfg::kStageBytes);
+                const uint32_t dst = smem_base + s * Cfg::kStageBytes;
+                tma_load_2d(dst, &tmap_w, full_bar(s), kb * kGemmBK, n0);
+                tma_load_2d(dst + Cfg::kWBytes, &tmap_x, full_bar(s), kb * kGemmBK, m0);
+            }
+            if (!ok) {
+                for (int i = 0; i < 64; ++i) __nanosleep(2000);  // let copies in flight land
+            }
+        }
+    } else if (warp == 1) {
+        if (elect_one()) {
+            constexpr uint32_t idesc = make_idesc_f16(Elem<T>::kIsBf16, 128, NB, 0, 0);
+            bool ok = true;
+            for (int kb = kb0; kb < kb1; ++kb) {
+                const int i = kb - kb0, s = i % STAGES;
+                if (!mbar_wait(full_bar(s), (uint32_t)((i / STAGES) & 1), abort_flag, 230)) { ok = false; break; }
+                tc_fence_after();
+                const uint32_t a_addr = smem_base + s * Cfg::kStageBytes;
+                const uint64_t a_desc = make_smem_desc_sw128(a_addr, 16, 1024);
+                const uint64_t b_desc = make_smem_desc_sw128(a_addr + Cfg::kWBytes, 16, 1024);
+#pragma unroll
+                for (int k = 0; k < kGemmBK / 16; ++k) tc_mma_ss(tmem_base, a_desc + 2 * k, b_desc + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+                tc_commit(empty_bar(s));
+            }
+            if (ok) tc_commit(done_bar);
+        }
+    } else if (mbar_wait(done_bar, 0, abort_flag, 330)) {
+        // every product of this CTA is complete, so the stages are free: the partial tile goes there, [x row][W row]
+        tc_fence_after();
+        const int q = warp & 3;  // tensor-memory quadrant: 32 rows of W
+        float* part = reinterpret_cast<float*>(smem) + q * 32 + lane;
+#pragma unroll 1
+        for (int c0 = 0; c0 < NB && m0 + c0 < M; c0 += 32) {
+            uint32_t r[32];
+            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+            tmem_ld_wait();
+#pragma unroll
+            for (int j = 0; j < 32; ++j) part[(c0 + j) * 128] = __uint_as_float(r[j]);
+        }
+        tc_fence_before();
+    }
+    __syncwarp();
+    cluster_sync_all();  // (a cluster of one: a CTA barrier)
+
+    // ---- this CTA's share of the tile: four outputs per thread, summed over the cluster in rank order
+    const bool gated = activation == KB_ACT_SWIGLU;
+    const int quads = gated ? 16 : 32;  // groups of four output columns of a tile row
+    const int total = min(NB, M - m0) * quads;
+    for (int i = rank * kClThreads + (int)threadIdx.x; i < total; i += splits * kClThreads) {
+        const int m = i / quads, q = i % quads;
+        // gated: W rows in blocks of eight gate and eight up rows; outputs 8 j .. from gate rows 16 j .., up rows 16 j + 8 ..
+        const int nl = gated ? (q >> 1) * 16 + (q & 1) * 4 : q * 4;
+        auto sum4 = [&](int n_local, float (&z)[4]) {
+            const uint32_t addr = smem_base + (uint32_t)((m * 128 + n_local) * 4);
+            z[0] = z[1] = z[2] = z[3] = 0.f;
+            for (int s = 0; s < splits; s += 4) {  // four loads on their way before the first is added
+                float4 f[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) f[e] = ld_cluster_f32x4(addr, (uint32_t)min(s + e, splits - 1));
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (s + e < splits) { z[0] += f[e].x; z[1] += f[e].y; z[2] += f[e].z; z[3] += f[e].w; }
+            }
+            if (bias != nullptr) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (n0 + n_local + e < N) z[e] += Elem<T>::to_f32(__ldg(bias + n0 + n_local + e));
+            }
+        };
+        if (n0 + nl >= N) continue;
+        float z[4];
+        sum4(nl, z);
+        const int64_t row = (int64_t)(m0 + m) * y_row_stride;
+        int n_out = n0 + nl, left = N - n_out;
+        if (gated) {
+            float up[4];
+            sum4(nl + 8, up);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) z[e] = act_silu(z[e]) * up[e];
+            n_out = (n0 >> 1) + (q >> 1) * 8 + (q & 1) * 4;
+            left = 4;
+        } else {
+            if (act_inputs != nullptr && skip == 0)
+                for (int e = 0; e < 4 && e < left; ++e) act_inputs[row + n_out + e] = Elem<T>::from_f32(z[e]);
+            apply_activation(z, activation);
+        }
+        if (skip != 0) continue;
+        T* dst = y + row + n_out;
+        if (left >= 4 && (((uintptr_t)dst) & 7) == 0) {
+            *reinterpret_cast<uint2*>(dst) = make_uint2(Elem<T>::pack2(z[0], z[1]), Elem<T>::pack2(z[2], z[3]));
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (e < left) dst[e] = Elem<T>::from_f32(z[e]);
+        }
+    }
+    __syncwarp();
+    cluster_sync_all();  // nobody leaves while its shared memory may still be read
+    if (warp == 1) tmem_dealloc(tmem_base, NB);
+}
+
+// Clusters of `splits` CTAs that are resident at once (asked once per device and size).
+template <typename T, int NB>
+static int linear_cluster_resident(int splits) {
+    static std::mutex mu;
+    static int resident[64][kClMaxSplits + 1] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lock(mu);
+    if (resident[dev][1] == 0) {
+        auto* kernel = linear_cluster_kernel<T, NB>;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ClCfg<NB>::kSmemBytes) != cudaSuccess ||
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+            return 0;
+        cudaLaunchConfig_t cfg = {};
+        cfg.blockDim = dim3(kClThreads);
+        cfg.dynamicSmemBytes = ClCfg<NB>::kSmemBytes;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        for (int s = kClMaxSplits; s >= 1; --s) {
+            int n = 0;
+            cfg.gridDim = dim3((unsigned)s);
+            attr[0].val.clusterDim.x = (unsigned)s;
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+                cudaGetLastError();
+                n = s > 8 ? 0 : 1;  // (not every device takes the large ones)
+            }
+            resident[dev][s] = n;
+        }
+    }
+    return resident[dev][splits];
+}
+
+template <typename T, int NB>
+static int launch_linear_cluster(const kb_linear_params& p, cudaStream_t stream, int splits) {
+    if (linear_cluster_resident<T, NB>(splits) == 0) return KB_ERR_LAUNCH;
+    CUtensorMap tmap_w, tmap_x;
+    {
+        const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.N};
+        const uint64_t strides[2] = {0, (uint64_t)p.K * 2};
+        const uint32_t box[2] = {kGemmBK, 128};
+        const int st = encode_tmap_16bit(&tmap_w, p.w, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
+        if (st != KB_OK) return st;
+    }
+    {
+        const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.M};
+        const uint64_t strides[2] = {0, (uint64_t)p.x_row_stride * 2};
+        const uint32_t box[2] = {kGemmBK, NB};
+        const int st = encode_tmap_16bit(&tmap_x, p.x, 2, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
+        if (st != KB_OK) return st;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(((p.M + NB - 1) / NB) * ((p.N + 127) / 128) * splits));
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = ClCfg<NB>::kSmemBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)splits;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 2u : 1u;
+    return cudaLaunchKernelEx(&cfg, linear_cluster_kernel<T, NB>, tmap_w, tmap_x, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)p.N,
+                              (int)p.K, p.y_row_stride, p.activation, splits) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
+}
+
+template <typename T>
+static int launch_linear_cluster_n(const kb_linear_params& p, cudaStream_t stream, int nb, int splits) {
+    if (nb == 32) return launch_linear_cluster<T, 32>(p, stream, splits);
+    if (nb == 64) return launch_linear_cluster<T, 64>(p, stream, splits);
+    return launch_linear_cluster<T, 128>(p, stream, splits);
+}
+
+
+// ---- which kernel a problem of 17 to 1024 rows goes to
+//
+// Estimates in us, fitted to times of the three kernels (graphs of calls with cold W) over 20 to 1000 rows and W
+// from 500 x 1000 to 12288 x 4096; off by up to a fifth, mostly by less than a tenth. An SM pulls about 118 bytes
+// per ns through its port to L2, shared by its CTAs; W comes from HBM at 6.5 bytes per ps at best.
+struct ClusterPlan {
+    int nb, splits;
+    double us;
+};
+template <typename T>
+static ClusterPlan linear_cluster_plan(const kb_linear_params& p) {
+    ClusterPlan best{0, 0, 1e300};
+    const int64_t num_k = (p.K + kGemmBK - 1) / kGemmBK, num_n = (p.N + 127) / 128;
+    const double w_bytes = (double)p.N * (double)p.K * 2.0, hbm = w_bytes / 6.5e6;
+    for (int nb : {32, 64, 128}) {
+        if (nb == 32 ? p.M > 256 : nb == 64 ? p.M <= 32 : p.M <= 64) continue;
+        const int64_t tiles = ((p.M + nb - 1) / nb) * num_n;
+        for (int s = 1; s <= kClMaxSplits && s <= num_k; ++s) {
+            const int resident = nb == 32 ? linear_cluster_resident<T, 32>(s) : nb == 64 ? linear_cluster_resident<T, 64>(s) : linear_cluster_resident<T, 128>(s);
+            if (resident == 0) continue;
+            const double waves = (double)((tiles + resident - 1) / resident);
+            const bool shared_sm = (tiles < resident ? tiles : resident) * s > sm_count();
+            const double load = (double)((num_k + s - 1) / s) * (16384.0 + (double)(p.M < nb ? p.M : nb) * 128.0) / (shared_sm ? 59e3 : 100e3);
+            const double body = waves * load > hbm ? waves * load : hbm;
+            const double us = 4.1 + (w_bytes > 8e6 ? 2.0 : 0.0) + body + waves * nb * 0.012;
+            if (us < best.us) best = ClusterPlan{nb, s, us};
+        }
+    }
+    return best;
+}
+static double linear_single_us(const kb_linear_params& p) {
+    const int bn = plan_linear_bn(p.M, p.N, p.K, 0);
+    const int64_t tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + bn - 1) / bn);
+    const double waves = (double)((tiles + gemm_sms() - 1) / gemm_sms());
+    return 3.0 + waves * ((double)(kGemmBM + bn) * (double)p.K * 2.0 / 118e3 + 0.006 * bn);
+}
+// (The cluster kernel has to be clearly ahead: where the two are close, its estimate is the less certain one.)
+template <typename T>
+static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
+    if (forced_bn == 0 && forced_splits <= 1) {
+        if (forced_splits == 0 && stream_layout(p) && p.M <= 16) return launch_linear_stream_t<T>(p, stream);
+        if (linear_pair_applicable(p)) return launch_linear_pair_t<T>(p, stream);
+        if (forced_splits == 0 && p.M <= 1024 && gemm_sms() == sm_count()) {
+            const double single = linear_single_us(p);
+            const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
+            const ClusterPlan cl = linear_cluster_plan<T>(p);
+            if (stream_us < single && stream_us < cl.us) return launch_linear_stream_t<T>(p, stream);
+            if (cl.us < 0.94 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+        }
+    } else if (forced_splits > 1) {
+        const int num_k = (int)((p.K + kGemmBK - 1) / kGemmBK), most = num_k < kClMaxSplits ? num_k : kClMaxSplits;
+        const int nb = forced_bn == 32 || forced_bn == 64 ? forced_bn : p.M <= 64 ? 32 : 128;
+        return launch_linear_cluster_n<T>(p, stream, nb, forced_splits < most ? forced_splits : most);
+    }
+    return launch_linear_single<T>(p, stream, forced_bn);
+}
+
+static int launch_linear(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
+    if (p.dtype == KB_F16) return launch_linear_t<__half>(p, stream, forced_bn, forced_splits);
+    if (p.dtype == KB_BF16) return launch_linear_t<__nv_bfloat16>(p, stream, forced_bn, forced_splits);
+    return KB_ERR_UNSUPPORTED;
+}
+
+}  // namespace kb

@@ -1,4 +1,4 @@
-// Linear layer for few rows (M <= 32): y = act(x · Wᵀ + bias), the decode-step shape.
+// Linear layer for few rows: y = act(x · Wᵀ + bias), the decode-step shape, and small problems of some more.
 //
 // With a handful of rows the op is a single pass over W from HBM (2·N·K bytes; x is a few dozen KB and
 // lives in L2), so what matters is how many bytes every SM keeps in flight, without a break, and how
@@ -29,10 +29,11 @@ namespace kb {
 constexpr int kStreamThreads = 128;
 constexpr int kStreamWarps = kStreamThreads / 32;
 constexpr int kStreamK = 64;  // elements of K per piece: 128-byte rows in shared memory
-constexpr int kStreamMaxM = 32;
+constexpr int kStreamMaxM = 32;  // rows of x per CTA; more rows are further CTAs (grid.y) over the same W
 constexpr int kStreamSmemBytes = 112 * 1024;  // rings and partial tiles of a CTA: two CTAs per SM
 
-constexpr int stream_red_bytes(int rmax, int nx) { return kStreamWarps * nx * 8 * (rmax + 1) * 4; }
+constexpr int stream_red_nx(int nx) { return nx > 2 ? 2 : nx; }  // 8-row tiles of x whose partial sums meet at a time
+constexpr int stream_red_bytes(int rmax, int nx) { return kStreamWarps * stream_red_nx(nx) * 8 * (rmax + 1) * 4; }
 
 // RMAX: most rows of W per tile (a multiple of 8), NX: 8-row tiles of x.
 template <int RMAX, int NX>
@@ -40,6 +41,7 @@ struct StreamCfg {
     static constexpr int kTiles16 = (RMAX + 15) / 16;  // 16-row operand tiles; rows beyond the tile's hold anything
     static constexpr int kWBytes = RMAX * kStreamK * 2;
     static constexpr int kStageBytes = kWBytes + NX * 8 * kStreamK * 2;
+    static constexpr int kRedNx = stream_red_nx(NX);
     static constexpr int kRedRow = RMAX + 1;  // partial tile of a warp: [x row][W row], rows padded
     static constexpr int kFit = (kStreamSmemBytes - stream_red_bytes(RMAX, NX)) / (kStreamWarps * kStageBytes);
     static constexpr int kStages = kFit > 10 ? 10 : kFit;
@@ -55,8 +57,15 @@ linear_stream_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* 
                      T* __restrict__ act_inputs, int M, int lines, int K, int64_t x_row_stride, int64_t y_row_stride,
                      int activation, int tiles) {
     using Cfg = StreamCfg<RMAX, NX>;
-    constexpr int STAGES = Cfg::kStages, MT = Cfg::kTiles16;
+    constexpr int STAGES = Cfg::kStages, MT = Cfg::kTiles16, RNX = Cfg::kRedNx;
     extern __shared__ __align__(128) uint8_t stream_smem[];
+    {
+        const int m0 = (int)blockIdx.y * kStreamMaxM;
+        x += m0 * x_row_stride;
+        y += m0 * y_row_stride;
+        if (act_inputs != nullptr) act_inputs += m0 * y_row_stride;
+        M = min(M - m0, kStreamMaxM);
+    }
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int g = lane >> 2, c = lane & 3;
     const uint32_t ring = smem_u32(stream_smem) + (uint32_t)(warp * STAGES * Cfg::kStageBytes);
@@ -133,6 +142,18 @@ linear_stream_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* 
 
     int slot = 0;
     for (int tile = 0; tile < tiles; ++tile) {
+        const int l0 = tile_begin(tile), n_lines = tile_begin(tile + 1) - l0;
+        constexpr int LH = (RMAX + 31) / 32;
+        float bias_r[LH], bias_up[LH];
+#pragma unroll
+        for (int h = 0; h < LH; ++h) {
+            const int r = h * 32 + lane;
+            bias_r[h] = bias_up[h] = 0.f;
+            if (bias != nullptr && r < n_lines) {
+                bias_r[h] = Elem<T>::to_f32(__ldg(bias + w_row(l0, n_lines, r)));
+                if (gated) bias_up[h] = Elem<T>::to_f32(__ldg(bias + w_row(l0, n_lines, n_lines + r)));
+            }
+        }
         float acc[2][MT][NX][4];  // two chains: a product waits for the one before the last
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
@@ -174,55 +195,56 @@ linear_stream_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* 
                         mma_16816<T>(acc[ks & 1][mt][nx], wf[ks][mt][0], wf[ks][mt][1], wf[ks][mt][2], wf[ks][mt][3], xf[nx][ks * 2], xf[nx][ks * 2 + 1]);
         }
         // c0, c1 -> (W row g, x rows 2c, 2c + 1); c2, c3 -> (W row g + 8, same)
+        // The sums of the four warps, 16 rows of x at a time. A lane keeps to its lines of the tile and a warp to its
+        // rows of x: no division, and bias is in registers since the tile began.
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
+        for (int nx0 = 0; nx0 < NX; nx0 += RNX) {
+            if (nx0 * 8 >= M) break;
 #pragma unroll
-            for (int nx = 0; nx < NX; ++nx)
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const int r = mt * 16 + g + 8 * (e >> 1);
-                    if (r < RMAX) red[(warp * NX * 8 + nx * 8 + 2 * c + (e & 1)) * Cfg::kRedRow + r] = acc[0][mt][nx][e] + acc[1][mt][nx][e];
+                for (int nx = 0; nx < RNX; ++nx)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int r = mt * 16 + g + 8 * (e >> 1);
+                        if (r < RMAX)
+                            red[(warp * RNX * 8 + nx * 8 + 2 * c + (e & 1)) * Cfg::kRedRow + r] = acc[0][mt][nx0 + nx][e] + acc[1][mt][nx0 + nx][e];
+                    }
+            __syncthreads();
+            auto sum = [&](int m, int r) {
+                float z = 0.f;
+#pragma unroll
+                for (int wi = 0; wi < kStreamWarps; ++wi) z += red[(wi * RNX * 8 + m) * Cfg::kRedRow + r];
+                return z;
+            };
+            const int m_live = min(M - nx0 * 8, RNX * 8);
+#pragma unroll
+            for (int h = 0; h < LH; ++h) {
+                const int r = h * 32 + lane;
+                if (r >= n_lines) break;
+                for (int m = warp; m < m_live; m += kStreamWarps) {
+                    const int64_t out = (int64_t)(nx0 * 8 + m) * y_row_stride + l0 + r;
+                    float z = sum(m, r) + bias_r[h];
+                    if (gated) {
+                        y[out] = Elem<T>::from_f32(act_silu(z) * (sum(m, n_lines + r) + bias_up[h]));
+                        continue;
+                    }
+                    if (act_inputs != nullptr) act_inputs[out] = Elem<T>::from_f32(z);
+                    switch (activation) {
+                        case KB_ACT_TANH: z = act_tanh(z); break;
+                        case KB_ACT_GELU: z = act_gelu(z); break;
+                        case KB_ACT_FAST_GELU: z = act_fast_gelu(z); break;
+                        case KB_ACT_RELU: z = fmaxf(z, 0.f); break;
+                        case KB_ACT_SILU: z = act_silu(z); break;
+                        default: break;
+                    }
+                    y[out] = Elem<T>::from_f32(z);
                 }
-        __syncthreads();
-        const int l0 = tile_begin(tile), n_lines = tile_begin(tile + 1) - l0;
-        auto sum = [&](int m, int r) {
-            float z = 0.f;
-#pragma unroll
-            for (int wi = 0; wi < kStreamWarps; ++wi) z += red[(wi * NX * 8 + m) * Cfg::kRedRow + r];
-            return z;
-        };
-        for (int i = tid; i < M * n_lines; i += kStreamThreads) {
-            const int m = i / n_lines, r = i % n_lines;
-            const int64_t out = (int64_t)m * y_row_stride + l0 + r;
-            float z = sum(m, r);
-            if (bias != nullptr) z += Elem<T>::to_f32(bias[w_row(l0, n_lines, r)]);
-            if (gated) {
-                float up = sum(m, n_lines + r);
-                if (bias != nullptr) up += Elem<T>::to_f32(bias[w_row(l0, n_lines, n_lines + r)]);
-                y[out] = Elem<T>::from_f32(act_silu(z) * up);
-                continue;
             }
-            if (act_inputs != nullptr) act_inputs[out] = Elem<T>::from_f32(z);
-            switch (activation) {
-                case KB_ACT_TANH: z = act_tanh(z); break;
-                case KB_ACT_GELU: z = act_gelu(z); break;
-                case KB_ACT_FAST_GELU: z = act_fast_gelu(z); break;
-                case KB_ACT_RELU: z = fmaxf(z, 0.f); break;
-                case KB_ACT_SILU: z = act_silu(z); break;
-                default: break;
-            }
-            y[out] = Elem<T>::from_f32(z);
+            __syncthreads();  // the partial sums are rewritten by the next pass
         }
-        __syncthreads();  // the partial tiles are rewritten by the next round
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-}
-
-static bool smallm_applicable(const kb_linear_params& p) {
-    return p.M >= 1 && p.M <= kStreamMaxM && p.K % 8 == 0 && p.x_row_stride % 8 == 0 && (((uintptr_t)p.x) & 15) == 0 &&
-           (((uintptr_t)p.w) & 15) == 0 && p.N <= (int64_t)0x7fffffff / 2 && p.K <= 0x7fffffff &&
-           // above 16 rows x weighs twice as much as W on the way from L2; a large W goes to the tcgen05 kernel
-           (p.M <= 16 || p.N * p.K <= (int64_t)20 << 20);
 }
 
 template <typename T, int RMAX, int NX>
@@ -232,7 +254,7 @@ static int launch_linear_stream(const kb_linear_params& p, cudaStream_t stream, 
     if (attr_once.first_time() &&
         cudaFuncSetAttribute(linear_stream_kernel<T, RMAX, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
         return KB_ERR_LAUNCH;
-    launch_pdl(linear_stream_kernel<T, RMAX, NX>, (unsigned)ctas, kStreamThreads, Cfg::kSmemBytes, stream, (const T*)p.x, (const T*)p.w,
+    launch_pdl(linear_stream_kernel<T, RMAX, NX>, dim3((unsigned)ctas, (unsigned)((p.M + kStreamMaxM - 1) / kStreamMaxM)), kStreamThreads, Cfg::kSmemBytes, stream, (const T*)p.x, (const T*)p.w,
                (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)lines, (int)p.K, p.x_row_stride, p.y_row_stride, p.activation, tiles);
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
@@ -243,29 +265,31 @@ static int stream_rows_in_flight(int r) {
     if (r <= 8) return (StreamCfg<8, NX>::kStages - 1) * r;
     if (r <= 16) return (StreamCfg<16, NX>::kStages - 1) * r;
     if (r <= 24) return (StreamCfg<24, NX>::kStages - 1) * r;
+    if (r <= 32) return (StreamCfg<32, NX>::kStages - 1) * r;
     if constexpr (NX < 4) {
-        if (r <= 32) return (StreamCfg<32, NX>::kStages - 1) * r;
         if (r <= 40) return (StreamCfg<40, NX>::kStages - 1) * r;
         return (StreamCfg<48, NX>::kStages - 1) * r;
     }
     return 0;
 }
 
-template <typename T, int NX>
-static int launch_linear_stream_n(const kb_linear_params& p, cudaStream_t stream) {
-    const bool gated = p.activation == KB_ACT_SWIGLU;
-    const int per_line = gated ? 2 : 1;
-    const int64_t lines = p.N / per_line;
-    // two CTAs per SM; fewer where that would leave a CTA less than eight rows (a whole mma.sync operand half)
-    int64_t ctas = 2 * (int64_t)sm_count();
-    if (lines * per_line < ctas * 8) ctas = (lines * per_line + 7) / 8;
-    const int64_t share = (lines + ctas - 1) / ctas * per_line;  // most rows of a CTA
-    // Tiles per CTA: the fewer the better (a tile costs a cross-warp sum, about as long as four pieces of a
-    // warp), as long as the tile's rows keep the ring full: below about 112 rows in flight per CTA the
-    // copies are bound by latency.
-    int best_tiles = 1, best_rows = 0;
+struct StreamPlan {
+    int64_t ctas;  // per 32 rows of x
+    int tiles, rows;
+    double us;     // above 16 rows: estimated time
+};
+
+// Up to 16 rows: W is what counts. Two CTAs per SM, fewer where that would leave a CTA less than eight rows
+// (a whole mma.sync operand half); tiles per CTA: the fewer the better (a tile costs a cross-warp sum, about as
+// long as four pieces of a warp), as long as the tile's rows keep the ring full: below about 112 rows in
+// flight per CTA the copies are bound by latency.
+template <int NX>
+static StreamPlan stream_plan_w(const kb_linear_params& p, int64_t lines, int per_line) {
+    StreamPlan best{2 * (int64_t)sm_count(), 1, 0, 0.0};
+    if (lines * per_line < best.ctas * 8) best.ctas = (lines * per_line + 7) / 8;
+    const int64_t share = (lines + best.ctas - 1) / best.ctas * per_line;  // most rows of a CTA
     double best_cost = 1e300;
-    const int max_rows = NX == 4 ? 24 : 48;
+    const int max_rows = 48;
     for (int64_t t = (share + max_rows - 1) / max_rows; t <= share && t <= (share + 7) / 8 + 1; ++t) {
         const int rows = (int)((share / per_line + t - 1) / t) * per_line;
         if (rows > max_rows) continue;
@@ -273,31 +297,57 @@ static int launch_linear_stream_n(const kb_linear_params& p, cudaStream_t stream
         const double cost = (double)share * p.K / (fill < 1.0 ? fill : 1.0) + (double)t * 16 * kStreamK * rows;
         if (cost < best_cost) {
             best_cost = cost;
-            best_tiles = (int)t;
-            best_rows = rows;
+            best.tiles = (int)t;
+            best.rows = rows;
         }
     }
-    if (best_rows <= 8) return launch_linear_stream<T, 8, NX>(p, stream, lines, ctas, best_tiles);
-    if (best_rows <= 16) return launch_linear_stream<T, 16, NX>(p, stream, lines, ctas, best_tiles);
-    if constexpr (NX < 4) {
-        if (best_rows > 40) return launch_linear_stream<T, 48, NX>(p, stream, lines, ctas, best_tiles);
-        if (best_rows > 32) return launch_linear_stream<T, 40, NX>(p, stream, lines, ctas, best_tiles);
-        if (best_rows > 24) return launch_linear_stream<T, 32, NX>(p, stream, lines, ctas, best_tiles);
+    return best;
+}
+
+// Above 16 rows: CTAs of 32 rows of x and `rows` of W, one tile each. A CTA pulls its rows through half an SM's
+// port to L2 (59 bytes per ns) and multiplies them at half an SM's mma.sync rate (0.49 products per ps); the
+// rest is fitted to times over 20 to 384 rows and W from 500 x 1000 to 4096 x 4096.
+static StreamPlan stream_plan_x(const kb_linear_params& p) {
+    const int per_line = p.activation == KB_ACT_SWIGLU ? 2 : 1;
+    const int64_t slots = 2 * (int64_t)sm_count(), groups = (p.M + kStreamMaxM - 1) / kStreamMaxM;
+    StreamPlan best{1, 1, 0, 1e300};
+    for (int rows = 8 * per_line; rows <= 32; rows += 8 * per_line) {
+        const int64_t ctas = (p.N + rows - 1) / rows;
+        const double load = (double)p.K * 2.0 * (rows + kStreamMaxM) / 59e3;
+        const double math = (double)((rows + 15) / 16 * 16) * kStreamMaxM * (double)p.K / 486e3;
+        const double us = 2.4 + 1.2 * (double)((ctas * groups + slots - 1) / slots) * (load + 0.5 * math + 0.3);
+        if (us < best.us) best = StreamPlan{ctas, 1, rows, us};
     }
-    return launch_linear_stream<T, 24, NX>(p, stream, lines, ctas, best_tiles);
+    const double hbm = (double)p.N * (double)p.K * 2.0 / 5.0e6;  // (with x in every ring, W does not come faster)
+    if (best.us < 2.4 + hbm) best.us = 2.4 + hbm;
+    return best;
+}
+
+static bool stream_layout(const kb_linear_params& p) {
+    return p.M >= 1 && p.K % 8 == 0 && p.x_row_stride % 8 == 0 && (((uintptr_t)p.x) & 15) == 0 && (((uintptr_t)p.w) & 15) == 0 &&
+           p.N <= (int64_t)0x7fffffff / 2 && p.K <= 0x7fffffff;
+}
+
+template <typename T, int NX>
+static int launch_linear_stream_n(const kb_linear_params& p, cudaStream_t stream) {
+    const int per_line = p.activation == KB_ACT_SWIGLU ? 2 : 1;
+    const int64_t lines = p.N / per_line;
+    const StreamPlan plan = NX == 4 ? stream_plan_x(p) : stream_plan_w<NX>(p, lines, per_line);
+    if (plan.rows <= 8) return launch_linear_stream<T, 8, NX>(p, stream, lines, plan.ctas, plan.tiles);
+    if (plan.rows <= 16) return launch_linear_stream<T, 16, NX>(p, stream, lines, plan.ctas, plan.tiles);
+    if (plan.rows <= 24) return launch_linear_stream<T, 24, NX>(p, stream, lines, plan.ctas, plan.tiles);
+    if constexpr (NX < 4) {
+        if (plan.rows > 40) return launch_linear_stream<T, 48, NX>(p, stream, lines, plan.ctas, plan.tiles);
+        if (plan.rows > 32) return launch_linear_stream<T, 40, NX>(p, stream, lines, plan.ctas, plan.tiles);
+    }
+    return launch_linear_stream<T, 32, NX>(p, stream, lines, plan.ctas, plan.tiles);
 }
 
 template <typename T>
-static int launch_linear_smallm_t(const kb_linear_params& p, cudaStream_t stream) {
+static int launch_linear_stream_t(const kb_linear_params& p, cudaStream_t stream) {
     if (p.M <= 8) return launch_linear_stream_n<T, 1>(p, stream);
     if (p.M <= 16) return launch_linear_stream_n<T, 2>(p, stream);
     return launch_linear_stream_n<T, 4>(p, stream);
-}
-
-static int launch_linear_smallm(const kb_linear_params& p, cudaStream_t stream) {
-    if (p.dtype == KB_F16) return launch_linear_smallm_t<__half>(p, stream);
-    if (p.dtype == KB_BF16) return launch_linear_smallm_t<__nv_bfloat16>(p, stream);
-    return KB_ERR_UNSUPPORTED;
 }
 
 }  // namespace kb

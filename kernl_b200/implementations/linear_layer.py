@@ -7,35 +7,7 @@ from kernl_b200 import _lib
 from kernl_b200.implementations._autocast import cast_if_autocast
 
 
-_WORKSPACE_BYTES = 32 * 1024 * 1024
-_workspaces = {}
 _padded_weights = {}
-
-
-def _workspace(device: torch.device) -> torch.Tensor:
-    """A zero-initialised scratch buffer for split-K partial sums per (device, stream), allocated on
-    first use and kept (a stable address, so CUDA graphs that captured it stay valid). The kernel
-    leaves it zero after every call. Calls on different streams get different buffers, so they may
-    overlap on the GPU; a graph replayed on a stream other than the one it was captured on keeps
-    using the capture stream's buffer."""
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    key = (index, torch.cuda.current_stream(device).cuda_stream)
-    ws = _workspaces.get(key)
-    if ws is None:
-        with torch.inference_mode(False):  # an ordinary tensor: it is zeroed in place again after an expired wait
-            ws = torch.zeros(_WORKSPACE_BYTES // 4, dtype=torch.float32, device=device)
-        _workspaces[key] = ws
-        _lib.native().register_workspace(*key, ws.data_ptr(), ws.numel() * 4)
-    return ws
-
-
-def _rezero_workspaces() -> None:
-    """A GEMM whose wait expired may have left partial sums behind; split-K needs zeros."""
-    for ws in _workspaces.values():
-        ws.zero_()
-
-
-_lib.on_wait_expired(_rezero_workspaces)
 
 
 def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -120,14 +92,11 @@ def linear_layer(
     if act_inputs is not None:
         assert act_inputs.shape == (M, N) and act_inputs.dtype == x.dtype and act_inputs.is_contiguous()
     if M > 0:
-        ws = _workspace(x.device) if _lib.load().kb_linear_workspace_bytes(M, N) <= _WORKSPACE_BYTES else None
         p = _lib.LinearParams(
             x=x_.data_ptr(), w=weight.data_ptr(), bias=bias.data_ptr() if bias is not None else None,
             y=outputs.data_ptr(), act_inputs=act_inputs.data_ptr() if act_inputs is not None else None,
             M=M, N=N, K=K, x_row_stride=x_.stride(0), y_row_stride=outputs.stride(0),
             activation=_lib.ACTIVATIONS[activation], dtype=_lib.dtype_code(x.dtype),
-            workspace=ws.data_ptr() if ws is not None else None,
-            workspace_bytes=ws.numel() * 4 if ws is not None else 0,
         )
         with torch.cuda.device(x.device):
             _lib.check(_lib.load().kb_linear_fwd(p, _lib.current_stream(x.device)), "linear_layer")

@@ -19,7 +19,6 @@ def test_linear_direct_or_general(lib, rows, k, shift, direct):
 
     x = _rand((rows * k + shift,))[shift:].view(rows, k)  # `shift` elements off a 16-byte boundary
     w, b = _rand((48, k), 0.1), _rand((48,))
-    linear_layer(x, w, b)  # registers the stream's workspace
     y = _lib.native().linear(x, w, b, _lib.ACTIVATIONS["relu"], None, None)
     assert (y is not None) == direct
     O.assert_parity(linear_layer(x, w, b, "relu"), O.linear(x.cpu(), w.cpu(), b.cpu(), "relu"), what="linear")
