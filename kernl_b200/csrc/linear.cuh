@@ -281,10 +281,14 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    // Launched with programmatic dependent launch: the barriers and the descriptor prefetch touch no
-    // global memory and may run while the previous kernel of the stream drains (a few-row GEMM of a
-    // latency-bound graph is itself only a few microseconds long).
+    // Launched with programmatic dependent launch: barriers, tensor memory and descriptors are set up, and the
+    // first tile's W is asked for in L2 (not read: it may be the output of the kernel ahead), while the
+    // previous kernel of the stream drains; a GEMM of a latency-bound graph is itself only a few microseconds long.
+    // A wait that expired in an earlier CTA or launch leaves the status word set: do no work until
+    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA.
+    __shared__ int s_skip;
     if (threadIdx.x == 0) {
+        s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
@@ -299,15 +303,9 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmap_x);
         tma_prefetch_desc(&tmap_w);
-    }
-    pdl_wait();
-    // A wait that expired in an earlier CTA or launch leaves the status word set: do no work until
-    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA.
-    {
-        __shared__ int s_skip;
-        if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
-        __syncthreads();
-        if (s_skip != 0) return;
+        int m_idx, n_idx;
+        tile_coords((int)blockIdx.x, (M + kGemmBM - 1) / kGemmBM, (N + BN - 1) / BN, m_idx, n_idx);
+        for (int kb = 0; kb < min(2 * STAGES, (K + kGemmBK - 1) / kGemmBK); ++kb) tma_prefetch_l2_2d(&tmap_w, kb * kGemmBK, n_idx * BN);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), Cfg::kTmemCols);
@@ -317,12 +315,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_wait();
+    const bool skip = s_skip != 0;
 
     const int num_m = (M + kGemmBM - 1) / kGemmBM;
     const int num_n = (N + BN - 1) / BN;
     const int num_tiles = num_m * num_n;
     const int num_k = (K + kGemmBK - 1) / kGemmBK;
-    if (warp == 0) {
+    if (skip) {
+        // (falls through to the teardown)
+    } else if (warp == 0) {
         if (elect_one()) {
             int stage = 0;
             uint32_t phase = 0;

@@ -35,9 +35,6 @@ struct ClCfg {  // NB: rows of x per tile
     static_assert(2 * (kSmemBytes + 1024) <= 227 * 1024, "two CTAs per SM");
 };
 
-__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* map, int x, int y) {
-    asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y) : "memory");
-}
 __device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t own_addr, uint32_t rank) {
     uint32_t a;
     float4 v;
