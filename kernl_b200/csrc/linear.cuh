@@ -485,11 +485,6 @@ static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream) {
     return KB_OK;
 }
 
-// Large problems go to CTA pairs on 256 x 256 tiles (linear_pair.cuh).
-static bool linear_pair_applicable(const kb_linear_params& p);
-template <typename T>
-static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream);
-
 template <typename T>
 static int launch_linear_single(const kb_linear_params& p, cudaStream_t stream, int forced_bn) {
     switch (plan_linear_bn(p.M, p.N, p.K, forced_bn)) {

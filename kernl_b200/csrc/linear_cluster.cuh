@@ -280,9 +280,9 @@ static int launch_linear_cluster_n(const kb_linear_params& p, cudaStream_t strea
 }
 
 
-// ---- which kernel a problem of 17 to 1024 rows goes to
+// ---- which kernel a problem goes to
 //
-// Estimates in us, fitted to times of the three kernels (graphs of calls with cold W) over 20 to 1000 rows and W
+// Estimates in us, fitted to times of the kernels (graphs of calls with cold W) over 20 to 3000 rows and W
 // from 500 x 1000 to 12288 x 4096; off by up to a fifth, mostly by less than a tenth. An SM pulls about 118 bytes
 // per ns through its port to L2, shared by its CTAs; W comes from HBM at 6.5 bytes per ps at best.
 struct ClusterPlan {
@@ -314,27 +314,37 @@ static double linear_single_us(const kb_linear_params& p) {
     const int bn = plan_linear_bn(p.M, p.N, p.K, 0);
     const int64_t tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + bn - 1) / bn);
     const double waves = (double)((tiles + gemm_sms() - 1) / gemm_sms());
-    return 3.0 + waves * ((double)(kGemmBM + bn) * (double)p.K * 2.0 / 118e3 + 0.006 * bn);
+    // 0.012: the epilogue of a column; a tile of which most rows lie outside x arrives later (zero fill): 5.5 us at
+    // 128 rows of [3072, 768], 6.9 at 33
+    return 2.8 + (p.M < 96 ? 1.3 : 0.0) + waves * ((double)(kGemmBM + bn) * (double)p.K * 2.0 / 118e3 + 0.012 * bn);
 }
-// (The cluster kernel has to be clearly ahead: where the two are close, its estimate is the less certain one.)
 template <typename T>
 static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
-    if (forced_bn == 0 && forced_splits <= 1) {
-        if (forced_splits == 0 && stream_layout(p) && p.M <= 16) return launch_linear_stream_t<T>(p, stream);
-        if (linear_pair_applicable(p)) return launch_linear_pair_t<T>(p, stream);
-        if (forced_splits == 0 && p.M <= 1024 && gemm_sms() == sm_count()) {
-            const double single = linear_single_us(p);
-            const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
-            const ClusterPlan cl = linear_cluster_plan<T>(p);
-            if (stream_us < single && stream_us < cl.us) return launch_linear_stream_t<T>(p, stream);
-            if (cl.us < 0.94 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
-        }
-    } else if (forced_splits > 1) {
+    if (forced_splits > 1) {
         const int num_k = (int)((p.K + kGemmBK - 1) / kGemmBK), most = num_k < kClMaxSplits ? num_k : kClMaxSplits;
         const int nb = forced_bn == 32 || forced_bn == 64 ? forced_bn : p.M <= 64 ? 32 : 128;
         return launch_linear_cluster_n<T>(p, stream, nb, forced_splits < most ? forced_splits : most);
     }
-    return launch_linear_single<T>(p, stream, forced_bn);
+    if (forced_bn != 0) return launch_linear_single<T>(p, stream, forced_bn);
+    if (stream_layout(p) && p.M <= 16) return launch_linear_stream_t<T>(p, stream);
+    const double single = linear_single_us(p);
+    if (p.M > 128 && p.N >= 128 && p.K >= 256 && g_linear_pair != 0) {
+        double pair;
+        const int bn = linear_pair_tile_width(p, &pair);
+        // (at thousands of rows the estimates no longer matter: the pair kernel pulls half as much W through each SM's port)
+        if (g_linear_pair != 1 || pair < 0.93 * single || (p.M > 4096 && p.N >= 256)) {
+            const ClusterPlan cl = p.M <= 1024 && g_linear_pair == 1 && gemm_sms() == sm_count() ? linear_cluster_plan<T>(p) : ClusterPlan{0, 0, 1e300};
+            if (pair <= cl.us) return launch_linear_pair_t<T>(p, stream, bn);
+        }
+    }
+    if (p.M <= 1024 && gemm_sms() == sm_count()) {
+        const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
+        const ClusterPlan cl = linear_cluster_plan<T>(p);
+        if (stream_us < single && stream_us < cl.us) return launch_linear_stream_t<T>(p, stream);
+        // (the cluster kernel has to be clearly ahead: where the two are close, its estimate is the less certain one)
+        if (cl.us < 0.94 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+    }
+    return launch_linear_single<T>(p, stream, 0);
 }
 
 static int launch_linear(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {

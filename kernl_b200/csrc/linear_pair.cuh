@@ -425,26 +425,27 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
 static int g_linear_pair = 1;  // test hook (kb_debug_linear_pair): 0 = never use the pair kernel, 192 / 256 = force that tile width
 
-// The pair kernel serves problems with at least one 256 x 256 tile per pair of SMs and no split-K.
-static bool linear_pair_applicable(const kb_linear_params& p) {
-    if (g_linear_pair == 0) return false;
-    const int64_t tiles = ((p.M + 255) / 256) * ((p.N + kPairBN - 1) / kPairBN);
-    return p.M >= 512 && p.N >= 256 && p.K >= 256 && tiles >= gemm_sms() / 2;
+// Estimated time in us of the pair kernel with tiles of 256 x `bn`: a fixed part, and rounds of tiles on the pairs of
+// (k-blocks x time of one + the part of an epilogue that the next tile does not hide). A k-block of 64 costs
+// 0.24 us (192 columns) or 0.285 us (256) while few pairs are busy, up to a quarter more when all of them pull
+// on L2. Fitted to 128 to 3000 rows, K from 768 to 11008; mostly within 8 %.
+static double linear_pair_us(const kb_linear_params& p, int bn) {
+    const int64_t pairs = gemm_sms() / 2 > 0 ? gemm_sms() / 2 : 1;
+    const int64_t tiles = ((p.M + 255) / 256) * ((p.N + bn - 1) / bn), rounds = (tiles + pairs - 1) / pairs;
+    const double busy = (double)tiles / (double)(rounds * pairs), num_k = (double)((p.K + kGemmBK - 1) / kGemmBK);
+    const double block = bn == 192 ? 0.24 + 0.05 * busy * busy : 0.285 + 0.09 * busy * busy;
+    return (bn == 192 ? 4.1 : 5.4) + (double)rounds * (num_k * block + 0.7);
 }
 
-// Tile width: rounds of tiles on the pairs x (columns of a tile + a fixed cost per tile, in columns).
-// 192 columns only where that is clearly cheaper (a launch of a few rounds whose last one is nearly
-// empty) and the epilogue can take its staged path (whole 16-byte pieces, no gated or pre-activation output).
-static int linear_pair_tile_width(const kb_linear_params& p, int pairs) {
-    if (g_linear_pair == 192 || g_linear_pair == 256) return g_linear_pair;
+// Tile width (192 or 256 columns), and the estimate that goes with it. 192 columns want the staged epilogue (whole
+// 16-byte pieces, no gated or pre-activation output); among close estimates the wide tile, which pulls less.
+static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
     const bool staged = p.activation != KB_ACT_SWIGLU && p.act_inputs == nullptr && (p.N & 7) == 0 && (p.y_row_stride & 7) == 0 &&
                         (((uintptr_t)p.y) & 15) == 0;
-    if (!staged) return 256;
-    auto cost = [&](int bn) {
-        const int64_t tiles = ((p.M + 255) / 256) * ((p.N + bn - 1) / bn);
-        return (double)((tiles + pairs - 1) / pairs) * (bn + 24);
-    };
-    return cost(192) < 0.95 * cost(256) ? 192 : 256;
+    const double wide = linear_pair_us(p, 256), narrow = linear_pair_us(p, 192);
+    const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : staged && narrow < 0.97 * wide ? 192 : 256;
+    *us = bn == 192 ? narrow : wide;
+    return bn;
 }
 
 template <typename T, int BN>
@@ -506,10 +507,8 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
 }
 
 template <typename T>
-static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream) {
-    const int pairs = gemm_sms() / 2;
-    if (linear_pair_tile_width(p, pairs > 0 ? pairs : 1) == 192) return launch_linear_pair_tb<T, 192>(p, stream);
-    return launch_linear_pair_tb<T, 256>(p, stream);
+static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream, int bn) {
+    return bn == 192 ? launch_linear_pair_tb<T, 192>(p, stream) : launch_linear_pair_tb<T, 256>(p, stream);
 }
 
 }  // namespace kb
