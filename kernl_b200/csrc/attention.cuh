@@ -114,15 +114,9 @@ static int attn_head_group(int64_t BH, int64_t N, int64_t D) {
 
 template <int D>
 struct AttnCfg {
-    static constexpr int kKvStages = D == 64 ? 3 : 2;
+    static constexpr int kKvStages = 2;
     static constexpr int kTileBytes = kAttnBlock * D * 2;  // one Q tile / one K block / one V block
-    // D = 64 only: the row sums of P come out of the tensor core. V gets 16 extra columns of ones
-    // (one 128-byte-swizzled slab of ones in shared memory, shared by every stage), so O has D+16
-    // columns and column D accumulates sum_k P[r,k] of exactly the 16-bit P that multiplies V.
-    static constexpr bool kSumOnTc = (D == 64);
-    static constexpr int kOnesBytes = kSumOnTc ? kAttnBlock * 128 : 0;
-    static constexpr int kOCols = kSumOnTc ? D + 16 : D;
-    static constexpr int kSmemBytes = (2 + 2 * kKvStages) * kTileBytes + kOnesBytes + 512 + 2048 + 1024;
+    static constexpr int kSmemBytes = (2 + 2 * kKvStages) * kTileBytes + 512 + 2048 + 1024;
 };
 
 __device__ __forceinline__ float mask_lowest(int mask_dtype) {
@@ -221,14 +215,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t q_smem = smem_u32(smem);
     const uint32_t k_smem = q_smem + 2 * TILE;
     const uint32_t v_smem = k_smem + KVS * TILE;
-    constexpr bool kSumOnTc = Cfg::kSumOnTc;
-    // With fp16 inputs the exponentials themselves are taken two at a time in half precision
-    // (ex2.approx.f16x2): the argument s - m_ref is at most 2^3 (lazy rescaling), where fp16 still
-    // resolves 2^-8, and P is rounded to fp16 for the tensor core anyway. bf16 keeps fp32 exponentials.
-    constexpr bool kHalfExp = kSumOnTc && !Elem<T>::kIsBf16;
-    constexpr int OCOLS = Cfg::kOCols;
-    const uint32_t ones_smem = v_smem + KVS * TILE;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (2 + 2 * KVS) * TILE + Cfg::kOnesBytes);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (2 + 2 * KVS) * TILE);
     const uint32_t bar_base = smem_u32(bars);
     // barrier slots
     auto q_full = [&](int t) { return bar_base + 8u * t; };
@@ -237,14 +224,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     auto v_full = [&](int s) { return bar_base + 8u * (2 + 2 * KVS + s); };
     auto v_empty = [&](int s) { return bar_base + 8u * (2 + 3 * KVS + s); };
     auto s_full = [&](int t) { return bar_base + 8u * (2 + 4 * KVS + t); };
-    auto p_full = [&](int t) { return bar_base + 8u * (4 + 4 * KVS + t); };
+    auto p_full = [&](int t, int half) { return bar_base + 8u * (16 + 4 * KVS + t * 2 + half); };  // keys [0, 64) / [64, 128) of P
     auto o_final = [&](int t) { return bar_base + 8u * (6 + 4 * KVS + t); };
     auto m_full = [&](int t, int bf) { return bar_base + 8u * (8 + 4 * KVS + t * 2 + bf); };
     auto m_empty = [&](int t, int bf) { return bar_base + 8u * (12 + 4 * KVS + t * 2 + bf); };
-    constexpr int kNumBars = 16 + 4 * KVS;
+    constexpr int kNumBars = 20 + 4 * KVS;
+    static_assert(kNumBars * 8 + 16 <= 512, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + Cfg::kOnesBytes + 512);  // [tile][buffer][128]
+    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // [tile][buffer][128]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -281,7 +269,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         for (int t = 0; t < 2; ++t) {
             mbar_init(q_full(t), 1);
             mbar_init(s_full(t), 1);
-            mbar_init(p_full(t), 4);
+            mbar_init(p_full(t, 0), 4);
+            mbar_init(p_full(t, 1), 4);
             mbar_init(o_final(t), 1);
             for (int bf = 0; bf < 2; ++bf) {
                 mbar_init(m_full(t, bf), 2);   // the two loader warps
@@ -297,12 +286,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         *abort_flag = 0;
         fence_mbar_init();
     }
-    if (kSumOnTc) {
-        const uint32_t one2 = Elem<T>::pack2(1.0f, 1.0f);
-        uint32_t* ones = reinterpret_cast<uint32_t*>(smem + (2 + 2 * KVS) * TILE);
-        for (int i = threadIdx.x; i < Cfg::kOnesBytes / 4; i += kAttnThreads) ones[i] = one2;
-        fence_proxy_async_smem();  // the tensor core reads shared memory through the async proxy
-    }
     if (warp == 9) {
         tmem_alloc(smem_u32(tmem_slot), kTmemCols);
         tmem_relinquish();
@@ -316,6 +299,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    // Launched with programmatic dependent launch: nothing of global memory but the status word is touched above
+    pdl_wait();
 
     if (warp >= 8) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kAttnRegsLow));
@@ -351,16 +336,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
             constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kIsBf16, 128, 128, 0, 0);
-            constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, OCOLS, 0, 1);
+            constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, D, 0, 1);
             bool ok = true;
             // Descriptor halves that never change: high word = stride offset 1024 B, version 1, 128-byte
             // swizzle; low word = address >> 4 (+ the leading offset for the N-major V operand).
             constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
             const uint32_t q_lo = (q_smem & 0x3FFFF) >> 4;
             const uint32_t k_lo = (k_smem & 0x3FFFF) >> 4;
-            // leading offset of the V operand = distance to the next 64-column slab along N: the second
-            // slab of D (D = 128) or the slab of ones (D = 64, added per stage below)
-            const uint32_t v_lo = ((v_smem & 0x3FFFF) >> 4) | (kSumOnTc ? 0u : ((uint32_t)(CHUNK >> 4) << 16));
+            // leading offset of the V operand = distance to the next 64-column slab along N
+            const uint32_t v_lo = ((v_smem & 0x3FFFF) >> 4) | ((uint32_t)(CHUNK >> 4) << 16);
             auto desc = [&](uint32_t lo) { return ((uint64_t)desc_hi << 32) | (uint64_t)lo; };
             auto issue_qk = [&](int t, int s) {
                 const uint32_t a_lo = q_lo + (uint32_t)(t * (TILE >> 4));
@@ -372,13 +356,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     tc_mma_ss(d_tmem, desc(a_lo + off), desc(b_lo + off), idesc_qk, ks > 0 ? 1u : 0u);
                 }
             };
-            auto issue_pv = [&](int t, int s, bool accumulate) {
-                uint32_t b_lo = v_lo + (uint32_t)(s * (TILE >> 4));
-                if (kSumOnTc) b_lo |= (uint32_t)((ones_smem - (v_smem + s * TILE)) >> 4) << 16;
+            auto issue_pv = [&](int t, int s, int half, bool accumulate) {
+                const uint32_t b_lo = v_lo + (uint32_t)(s * (TILE >> 4));
                 const uint32_t d_tmem = tmem_base + (uint32_t)(256 + t * 128);
                 const uint32_t a_tmem = tmem_base + (uint32_t)(t * 128);
 #pragma unroll
-                for (int ks = 0; ks < kAttnBlock / 16; ++ks) {
+                for (int k4 = 0; k4 < kAttnBlock / 32; ++k4) {
+                    const int ks = half * (kAttnBlock / 32) + k4;
                     // 16 keys = 16 rows of 128 bytes = 2048 B; the second 64-wide slab of D is CHUNK bytes away
                     tc_mma_ts(d_tmem, a_tmem + (uint32_t)(ks * 8), desc(b_lo + (uint32_t)(ks * (2048 >> 4))), idesc_pv,
                               (accumulate || ks > 0) ? 1u : 0u);
@@ -410,9 +394,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 }
                 for (int t = 0; t < ntl; ++t) {
                     if (j >= nblk[t]) continue;
-                    if (!mbar_wait(p_full(t), (uint32_t)(j & 1), abort_flag, 204)) { ok = false; break; }
+                    // P in halves: the first product runs while the second half's exponentials are taken
+                    if (!mbar_wait(p_full(t, 0), (uint32_t)(j & 1), abort_flag, 204)) { ok = false; break; }
                     tc_fence_after();
-                    issue_pv(t, s, j > 0);
+                    issue_pv(t, s, 0, j > 0);
+                    if (!mbar_wait(p_full(t, 1), (uint32_t)(j & 1), abort_flag, 205)) { ok = false; break; }
+                    tc_fence_after();
+                    issue_pv(t, s, 1, true);
                     if (j + 1 < nblk[t]) {
                         issue_qk(t, s1);
                         tc_commit(s_full(t));
@@ -555,7 +543,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 if (j > 0 && __any_sync(0xffffffffu, grow)) {
                     // S_j complete implies P·V of block j-1 complete (issued earlier, same thread), so O is quiescent.
 #pragma unroll
-                    for (int dch = 0; dch < OCOLS / 16; ++dch) {
+                    for (int dch = 0; dch < D / 16; ++dch) {
                         uint32_t orr[16];
                         tmem_ld_32x16(o_addr + dch * 16, orr);
                         tmem_ld_wait();
@@ -567,41 +555,33 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 // ---- exponentials, row sum (four independent partial sums), pack to 16 bit, write P over
                 //      the first 64 columns of S
                 const float neg_ref = -m_ref * unit;
-                float lp[4] = {0.f, 0.f, 0.f, 0.f};
+                const float2 unit2 = make_float2(unit, unit), neg2 = make_float2(neg_ref, neg_ref);
+                float2 lp[2] = {{0.f, 0.f}, {0.f, 0.f}};
 #pragma unroll
                 for (int cch = 0; cch < 4; ++cch) {
                     uint32_t pk[16];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
-                        const float a0 = fmaf(__uint_as_float(sr[cch][2 * i]), unit, neg_ref);
-                        const float a1 = fmaf(__uint_as_float(sr[cch][2 * i + 1]), unit, neg_ref);
-                        if (kHalfExp) {
-                            const uint32_t h2 = Elem<T>::pack2(a0, a1);
-                            asm("ex2.approx.f16x2 %0, %1;" : "=r"(pk[i]) : "r"(h2));
-                        } else {
-                            const float e0 = fast_exp2(a0);
-                            const float e1 = fast_exp2(a1);
-                            if (!kSumOnTc) lp[i & 3] += e0 + e1;
-                            pk[i] = Elem<T>::pack2(e0, e1);
-                        }
+                        const float2 a = __ffma2_rn(make_float2(__uint_as_float(sr[cch][2 * i]), __uint_as_float(sr[cch][2 * i + 1])), unit2, neg2);
+                        // (a quarter to a half of them on the FMA pipe instead was no faster: the unit is half idle)
+                        const float2 e = make_float2(fast_exp2(a.x), fast_exp2(a.y));
+                        lp[i & 1] = __fadd2_rn(lp[i & 1], e);
+                        pk[i] = Elem<T>::pack2(e.x, e.y);
                     }
                     tmem_st_32x16(s_addr + cch * 16, pk);
+                    if (cch & 1) {
+                        tmem_st_wait();
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(p_full(t, cch >> 1));
+                    }
                 }
-                if (!kSumOnTc) l += (lp[0] + lp[1]) + (lp[2] + lp[3]);
-                tmem_st_wait();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_full(t));
+                l += (lp[0].x + lp[0].y) + (lp[1].x + lp[1].y);
             }
+            pdl_launch_dependents();  // the key loop is over: a dependent launch may take the slots that free up
             // ---- epilogue: O / l -> global
             if (ok && mbar_wait(o_final(t), 0, abort_flag, 310 + t)) {
                 tc_fence_after();
-                if (kSumOnTc) {
-                    uint32_t lr[16];
-                    tmem_ld_32x16(o_addr + D, lr);
-                    tmem_ld_wait();
-                    l = __uint_as_float(lr[0]);
-                }
                 const float inv_l = 1.0f / l;
                 T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                            (int64_t)row * p.o_strides[2];
@@ -687,7 +667,8 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     }
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
-    attention_tc_kernel<T, D, MODE><<<(unsigned)grid, kAttnThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, d);
+    if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads, Cfg::kSmemBytes, stream, tq, tk, tv, d) != cudaSuccess)
+        return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
 
