@@ -116,7 +116,10 @@ template <int D>
 struct AttnCfg {
     static constexpr int kKvStages = 2;
     static constexpr int kTileBytes = kAttnBlock * D * 2;  // one Q tile / one K block / one V block
-    static constexpr int kSmemBytes = (2 + 2 * kKvStages) * kTileBytes + 512 + 2048 + 1024;
+    static constexpr int kSmemBase = (2 + 2 * kKvStages) * kTileBytes + 512 + 1024;
+    static constexpr int kMaskMaxN = 7168;  // MODE 1: the longest mask row that fits behind the tiles
+    static constexpr int kSmemMax = kSmemBase + kMaskMaxN * 4;
+    static_assert(kSmemMax <= 227 * 1024 - 256, "shared memory of one CTA");
 };
 
 __device__ __forceinline__ float mask_lowest(int mask_dtype) {
@@ -195,10 +198,41 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// Key blocks of a MODE 1 launch whose mask is "minus infinity" for every key (the padding behind a
+// sequence) contribute exp(-65504 + ...) = 0 to every row and are skipped: not loaded, not multiplied,
+// not exponentiated. A block is skipped only if all of its mask values are below kSkipBelow (in the
+// log2 domain), far beyond where fp32 exp underflows for any score difference up to 2^14; if the
+// whole row is like that (a fully padded sequence, where the mask cancels and the reference
+// returns a plain softmax) nothing is skipped. At most 128 blocks (N <= 8192): a 128-bit set.
+constexpr float kSkipBelow = -30000.0f * 1.4426950408889634f;
+__device__ __forceinline__ int bits_next(const uint32_t (&w)[4], int from) {  // smallest set bit >= from
+    int r = 1 << 20;
+#pragma unroll
+    for (int wi = 3; wi >= 0; --wi) {
+        uint32_t m = w[wi];
+        const int lo = from - wi * 32;
+        if (lo >= 32) m = 0u;
+        else if (lo > 0) m &= 0xffffffffu << lo;
+        if (m != 0u) r = wi * 32 + __ffs((int)m) - 1;
+    }
+    return r;
+}
+__device__ __forceinline__ int bits_count_below(const uint32_t (&w)[4], int limit) {  // set bits with index < limit
+    int n = 0;
+#pragma unroll
+    for (int wi = 0; wi < 4; ++wi) {
+        const int hi = limit - wi * 32;
+        uint32_t m = w[wi];
+        if (hi <= 0) m = 0u;
+        else if (hi < 32) m &= (1u << hi) - 1u;
+        n += __popc(m);
+    }
+    return n;
+}
 // MODE 0: no mask and positive scale (maximum taken on raw scores, one FFMA + EX2 per element);
-// MODE 1: additive mask that is the same for every query row (padding masks): warps 10-11 stage
-//         it per key block in shared memory, already clamped, scaled by log2(e) and with -inf for
-//         columns beyond N; MODE 2: anything else (per-row masks read from global memory with
+// MODE 1: additive mask that is the same for every query row (padding masks): all threads stage it in
+//         shared memory during set-up, already clamped, scaled by log2(e) and with -inf for columns
+//         beyond N, and key blocks that are masked throughout are not visited; MODE 2: anything else (per-row masks read from global memory with
 //         128-bit loads where the layout allows, non-positive scale).
 template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kAttnThreads, 1)
@@ -224,15 +258,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     auto v_full = [&](int s) { return bar_base + 8u * (2 + 2 * KVS + s); };
     auto v_empty = [&](int s) { return bar_base + 8u * (2 + 3 * KVS + s); };
     auto s_full = [&](int t) { return bar_base + 8u * (2 + 4 * KVS + t); };
-    auto p_full = [&](int t, int half) { return bar_base + 8u * (16 + 4 * KVS + t * 2 + half); };  // keys [0, 64) / [64, 128) of P
+    auto p_full = [&](int t, int half) { return bar_base + 8u * (8 + 4 * KVS + t * 2 + half); };  // keys [0, 64) / [64, 128) of P
     auto o_final = [&](int t) { return bar_base + 8u * (6 + 4 * KVS + t); };
-    auto m_full = [&](int t, int bf) { return bar_base + 8u * (8 + 4 * KVS + t * 2 + bf); };
-    auto m_empty = [&](int t, int bf) { return bar_base + 8u * (12 + 4 * KVS + t * 2 + bf); };
-    constexpr int kNumBars = 20 + 4 * KVS;
-    static_assert(kNumBars * 8 + 16 <= 512, "barrier area too small");
+    constexpr int kNumBars = 12 + 4 * KVS;
+    static_assert(kNumBars * 8 + 32 <= 512, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // [tile][buffer][128]
+    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // MODE 1: [N rounded up to 128]
+    uint32_t* act_bits = tmem_slot + 2;  // MODE 1: key blocks with an unmasked key
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -272,10 +305,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             mbar_init(p_full(t, 0), 4);
             mbar_init(p_full(t, 1), 4);
             mbar_init(o_final(t), 1);
-            for (int bf = 0; bf < 2; ++bf) {
-                mbar_init(m_full(t, bf), 2);   // the two loader warps
-                mbar_init(m_empty(t, bf), 4);  // the four warps of the tile's softmax group
-            }
         }
         for (int s = 0; s < KVS; ++s) {
             mbar_init(k_full(s), 1);
@@ -284,6 +313,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             mbar_init(v_empty(s), 1);
         }
         *abort_flag = 0;
+        for (int i = 0; i < 4; ++i) act_bits[i] = 0u;
         fence_mbar_init();
     }
     if (warp == 9) {
@@ -301,6 +331,39 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const uint32_t tmem_base = *tmem_slot;
     // Launched with programmatic dependent launch: nothing of global memory but the status word is touched above
     pdl_wait();
+    if (warp == 8 && lane == 0) {
+        for (int t = 0; t < ntl; ++t) {
+            mbar_arrive_expect_tx(q_full(t), TILE);
+            for (int c = 0; c < D / 64; ++c)
+                tma_load_4d(q_smem + t * TILE + c * CHUNK, &tmap_q, q_full(t), c * 64, mt[t] * kAttnBlock, h, b);
+        }
+    }
+    uint32_t act[4] = {0u, 0u, 0u, 0u};
+    if (MODE == 1) {
+        const float mlow = mask_lowest(p.mask_dtype);
+        const int64_t moff = (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1];
+        const int cols = max_blk * kAttnBlock;
+        for (int c0 = 0; c0 < cols; c0 += kAttnThreads) {
+            const int col = c0 + (int)threadIdx.x;  // a warp's 32 columns lie in one key block
+            const bool inside = col < p.N && col < cols;
+            const float v = inside ? fmaxf(mask_load(p.mask, moff + (int64_t)col * p.mask_strides[3], p.mask_dtype), mlow) * kLog2e : -INFINITY;
+            if (col < cols) mask_smem[col] = v;
+            if (__any_sync(0xffffffffu, inside && v > kSkipBelow) && lane == 0) atomicOr(&act_bits[col >> 12], 1u << ((col >> 7) & 31));
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) act[i] = act_bits[i];
+        // nothing is skipped when everything is masked, nor for causal rows, which may see masked keys only
+        if ((act[0] | act[1] | act[2] | act[3]) == 0u || p.is_causal) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) act[i] = 0xffffffffu;
+        }
+        nblk[0] = bits_count_below(act, nblk[0]);
+        nblk[1] = bits_count_below(act, nblk[1]);
+    }
+    // from here on nblk counts the blocks that a tile visits; both tiles visit a prefix of the same list
+    const int visits = max(nblk[0], nblk[1]);
+    auto next_blk = [&](int from) { return MODE == 1 ? bits_next(act, from) : from; };
 
     if (warp >= 8) {
       asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kAttnRegsLow));
@@ -308,25 +371,20 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         // ------------------------------------------------------------------ TMA producer
         if (elect_one()) {
             bool ok = true;
-            for (int t = 0; t < ntl; ++t) {
-                mbar_arrive_expect_tx(q_full(t), TILE);
-                for (int c = 0; c < D / 64; ++c)
-                    tma_load_4d(q_smem + t * TILE + c * CHUNK, &tmap_q, q_full(t), c * 64,
-                                mt[t] * kAttnBlock, h, b);
-            }
-            for (int j = 0; j < max_blk && ok; ++j) {
+            int jb = next_blk(0);
+            for (int j = 0; j < visits && ok; ++j, jb = next_blk(jb + 1)) {
                 const int s = j % KVS;
                 const uint32_t ph = (uint32_t)((j / KVS) & 1);
                 if (!mbar_wait(k_empty(s), ph ^ 1, abort_flag, 100)) { ok = false; break; }
                 mbar_arrive_expect_tx(k_full(s), TILE);
                 for (int c = 0; c < D / 64; ++c)
                     tma_load_4d(k_smem + s * TILE + c * CHUNK, &tmap_k, k_full(s), c * 64,
-                                j * kAttnBlock, h / p.kv_group, b);
+                                jb * kAttnBlock, h / p.kv_group, b);
                 if (!mbar_wait(v_empty(s), ph ^ 1, abort_flag, 101)) { ok = false; break; }
                 mbar_arrive_expect_tx(v_full(s), TILE);
                 for (int c = 0; c < D / 64; ++c)
                     tma_load_4d(v_smem + s * TILE + c * CHUNK, &tmap_v, v_full(s), c * 64,
-                                j * kAttnBlock, h / p.kv_group, b);
+                                jb * kAttnBlock, h / p.kv_group, b);
             }
             if (!ok) {
                 for (int i = 0; i < 64; ++i) __nanosleep(2000);
@@ -370,7 +428,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             };
             for (int t = 0; t < ntl && ok; ++t)
                 if (!mbar_wait(q_full(t), 0, abort_flag, 200)) ok = false;
-            if (ok && max_blk > 0) {
+            if (ok && visits > 0) {
                 if (!mbar_wait(k_full(0), 0, abort_flag, 201)) ok = false;
                 if (ok) {
                     tc_fence_after();
@@ -383,13 +441,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     tc_commit(k_empty(0));
                 }
             }
-            for (int j = 0; j < max_blk && ok; ++j) {
+            for (int j = 0; j < visits && ok; ++j) {
                 const int s = j % KVS;
                 const uint32_t ph = (uint32_t)((j / KVS) & 1);
                 const int s1 = (j + 1) % KVS;
                 const uint32_t ph1 = (uint32_t)(((j + 1) / KVS) & 1);
                 if (!mbar_wait(v_full(s), ph, abort_flag, 202)) { ok = false; break; }
-                if (j + 1 < max_blk) {
+                if (j + 1 < visits) {
                     if (!mbar_wait(k_full(s1), ph1, abort_flag, 203)) { ok = false; break; }
                 }
                 for (int t = 0; t < ntl; ++t) {
@@ -410,32 +468,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 }
                 if (!ok) break;
                 tc_commit(v_empty(s));
-                if (j + 1 < max_blk) tc_commit(k_empty(s1));
-            }
-        }
-      } else if (MODE == 1) {
-        // ------------------------------------------------------------------ mask loaders (warps 10, 11)
-        const int li = (int)threadIdx.x - 320;  // 0..63, two columns each
-        const float mlow = mask_lowest(p.mask_dtype);
-        const int64_t moff = (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1];
-        bool ok = true;
-        for (int j = 0; j < max_blk && ok; ++j) {
-            const int bf = j & 1;
-            const uint32_t ph = (uint32_t)((j >> 1) & 1);
-            for (int t = 0; t < ntl && ok; ++t) {
-                if (j >= nblk[t]) continue;
-                if (!mbar_wait(m_empty(t, bf), ph ^ 1, abort_flag, 400 + t)) { ok = false; break; }
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    const int idx = li + e * 64;
-                    const int col = j * kAttnBlock + idx;
-                    float a = -INFINITY;
-                    if (col < p.N)
-                        a = fmaxf(mask_load(p.mask, moff + (int64_t)col * p.mask_strides[3], p.mask_dtype), mlow) * kLog2e;
-                    mask_smem[(t * 2 + bf) * kAttnBlock + idx] = a;
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(m_full(t, bf));
+                if (j + 1 < visits) tc_commit(k_empty(s1));
             }
         }
       }
@@ -461,7 +494,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             float m_ref = -INFINITY;
             float l = 0.f;
             bool ok = true;
-            for (int j = 0; j < nblk[t]; ++j) {
+            int jb = next_blk(0);
+            for (int j = 0; j < nblk[t]; ++j, jb = next_blk(jb + 1)) {
                 if (!mbar_wait(s_full(t), (uint32_t)(j & 1), abort_flag, 300 + t)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t sr[4][32];
@@ -469,12 +503,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 for (int cch = 0; cch < 4; ++cch) tmem_ld_32x32(s_addr + cch * 32, sr[cch]);
                 tmem_ld_wait();
 
-                const int col0 = j * kAttnBlock;
+                const int col0 = jb * kAttnBlock;
                 const bool causal_edge = p.is_causal && col0 + kAttnBlock - 1 > mt[t] * kAttnBlock;
                 if (MODE == 1) {
-                    const int bf = j & 1;
-                    if (!mbar_wait(m_full(t, bf), (uint32_t)((j >> 1) & 1), abort_flag, 320 + t)) { ok = false; break; }
-                    const float4* ms = reinterpret_cast<const float4*>(mask_smem + (t * 2 + bf) * kAttnBlock);
+                    const float4* ms = reinterpret_cast<const float4*>(mask_smem + col0);
 #pragma unroll
                     for (int cch = 0; cch < 4; ++cch) {
 #pragma unroll
@@ -486,8 +518,6 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                             sr[cch][v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[cch][v4 * 4 + 3]), c, a.w));
                         }
                     }
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(m_empty(t, bf));
                 } else if (MODE == 2) {
                     if (p.mask == nullptr) {
 #pragma unroll
@@ -662,12 +692,13 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     static PerDeviceOnce attr_once;
     if (attr_once.first_time()) {
         if (cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg::kSmemBytes) != cudaSuccess)
+                                 MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase) != cudaSuccess)
             return KB_ERR_LAUNCH;
     }
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
-    if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads, Cfg::kSmemBytes, stream, tq, tk, tv, d) != cudaSuccess)
+    if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads,
+                   (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : 0), stream, tq, tk, tv, d) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
@@ -675,7 +706,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
 template <typename T, int D>
 static int launch_attention_td(const kb_attn_params& p, cudaStream_t stream) {
     if (p.mask == nullptr && p.sm_scale > 0.f) return launch_attention_tdm<T, D, 0>(p, stream);
-    if (p.mask != nullptr && p.mask_strides[2] == 0) return launch_attention_tdm<T, D, 1>(p, stream);
+    if (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnCfg<D>::kMaskMaxN) return launch_attention_tdm<T, D, 1>(p, stream);
     return launch_attention_tdm<T, D, 2>(p, stream);
 }
 

@@ -321,9 +321,9 @@ static bool attention_short_applicable(const kb_attn_params& p) {
     const bool d80 = p.D <= 80;
     const double mine = estimate(tiles64, 2300.0 + (d80 ? 1080.0 : 1650.0) * fb * live, (d80 ? 9.5 : 11.0) + 2 * fa + (d80 ? 5.0 : 7.2) * fb * live);
     const double pairs = bh * (double)((p.M + 255) / 256), b128 = (double)((p.N + 127) / 128);
-    const double live128 = p.is_causal ? (b128 + 1) / 2 : b128;
+    const double live128 = p.is_causal ? (b128 + 1) / 2 : row_mask && b128 > 1 ? 0.33 + 0.67 * b128 : b128;
     const bool ragged = full_mask && (p.mask_strides[2] % 8 != 0 || p.mask_strides[3] != 1);
-    const double slow = ragged ? 2.6 : full_mask ? 1.8 : row_mask ? 1.3 : 1.0;  // masks cost that kernel's softmax warps, and it skips no blocks
+    const double slow = ragged ? 2.6 : full_mask ? 1.8 : row_mask ? 1.15 : 1.0;  // masks cost that kernel's softmax warps
     const double other = estimate(pairs, (5000.0 + 2500.0 * live128) * slow, (p.M > 128 ? 57.0 : 35.0) * (full_mask ? 1.5 : 1.0) + 13.0 * live128 * slow);
     return mine < other;
 }

@@ -46,37 +46,6 @@ struct SplitShape {
 static int g_split_tiles = 0;  // test hook: 0 = by launch size, 1 / 2 = force the number of query tiles per CTA
 static int g_attn_persistent = -1;  // test hook: -1 = dispatcher's choice, 0 = one CTA per tile, 1 = persistent CTAs
 
-// Key blocks of a MODE 1 launch whose mask is "minus infinity" for every key (the padding behind a
-// sequence) contribute exp(-65504 + ...) = 0 to every row and are skipped: not loaded, not multiplied,
-// not exponentiated. A block is skipped only if all of its mask values are below kSkipBelow (in the
-// log2 domain), far beyond where fp32 exp underflows for any score difference up to 2^14; if the
-// whole row is like that (a fully padded sequence, where the mask cancels and the reference
-// returns a plain softmax) nothing is skipped. At most 128 blocks (N <= 8192): a 128-bit set.
-constexpr float kSkipBelow = -30000.0f * 1.4426950408889634f;
-__device__ __forceinline__ int bits_next(const uint32_t (&w)[4], int from) {  // smallest set bit >= from
-    int r = 1 << 20;
-#pragma unroll
-    for (int wi = 3; wi >= 0; --wi) {
-        uint32_t m = w[wi];
-        const int lo = from - wi * 32;
-        if (lo >= 32) m = 0u;
-        else if (lo > 0) m &= 0xffffffffu << lo;
-        if (m != 0u) r = wi * 32 + __ffs((int)m) - 1;
-    }
-    return r;
-}
-__device__ __forceinline__ int bits_count_below(const uint32_t (&w)[4], int limit) {  // set bits with index < limit
-    int n = 0;
-#pragma unroll
-    for (int wi = 0; wi < 4; ++wi) {
-        const int hi = limit - wi * 32;
-        uint32_t m = w[wi];
-        if (hi <= 0) m = 0u;
-        else if (hi < 32) m &= (1u << hi) - 1u;
-        n += __popc(m);
-    }
-    return n;
-}
 __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
     asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];" ::"l"(
                      reinterpret_cast<uint64_t>(map)),
