@@ -687,10 +687,6 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             const int b = bh / p.H, h = bh % p.H;
             const int row = mt * kAttnBlock + r_in_tile;
             const float* mask_row = mask_smem + slot * mask_cols;
-            const int64_t mask_row_off =
-                (MODE == 2 && p.mask != nullptr)
-                    ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)min(row, p.M - 1) * p.mask_strides[2]
-                    : 0;
             float m_ref = -INFINITY;
             float l = 0.f;
             int jb = (MODE == 1) ? bits_next(act, 0) : 0;  // key-block number of visit j
@@ -719,23 +715,6 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                         sr[v4 * 4 + 1] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 1]), c, a.y));
                         sr[v4 * 4 + 2] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 2]), c, a.z));
                         sr[v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 3]), c, a.w));
-                    }
-                } else if (MODE == 2) {
-                    if (p.mask == nullptr) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) sr[i] = __float_as_uint(__uint_as_float(sr[i]) * c);
-                    } else {
-#pragma unroll
-                        for (int hc = 0; hc < 2; ++hc) {
-                            const int colc = col0 + hc * 16;
-                            float mvals[16];
-                            mask_values(p, mask_row_off, colc, mvals);
-#pragma unroll
-                            for (int i = 0; i < 16; ++i) {
-                                uint32_t& sv = sr[hc * 16 + i];
-                                sv = __float_as_uint(fmaf(fmaxf(mvals[i], mlow), kLog2e, __uint_as_float(sv) * c));
-                            }
-                        }
                     }
                 }
                 const bool causal_edge = p.is_causal && col0 + 31 > mt * kAttnBlock;
@@ -914,7 +893,6 @@ static unsigned int* attention_queue_slot() {
 template <typename T, int MODE>
 static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream) {
     using Cfg = AttnPersistCfg;
-    constexpr int D = 64;
     CUtensorMap tq, tk, tv;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;

@@ -200,19 +200,23 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     if (warp == 1) tmem_dealloc(tmem_base, NB);
 }
 
-// Clusters of `splits` CTAs that are resident at once (asked once per device and size).
+// Clusters that are resident at once on the current device, by size (asked once per device; null: no device).
+// A plain pointer to the table: a plan looks at all sizes of three kernels, and a lock and a device query for
+// each of them were 2.5 us of host time per call.
 template <typename T, int NB>
-static int linear_cluster_resident(int splits) {
-    static std::mutex mu;
+static const int* linear_cluster_resident() {
     static int resident[64][kClMaxSplits + 1] = {};
+    static std::atomic<bool> known[64] = {};
+    static std::mutex mu;
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    if (known[dev].load(std::memory_order_acquire)) return resident[dev];
     std::lock_guard<std::mutex> lock(mu);
-    if (resident[dev][1] == 0) {
+    if (!known[dev].load(std::memory_order_relaxed)) {
         auto* kernel = linear_cluster_kernel<T, NB>;
         if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, ClCfg<NB>::kSmemBytes) != cudaSuccess ||
             cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-            return 0;
+            return nullptr;
         cudaLaunchConfig_t cfg = {};
         cfg.blockDim = dim3(kClThreads);
         cfg.dynamicSmemBytes = ClCfg<NB>::kSmemBytes;
@@ -232,13 +236,15 @@ static int linear_cluster_resident(int splits) {
             }
             resident[dev][s] = n;
         }
+        known[dev].store(true, std::memory_order_release);
     }
-    return resident[dev][splits];
+    return resident[dev];
 }
 
 template <typename T, int NB>
 static int launch_linear_cluster(const kb_linear_params& p, cudaStream_t stream, int splits) {
-    if (linear_cluster_resident<T, NB>(splits) == 0) return KB_ERR_LAUNCH;
+    const int* table = linear_cluster_resident<T, NB>();  // (also sets the kernel's attributes)
+    if (table == nullptr || table[splits] == 0) return KB_ERR_LAUNCH;
     CUtensorMap tmap_w, tmap_x;
     {
         const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.N};
@@ -297,8 +303,10 @@ static ClusterPlan linear_cluster_plan(const kb_linear_params& p) {
     for (int nb : {32, 64, 128}) {
         if (nb == 32 ? p.M > 256 : nb == 64 ? p.M <= 32 : p.M <= 64) continue;
         const int64_t tiles = ((p.M + nb - 1) / nb) * num_n;
+        const int* table = nb == 32 ? linear_cluster_resident<T, 32>() : nb == 64 ? linear_cluster_resident<T, 64>() : linear_cluster_resident<T, 128>();
+        if (table == nullptr) continue;
         for (int s = 1; s <= kClMaxSplits && s <= num_k; ++s) {
-            const int resident = nb == 32 ? linear_cluster_resident<T, 32>(s) : nb == 64 ? linear_cluster_resident<T, 64>(s) : linear_cluster_resident<T, 128>(s);
+            const int resident = table[s];
             if (resident == 0) continue;
             const double waves = (double)((tiles + resident - 1) / resident);
             const bool shared_sm = (tiles < resident ? tiles : resident) * s > sm_count();
@@ -328,18 +336,17 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
     if (forced_bn != 0) return launch_linear_single<T>(p, stream, forced_bn);
     if (stream_layout(p) && p.M <= 16) return launch_linear_stream_t<T>(p, stream);
     const double single = linear_single_us(p);
+    const ClusterPlan cl = p.M <= 1024 && g_linear_pair == 1 && gemm_sms() == sm_count() ? linear_cluster_plan<T>(p) : ClusterPlan{0, 0, 1e300};
     if (p.M > 128 && p.N >= 128 && p.K >= 256 && g_linear_pair != 0) {
         double pair;
         const int bn = linear_pair_tile_width(p, &pair);
         // (at thousands of rows the estimates no longer matter: the pair kernel pulls half as much W through each SM's port)
         if (g_linear_pair != 1 || pair < 0.93 * single || (p.M > 4096 && p.N >= 256)) {
-            const ClusterPlan cl = p.M <= 1024 && g_linear_pair == 1 && gemm_sms() == sm_count() ? linear_cluster_plan<T>(p) : ClusterPlan{0, 0, 1e300};
             if (pair <= cl.us) return launch_linear_pair_t<T>(p, stream, bn);
         }
     }
     if (p.M <= 1024 && gemm_sms() == sm_count()) {
         const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
-        const ClusterPlan cl = linear_cluster_plan<T>(p);
         if (stream_us < single && stream_us < cl.us) return launch_linear_stream_t<T>(p, stream);
         // (the cluster kernel has to be clearly ahead: where the two are close, its estimate is the less certain one)
         if (cl.us < 0.94 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);

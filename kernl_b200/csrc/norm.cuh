@@ -38,7 +38,11 @@ constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
 // and left twelve warps on an SM, all of them loading, then all computing, then all storing:
 // [16384, 4096] bf16 add + RMSNorm 120.9 us (4.4 TB/s), with four warps per row 89.2 us (6.0 TB/s).
 // Vector c of lane l of warp w covers columns ((c*WPR + w)*32 + l)*8 .. +8. cols must be a multiple of 8.
-template <typename T, int CHUNKS, bool RMS, int WPR = 1>
+// CHAIN (RMSNorm, many rows, four warps): the warps own consecutive parts of the row and pass each lane's sum of
+// squares on from warp to warp, so that the row is summed in the order of one warp walking it: a decoder's
+// hidden states, and with them its greedy tokens, do not depend on how many warps share a row. The hand-over is
+// hidden behind the other CTAs of the SM.
+template <typename T, int CHUNKS, bool RMS, int WPR = 1, bool CHAIN = false>
 __global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
 norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ gamma,
                         const T* __restrict__ beta, float* __restrict__ mean_out,
@@ -48,13 +52,14 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
     pdl_wait();
     pdl_launch_dependents();
     __shared__ float red_s[2][8];
+    __shared__ float chain_s[CHAIN ? 32 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wir = warp % WPR;  // this warp's position inside its row
     const int64_t row = WPR == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
     if (row >= rows) return;  // (WPR > 1: the whole CTA leaves together)
     const T* xr = x + row * x_row_stride;
     T* yr = y + row * y_row_stride;
-#define KB_NORM_COL(c) ((((c) * WPR + wir) * 32 + lane) * 8)
+#define KB_NORM_COL(c) (((CHAIN ? wir * CHUNKS + (c) : (c) * WPR + wir) * 32 + lane) * 8)
 
     uint4 v[CHUNKS];
 #pragma unroll
@@ -113,30 +118,62 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
         if (!RMS) shift = __shfl_sync(0xffffffffu, Elem<T>::unpack2(v[0].x).x, 0);
         // (two values per instruction: at 4096 columns a third of the issue slots went into this sweep and the
         // last one, and a LayerNorm row took a quarter longer than an RMSNorm row)
-        float2 p1 = make_float2(0.f, 0.f), p2 = make_float2(0.f, 0.f);
-        const float2 neg_shift = make_float2(-shift, -shift);
+        // (RMSNorm keeps one scalar chain per lane: it needs half the instructions, and its order is kept, see CHAIN)
+        float s1 = 0.f, s2 = 0.f;
+        auto add_squares = [&]() {
 #pragma unroll
-        for (int c = 0; c < CHUNKS; ++c) {
-            const int col = KB_NORM_COL(c);
-            if (col < cols) {
-                const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+            for (int c = 0; c < CHUNKS; ++c) {
+                if (KB_NORM_COL(c) < cols) {
+                    const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float2 f = Elem<T>::unpack2(w[i]);
-                    if (!RMS) {
-                        f = __fadd2_rn(f, neg_shift);
-                        p1 = __fadd2_rn(p1, f);
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = Elem<T>::unpack2(w[i]);
+                        s2 = fmaf(f.x, f.x, fmaf(f.y, f.y, s2));
                     }
-                    p2 = __ffma2_rn(f, f, p2);
                 }
             }
+        };
+        if (CHAIN) {
+#pragma unroll
+            for (int w = 0; w < WPR; ++w) {
+                if (wir == w) {
+                    if (w > 0) s2 = chain_s[lane];
+                    add_squares();
+                    chain_s[lane] = s2;
+                }
+                __syncthreads();
+            }
+            s2 = chain_s[lane];
+        } else if (RMS) {
+            add_squares();
+        } else {
+            float2 p1 = make_float2(0.f, 0.f), p2 = make_float2(0.f, 0.f);
+            const float2 neg_shift = make_float2(-shift, -shift);
+#pragma unroll
+            for (int c = 0; c < CHUNKS; ++c) {
+                if (KB_NORM_COL(c) < cols) {
+                    const uint32_t w[4] = {v[c].x, v[c].y, v[c].z, v[c].w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const float2 f = __fadd2_rn(Elem<T>::unpack2(w[i]), neg_shift);
+                        p1 = __fadd2_rn(p1, f);
+                        p2 = __ffma2_rn(f, f, p2);
+                    }
+                }
+            }
+            s1 = p1.x + p1.y;
+            s2 = p2.x + p2.y;
         }
-        float s1 = p1.x + p1.y, s2 = p2.x + p2.y;
         s2 = warp_sum(s2);
         if (!RMS) s1 = warp_sum(s1);
-        if (WPR > 1) {
-            // the warps of a row meet: their sums, or (LayerNorm) their means and squared deviations, whose
-            // combination needs no common shift
+        if (WPR > 1 && RMS && !CHAIN) {
+            if (lane == 0) red_s[1][warp] = s2;
+            __syncthreads();
+            s2 = (red_s[1][0] + red_s[1][1]) + (red_s[1][2] + red_s[1][3]);
+            if (WPR == 8) s2 += (red_s[1][4] + red_s[1][5]) + (red_s[1][6] + red_s[1][7]);
+            s2 *= inv_n;
+        } else if (WPR > 1 && !RMS) {
+            // the warps of a row meet: their means and squared deviations, whose combination needs no common shift
             auto columns_of = [&](int w) {
                 int n = 0;
 #pragma unroll
@@ -146,22 +183,17 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
             if (lane == 0) {
                 const float n = columns_of(warp), d = n > 0.f ? s1 / n : 0.f;
                 red_s[0][warp] = shift + d;
-                red_s[1][warp] = RMS ? s2 : fmaxf(s2 - s1 * d, 0.f);
+                red_s[1][warp] = fmaxf(s2 - s1 * d, 0.f);
             }
             __syncthreads();
             float total = 0.f, m2 = 0.f;
-            if (!RMS) {
 #pragma unroll
-                for (int w = 0; w < WPR; ++w) total = fmaf(columns_of(w), red_s[0][w], total);
-                mean = total * inv_n;
-            }
+            for (int w = 0; w < WPR; ++w) total = fmaf(columns_of(w), red_s[0][w], total);
+            mean = total * inv_n;
 #pragma unroll
             for (int w = 0; w < WPR; ++w) {
-                m2 += red_s[1][w];
-                if (!RMS) {
-                    const float d = red_s[0][w] - mean;
-                    m2 = fmaf(columns_of(w) * d, d, m2);
-                }
+                const float d = red_s[0][w] - mean;
+                m2 = fmaf(columns_of(w) * d, d, m2 + red_s[1][w]);
             }
             s2 = m2 * inv_n;
         } else {
@@ -262,8 +294,8 @@ static int launch_norm_t(const kb_norm_params& p, cudaStream_t stream) {
                         ((uintptr_t)p.x % 16) == 0 && ((uintptr_t)p.y % 16) == 0 &&
                         ((uintptr_t)p.gamma % 16) == 0 &&
                         (p.beta == nullptr || ((uintptr_t)p.beta % 16) == 0) && p.cols <= kNormMaxCols;
-#define KB_NORM_LAUNCH(C, W)                                                                      \
-    return launch_pdl(norm_fwd_rowwarp_kernel<T, C, RMS, W>, W == 1 ? grid : (unsigned)p.rows, W == 8 ? 256 : 128, 0, stream, \
+#define KB_NORM_LAUNCH(C, W, ...)                                                                 \
+    return launch_pdl(norm_fwd_rowwarp_kernel<T, C, RMS, W, ##__VA_ARGS__>, W == 1 ? grid : (unsigned)p.rows, W == 8 ? 256 : 128, 0, stream, \
                       x, y, g, b, p.mean, p.rstd, p.rows, (int)p.cols, p.x_row_stride, p.y_row_stride, p.eps,                  \
                       (const T*)p.residual, (T*)p.sum_out) == cudaSuccess ? KB_OK : KB_ERR_LAUNCH
     if (vec_ok && p.cols > 4096) {
@@ -271,11 +303,16 @@ static int launch_norm_t(const kb_norm_params& p, cudaStream_t stream) {
         if (p.cols <= 4 * 2048) KB_NORM_LAUNCH(4, 8);
         KB_NORM_LAUNCH(8, 8);
     }
-    if (vec_ok && (p.cols > 1024 || p.rows <= 1024)) {
+    if (vec_ok && p.rows <= 1024) {
         if (p.cols <= 1024) KB_NORM_LAUNCH(1, 4);
         if (p.cols <= 2 * 1024) KB_NORM_LAUNCH(2, 4);
         if (p.cols <= 3 * 1024) KB_NORM_LAUNCH(3, 4);
         KB_NORM_LAUNCH(4, 4);
+    }
+    if (vec_ok && p.cols > 1024) {
+        if (p.cols <= 2 * 1024) KB_NORM_LAUNCH(2, 4, RMS);
+        if (p.cols <= 3 * 1024) KB_NORM_LAUNCH(3, 4, RMS);
+        KB_NORM_LAUNCH(4, 4, RMS);
     }
     if (vec_ok) {
         if (p.cols <= 256) KB_NORM_LAUNCH(1, 1);
