@@ -586,23 +586,21 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 //      the first 64 columns of S
                 const float neg_ref = -m_ref * unit;
                 const float2 unit2 = make_float2(unit, unit), neg2 = make_float2(neg_ref, neg_ref);
-                // Row sum: four chains over the pair sums e0 + e1, in the order of a scalar loop (pair i adds to chain
-                // i & 3), so that the result does not depend on the arithmetic being packed two by two.
-                float2 lp01 = {0.f, 0.f}, lp23 = {0.f, 0.f};
+                // Row sum: four scalar chains (pair i adds to chain i & 3), taken after P has been handed over. Two values
+                // per instruction would save issue slots (155 us instead of 164 at [4, 32 over 8, 2048, 128] causal) but
+                // add in another order, and a decoder's greedy tokens should not depend on that. (A quarter to a half
+                // of the exponentials on the FMA pipe was no faster: the special-function unit is half idle.)
+                float lp[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
                 for (int cch = 0; cch < 4; ++cch) {
                     uint32_t pk[16];
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        // (a quarter to a half of the exponentials on the FMA pipe instead was no faster: the unit is half idle)
-                        const float2 a0 = __ffma2_rn(make_float2(__uint_as_float(sr[cch][2 * i]), __uint_as_float(sr[cch][2 * i + 1])), unit2, neg2);
-                        const float2 a1 = __ffma2_rn(make_float2(__uint_as_float(sr[cch][2 * i + 2]), __uint_as_float(sr[cch][2 * i + 3])), unit2, neg2);
-                        const float2 e0 = make_float2(fast_exp2(a0.x), fast_exp2(a1.x)), e1 = make_float2(fast_exp2(a0.y), fast_exp2(a1.y));
-                        const float2 both = __fadd2_rn(e0, e1);
-                        if (i & 2) lp23 = __fadd2_rn(lp23, both);
-                        else lp01 = __fadd2_rn(lp01, both);
-                        pk[i] = Elem<T>::pack2(e0.x, e1.x);
-                        pk[i + 1] = Elem<T>::pack2(e0.y, e1.y);
+                    for (int i = 0; i < 16; ++i) {
+                        const float2 a = __ffma2_rn(make_float2(__uint_as_float(sr[cch][2 * i]), __uint_as_float(sr[cch][2 * i + 1])), unit2, neg2);
+                        const float e0 = fast_exp2(a.x), e1 = fast_exp2(a.y);
+                        sr[cch][2 * i] = __float_as_uint(e0);
+                        sr[cch][2 * i + 1] = __float_as_uint(e1);
+                        pk[i] = Elem<T>::pack2(e0, e1);
                     }
                     tmem_st_32x16(s_addr + cch * 16, pk);
                     if (cch & 1) {
@@ -612,7 +610,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         if (lane == 0) mbar_arrive(p_full(t, cch >> 1));
                     }
                 }
-                l += (lp01.x + lp01.y) + (lp23.x + lp23.y);
+#pragma unroll
+                for (int cch = 0; cch < 4; ++cch) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) lp[i & 3] += __uint_as_float(sr[cch][2 * i]) + __uint_as_float(sr[cch][2 * i + 1]);
+                }
+                l += (lp[0] + lp[1]) + (lp[2] + lp[3]);
             }
             pdl_launch_dependents();  // the key loop is over: a dependent launch may take the slots that free up
             // ---- epilogue: O / l -> global
