@@ -699,11 +699,11 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     d.d_out = (int)p.D;
 
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) {
-        if (cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase) != cudaSuccess)
-            return KB_ERR_LAUNCH;
-    }
+    if (!attr_once.run([] {
+            return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase) == cudaSuccess;
+        }))
+        return KB_ERR_LAUNCH;
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads,

@@ -932,7 +932,7 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
     d.kv_group = (int)kv_group;
     d.d_out = (int)p.D;
-    static int regs_ok = 0;  // 0 = not checked, 1 = usable, -1 = register allocation does not fit
+    static std::atomic<int> regs_ok{0};  // 0 = not checked, 1 = usable, -1 = register allocation does not fit
     if (regs_ok == 0) {
         // setmaxnreg.inc blocks until the CTA's pool holds the registers: refuse to launch a build
         // whose launch allocation is smaller than the redistribution assumes.
@@ -944,14 +944,13 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     const int mask_cols = MODE == 1 ? attention_persist_mask_cols(p.N) : 0;
     const size_t smem_bytes = (size_t)Cfg::kSmemBase + (size_t)mask_cols * 8;
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) {
-        // two CTAs of up to 113 KB share an SM: that needs the largest shared-memory carve-out
-        if (cudaFuncSetAttribute(attention_persist_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg::kSmemLimit) != cudaSuccess ||
-            cudaFuncSetAttribute(attention_persist_kernel<T, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 (int)cudaSharedmemCarveoutMaxShared) != cudaSuccess)
-            return KB_ERR_LAUNCH;
-    }
+    if (!attr_once.run([] {
+            // two CTAs of up to 113 KB share an SM: that needs the largest shared-memory carve-out
+            return cudaFuncSetAttribute(attention_persist_kernel<T, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemLimit) == cudaSuccess &&
+                   cudaFuncSetAttribute(attention_persist_kernel<T, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                        (int)cudaSharedmemCarveoutMaxShared) == cudaSuccess;
+        }))
+        return KB_ERR_LAUNCH;
     if (smem_bytes > (size_t)Cfg::kSmemLimit) return KB_ERR_UNSUPPORTED;
     const int64_t tiles = (int64_t)d.num_pairs * p.B * p.H;
     const int64_t grid = tiles < 2 * (int64_t)sm_count() ? tiles : 2 * (int64_t)sm_count();

@@ -360,8 +360,10 @@ static int launch_attention_short_t(const kb_attn_params& p, cudaStream_t stream
     d.d_out = (int)p.D;
     s.trigger_early = grid <= (int64_t)sm_count() * Cfg::ctas(MODE) ? 1 : 0;
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time() && cudaFuncSetAttribute(attention_short_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       Cfg::kSmemBytes + (MODE == 1 ? kShortMaskCols * 4 : 0)) != cudaSuccess)
+    if (!attr_once.run([] {
+            return cudaFuncSetAttribute(attention_short_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        Cfg::kSmemBytes + (MODE == 1 ? kShortMaskCols * 4 : 0)) == cudaSuccess;
+        }))
         return KB_ERR_LAUNCH;
     const size_t smem = (size_t)Cfg::kSmemBytes + (MODE == 1 ? (size_t)((p.N + 63) / 64) * 64 * 4 : 0);
     if (launch_pdl(attention_short_kernel<T, D, MODE>, (unsigned)grid, kShortThreads, smem, stream, s) != cudaSuccess) return KB_ERR_LAUNCH;

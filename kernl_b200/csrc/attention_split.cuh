@@ -665,7 +665,7 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
     d.kv_group = (int)kv_group;
     d.d_out = (int)p.D;
-    static int regs_ok = 0;  // 0 = not checked, 1 = usable, -1 = register allocation does not fit
+    static std::atomic<int> regs_ok{0};  // 0 = not checked, 1 = usable, -1 = register allocation does not fit
     if (regs_ok == 0) {
         // setmaxnreg.inc blocks until the CTA's pool holds the registers: refuse to launch a build
         // whose launch allocation is smaller than the redistribution assumes.
@@ -675,11 +675,10 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
     }
     if (regs_ok < 0) return KB_ERR_UNSUPPORTED;
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) {
-        if (cudaFuncSetAttribute(attention_split_kernel<T, MODE, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 Cfg::kSmemMax) != cudaSuccess)
-            return KB_ERR_LAUNCH;
-    }
+    if (!attr_once.run([] {
+            return cudaFuncSetAttribute(attention_split_kernel<T, MODE, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemMax) == cudaSuccess;
+        }))
+        return KB_ERR_LAUNCH;
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     const int num_n_blocks = (int)((p.N + kBlkN - 1) / kBlkN);

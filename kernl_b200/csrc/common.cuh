@@ -9,6 +9,9 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/kernl_b200.h"
 
 namespace kb {
@@ -111,14 +114,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
 }
 
 // Function attributes (dynamic shared memory size) are per device: a process that drives several
-// GPUs has to set them once on each. Not synchronised: setting an attribute twice is harmless.
+// GPUs has to set them once on each. `set` returns whether it succeeded; a thread that comes second waits until
+// the first has set them (launched before that, a kernel is refused for its shared memory), and a failure is
+// tried again at the next call.
 struct PerDeviceOnce {
-    bool done[64] = {};
-    bool first_time() {
+    std::atomic<bool> done[64] = {};
+    std::mutex mu;
+    template <typename F>
+    bool run(F&& set) {
         int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return true;
-        if (done[dev]) return false;
-        done[dev] = true;
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set();
+        if (done[dev].load(std::memory_order_acquire)) return true;
+        std::lock_guard<std::mutex> lock(mu);
+        if (done[dev].load(std::memory_order_relaxed)) return true;
+        if (!set()) return false;
+        done[dev].store(true, std::memory_order_release);
         return true;
     }
 };

@@ -67,7 +67,7 @@ int encode_tmap_16bit(CUtensorMap* out, const void* base, int rank, const uint64
 
 // Both answers are per device (a process may drive several GPUs), cached per device index.
 int sm_count() {
-    static int cached[64] = {};
+    static std::atomic<int> cached[64] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 148;
     if (dev >= 0 && dev < 64 && cached[dev] > 0) return cached[dev];
@@ -84,7 +84,7 @@ int gemm_sms() {
 }
 
 static int check_device() {
-    static int state[64] = {};  // per device: 0 unknown, 1 ok, -1 not an sm_100 device
+    static std::atomic<int> state[64] = {};  // per device: 0 unknown, 1 ok, -1 not an sm_100 device
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();

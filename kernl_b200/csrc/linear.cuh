@@ -470,11 +470,10 @@ static int launch_linear_bn(const kb_linear_params& p, cudaStream_t stream) {
         if (st != KB_OK) return st;
     }
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time()) {
-        cudaError_t e = cudaFuncSetAttribute(linear_tc_kernel<T, BN>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-        if (e != cudaSuccess) return KB_ERR_LAUNCH;
-    }
+    if (!attr_once.run([] {
+            return cudaFuncSetAttribute(linear_tc_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) == cudaSuccess;
+        }))
+        return KB_ERR_LAUNCH;
     const int64_t num_tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + BN - 1) / BN);
     const int grid = (int)(num_tiles < gemm_sms() ? num_tiles : gemm_sms());
     const cudaError_t le = launch_pdl(linear_tc_kernel<T, BN>, dim3((unsigned)grid), dim3(kGemmThreads), (size_t)Cfg::kSmemBytes, stream, tmap_x,

@@ -481,10 +481,11 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // pairs that can be resident at once, per device (the grid is persistent: one pair per slot)
-    static int max_pairs[64] = {};
+    static std::atomic<int> max_pairs[64] = {};  // (set after the attribute; two threads that ask at once get the same answer)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return KB_ERR_LAUNCH;
-    if (max_pairs[dev] == 0) {
+    int resident = max_pairs[dev].load(std::memory_order_acquire);
+    if (resident == 0) {
         if (cudaFuncSetAttribute(linear_pair_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) != cudaSuccess)
             return KB_ERR_LAUNCH;
         cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
@@ -493,10 +494,11 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
             cudaGetLastError();
             return KB_ERR_LAUNCH;
         }
-        max_pairs[dev] = n < sm_count() / 2 ? n : sm_count() / 2;
+        resident = n < sm_count() / 2 ? n : sm_count() / 2;
+        max_pairs[dev].store(resident, std::memory_order_release);
     }
     const int64_t tiles = ((p.M + 255) / 256) * ((p.N + BN - 1) / BN);
-    int pairs = (int)(tiles < max_pairs[dev] ? tiles : max_pairs[dev]);
+    int pairs = (int)(tiles < resident ? tiles : resident);
     if (pairs > gemm_sms() / 2) pairs = gemm_sms() / 2;  // a caller-set limit leaves SMs to a concurrent collective
     cfg.gridDim = dim3(2 * (unsigned)pairs);
     cfg.numAttrs = g_use_pdl ? 2u : 1u;

@@ -251,8 +251,9 @@ template <typename T, int RMAX, int NX>
 static int launch_linear_stream(const kb_linear_params& p, cudaStream_t stream, int64_t lines, int64_t ctas, int tiles) {
     using Cfg = StreamCfg<RMAX, NX>;
     static PerDeviceOnce attr_once;
-    if (attr_once.first_time() &&
-        cudaFuncSetAttribute(linear_stream_kernel<T, RMAX, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+    if (!attr_once.run([] {
+            return cudaFuncSetAttribute(linear_stream_kernel<T, RMAX, NX>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) == cudaSuccess;
+        }))
         return KB_ERR_LAUNCH;
     launch_pdl(linear_stream_kernel<T, RMAX, NX>, dim3((unsigned)ctas, (unsigned)((p.M + kStreamMaxM - 1) / kStreamMaxM)), kStreamThreads, Cfg::kSmemBytes, stream, (const T*)p.x, (const T*)p.w,
                (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M, (int)lines, (int)p.K, p.x_row_stride, p.y_row_stride, p.activation, tiles);
