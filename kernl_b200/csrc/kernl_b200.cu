@@ -59,9 +59,18 @@ int encode_tmap_16bit(CUtensorMap* out, const void* base, int rank, const uint64
         }
     }
     // CU_TENSOR_MAP_DATA_TYPE_FLOAT16 and BFLOAT16 move bytes identically; zero fill for OOB.
-    CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank, const_cast<void*>(base), gdims,
-                    gstrides, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, l2,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    auto encode = [&] {
+        return fn(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (cuuint32_t)rank, const_cast<void*>(base), gdims, gstrides, gbox, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swz, l2, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT || r == CUDA_ERROR_NOT_INITIALIZED) {
+        // The driver's call wants a current context, and a thread has none before its first runtime call that needs
+        // one: setting the device it is on makes that device's context current.
+        int dev = 0;
+        if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return KB_ERR_NO_DEVICE;
+        r = encode();
+    }
     return r == CUDA_SUCCESS ? KB_OK : KB_ERR_UNSUPPORTED;
 }
 
