@@ -49,6 +49,15 @@ PyObject* failed(const char* what, int status) {
     return nullptr;
 }
 
+// The GIL is given up around allocation and launch: a launch into a full queue blocks until the GPU has caught up, and a
+// cudaMalloc for seconds, and a serving process has other threads to run meanwhile.
+struct WithoutGil {
+    PyThreadState* const state = PyEval_SaveThread();
+    WithoutGil() = default;
+    WithoutGil(const WithoutGil&) = delete;
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 bool arity(Py_ssize_t got, Py_ssize_t want, const char* name) {
     if (got == want) return true;
     PyErr_Format(PyExc_TypeError, "%s takes %zd arguments, got %zd", name, want, got);
@@ -93,23 +102,26 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n) {
             Py_RETURN_NONE;
         y = *out;
     }
-    void* const stream = stream_of(*x);
     kb_linear_params p{};
-    const c10::cuda::CUDAGuard guard(x->device());
-    if (!y.defined()) y = dim == 2 ? empty({M, n_out}, *x) : empty({x->size(0), x->size(1), n_out}, *x);
     p.x = x->data_ptr();
     p.w = w->data_ptr();
     p.bias = bias != nullptr ? bias->data_ptr() : nullptr;
-    p.y = y.data_ptr();
     p.act_inputs = pre != nullptr ? pre->data_ptr() : nullptr;
     p.M = M;
     p.N = N;
     p.K = K;
     p.x_row_stride = x_stride;
-    p.y_row_stride = dim == 2 ? y.stride(0) : n_out;
     p.activation = act;
     p.dtype = dtype_code(x->scalar_type());
-    const int st = kb_linear_fwd(&p, stream);
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(x->device());
+        if (!y.defined()) y = dim == 2 ? empty({M, n_out}, *x) : empty({x->size(0), x->size(1), n_out}, *x);
+        p.y = y.data_ptr();
+        p.y_row_stride = dim == 2 ? y.stride(0) : n_out;
+        st = kb_linear_fwd(&p, stream_of(*x));
+    }
     if (st != KB_OK) return failed("linear_layer", st);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS
@@ -147,12 +159,8 @@ PyObject* layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (out == nullptr || !like(*out, *x) || !out->sizes().equals(x->sizes()) || !out->is_contiguous()) Py_RETURN_NONE;
         y = *out;
     }
-    const c10::cuda::CUDAGuard guard(x->device());
-    if (!y.defined()) y = empty(x->sizes(), *x);
-    if (residual != nullptr && with_sum) sum = empty(x->sizes(), *x);
     kb_norm_params p{};
     p.x = x->data_ptr();
-    p.y = y.data_ptr();
     p.gamma = w->data_ptr();
     p.beta = bias != nullptr ? bias->data_ptr() : nullptr;
     p.rows = x->numel() / cols;
@@ -163,8 +171,16 @@ PyObject* layer_norm(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.is_rms = rms;
     p.dtype = dtype_code(x->scalar_type());
     p.residual = residual != nullptr ? residual->data_ptr() : nullptr;
-    p.sum_out = sum.defined() ? sum.data_ptr() : nullptr;
-    const int st = kb_norm_fwd(&p, stream_of(*x));
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(x->device());
+        if (!y.defined()) y = empty(x->sizes(), *x);
+        if (residual != nullptr && with_sum) sum = empty(x->sizes(), *x);
+        p.y = y.data_ptr();
+        p.sum_out = sum.defined() ? sum.data_ptr() : nullptr;
+        st = kb_norm_fwd(&p, stream_of(*x));
+    }
     if (st != KB_OK) return failed("layer_norm", st);
     if (!sum.defined()) return THPVariable_Wrap(std::move(y));
     PyObject* pair = PyTuple_New(2);
@@ -241,8 +257,12 @@ PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
         for (int i = 0; i < 3; ++i)
             if (sizes[i] > 1 && strides[t][i] % 8 != 0) Py_RETURN_NONE;
     }
-    const c10::cuda::CUDAGuard guard(q->device());
-    const int st = kb_attention_fwd(&p, stream_of(*q));
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(q->device());
+        st = kb_attention_fwd(&p, stream_of(*q));
+    }
     if (st != KB_OK) return failed("attention_forward", st);
     Py_INCREF(a[3]);
     return a[3];
@@ -263,8 +283,12 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (len == nullptr || len->scalar_type() != at::kLong || len->numel() != 1 || len->device() != q->device()) Py_RETURN_NONE;
         p.kv_len_dev = len->data_ptr<int64_t>();
     }
-    const c10::cuda::CUDAGuard guard(q->device());
-    const int st = kb_attention_decode_fwd(&p, nullptr, 0, stream_of(*q));
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(q->device());
+        st = kb_attention_decode_fwd(&p, nullptr, 0, stream_of(*q));
+    }
     if (st == KB_ERR_BAD_ARG) Py_RETURN_NONE;  // a layout that needs scratch, which the general path allocates
     if (st != KB_OK) return failed("skinny_attention_forward", st);
     Py_INCREF(a[3]);
@@ -298,10 +322,7 @@ PyObject* rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
         if (pos == nullptr || pos->scalar_type() != at::kLong || pos->numel() != 1 || pos->device() != qkv.device()) Py_RETURN_NONE;
         p.pos_dev = pos->data_ptr<int64_t>();
     }
-    const c10::cuda::CUDAGuard guard(qkv.device());
-    at::Tensor q = empty({batch, seq, H, D}, qkv);
     p.qkv = qkv.data_ptr();
-    p.q_out = q.data_ptr();
     p.k_cache = kc.data_ptr();
     p.v_cache = vc.data_ptr();
     p.cos = cos.data_ptr<float>();
@@ -312,7 +333,15 @@ PyObject* rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
     p.D = D;
     p.max_seq = max_seq;
     p.dtype = dtype_code(qkv.scalar_type());
-    const int st = kb_rope_kv_write(&p, stream_of(qkv));
+    at::Tensor q;
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(qkv.device());
+        q = empty({batch, seq, H, D}, qkv);
+        p.q_out = q.data_ptr();
+        st = kb_rope_kv_write(&p, stream_of(qkv));
+    }
     if (st != KB_OK) return failed("rope_kv_write", st);
     return THPVariable_Wrap(std::move(q));
     END_HANDLE_TH_ERRORS
