@@ -831,7 +831,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 
     tc_fence_before();
     __syncthreads();
-    if (!skip && warp == 9) {
+    if (warp == 9) {  // (also when the work was skipped: tensor memory is allocated before that is known)
         __syncwarp();
         tmem_dealloc(*tmem_slot, kTmemCols);
     }

@@ -67,3 +67,45 @@ def test_expired_wait_sets_the_status_word_and_the_library_recovers(lib):
     assert _lib.device_status()[0] == 0
     want = (bufs[0].float() + bufs[1].float() + residual.float()).bfloat16()
     assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("kernel", ["gemm_single", "gemm_pair", "gemm_cluster", "attn_d128", "attn_split", "attn_persistent", "attn_short"])
+def test_kernels_with_waits_store_nothing_after_an_expiry(lib, kernel):
+    from kernl_b200 import _lib
+    from kernl_b200.implementations.attention import attention_forward
+    from kernl_b200.implementations.linear_layer import linear_layer
+
+    dev = torch.device("cuda", 0)
+    bufs = [torch.zeros(4096, dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    flags = [torch.zeros(64, dtype=torch.int32, device=dev) for _ in range(2)]
+    out = torch.zeros(4096, dtype=torch.bfloat16, device=dev)
+    if kernel.startswith("gemm"):
+        x, w = torch.randn((600, 256), device=dev).half(), torch.randn((512, 256), device=dev).half()
+        result = torch.full((600, 512), 7.0, dtype=torch.float16, device=dev)
+        call = lambda: linear_layer(x, w, None, "", out=result)
+    else:
+        q = torch.randn((2, 2, 300, 128 if kernel == "attn_d128" else 64), device=dev).half()
+        result = torch.full_like(q, 7.0)
+        call = lambda: attention_forward(q, q, q, result, 0.1)
+    hooks = {"gemm_single": [(lib.kb_debug_force_bn, 64, 0)], "gemm_pair": [(lib.kb_debug_linear_pair, 256, 1)],
+             "gemm_cluster": [(lib.kb_debug_force_splits, 2, 0)], "attn_persistent": [(lib.kb_debug_attention_persistent, 1, -1)],
+             "attn_short": [(lib.kb_debug_attention_short, 1, -1)], "attn_d128": [(lib.kb_debug_attention_short, 0, -1)],
+             "attn_split": [(lib.kb_debug_attention_short, 0, -1), (lib.kb_debug_attention_persistent, 0, -1)]}[kernel]
+    _lib.device_status()
+    for hook, on, _ in hooks:
+        hook(on)
+    try:
+        call()  # (the kernel's one-time set-up is not part of the test)
+        result.fill_(7.0)
+        assert lib.kb_debug_wait_limit(0, 20000) == 0
+        assert lib.kb_allreduce_residual_fwd(_params(bufs, flags, out, out), _lib.current_stream(dev)) == 0
+        call()
+        with pytest.raises(RuntimeError, match="wait expired"):
+            _lib.device_status()
+        assert bool((result == 7.0).all())
+        call()
+        assert _lib.device_status()[0] == 0 and not bool((result == 7.0).all())
+    finally:
+        assert lib.kb_debug_wait_limit(0, 0) == 0
+        for hook, _, off in hooks:
+            hook(off)
