@@ -211,9 +211,11 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     // A wait that expired in an earlier launch leaves the status word set: such a launch does no
     // work. The word is read here and looked at after the set-up barrier, so that its latency
     // overlaps the set-up instead of preceding it.
+    // One thread reads it, the one that issues the first loads: two that read it at different times may differ, and a
+    // CTA must not leave with copies in flight.
     __shared__ int s_skip;
     int status_early = 0;
-    if (threadIdx.x == 0 || threadIdx.x == 8 * 32) status_early = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+    if (threadIdx.x == 8 * 32) status_early = *reinterpret_cast<volatile int*>(&g_device_status[0]);
 
     const int BH = p.B * p.H;
     const int num_n_blocks = (p.N + kBlkN - 1) / kBlkN;
@@ -302,10 +304,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             if (lane == 2) mbar_init(o_final, 1);
             if (lane == 3) mbar_init(o_free, 8);
             if (lane >= 4 && lane < 8) mbar_init(ep_bar(lane - 4), 2);
-            if (lane == 0) {
-                *abort_flag = 0;
-                s_skip = status_early;
-            }
+            if (lane == 0) *abort_flag = 0;
             fence_mbar_init();
         } else if (warp == 9) {
             tmem_alloc(smem_u32(tmem_slot), kTmemCols);
@@ -455,7 +454,10 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             mbar_arrive(item_full(0));
         }
     }
-    if (!(MODE == 1 && sort_batches) && warp == 8 && lane == 0) *setup_issued = first_kv;
+    if (warp == 8 && lane == 0) {
+        s_skip = status_early;
+        if (!(MODE == 1 && sort_batches)) *setup_issued = first_kv;
+    }
 #ifdef KB_ATTN_TRACE
     if (threadIdx.x == 0) KB_TRACE(kTraceTiles, 4, trace_now());
 #endif
