@@ -833,7 +833,13 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 
     tc_fence_before();
     __syncthreads();
-    if (warp == 9) {  // (also when the work was skipped: tensor memory is allocated before that is known)
+    // Tensor memory is allocated before it is known whether the work is skipped. (Freed in two places: with one branch for
+    // both ways the compiler arranges the key loop otherwise, 20.1 -> 20.8 us at [8, 12, 512, 64] with padding.)
+    if (!skip && warp == 9) {
+        __syncwarp();
+        tmem_dealloc(*tmem_slot, kTmemCols);
+    }
+    if (skip && warp == 9) {
         __syncwarp();
         tmem_dealloc(*tmem_slot, kTmemCols);
     }
