@@ -191,8 +191,9 @@ def current_stream(device: torch.device) -> int:
 
 def device_status() -> list:
     """Synchronise the device and return (and clear) the kernels' status word; raises when a
-    bounded device-side wait expired. Kernels launched between the expiry and this call did no
-    work, so call it at every point where results leave the GPU (end of a generation loop, after
+    bounded device-side wait expired. Kernels that have such waits (the tcgen05 GEMMs, fused attention) and
+    were launched between the expiry and this call stored nothing; the others (norms, few-row linear, decode
+    attention, rotary) ran on what they found. So call it at every point where results leave the GPU (end of a generation loop, after
     replaying captured graphs, before closing peer buffers)."""
     out = (c_int32 * 4)()
     st = load().kb_device_status_read(out)

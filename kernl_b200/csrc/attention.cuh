@@ -270,12 +270,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // A wait that expired in an earlier CTA or launch leaves the status word set: do no work until
-    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA.
+    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA. What is read here may be
+    // too early (status_word()); the epilogue looks again before it stores.
+    __shared__ int s_expired;
     {
         __shared__ int s_skip;
-        if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+        if (threadIdx.x == 0) s_skip = status_word();
         __syncthreads();
-        if (s_skip != 0) return;
+        if (s_skip != 0) {
+            pdl_wait();
+            return;
+        }
     }
 
     // Work assignment: heavy (late) query tiles first so that causal work is balanced.
@@ -304,7 +309,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             mbar_init(s_full(t), 1);
             mbar_init(p_full(t, 0), 4);
             mbar_init(p_full(t, 1), 4);
-            mbar_init(o_final(t), 1);
+            mbar_init(o_final(t), 2);  // the last product, and the issuer itself, for s_expired
         }
         for (int s = 0; s < KVS; ++s) {
             mbar_init(k_full(s), 1);
@@ -393,6 +398,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     } else if (warp == 9) {
         // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
+            s_expired = status_word();
             constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kIsBf16, 128, 128, 0, 0);
             constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, D, 0, 1);
             bool ok = true;
@@ -463,6 +469,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         issue_qk(t, s1);
                         tc_commit(s_full(t));
                     } else {
+                        mbar_arrive(o_final(t));
                         tc_commit(o_final(t));
                     }
                 }
@@ -621,6 +628,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             // ---- epilogue: O / l -> global
             if (ok && mbar_wait(o_final(t), 0, abort_flag, 310 + t)) {
                 tc_fence_after();
+                const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
                 const float inv_l = 1.0f / l;
                 T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                            (int64_t)row * p.o_strides[2];
@@ -630,7 +638,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     uint32_t orr[32];
                     tmem_ld_32x32(o_addr + dch * 32, orr);
                     tmem_ld_wait();
-                    if (row < p.M) {
+                    if (row < m_end) {
                         float val[32];
 #pragma unroll
                         for (int i = 0; i < 32; ++i) val[i] = __uint_as_float(orr[i]) * inv_l;

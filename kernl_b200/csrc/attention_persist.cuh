@@ -210,12 +210,13 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #endif
     // A wait that expired in an earlier launch leaves the status word set: such a launch does no
     // work. The word is read here and looked at after the set-up barrier, so that its latency
-    // overlaps the set-up instead of preceding it.
+    // overlaps the set-up instead of preceding it. It may be too early (status_word()); every tile's
+    // epilogue looks again before it stores.
     // One thread reads it, the one that issues the first loads: two that read it at different times may differ, and a
     // CTA must not leave with copies in flight.
-    __shared__ int s_skip;
+    __shared__ int s_skip, s_expired;  // s_expired: read by the issuer behind pdl_wait()
     int status_early = 0;
-    if (threadIdx.x == 8 * 32) status_early = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+    if (threadIdx.x == 8 * 32) status_early = status_word();
 
     const int BH = p.B * p.H;
     const int num_n_blocks = (p.N + kBlkN - 1) / kBlkN;
@@ -236,15 +237,15 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     auto locate_sorted = [&](int idx, int& bh, int& mt) {
         if (!sort_batches) {
             locate(idx, bh, mt);
-            return;
+        } else {
+            // batch-major: all tiles of the longest batch, then of the next one, ...; inside a batch
+            // the heads of one query tile are neighbours (they share no K/V, but a batch's K/V of all
+            // heads is small next to L2)
+            const int per_batch = p.H * p.num_pairs;
+            const int r = idx / per_batch, rem = idx % per_batch;
+            mt = p.num_pairs - 1 - rem / p.H;
+            bh = batch_order[r] * p.H + rem % p.H;
         }
-        // batch-major: all tiles of the longest batch, then of the next one, ...; inside a batch
-        // the heads of one query tile are neighbours (they share no K/V, but a batch's K/V of all
-        // heads is small next to L2)
-        const int per_batch = p.H * p.num_pairs;
-        const int r = idx / per_batch, rem = idx % per_batch;
-        mt = p.num_pairs - 1 - rem / p.H;
-        bh = batch_order[r] * p.H + rem % p.H;
     };
     // The CTA's first tile is its block index: known without the queue, so its operands are
     // requested during set-up and its mask row is staged by all threads at once.
@@ -301,7 +302,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 mbar_init(p_full(lane), 8);
                 mbar_init(pv_done(lane), 1);
             }
-            if (lane == 2) mbar_init(o_final, 1);
+            if (lane == 2) mbar_init(o_final, 2);  // a tile's last product, and the issuer itself, for s_expired
             if (lane == 3) mbar_init(o_free, 8);
             if (lane >= 4 && lane < 8) mbar_init(ep_bar(lane - 4), 2);
             if (lane == 0) *abort_flag = 0;
@@ -588,6 +589,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
         } else if (warp == 9) {
             // -------------------------------------------------------------- tcgen05 issuer
             if (elect_one()) {
+                s_expired = status_word();
                 constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kIsBf16, 128, kBlkN, 0, 0);
                 constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, D, 0, 1);
                 constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
@@ -653,7 +655,10 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                         issue_pv(j);
                         tc_commit(pv_done((g + j) & 1));
                         if (j2 < nb) issue_qk(j2);  // into the slot that P_j has just been read from (in-order execution)
-                        if (j + 1 == nb) tc_commit(o_final);
+                        if (j + 1 == nb) {
+                            mbar_arrive(o_final);
+                            tc_commit(o_final);
+                        }
                         tc_commit(v_empty(kr % KVS));
                     }
                     g += nb;
@@ -799,6 +804,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             const uint32_t tph = (uint32_t)(it & 1);
             if (!(mbar_wait(ep_bar(q), tph, abort_flag, 733) && mbar_wait(o_final, tph, abort_flag, 734))) { ok = false; break; }
             tc_fence_after();
+            const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
             const float2 other = xrow[(hf ^ 1) * kAttnBlock + r_in_tile];
             float m_all = fmaxf(m_own, other.x);
             if (m_all == -INFINITY) m_all = 0.f;
@@ -817,7 +823,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                        (int64_t)row * p.o_strides[2];
             const bool vec = p.o_strides[3] == 1 && ((((uintptr_t)o_row) & 15) == 0);
-            if (row < p.M) {
+            if (row < m_end) {
                 float val[32];
 #pragma unroll
                 for (int i = 0; i < 32; ++i) val[i] = fmaf(__uint_as_float(oa[i]), wa, __uint_as_float(ob[i]) * wb);

@@ -86,7 +86,7 @@ attention_short_kernel(const AttnShortDev s) {
     pdl_wait();
     if (s.trigger_early) pdl_launch_dependents();
     // set by a wait that expired in an earlier launch: nothing is stored then (looked at in the end, off the path of the loads)
-    const int skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+    const int skip = status_word();
     load_rows(q_s, qp, s.q_strides[2], row0, p.M);
     asm volatile("cp.async.commit_group;" ::: "memory");
     uint32_t act[4] = {0u, 0u, 0u, 0u};

@@ -166,12 +166,16 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const bool mask_async = Cfg::kMaskRing && p.mask_async;
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ int s_expired[TILES];  // a tile's issuer reads the status word behind pdl_wait()
     {
         __shared__ int s_skip;
-        if (threadIdx.x == 0) s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+        if (threadIdx.x == 0) s_skip = status_word();  // (the epilogue looks again before it stores)
         if (MODE == 1 && threadIdx.x < 4) act_bits[threadIdx.x] = 0u;
         __syncthreads();
-        if (s_skip != 0) return;
+        if (s_skip != 0) {
+            pdl_wait();
+            return;
+        }
     }
 
     const int BH = p.B * p.H;
@@ -239,7 +243,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             }
         }
     } else if (warp == 0) {
-        if (lane < 2) mbar_init(o_final(lane), 1);
+        if (lane < 2) mbar_init(o_final(lane), 2);  // the last product, and the issuer itself, for s_expired
         if (lane < 4) {
             mbar_init(p_full(lane >> 1, lane & 1), 8);
             mbar_init(s_full(lane >> 1, lane & 1), 1);
@@ -331,6 +335,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // ------------------------------------------------------------------ MMA issuers, one per tile
         const int t = warp - (W0 + 1);
         if (elect_one()) {
+            s_expired[t] = status_word();
             constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kIsBf16, 128, kBlkN, 0, 0);
             constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, D, 0, 1);
             constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
@@ -392,7 +397,10 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         issue_qk(j2);  // into the slot that P_j has just been read from (in-order execution)
                         tc_commit(s_full(t, j & 1));
                     }
-                    if (j + 1 == my_blk) tc_commit(o_final(t));
+                    if (j + 1 == my_blk) {
+                        mbar_arrive(o_final(t));
+                        tc_commit(o_final(t));
+                    }
                     tc_commit(v_empty(s));
                     if (j2 < max_blk) {
                         if (j2 < my_blk) tc_commit(k_empty(j2 % KVS));
@@ -586,6 +594,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             if (lane == 0) mbar_arrive(ep_bar(t, q));
             if (ok && mbar_wait(ep_bar(t, q), 0, abort_flag, 660 + t) && mbar_wait(o_final(t), 0, abort_flag, 670 + t)) {
                 tc_fence_after();
+                const int m_end = s_expired[t] == 0 ? p.M : 0;  // rows that may be stored
                 const float2 other = xch[(t * 2 + (hf ^ 1)) * kAttnBlock + r_in_tile];
                 float m_all = fmaxf(m_own, other.x);
                 if (m_all == -INFINITY) m_all = 0.f;
@@ -601,7 +610,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                            (int64_t)row * p.o_strides[2];
                 const bool vec = p.o_strides[3] == 1 && ((((uintptr_t)o_row) & 15) == 0);
-                if (row < p.M) {
+                if (row < m_end) {
                     float val[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) val[i] = fmaf(__uint_as_float(oa[i]), wa, __uint_as_float(ob[i]) * wb);

@@ -285,10 +285,11 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     // first tile's W is asked for in L2 (not read: it may be the output of the kernel ahead), while the
     // previous kernel of the stream drains; a GEMM of a latency-bound graph is itself only a few microseconds long.
     // A wait that expired in an earlier CTA or launch leaves the status word set: do no work until
-    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA.
-    __shared__ int s_skip;
+    // the host has read (and cleared) it, so that one failure cannot cost a second per CTA. What is read here may be
+    // too early (status_word()); the epilogue looks again before it stores.
+    __shared__ int s_skip, s_expired;
     if (threadIdx.x == 0) {
-        s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+        s_skip = status_word();
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
@@ -390,12 +391,16 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
+        if (threadIdx.x == 64) s_expired = status_word();
+        named_barrier(1, kGemmEpilogueWarps * 32);
+        const int m_end = s_expired == 0 ? M : 0;  // rows that may be stored
         for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
             int m_idx, n_idx;
             tile_coords(w, num_m, num_n, m_idx, n_idx);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 300)) { ok = false; break; }
             tc_fence_after();
             const int row = m_idx * kGemmBM + q * 32 + lane;
+            const bool row_ok = row < m_end;
             const int n0 = n_idx * BN;
             T* y_row = y + (int64_t)row * y_row_stride;
             T* a_row = act_inputs ? act_inputs + (int64_t)row * y_row_stride : nullptr;
@@ -409,8 +414,8 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 float accv[32];
 #pragma unroll
                 for (int j = 0; j < 32; ++j) accv[j] = __uint_as_float(r[j]);
-                if (activation == KB_ACT_SWIGLU) epilogue_chunk_swiglu<T>(accv, bias, y_row, col0, N, row < M);
-                else epilogue_chunk<T>(accv, bias, y_row, a_row, col0, N, row < M, activation);
+                if (activation == KB_ACT_SWIGLU) epilogue_chunk_swiglu<T>(accv, bias, y_row, col0, N, row_ok);
+                else epilogue_chunk<T>(accv, bias, y_row, a_row, col0, N, row_ok, activation);
             }
             tc_fence_before();
             __syncwarp();

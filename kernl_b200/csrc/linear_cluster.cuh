@@ -91,7 +91,7 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     pdl_launch_dependents();
     // set by a wait that expired in an earlier launch: nothing is stored then (looked at in the end, so that the
     // CTAs of a cluster, which may read it at different times, take the same way through its barriers)
-    const int skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+    const int skip = status_word();
 
     if (warp == 0) {
         if (elect_one()) {

@@ -168,11 +168,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
     // A wait that expired earlier leaves the status word set: such a launch does no work. Both CTAs
     // of a pair must take the same decision (they allocate tensor memory together), so the leader's
-    // reading counts for both: it is exchanged through the cluster barrier below.
-    __shared__ int s_skip;
+    // reading counts for both: it is exchanged through the cluster barrier below. It may be too early
+    // (status_word()); the epilogue looks again before it stores.
+    __shared__ int s_skip, s_expired;
     if (threadIdx.x == 0) {
         KB_GTRACE(0, 7);
-        s_skip = *reinterpret_cast<volatile int*>(&g_device_status[0]);
+        s_skip = status_word();
         for (int s = 0; s < STAGES; ++s) {
             mbar_init(full_bar(s), 1);
             mbar_init(empty_bar(s), 1);
@@ -305,6 +306,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
             return b2;
         };
         if (staged) reinterpret_cast<float2*>(bias_s)[lane] = load_bias(pair);
+        if (threadIdx.x == 64) s_expired = status_word();
+        named_barrier(1, kPairEpilogueWarps * 32);
+        const int m_end = s_expired == 0 ? M : 0;  // rows that may be stored
         for (int t = pair; t < num_tiles && ok; t += num_pairs, ++ti) {
             int m_idx, n_idx;
             tile_coords(t, num_m, num_n, m_idx, n_idx);
@@ -378,7 +382,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         const int rr = it * kRowsPerStore + lane / kPieces, pc = lane % kPieces;
                         const uint4 o = *reinterpret_cast<const uint4*>(mine + pair_stage_offset(rr, pc));
                         const int grow = row_base + rr, gcol = n0 + pc0 + pc * 8;
-                        if (grow < M && gcol < N) *reinterpret_cast<uint4*>(y + (int64_t)grow * y_row_stride + gcol) = o;
+                        if (grow < m_end && gcol < N) *reinterpret_cast<uint4*>(y + (int64_t)grow * y_row_stride + gcol) = o;
                     }
                     if (warp == 2 && lane == 0 && ps == 0) KB_GTRACE(ti, 6);
                     __syncwarp();
@@ -399,8 +403,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     float accv[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) accv[j] = __uint_as_float(r[j]);
-                    if (activation == KB_ACT_SWIGLU) epilogue_chunk_swiglu<T>(accv, bias, y_row, n0 + c0, N, row < M);
-                    else epilogue_chunk<T>(accv, bias, y_row, a_row, n0 + c0, N, row < M, activation);
+                    if (activation == KB_ACT_SWIGLU) epilogue_chunk_swiglu<T>(accv, bias, y_row, n0 + c0, N, row < m_end);
+                    else epilogue_chunk<T>(accv, bias, y_row, a_row, n0 + c0, N, row < m_end, activation);
                 }
                 tc_fence_before();
                 __syncwarp();

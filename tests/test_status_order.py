@@ -1,6 +1,9 @@
 """Kernels that are launched programmatically and wait on the device: how they read the status word.
 
-It cannot be shown on a GPU without a wait that runs out inside a kernel in flight, so it is read from the source.
+Such a kernel may set itself up while the kernel ahead of it still runs, and a wait of that one may yet expire. So it has to
+read the status word behind pdl_wait() before it stores, and must not return ahead of pdl_wait(): the kernel behind
+it would find it complete while the kernel ahead is not. Neither can be shown on a GPU without a wait that runs
+out inside a kernel in flight, so the order is read from the source.
 """
 import os
 import re
@@ -36,6 +39,19 @@ WAITING = sorted(k for k, body in KERNELS.items() if "mbar_wait(" in body and "p
 def test_the_kernels_are_found():
     assert {"linear_tc_kernel", "linear_pair_kernel", "linear_cluster_kernel", "attention_tc_kernel", "attention_split_kernel",
             "attention_persist_kernel"} <= set(WAITING)
+
+
+@pytest.mark.parametrize("kernel", WAITING)
+def test_status_is_read_behind_the_wait_for_the_kernel_ahead(kernel):
+    body = KERNELS[kernel]
+    wait = body.rindex("pdl_wait();")
+    assert re.search(r"status_word\(\)|g_device_status", body[wait:]), "the status word is read ahead of pdl_wait() only"
+
+
+@pytest.mark.parametrize("kernel", sorted(k for k, body in KERNELS.items() if "pdl_wait()" in body))
+def test_no_return_ahead_of_the_wait_for_the_kernel_ahead(kernel):
+    body = KERNELS[kernel]
+    assert "return;" not in body[: body.index("pdl_wait();")]
 
 
 @pytest.mark.parametrize("kernel", WAITING)
