@@ -78,6 +78,28 @@ struct AttnSplitCfgT {
 
 using AttnSplitCfg = AttnSplitCfgT<2>;
 
+// A staged mask row begins at byte `lead` of its nine chunks, where `lead` is its address modulo 16, so that every
+// aligned chunk of global memory is a chunk here. How much of chunk `c` belongs to the row, from the chunk's first byte on,
+// for a row of `len` bytes (an even number, at most 128). What a chunk holds ahead of its row is not looked at.
+__host__ __device__ constexpr int mask_chunk_bytes(int lead, int c, int len) {
+    const int n = lead + len - 16 * c;
+    return n < 0 ? 0 : n < 16 ? n : 16;
+}
+constexpr bool mask_chunks_cover_a_row() {
+    for (int lead = 0; lead < 16; lead += 2)
+        for (int len = 2; len <= 2 * kBlkN; len += 2) {
+            int end = 0;
+            for (int c = 0; c < 9; ++c) {
+                const int n = mask_chunk_bytes(lead, c, len);
+                if (n > 0 && (end != 16 * c || n > 16)) return false;
+                if (n > 0) end = 16 * c + n;
+            }
+            if (end != lead + len) return false;
+        }
+    return true;
+}
+static_assert(mask_chunks_cover_a_row(), "the chunks of a staged mask row end with the row");
+
 // Adds sixteen mask values of a staged row to scores, in score units: s += max(mask, lowest) * inv_scale, two
 // values per instruction. `src` is the 16-byte chunk in which the row's 32 bytes begin, `shift` (0..7
 // elements) where in it: rows of a mask whose length is no multiple of eight all start differently.
@@ -118,7 +140,8 @@ __device__ __forceinline__ void add_staged_mask(const AttnDev& p, const uint8_t*
     }
 }
 
-template <typename T, int MODE, int TILES>
+// EDGE (MODE 2): the mask begins or ends inside a 16-byte chunk, and copies of whole chunks would read outside it.
+template <typename T, int MODE, int TILES, bool EDGE = false>
 __global__ void __launch_bounds__(SplitShape<TILES>::kThreads, TILES == 2 ? 1 : 2)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, const AttnDev p) {
@@ -251,7 +274,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         }
         if (lane < 8) mbar_init(ep_bar(lane >> 2, lane & 3), 2);
         if (Cfg::kMaskRing && lane < 2) {
-            mbar_init(m_full(lane), 64);  // the threads of the two loader warps
+            mbar_init(m_full(lane), EDGE ? 128 : 64);  // the threads of the two loader warps: their copies (and their own stores)
             mbar_init(m_empty(lane), 8);
         }
         if (lane == 0) *abort_flag = 0;
@@ -416,7 +439,11 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // ------------------------------------------------------------------ mask loaders (two warps)
         // Eight threads in a row read neighbouring chunks of one mask row. (Every softmax thread fetching its own
         // row touched 32 cache lines per instruction: a block with a mask took twice as long as one without.)
-        // Thread (r0, ch) of 7 x 9 takes chunk ch of rows r0, r0 + 7, ...: pointers advance by a constant.
+        // Thread (r0, ch) of 7 x 9 takes chunk ch of rows r0, r0 + 7, ...: pointers advance by a constant. Nothing outside
+        // the mask, from its first value to its last, is read: whole chunks lie inside it where it begins and ends with
+        // one, and else (EDGE) a copy ends with its row and the chunk in which the mask begins is taken value by value.
+        // (EDGE costs 3 to 8 %: 12.2 -> 12.6 us at [3, 12, 333, 64], 30.2 -> 32.0 at [8, 12, 512, 64]. Rows read byte for
+        // byte, with their heads word by word, took 15.7 and 31.0.)
         const int lt = (int)threadIdx.x - (W0 + 2) * 32;
         const int r0 = lt / 9, ch = lt % 9;
         const int rows = lt < 63 ? min(kAttnBlock, p.M - mt[0] * kAttnBlock) : 0;
@@ -429,15 +456,40 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             const uint32_t dst = dst0 + (uint32_t)((j & 1) * Cfg::kMaskSlotBytes);
             const uint8_t* first = base + j * (kBlkN * 2);
             const int bytes = 2 * min(kBlkN, p.N - j * kBlkN) - ch * 16;  // of the row, from chunk ch of an aligned row on
+            if (!EDGE) {
 #pragma unroll
-            for (int it = 0; it < (kAttnBlock + 6) / 7; ++it) {
-                const uint32_t lead = (uint32_t)(uintptr_t)first & 15u;
-                // a chunk is fetched if it holds a value of the row; what else it holds is not looked at
-                if (it * 7 + r0 < rows && (int)(0u - lead) < bytes)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(it * 7 * Cfg::kMaskRowBytes)), "l"(first - lead + ch * 16) : "memory");
-                first += step;
+                for (int it = 0; it < (kAttnBlock + 6) / 7; ++it) {
+                    const uint32_t lead = (uint32_t)(uintptr_t)first & 15u;
+                    // a chunk is fetched if it holds a value of the row; what else it holds is not looked at
+                    if (it * 7 + r0 < rows && (int)(0u - lead) < bytes)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (uint32_t)(it * 7 * Cfg::kMaskRowBytes)), "l"(first - lead + ch * 16) : "memory");
+                    first += step;
+                }
+            } else if (j > 0 || p.mask_lead == 0) {
+                const int len = 2 * min(kBlkN, p.N - j * kBlkN);
+#pragma unroll
+                for (int it = 0; it < (kAttnBlock + 6) / 7; ++it) {
+                    const int lead = (int)((uintptr_t)first & 15u), n = mask_chunk_bytes(lead, ch, len);
+                    if (it * 7 + r0 < rows && n > 0)
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst + (uint32_t)(it * 7 * Cfg::kMaskRowBytes)), "l"(first - lead + ch * 16), "r"(n) : "memory");
+                    first += step;
+                }
+            } else {
+                // rows that begin in the same chunk as the mask itself: value by value up to the next one
+                const int len = 2 * min(kBlkN, p.N);
+#pragma unroll 1
+                for (int r = r0; r < rows; r += 7, first += step) {
+                    const int lead = (int)((uintptr_t)first & 15u), n = mask_chunk_bytes(lead, ch, len);
+                    const uint32_t to = dst + (uint32_t)((r - r0) * Cfg::kMaskRowBytes);
+                    if (n > 0 && first - lead + ch * 16 >= reinterpret_cast<const uint8_t*>(p.mask))
+                        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to), "l"(first - lead + ch * 16), "r"(n) : "memory");
+                    else
+                        for (int e = lead; e < n; e += 2)
+                            asm volatile("st.shared.u16 [%0], %1;" ::"r"(to + (uint32_t)e), "h"(__ldg(reinterpret_cast<const uint16_t*>(first - lead + e))) : "memory");
+                }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(m_full(j & 1)) : "memory");
+            if (EDGE) mbar_arrive(m_full(j & 1));  // for the values that the thread has stored itself
         }
         asm volatile("cp.async.wait_all;" ::: "memory");
       }
@@ -629,7 +681,18 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
 }
 
-template <typename T, int MODE, int TILES>
+// Whether the rows of a per-row mask are staged: 16-bit values side by side, the first one at the lowest address.
+static bool mask_is_staged(const kb_attn_params& p) {
+    return p.mask != nullptr && p.mask_dtype != KB_F32 && p.mask_strides[3] == 1 && p.sm_scale > 0.f && p.mask_strides[0] >= 0 &&
+           p.mask_strides[1] >= 0 && p.mask_strides[2] >= 0;
+}
+// Whether a mask whose rows are staged begins or ends inside a 16-byte chunk.
+static bool mask_has_edges(const kb_attn_params& p) {
+    const int64_t last = (p.B - 1) * p.mask_strides[0] + (p.H - 1) * p.mask_strides[1] + (p.M - 1) * p.mask_strides[2] + p.N;  // values from the first on
+    return ((((uintptr_t)p.mask) | ((uintptr_t)p.mask + 2 * (uintptr_t)last)) & 15) != 0;
+}
+
+template <typename T, int MODE, int TILES, bool EDGE = false>
 static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stream) {
     using Cfg = AttnSplitCfgT<TILES, MODE>;
     using Shape = SplitShape<TILES>;
@@ -668,7 +731,8 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
         const int64_t per16 = (p.mask_dtype == KB_F32) ? 4 : 8;
         d.mask_vec = (p.mask_strides[0] % per16 == 0 && p.mask_strides[1] % per16 == 0 && p.mask_strides[2] % per16 == 0) ? 1 : 0;
     }
-    d.mask_async = p.mask != nullptr && p.mask_dtype != KB_F32 && p.mask_strides[3] == 1 && p.sm_scale > 0.f ? 1 : 0;
+    d.mask_async = MODE == 2 && mask_is_staged(p) ? 1 : 0;
+    d.mask_lead = p.mask != nullptr ? (int)((uintptr_t)p.mask & 15) : 0;
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
     d.num_pairs = (num_m_tiles + TILES - 1) / TILES;  // work items per (batch, head): tile pairs, or tiles
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
@@ -679,20 +743,20 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
         // setmaxnreg.inc blocks until the CTA's pool holds the registers: refuse to launch a build
         // whose launch allocation is smaller than the redistribution assumes.
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, attention_split_kernel<T, MODE, TILES>) != cudaSuccess) return KB_ERR_LAUNCH;
+        if (cudaFuncGetAttributes(&fa, attention_split_kernel<T, MODE, TILES, EDGE>) != cudaSuccess) return KB_ERR_LAUNCH;
         regs_ok = (fa.numRegs < Shape::kRegsLaunch) ? -1 : 1;
     }
     if (regs_ok < 0) return KB_ERR_UNSUPPORTED;
     static PerDeviceOnce attr_once;
     if (!attr_once.run([] {
-            return cudaFuncSetAttribute(attention_split_kernel<T, MODE, TILES>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemMax) == cudaSuccess;
+            return cudaFuncSetAttribute(attention_split_kernel<T, MODE, TILES, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemMax) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     const int num_n_blocks = (int)((p.N + kBlkN - 1) / kBlkN);
     const size_t smem_bytes = (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)num_n_blocks * kBlkN * 4 : 0);
-    if (launch_pdl(attention_split_kernel<T, MODE, TILES>, (unsigned)grid, (unsigned)Shape::kThreads, smem_bytes, stream, tq,
+    if (launch_pdl(attention_split_kernel<T, MODE, TILES, EDGE>, (unsigned)grid, (unsigned)Shape::kThreads, smem_bytes, stream, tq,
                    tk, tv, d) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
@@ -705,6 +769,9 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
 template <typename T, int MODE>
 static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t stream) {
     if (g_split_tiles == 2) return launch_attention_split_tmt<T, MODE, 2>(p, stream);
+    if constexpr (MODE == 2) {
+        if (mask_is_staged(p) && mask_has_edges(p)) return launch_attention_split_tmt<T, MODE, 1, true>(p, stream);
+    }
     return launch_attention_split_tmt<T, MODE, 1>(p, stream);
 }
 

@@ -1,0 +1,33 @@
+"""Per-row masks at head dimension 64, staged row by row: where a row starts and ends in its 16-byte chunks."""
+import pytest
+import torch
+
+from oracle import kernl_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("shift", range(8))
+@pytest.mark.parametrize("M, N, gap", [(130, 333, 0), (128, 64, 8), (9, 65, 3), (257, 455, 1)])
+def test_staged_mask_rows(lib, dtype, shift, M, N, gap):
+    """The mask is a view into a larger buffer that holds NaN everywhere else, `shift` elements off a 16-byte boundary
+    and with `gap` elements between its rows."""
+    from kernl_b200.implementations.attention import attention_forward
+
+    g = torch.Generator().manual_seed(M + shift)
+    H, row = 2, N + gap
+    q, k, v = (torch.randn((2, H, s, 64), generator=g).to(dtype) for s in (M, N, N))
+    buffer = torch.full((16 + H * M * row + 16,), float("nan"), dtype=dtype)
+    strides = (0, M * row, row, 1)
+    values = torch.randn((1, H, M, N), generator=g).to(dtype)
+    values[:, :, :, N // 2] = float("-inf")
+    buffer.as_strided((1, H, M, N), strides, 8 + shift).copy_(values)
+    on_gpu = buffer.cuda()
+    mask = on_gpu.as_strided((1, H, M, N), strides, 8 + shift)
+    lib.kb_debug_attention_short(0)
+    try:
+        out = attention_forward(q.cuda(), k.cuda(), v.cuda(), torch.empty_like(q, device="cuda"), 0.125, False, mask)
+    finally:
+        lib.kb_debug_attention_short(-1)
+    O.assert_parity(out, O.attention(q, k, v, 0.125, False, values), max_abs=1e-2 if dtype == torch.float16 else 3e-2, what="staged mask")
