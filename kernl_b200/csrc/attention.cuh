@@ -53,8 +53,7 @@ struct AttnDev {
     int is_causal;
     int mask_dtype;
     int mask_vec;   // mask rows can be read with aligned 128-bit loads
-    int mask_async; // MODE 2, head dimension 64: mask tiles are staged in shared memory (16-bit values, unit column stride)
-    int mask_lead;  // the mask's address modulo 16 (read where mask_async is set)
+    int mask_lead;  // the mask's address modulo 16 (head dimension 64, staged per-row masks)
     int num_pairs;  // ceil(ceil(M/128)/2)
     int head_group; // heads whose CTAs are interleaved (see attn_work_item)
     int kv_group;   // query heads per K/V head (grouped-query attention), >= 1

@@ -694,6 +694,10 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             const int b = bh / p.H, h = bh % p.H;
             const int row = mt * kAttnBlock + r_in_tile;
             const float* mask_row = mask_smem + slot * mask_cols;
+            const int64_t mask_row_off =
+                (MODE == 2 && p.mask != nullptr)
+                    ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)min(row, p.M - 1) * p.mask_strides[2]
+                    : 0;
             float m_ref = -INFINITY;
             float l = 0.f;
             int jb = (MODE == 1) ? bits_next(act, 0) : 0;  // key-block number of visit j
@@ -722,6 +726,23 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                         sr[v4 * 4 + 1] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 1]), c, a.y));
                         sr[v4 * 4 + 2] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 2]), c, a.z));
                         sr[v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 3]), c, a.w));
+                    }
+                } else if (MODE == 2) {
+                    if (p.mask == nullptr) {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) sr[i] = __float_as_uint(__uint_as_float(sr[i]) * c);
+                    } else {
+#pragma unroll
+                        for (int hc = 0; hc < 2; ++hc) {
+                            const int colc = col0 + hc * 16;
+                            float mvals[16];
+                            mask_values(p, mask_row_off, colc, mvals);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                uint32_t& sv = sr[hc * 16 + i];
+                                sv = __float_as_uint(fmaf(fmaxf(mvals[i], mlow), kLog2e, __uint_as_float(sv) * c));
+                            }
+                        }
                     }
                 }
                 const bool causal_edge = p.is_causal && col0 + 31 > mt * kAttnBlock;
@@ -863,6 +884,8 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
     }
 }
 
+// Masks that are not staged (MODE 2 of attention_split.cuh) are read by the softmax warps here too: [8, 12, 2048, 64] with an
+// fp32 bias 528 us, 641 with a CTA per tile; a row mask of 8256 keys at [2, 12] 1124 and 1301.
 // Whether the persistent kernel serves a call: a launch of more tiles than CTA slots (otherwise
 // every CTA would draw one tile and the queue buys nothing), and for row-broadcast masks a mask
 // row short enough for two of them to sit in shared memory next to two CTAs' tiles.
@@ -873,7 +896,7 @@ static int attention_persist_mask_cols(int64_t N) {  // one staged mask row: who
 
 static bool attention_persist_applicable(const kb_attn_params& p, int mode) {
     const int64_t tiles = ((p.M + kAttnBlock - 1) / kAttnBlock) * p.B * p.H;
-    if (g_attn_persistent == 0 || mode == 2) return false;  // per-row masks: attention_split.cuh stages them by tile
+    if (g_attn_persistent == 0 || mode == 3) return false;  // staged per-row masks: their ring takes the room of a second Q tile
     if (mode == 1 && (p.N > 8192 || attention_persist_mask_cols(p.N) > AttnPersistCfg::kMaskMaxCols)) return false;
     if (tiles > 0x3fffffff) return false;
     if (g_attn_persistent == 1) return true;

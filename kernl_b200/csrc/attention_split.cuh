@@ -55,10 +55,11 @@ __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c
 
 template <int TILES, int MODE = 0>
 struct AttnSplitCfgT {
-    // MODE 2, one tile: mask tiles of 128 rows x 64 keys through two slots of shared memory, for which the
+    // MODE 3: mask tiles of 128 rows x 64 keys through two slots of shared memory, for which the
     // K/V ring gives up a stage (two CTAs per SM). A row is staged as the nine 16-byte chunks that hold its
     // 128 bytes wherever they start.
-    static constexpr bool kMaskRing = MODE == 2 && TILES == 1;
+    static constexpr bool kMaskRing = MODE == 3;
+    static_assert(!kMaskRing || TILES == 1, "staged masks: one tile per CTA");
     static constexpr int kMaskRowBytes = 9 * 16;
     static constexpr int kMaskSlotBytes = kMaskRing ? kAttnBlock * kMaskRowBytes : 0;
     static constexpr int kKvStages = TILES == 2 ? 8 : kMaskRing ? 3 : 4;
@@ -68,7 +69,7 @@ struct AttnSplitCfgT {
     static constexpr int kBarBytes = 1024;
     static constexpr int kXchBytes = 2 * 2 * kAttnBlock * 8;  // [tile][half][row] (m, l)
     // MODE 1 keeps the whole row-broadcast mask of its (batch, head) in shared memory, as fp32 in the
-    // log2 domain, staged by all threads during set-up; longer rows take the general path (MODE 2)
+    // log2 domain, staged by all threads during set-up; longer rows are read like per-row masks (MODE 2)
     static constexpr int kMaskMaxN = 8192;
     static constexpr int kMaskLoads = (kMaskMaxN + SplitShape<TILES>::kThreads - 1) / SplitShape<TILES>::kThreads;  // per thread
     static constexpr int kSmemBase = kTilesBytes + kBarBytes + kXchBytes + 2 * kMaskSlotBytes + 1024;
@@ -140,7 +141,10 @@ __device__ __forceinline__ void add_staged_mask(const AttnDev& p, const uint8_t*
     }
 }
 
-// EDGE (MODE 2): the mask begins or ends inside a 16-byte chunk, and copies of whole chunks would read outside it.
+// MODE 0, 1: as in attention.cuh. MODE 2: no positive scale, or a mask of which every softmax thread reads its own row: 32-bit
+// values, values apart, rows of more than kMaskMaxN keys. MODE 3: per-row masks of 16-bit values side by side, staged by two
+// loader warps. (A kernel each: with both in one, the general masks shared the registers and the smaller K/V ring of the staged
+// ones. fp32 masks at [2, 12, 512, 64] 23.0 -> 16.8 us, staged ones at [8, 12, 512, 64] 31.0 -> 29.0.) EDGE (MODE 3): the mask begins or ends inside a 16-byte chunk, and copies of whole chunks would read outside it.
 template <typename T, int MODE, int TILES, bool EDGE = false>
 __global__ void __launch_bounds__(SplitShape<TILES>::kThreads, TILES == 2 ? 1 : 2)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -185,8 +189,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     uint32_t* act_bits = tmem_slot + 4;  // MODE 1: which key blocks have at least one unmasked key
     float2* xch = reinterpret_cast<float2*>(smem + Cfg::kTilesBytes + Cfg::kBarBytes);
     float* mask_smem = reinterpret_cast<float*>(smem + Cfg::kTilesBytes + Cfg::kBarBytes + Cfg::kXchBytes);  // MODE 1: [N rounded up to 64]
-    uint8_t* mask_ring = reinterpret_cast<uint8_t*>(mask_smem);  // MODE 2: two slots of kMaskSlotBytes
-    const bool mask_async = Cfg::kMaskRing && p.mask_async;
+    uint8_t* mask_ring = reinterpret_cast<uint8_t*>(mask_smem);  // MODE 3: two slots of kMaskSlotBytes
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     __shared__ int s_expired[TILES];  // a tile's issuer reads the status word behind pdl_wait()
@@ -435,15 +438,15 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 }
             }
         }
-      } else if (Cfg::kMaskRing && mask_async && warp >= W0 + 2) {
+      } else if (Cfg::kMaskRing && warp >= W0 + 2) {
         // ------------------------------------------------------------------ mask loaders (two warps)
         // Eight threads in a row read neighbouring chunks of one mask row. (Every softmax thread fetching its own
         // row touched 32 cache lines per instruction: a block with a mask took twice as long as one without.)
         // Thread (r0, ch) of 7 x 9 takes chunk ch of rows r0, r0 + 7, ...: pointers advance by a constant. Nothing outside
         // the mask, from its first value to its last, is read: whole chunks lie inside it where it begins and ends with
         // one, and else (EDGE) a copy ends with its row and the chunk in which the mask begins is taken value by value.
-        // (EDGE costs 3 to 8 %: 12.2 -> 12.6 us at [3, 12, 333, 64], 30.2 -> 32.0 at [8, 12, 512, 64]. Rows read byte for
-        // byte, with their heads word by word, took 15.7 and 31.0.)
+        // (EDGE copies are a little slower; rows read byte for byte, with their heads word by word, took 15.7 us at
+        // [3, 12, 333, 64] where EDGE takes 12.0.)
         const int lt = (int)threadIdx.x - (W0 + 2) * 32;
         const int r0 = lt / 9, ch = lt % 9;
         const int rows = lt < 63 ? min(kAttnBlock, p.M - mt[0] * kAttnBlock) : 0;
@@ -508,13 +511,13 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             const float c = p.scale_log2;
             const float mlow = mask_lowest(p.mask_dtype);
             const int64_t mask_row_off =
-                (MODE == 2 && p.mask != nullptr)
+                (MODE >= 2 && p.mask != nullptr)
                     ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)min(row, p.M - 1) * p.mask_strides[2]
                     : 0;
             // where this row starts in its staged chunks, in elements
             const int mask_shift = (int)(((uintptr_t)p.mask + 2 * (uintptr_t)mask_row_off) >> 1) & 7;
             // MODE 0 and staged masks: scores stay in their own units, the exponent is (s - m) * c; else log2 domain
-            const float unit = (MODE == 0 || mask_async) ? c : 1.0f;
+            const float unit = (MODE == 0 || MODE == 3) ? c : 1.0f;
             const float inv_scale = kLog2e / c;
             float m_ref = -INFINITY;
             float l = 0.f;
@@ -541,15 +544,15 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         sr[v4 * 4 + 2] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 2]), c, a.z));
                         sr[v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[v4 * 4 + 3]), c, a.w));
                     }
+                } else if (MODE == 3) {
+                    if (!mbar_wait(m_full(bf), ph, abort_flag, 641)) { ok = false; break; }
+                    const uint8_t* src = mask_ring + bf * Cfg::kMaskSlotBytes + r_in_tile * Cfg::kMaskRowBytes + hf * 64;
+                    add_staged_mask(p, src, mask_shift, inv_scale, sr);
+                    add_staged_mask(p, src + 32, mask_shift, inv_scale, sr + 16);
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(m_empty(bf));
                 } else if (MODE == 2) {
-                    if (mask_async) {
-                        if (!mbar_wait(m_full(bf), ph, abort_flag, 641)) { ok = false; break; }
-                        const uint8_t* src = mask_ring + bf * Cfg::kMaskSlotBytes + r_in_tile * Cfg::kMaskRowBytes + hf * 64;
-                        add_staged_mask(p, src, mask_shift, inv_scale, sr);
-                        add_staged_mask(p, src + 32, mask_shift, inv_scale, sr + 16);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(m_empty(bf));
-                    } else if (p.mask == nullptr) {
+                    if (p.mask == nullptr) {
 #pragma unroll
                         for (int i = 0; i < 32; ++i) sr[i] = __float_as_uint(__uint_as_float(sr[i]) * c);
                     } else {
@@ -731,7 +734,6 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
         const int64_t per16 = (p.mask_dtype == KB_F32) ? 4 : 8;
         d.mask_vec = (p.mask_strides[0] % per16 == 0 && p.mask_strides[1] % per16 == 0 && p.mask_strides[2] % per16 == 0) ? 1 : 0;
     }
-    d.mask_async = MODE == 2 && mask_is_staged(p) ? 1 : 0;
     d.mask_lead = p.mask != nullptr ? (int)((uintptr_t)p.mask & 15) : 0;
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
     d.num_pairs = (num_m_tiles + TILES - 1) / TILES;  // work items per (batch, head): tile pairs, or tiles
@@ -769,9 +771,6 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
 template <typename T, int MODE>
 static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t stream) {
     if (g_split_tiles == 2) return launch_attention_split_tmt<T, MODE, 2>(p, stream);
-    if constexpr (MODE == 2) {
-        if (mask_is_staged(p) && mask_has_edges(p)) return launch_attention_split_tmt<T, MODE, 1, true>(p, stream);
-    }
     return launch_attention_split_tmt<T, MODE, 1>(p, stream);
 }
 
@@ -783,14 +782,17 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
 template <typename T>
 static int launch_attention_split_t(const kb_attn_params& p, cudaStream_t stream) {
     const int mode = (p.mask == nullptr && p.sm_scale > 0.f) ? 0
-                     : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg::kMaskMaxN) ? 1 : 2;
+                     : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg::kMaskMaxN) ? 1
+                     : (g_split_tiles != 2 && p.mask_strides[2] != 0 && mask_is_staged(p)) ? 3 : 2;
     if (g_split_tiles == 0 && attention_persist_applicable(p, mode)) {
         if (mode == 0) return launch_attention_persist_tm<T, 0>(p, stream);
-        return launch_attention_persist_tm<T, 1>(p, stream);
+        if (mode == 1) return launch_attention_persist_tm<T, 1>(p, stream);
+        return launch_attention_persist_tm<T, 2>(p, stream);
     }
     if (mode == 0) return launch_attention_split_tm<T, 0>(p, stream);
     if (mode == 1) return launch_attention_split_tm<T, 1>(p, stream);
-    return launch_attention_split_tm<T, 2>(p, stream);
+    if (mode == 2) return launch_attention_split_tm<T, 2>(p, stream);
+    return mask_has_edges(p) ? launch_attention_split_tmt<T, 3, 1, true>(p, stream) : launch_attention_split_tmt<T, 3, 1>(p, stream);
 }
 
 static int launch_attention_split(const kb_attn_params& p, cudaStream_t stream) {

@@ -31,3 +31,34 @@ def test_staged_mask_rows(lib, dtype, shift, M, N, gap):
     finally:
         lib.kb_debug_attention_short(-1)
     O.assert_parity(out, O.attention(q, k, v, 0.125, False, values), max_abs=1e-2 if dtype == torch.float16 else 3e-2, what="staged mask")
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("kind, B, H, M, N", [("float32", 13, 12, 257, 130), ("apart", 13, 12, 257, 130), ("float32", 2, 3, 130, 333), ("apart", 2, 3, 130, 65),
+                                              ("negative", 13, 12, 257, 130), ("negative", 1, 2, 130, 200), ("row", 1, 2, 140, 8200), ("row32", 1, 2, 300, 8257)])
+@pytest.mark.parametrize("persistent", [-1, 0, 1])
+def test_masks_that_are_not_staged(lib, dtype, kind, B, H, M, N, persistent):
+    """32-bit values, values that are not side by side, a scale that is not positive, rows of more than 8192 keys: in launches of
+    few tiles and of many, with a CTA per tile and with CTAs that draw their tiles."""
+    from kernl_b200.implementations.attention import attention_forward
+
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn((B, H, s, 64), generator=g).to(dtype) for s in (M, N, N))
+    scale = -0.125 if kind == "negative" else 0.125
+    mask = None
+    if kind in ("float32", "apart"):
+        mask = torch.randn((1, H, M, 2 * N if kind == "apart" else N), generator=g).to(dtype if kind == "apart" else torch.float32)
+        mask[..., 7] = float("-inf")
+    elif kind != "negative":
+        mask = torch.where(torch.arange(N) < N - 300, 0.0, float("-inf")).reshape(1, 1, 1, N).to(torch.float32 if kind == "row32" else dtype)
+    on_gpu = mask.cuda() if mask is not None else None
+    if kind == "apart":
+        mask, on_gpu = mask[..., ::2], on_gpu[..., ::2]
+    lib.kb_debug_attention_short(0)
+    lib.kb_debug_attention_persistent(persistent)
+    try:
+        out = attention_forward(q.cuda(), k.cuda(), v.cuda(), torch.empty_like(q, device="cuda"), scale, False, on_gpu)
+    finally:
+        lib.kb_debug_attention_short(-1)
+        lib.kb_debug_attention_persistent(-1)
+    O.assert_parity(out, O.attention(q, k, v, scale, False, mask), max_abs=1e-2 if dtype == torch.float16 else 3e-2, what=kind)
