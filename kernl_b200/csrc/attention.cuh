@@ -118,6 +118,7 @@ struct AttnCfg {
     static constexpr int kTileBytes = kAttnBlock * D * 2;  // one Q tile / one K block / one V block
     static constexpr int kSmemBase = (2 + 2 * kKvStages) * kTileBytes + 512 + 1024;
     static constexpr int kMaskMaxN = 7168;  // MODE 1: the longest mask row that fits behind the tiles
+    static constexpr int kMaskRingBytes = 2 * 2 * kAttnBlock * 4;  // MODE 3
     static constexpr int kSmemMax = kSmemBase + kMaskMaxN * 4;
     static_assert(kSmemMax <= 227 * 1024 - 256, "shared memory of one CTA");
 };
@@ -233,7 +234,9 @@ __device__ __forceinline__ int bits_count_below(const uint32_t (&w)[4], int limi
 // MODE 1: additive mask that is the same for every query row (padding masks): all threads stage it in
 //         shared memory during set-up, already clamped, scaled by log2(e) and with -inf for columns
 //         beyond N, and key blocks that are masked throughout are not visited; MODE 2: anything else (per-row masks read from global memory with
-//         128-bit loads where the layout allows, non-positive scale).
+//         128-bit loads where the layout allows, non-positive scale); MODE 3: a row mask too long to be staged whole: the two
+//         idle warps keep two key blocks of it in shared memory, and every block is visited ([1, 16, 8192, 128] padded
+//         1265 us with every thread reading the row for itself).
 template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -260,11 +263,13 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     auto s_full = [&](int t) { return bar_base + 8u * (2 + 4 * KVS + t); };
     auto p_full = [&](int t, int half) { return bar_base + 8u * (8 + 4 * KVS + t * 2 + half); };  // keys [0, 64) / [64, 128) of P
     auto o_final = [&](int t) { return bar_base + 8u * (6 + 4 * KVS + t); };
-    constexpr int kNumBars = 12 + 4 * KVS;
+    auto m_full = [&](int t, int bf) { return bar_base + 8u * (12 + 4 * KVS + t * 2 + bf); };  // MODE 3
+    auto m_empty = [&](int t, int bf) { return bar_base + 8u * (16 + 4 * KVS + t * 2 + bf); };
+    constexpr int kNumBars = 20 + 4 * KVS;
     static_assert(kNumBars * 8 + 32 <= 512, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // MODE 1: [N rounded up to 128]
+    float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // MODE 1: [N rounded up to 128]; MODE 3: [tile][two blocks][128]
     uint32_t* act_bits = tmem_slot + 2;  // MODE 1: key blocks with an unmasked key
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -309,6 +314,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             mbar_init(s_full(t), 1);
             mbar_init(p_full(t, 0), 4);
             mbar_init(p_full(t, 1), 4);
+            for (int bf = 0; MODE == 3 && bf < 2; ++bf) {
+                mbar_init(m_full(t, bf), 2);  // the loader warps
+                mbar_init(m_empty(t, bf), 4);  // the tile's softmax warps
+            }
             mbar_init(o_final(t), 2);  // the last product, and the issuer itself, for s_expired
         }
         for (int s = 0; s < KVS; ++s) {
@@ -478,6 +487,28 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 if (j + 1 < visits) tc_commit(k_empty(s1));
             }
         }
+      } else if (MODE == 3) {
+        // ------------------------------------------------------------------ mask loaders (warps 10, 11)
+        const int li = (int)threadIdx.x - 320;  // 0 ... 63, two columns each
+        const float mlow = mask_lowest(p.mask_dtype);
+        const int64_t moff = (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1];
+        bool ok = true;
+        for (int j = 0; j < visits && ok; ++j) {
+            float a[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int col = j * kAttnBlock + li + e * 64;
+                a[e] = col < p.N ? fmaxf(mask_load(p.mask, moff + (int64_t)col * p.mask_strides[3], p.mask_dtype), mlow) * kLog2e : -INFINITY;
+            }
+            for (int t = 0; t < ntl && ok; ++t) {
+                if (j >= nblk[t]) continue;
+                if (!mbar_wait(m_empty(t, j & 1), (uint32_t)((j >> 1) & 1) ^ 1u, abort_flag, 400 + t)) { ok = false; break; }
+                mask_smem[(t * 2 + (j & 1)) * kAttnBlock + li] = a[0];
+                mask_smem[(t * 2 + (j & 1)) * kAttnBlock + li + 64] = a[1];
+                __syncwarp();
+                if (lane == 0) mbar_arrive(m_full(t, j & 1));
+            }
+        }
       }
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kAttnRegsHigh));
@@ -512,8 +543,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 
                 const int col0 = jb * kAttnBlock;
                 const bool causal_edge = p.is_causal && col0 + kAttnBlock - 1 > mt[t] * kAttnBlock;
-                if (MODE == 1) {
-                    const float4* ms = reinterpret_cast<const float4*>(mask_smem + col0);
+                if (MODE == 1 || MODE == 3) {
+                    if (MODE == 3 && !mbar_wait(m_full(t, j & 1), (uint32_t)((j >> 1) & 1), abort_flag, 320 + t)) { ok = false; break; }
+                    const float4* ms = reinterpret_cast<const float4*>(mask_smem + (MODE == 1 ? col0 : (t * 2 + (j & 1)) * kAttnBlock));
 #pragma unroll
                     for (int cch = 0; cch < 4; ++cch) {
 #pragma unroll
@@ -524,6 +556,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                             sr[cch][v4 * 4 + 2] = __float_as_uint(fmaf(__uint_as_float(sr[cch][v4 * 4 + 2]), c, a.z));
                             sr[cch][v4 * 4 + 3] = __float_as_uint(fmaf(__uint_as_float(sr[cch][v4 * 4 + 3]), c, a.w));
                         }
+                    }
+                    if (MODE == 3) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(m_empty(t, j & 1));
                     }
                 } else if (MODE == 2) {
                     if (p.mask == nullptr) {
@@ -546,8 +582,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         }
                     }
                 }
-                // columns beyond N (already -inf in MODE 1) and, on the diagonal block, above the diagonal
-                if ((MODE != 1 && col0 + kAttnBlock > p.N) || causal_edge) {
+                // columns beyond N (already -inf in MODE 1 and 3) and, on the diagonal block, above the diagonal
+                if ((MODE != 1 && MODE != 3 && col0 + kAttnBlock > p.N) || causal_edge) {
 #pragma unroll
                     for (int cch = 0; cch < 4; ++cch) {
 #pragma unroll
@@ -709,13 +745,13 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     static PerDeviceOnce attr_once;
     if (!attr_once.run([] {
             return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase) == cudaSuccess;
+                                        MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase + (MODE == 3 ? Cfg::kMaskRingBytes : 0)) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads,
-                   (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : 0), stream, tq, tk, tv, d) != cudaSuccess)
+                   (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : MODE == 3 ? Cfg::kMaskRingBytes : 0), stream, tq, tk, tv, d) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
@@ -723,7 +759,8 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
 template <typename T, int D>
 static int launch_attention_td(const kb_attn_params& p, cudaStream_t stream) {
     if (p.mask == nullptr && p.sm_scale > 0.f) return launch_attention_tdm<T, D, 0>(p, stream);
-    if (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnCfg<D>::kMaskMaxN) return launch_attention_tdm<T, D, 1>(p, stream);
+    if (p.mask != nullptr && p.mask_strides[2] == 0)
+        return p.N <= AttnCfg<D>::kMaskMaxN ? launch_attention_tdm<T, D, 1>(p, stream) : launch_attention_tdm<T, D, 3>(p, stream);
     return launch_attention_tdm<T, D, 2>(p, stream);
 }
 

@@ -62,3 +62,25 @@ def test_masks_that_are_not_staged(lib, dtype, kind, B, H, M, N, persistent):
         lib.kb_debug_attention_short(-1)
         lib.kb_debug_attention_persistent(-1)
     O.assert_parity(out, O.attention(q, k, v, scale, False, mask), max_abs=1e-2 if dtype == torch.float16 else 3e-2, what=kind)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B, M, N, D, causal, wide", [(2, 130, 7168, 128, False, False), (2, 130, 7169, 128, False, False), (2, 300, 7300, 80, False, True),
+                                                      (1, 20, 9000, 128, False, True), (1, 400, 7200, 128, True, False)])
+def test_long_row_masks_at_wide_heads(lib, dtype, B, M, N, D, causal, wide):
+    """Row masks up to what fits in shared memory and beyond, one tile and two per CTA, the last key block cut; a sequence
+    of which every key is masked."""
+    from kernl_b200.implementations.attention import attention_forward
+
+    g = torch.Generator().manual_seed(N)
+    q, k, v = (torch.randn((B, 2, s, D), generator=g).to(dtype) for s in (M, N, N))
+    live = torch.arange(N)[None, :] < torch.tensor([N - 200, 0])[:B, None]
+    mask = torch.where(live, torch.randn((B, N), generator=g), torch.tensor(float("-inf"))).reshape(B, 1, 1, N).to(torch.float16 if not wide else torch.float32)
+    if mask.dtype != torch.float16:
+        mask[B - 1, 0, 0, :9] = 0.0  # (the lowest 32-bit value leaves nothing of the scores it is added to)
+    lib.kb_debug_attention_short(0)
+    try:
+        out = attention_forward(q.cuda(), k.cuda(), v.cuda(), torch.empty_like(q, device="cuda"), D ** -0.5, causal, mask.cuda())
+    finally:
+        lib.kb_debug_attention_short(-1)
+    O.assert_parity(out, O.attention(q, k, v, D ** -0.5, causal, mask), max_abs=1e-2 if dtype == torch.float16 else 4e-2, what="long row mask")
