@@ -38,9 +38,11 @@ constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
 // and left twelve warps on an SM, all of them loading, then all computing, then all storing:
 // [16384, 4096] bf16 add + RMSNorm 120.9 us (4.4 TB/s), with four warps per row 89.2 us (6.0 TB/s).
 // Vector c of lane l of warp w covers columns ((c*WPR + w)*32 + l)*8 .. +8. cols must be a multiple of 8.
-// CHAIN (RMSNorm, many rows, four warps): the warps own consecutive parts of the row and pass each lane's sum of
-// squares on from warp to warp, so that the row is summed in the order of one warp walking it: a decoder's
-// hidden states, and with them its greedy tokens, do not depend on how many warps share a row. The hand-over is
+// CHAIN (RMSNorm of 1025 to 4096 columns, more than 1024 rows): the warps own consecutive parts of the row and pass each
+// lane's sum of squares on from warp to warp, so that the row is summed in the order of one warp walking it, the order a
+// decoder's prefill at these widths has always had: another one moves its hidden states by roundings, and near-ties of
+// its greedy tokens with them. Nothing more is promised: the same row in a launch of up to 1024 rows, longer rows
+// (eight warps) and LayerNorm add up their warps' sums pairwise. The hand-over is
 // hidden behind the other CTAs of the SM.
 template <typename T, int CHUNKS, bool RMS, int WPR = 1, bool CHAIN = false>
 __global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
