@@ -17,7 +17,8 @@ extern "C" {
 void kb_debug_force_bn(int bn);
 /* Force the number of CTAs that divide K (0 = heuristic, at most 16). */
 void kb_debug_force_splits(int splits);
-/* Query tiles per CTA of the head-dimension-64 attention kernel (0 = dispatcher's choice, 1, 2). */
+/* 1 = the head-dimension-64 attention kernel with a CTA per query tile, whatever the size of the launch;
+ * 0 = dispatcher's choice. */
 void kb_debug_split_tiles(int tiles);
 /* Work scheduling of the head-dimension-64 attention kernel: 1 = persistent CTAs that pull query
  * tiles from a device-side queue, 2 = the same without the longest-batch-first tile order,

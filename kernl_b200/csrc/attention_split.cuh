@@ -1,7 +1,7 @@
 // Fused attention forward for sm_100a, head dimension 64, "split-row" variant.
 //
-// Two 128-row query tiles per CTA, keys in blocks of 64, K/V through an 8-stage TMA ring, one
-// tcgen05 issuer warp per tile, and SIXTEEN softmax warps: every query row is shared by two
+// One 128-row query tile per CTA, two CTAs per SM, keys in blocks of 64, K/V through a 4-stage TMA
+// ring, one tcgen05 issuer warp, and EIGHT softmax warps: every query row is shared by two
 // threads of different warps, one owning key columns
 // [0,32) of each block, the other [32,64). The two halves never talk to each other inside the key
 // loop: each keeps its own running maximum and row sum, writes its own half of P, and its P·V goes
@@ -16,9 +16,11 @@
 // sub-partition. Clock stamps taken inside the kernel showed a block taking ~2200 cycles of which
 // the special-function unit was busy for 512. Four warps per sub-partition overlap those chains.
 //
-// Warps (640 threads): 0..7 tile 0 (0..3 first halves, 4..7 second halves), 8..15 tile 1,
-// 16 TMA producer, 17/18 tcgen05 issuers of tile 0/1, 19 mask loader (MODE 1).
-// TMEM columns per tile t (base 256·t): S ring slot s at 64·s (s = 0,1; 64 fp32 columns; P of the
+// Two independent CTAs on an SM also hide each other's fixed costs (set-up, first loads from DRAM, epilogue, exit), and
+// the second wave starts per tile: one CTA of two tiles that shares K/V was 2 % (B8 H12 S4096) to 20 % (B64 H12 S512) slower.
+//
+// Warps (384 threads): 0..7 softmax (0..3 first halves, 4..7 second halves), 8 TMA producer, 9 tcgen05 issuer, 10..11 mask
+// loaders (MODE 3). TMEM columns (256 of 512): S ring slot s at 64·s (s = 0,1; 64 fp32 columns; P of the
 // first half overwrites columns [0,16), P of the second half columns [32,48) of the same slot),
 // O_a at 128, O_b at 192.
 #pragma once
@@ -26,24 +28,16 @@
 
 namespace kb {
 
-// TILES = 2: the CTA described above (640 threads, all 512 TMEM columns, one CTA per SM). TILES = 1:
-// half of it (one query tile, 8 softmax warps + TMA + one issuer = 384 threads, 256 TMEM columns, a
-// 4-stage K/V ring), so that TWO CTAs share an SM. A launch that is only one or two waves of
-// two-tile CTAs spends a third of its time in per-CTA fixed costs (set-up, first loads from DRAM,
-// epilogue, exit) with the SM idle; with two independent CTAs per SM one CTA's fixed costs overlap
-// the other's key loop, and the second wave starts per tile, not per pair. Measured faster at every
-// launch size, so TILES = 1 is what the dispatcher picks; TILES = 2 loads K/V once for two tiles.
-template <int TILES>
 struct SplitShape {
-    static constexpr int kThreads = TILES * 256 + 128;
-    static constexpr int kAuxWarp = TILES * 8;  // first non-softmax warp: TMA producer; issuers follow
-    static constexpr int kRegsLaunch = TILES == 2 ? 96 : 80;  // 65536 / 640 and 65536 / (2 x 384), rounded down to 8
-    static constexpr int kRegsHigh = TILES == 2 ? 104 : 96;
-    static constexpr int kRegsLow = TILES == 2 ? 64 : 48;
-    static_assert(TILES * 2 * kRegsHigh + kRegsLow <= (TILES * 2 + 1) * kRegsLaunch, "setmaxnreg totals exceed the CTA's register pool");
+    static constexpr int kThreads = 384;
+    static constexpr int kAuxWarp = 8;  // first non-softmax warp: TMA producer; the issuer follows
+    static constexpr int kRegsLaunch = 80;  // 65536 / (2 x 384), rounded down to 8
+    static constexpr int kRegsHigh = 96;
+    static constexpr int kRegsLow = 48;
+    static_assert(2 * kRegsHigh + kRegsLow <= 3 * kRegsLaunch, "setmaxnreg totals exceed the CTA's register pool");
     static_assert(kRegsHigh % 8 == 0 && kRegsLow % 8 == 0, "setmaxnreg wants multiples of 8");
 };
-static int g_split_tiles = 0;  // test hook: 0 = by launch size, 1 / 2 = force the number of query tiles per CTA
+static int g_split_tiles = 0;  // test hook: 1 = this kernel whatever the size of the launch
 static int g_attn_persistent = -1;  // test hook: -1 = dispatcher's choice, 0 = one CTA per tile, 1 = persistent CTAs
 
 __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
@@ -53,31 +47,28 @@ __device__ __forceinline__ void tma_prefetch_l2_4d(const CUtensorMap* map, int c
                  : "memory");
 }
 
-template <int TILES, int MODE = 0>
-struct AttnSplitCfgT {
+template <int MODE>
+struct AttnSplitCfg {
     // MODE 3: mask tiles of 128 rows x 64 keys through two slots of shared memory, for which the
     // K/V ring gives up a stage (two CTAs per SM). A row is staged as the nine 16-byte chunks that hold its
     // 128 bytes wherever they start.
     static constexpr bool kMaskRing = MODE == 3;
-    static_assert(!kMaskRing || TILES == 1, "staged masks: one tile per CTA");
     static constexpr int kMaskRowBytes = 9 * 16;
     static constexpr int kMaskSlotBytes = kMaskRing ? kAttnBlock * kMaskRowBytes : 0;
-    static constexpr int kKvStages = TILES == 2 ? 8 : kMaskRing ? 3 : 4;
+    static constexpr int kKvStages = kMaskRing ? 3 : 4;
     static constexpr int kQTileBytes = kAttnBlock * 64 * 2;
     static constexpr int kKvBytes = kBlkN * 64 * 2;
-    static constexpr int kTilesBytes = TILES * kQTileBytes + 2 * kKvStages * kKvBytes;
+    static constexpr int kTilesBytes = kQTileBytes + 2 * kKvStages * kKvBytes;
     static constexpr int kBarBytes = 1024;
-    static constexpr int kXchBytes = 2 * 2 * kAttnBlock * 8;  // [tile][half][row] (m, l)
+    static constexpr int kXchBytes = 2 * kAttnBlock * 8;  // [half][row] (m, l)
     // MODE 1 keeps the whole row-broadcast mask of its (batch, head) in shared memory, as fp32 in the
     // log2 domain, staged by all threads during set-up; longer rows are read like per-row masks (MODE 2)
     static constexpr int kMaskMaxN = 8192;
-    static constexpr int kMaskLoads = (kMaskMaxN + SplitShape<TILES>::kThreads - 1) / SplitShape<TILES>::kThreads;  // per thread
+    static constexpr int kMaskLoads = (kMaskMaxN + SplitShape::kThreads - 1) / SplitShape::kThreads;  // per thread
     static constexpr int kSmemBase = kTilesBytes + kBarBytes + kXchBytes + 2 * kMaskSlotBytes + 1024;
     static constexpr int kSmemMax = kSmemBase + (MODE == 1 ? kMaskMaxN * 4 : 0);
     static_assert(!kMaskRing || 2 * (kSmemMax + 1024) <= 227 * 1024, "two CTAs per SM");
 };
-
-using AttnSplitCfg = AttnSplitCfgT<2>;
 
 // A staged mask row begins at byte `lead` of its nine chunks, where `lead` is its address modulo 16, so that every
 // aligned chunk of global memory is a chunk here. How much of chunk `c` belongs to the row, from the chunk's first byte on,
@@ -145,12 +136,12 @@ __device__ __forceinline__ void add_staged_mask(const AttnDev& p, const uint8_t*
 // values, values apart, rows of more than kMaskMaxN keys. MODE 3: per-row masks of 16-bit values side by side, staged by two
 // loader warps. (A kernel each: with both in one, the general masks shared the registers and the smaller K/V ring of the staged
 // ones. fp32 masks at [2, 12, 512, 64] 23.0 -> 16.8 us, staged ones at [8, 12, 512, 64] 31.0 -> 29.0.) EDGE (MODE 3): the mask begins or ends inside a 16-byte chunk, and copies of whole chunks would read outside it.
-template <typename T, int MODE, int TILES, bool EDGE = false>
-__global__ void __launch_bounds__(SplitShape<TILES>::kThreads, TILES == 2 ? 1 : 2)
+template <typename T, int MODE, bool EDGE = false>
+__global__ void __launch_bounds__(SplitShape::kThreads, 2)
 attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                        const __grid_constant__ CUtensorMap tmap_v, const AttnDev p) {
-    using Cfg = AttnSplitCfgT<TILES, MODE>;
-    using Shape = SplitShape<TILES>;
+    using Cfg = AttnSplitCfg<MODE>;
+    using Shape = SplitShape;
     constexpr int kThreads = Shape::kThreads;
     constexpr int W0 = Shape::kAuxWarp;
     constexpr int D = 64;
@@ -158,24 +149,22 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     constexpr int QTILE = Cfg::kQTileBytes;
     constexpr int KVB = Cfg::kKvBytes;
     constexpr int NB = 2;
-    constexpr uint32_t kTmemCols = TILES * 256;
+    constexpr uint32_t kTmemCols = 256;
 
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     const uint32_t q_smem = smem_u32(smem);
-    const uint32_t k_smem = q_smem + TILES * QTILE;
+    const uint32_t k_smem = q_smem + QTILE;
     const uint32_t v_smem = k_smem + KVS * KVB;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kTilesBytes);
     const uint32_t bar_base = smem_u32(bars);
-    // q_full[2] | o_final[2] | p_full, s_full, pv_done [2][2] each | ep[2][4] |
-    // k_full, k_empty, v_full, v_empty [KVS] each
-    auto q_full = [&](int t) { return bar_base + 8u * t; };
-    auto o_final = [&](int t) { return bar_base + 8u * (2 + t); };
-    auto p_full = [&](int t, int bf) { return bar_base + 8u * (4 + t * NB + bf); };
-    auto s_full = [&](int t, int bf) { return bar_base + 8u * (8 + t * NB + bf); };
-    auto pv_done = [&](int t, int bf) { return bar_base + 8u * (12 + t * NB + bf); };
-    auto ep_bar = [&](int t, int q) { return bar_base + 8u * (16 + t * 4 + q); };
-    constexpr int kKvBar = 24;
+    // q_full | o_final | p_full, s_full, pv_done [2] each | ep[4] | k_full, k_empty, v_full, v_empty [KVS] each | m_full, m_empty [2]
+    const uint32_t q_full = bar_base, o_final = bar_base + 8u;
+    auto p_full = [&](int bf) { return bar_base + 8u * (2 + bf); };
+    auto s_full = [&](int bf) { return bar_base + 8u * (4 + bf); };
+    auto pv_done = [&](int bf) { return bar_base + 8u * (6 + bf); };
+    auto ep_bar = [&](int q) { return bar_base + 8u * (8 + q); };
+    constexpr int kKvBar = 12;
     auto k_full = [&](int s) { return bar_base + 8u * (kKvBar + s); };
     auto k_empty = [&](int s) { return bar_base + 8u * (kKvBar + KVS + s); };
     auto v_full = [&](int s) { return bar_base + 8u * (kKvBar + 2 * KVS + s); };
@@ -192,7 +181,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     uint8_t* mask_ring = reinterpret_cast<uint8_t*>(mask_smem);  // MODE 3: two slots of kMaskSlotBytes
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    __shared__ int s_expired[TILES];  // a tile's issuer reads the status word behind pdl_wait()
+    __shared__ int s_expired;  // the issuer reads the status word behind pdl_wait()
     {
         __shared__ int s_skip;
         if (threadIdx.x == 0) s_skip = status_word();  // (the epilogue looks again before it stores)
@@ -205,24 +194,12 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     }
 
     const int BH = p.B * p.H;
-    int bh, pair;
-    attn_work_item(p, BH, bh, pair);
+    int bh, mt;  // (batch, head) and query tile
+    attn_work_item(p, BH, bh, mt);
     const int b = bh / p.H, h = bh % p.H;
     const int hk = h / p.kv_group;  // K/V head of this query head
-    const int num_m_tiles = (p.M + kAttnBlock - 1) / kAttnBlock;
     const int num_n_blocks = (p.N + kBlkN - 1) / kBlkN;
-    int mt[2], nblk[2];
-    int ntl = 0;
-    for (int t = 0; t < 2; ++t) {
-        mt[t] = pair * TILES + t;
-        if (t < TILES && mt[t] < num_m_tiles) {
-            ntl = t + 1;
-            nblk[t] = p.is_causal ? min(num_n_blocks, (mt[t] + 1) * (kAttnBlock / kBlkN)) : num_n_blocks;
-        } else {
-            nblk[t] = 0;
-        }
-    }
-    const int max_blk = max(nblk[0], nblk[1]);
+    const int max_blk = p.is_causal ? min(num_n_blocks, (mt + 1) * (kAttnBlock / kBlkN)) : num_n_blocks;
 
     // Set-up is spread over three warps so that the first loads are in flight as early as possible:
     // the TMA warp initialises the barriers its loads complete on and issues both Q tiles and the
@@ -236,28 +213,26 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             tma_prefetch_desc(&tmap_q);
             tma_prefetch_desc(&tmap_k);
             tma_prefetch_desc(&tmap_v);
-            for (int t = 0; t < 2; ++t) mbar_init(q_full(t), 1);
+            mbar_init(q_full, 1);
             for (int s = 0; s < KVS; ++s) {
                 mbar_init(k_full(s), 1);
-                mbar_init(k_empty(s), ntl);  // one arrival per live tile's issuer
+                mbar_init(k_empty(s), 1);
                 mbar_init(v_full(s), 1);
-                mbar_init(v_empty(s), ntl);
+                mbar_init(v_empty(s), 1);
             }
             fence_mbar_init();
             pdl_wait();  // q/k/v may be the output of the kernel before this one
-            for (int t = 0; t < ntl; ++t) {
-                mbar_arrive_expect_tx(q_full(t), QTILE);
-                tma_load_4d(q_smem + t * QTILE, &tmap_q, q_full(t), 0, mt[t] * kAttnBlock, h, b);
-                if (MODE == 1 && t == 0) {
-                    for (int j = 0; j < min(KVS, max_blk); ++j) {
-                        tma_prefetch_l2_4d(&tmap_k, 0, j * kBlkN, hk, b);
-                        tma_prefetch_l2_4d(&tmap_v, 0, j * kBlkN, hk, b);
-                    }
+            mbar_arrive_expect_tx(q_full, QTILE);
+            tma_load_4d(q_smem, &tmap_q, q_full, 0, mt * kAttnBlock, h, b);
+            if (MODE == 1) {
+                for (int j = 0; j < min(KVS, max_blk); ++j) {
+                    tma_prefetch_l2_4d(&tmap_k, 0, j * kBlkN, hk, b);
+                    tma_prefetch_l2_4d(&tmap_v, 0, j * kBlkN, hk, b);
                 }
-                if (t == 0 && first_kv > 0) {  // K_0 right behind the first Q tile: the first Q·Kᵀ needs just these two
-                    mbar_arrive_expect_tx(k_full(0), KVB);
-                    tma_load_4d(k_smem, &tmap_k, k_full(0), 0, 0, hk, b);
-                }
+            }
+            if (first_kv > 0) {  // K_0 right behind Q: the first Q·Kᵀ needs just these two
+                mbar_arrive_expect_tx(k_full(0), KVB);
+                tma_load_4d(k_smem, &tmap_k, k_full(0), 0, 0, hk, b);
             }
             for (int j = 0; j < first_kv; ++j) {
                 if (j > 0) {
@@ -269,13 +244,13 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             }
         }
     } else if (warp == 0) {
-        if (lane < 2) mbar_init(o_final(lane), 2);  // the last product, and the issuer itself, for s_expired
-        if (lane < 4) {
-            mbar_init(p_full(lane >> 1, lane & 1), 8);
-            mbar_init(s_full(lane >> 1, lane & 1), 1);
-            mbar_init(pv_done(lane >> 1, lane & 1), 1);
+        if (lane == 0) mbar_init(o_final, 2);  // the last product, and the issuer itself, for s_expired
+        if (lane < 2) {
+            mbar_init(p_full(lane), 8);
+            mbar_init(s_full(lane), 1);
+            mbar_init(pv_done(lane), 1);
         }
-        if (lane < 8) mbar_init(ep_bar(lane >> 2, lane & 3), 2);
+        if (lane < 4) mbar_init(ep_bar(lane), 2);
         if (Cfg::kMaskRing && lane < 2) {
             mbar_init(m_full(lane), EDGE ? 128 : 64);  // the threads of the two loader warps: their copies (and their own stores)
             mbar_init(m_empty(lane), 8);
@@ -319,7 +294,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     const uint32_t tmem_base = *tmem_slot;
     // the key blocks this CTA visits: all of them, or (MODE 1) those with an unmasked key
     uint32_t act[4] = {0u, 0u, 0u, 0u};
-    int n_union = max_blk, n_tile[2] = {nblk[0], nblk[1]};
+    int visits = max_blk;
     if (MODE == 1) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) act[i] = act_bits[i];
@@ -329,9 +304,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 #pragma unroll
             for (int i = 0; i < 4; ++i) act[i] = 0xffffffffu;
         }
-        n_union = bits_count_below(act, max_blk);
-        n_tile[0] = bits_count_below(act, nblk[0]);
-        n_tile[1] = bits_count_below(act, nblk[1]);
+        visits = bits_count_below(act, max_blk);
     }
     auto next_blk = [&](int from) { return MODE == 1 ? bits_next(act, from) : from; };
 
@@ -342,7 +315,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         if (elect_one()) {
             bool ok = true;
             int jb = next_blk(first_kv);
-            for (int i = first_kv; i < n_union && ok; ++i) {  // (MODE 0/2: the first ring was issued during set-up)
+            for (int i = first_kv; i < visits && ok; ++i) {  // (MODE 0/2: the first ring was issued during set-up)
                 const int s = i % KVS;
                 const uint32_t ph = (uint32_t)((i / KVS) & 1);
                 if (!mbar_wait(k_empty(s), ph ^ 1, abort_flag, 600)) { ok = false; break; }
@@ -357,22 +330,20 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 for (int i = 0; i < 64; ++i) __nanosleep(2000);
             }
         }
-      } else if (warp >= W0 + 1 && warp <= W0 + TILES) {
-        // ------------------------------------------------------------------ MMA issuers, one per tile
-        const int t = warp - (W0 + 1);
+      } else if (warp == W0 + 1) {
+        // ------------------------------------------------------------------ MMA issuer
         if (elect_one()) {
-            s_expired[t] = status_word();
+            s_expired = status_word();
             constexpr uint32_t idesc_qk = make_idesc_f16(Elem<T>::kIsBf16, 128, kBlkN, 0, 0);
             constexpr uint32_t idesc_pv = make_idesc_f16(Elem<T>::kIsBf16, 128, D, 0, 1);
             constexpr uint32_t desc_hi = (1024u >> 4) | (1u << 14) | (2u << 29);
-            const uint32_t q_lo = ((q_smem + t * QTILE) & 0x3FFFF) >> 4;
+            const uint32_t q_lo = (q_smem & 0x3FFFF) >> 4;
             const uint32_t k_lo = (k_smem & 0x3FFFF) >> 4;
             const uint32_t v_lo = (v_smem & 0x3FFFF) >> 4;
-            const uint32_t t_base = tmem_base + (uint32_t)(t * 256);
             auto desc = [&](uint32_t lo) { return ((uint64_t)desc_hi << 32) | (uint64_t)lo; };
-            auto issue_qk = [&](int j) {  // S[t][j & 1] = Q_t · K_jᵀ
+            auto issue_qk = [&](int j) {  // S[j & 1] = Q · K_jᵀ
                 const uint32_t b_lo = k_lo + (uint32_t)((j % KVS) * (KVB >> 4));
-                const uint32_t d_tmem = t_base + (uint32_t)((j & 1) * kBlkN);
+                const uint32_t d_tmem = tmem_base + (uint32_t)((j & 1) * kBlkN);
 #pragma unroll
                 for (int ks = 0; ks < D / 16; ++ks)
                     tc_mma_ss(d_tmem, desc(q_lo + (uint32_t)((ks * 32) >> 4)), desc(b_lo + (uint32_t)((ks * 32) >> 4)), idesc_qk,
@@ -380,62 +351,46 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             };
             auto issue_pv = [&](int j) {  // O_a += P_j[:, 0:32] · V_j[0:32, :],  O_b += P_j[:, 32:64] · V_j[32:64, :]
                 const uint32_t b_lo = v_lo + (uint32_t)((j % KVS) * (KVB >> 4));
-                const uint32_t s_tmem = t_base + (uint32_t)((j & 1) * kBlkN);
+                const uint32_t s_tmem = tmem_base + (uint32_t)((j & 1) * kBlkN);
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
 #pragma unroll
                     for (int ks = 0; ks < 2; ++ks) {
-                        tc_mma_ts(t_base + (uint32_t)(128 + hf * 64), s_tmem + (uint32_t)(hf * 32 + ks * 8),
+                        tc_mma_ts(tmem_base + (uint32_t)(128 + hf * 64), s_tmem + (uint32_t)(hf * 32 + ks * 8),
                                   desc(b_lo + (uint32_t)((hf * 2 + ks) * (2048 >> 4))), idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
                     }
                 }
             };
-            // j below counts visited blocks (ring positions), not key-block numbers; a tile's blocks are
-            // a prefix of the CTA's visit list (causal tiles stop early)
-            const int my_blk = (t < ntl) ? n_tile[t] : 0;
-            const int max_blk = n_union;
-            bool ok = true;
-            if (t < ntl && !mbar_wait(q_full(t), 0, abort_flag, 610)) ok = false;
-            for (int jj = 0; jj < NB && jj < max_blk && ok && t < ntl; ++jj) {
+            // j counts visited blocks (ring positions), not key-block numbers
+            bool ok = mbar_wait(q_full, 0, abort_flag, 610);
+            for (int jj = 0; jj < NB && jj < visits && ok; ++jj) {
                 if (!mbar_wait(k_full(jj % KVS), (uint32_t)((jj / KVS) & 1), abort_flag, 611)) { ok = false; break; }
-                if (jj < my_blk) {
-                    tc_fence_after();
-                    issue_qk(jj);
-                    tc_commit(s_full(t, jj & 1));
-                    tc_commit(k_empty(jj % KVS));
-                } else {
-                    mbar_arrive(k_empty(jj % KVS));  // a block this tile does not need (shorter causal range)
-                }
+                tc_fence_after();
+                issue_qk(jj);
+                tc_commit(s_full(jj & 1));
+                tc_commit(k_empty(jj % KVS));
             }
-            for (int j = 0; j < max_blk && ok && t < ntl; ++j) {
+            for (int j = 0; j < visits && ok; ++j) {
                 const int s = j % KVS;
                 if (!mbar_wait(v_full(s), (uint32_t)((j / KVS) & 1), abort_flag, 612)) { ok = false; break; }
                 const int j2 = j + NB;
-                if (j2 < max_blk) {
+                if (j2 < visits) {
                     if (!mbar_wait(k_full(j2 % KVS), (uint32_t)((j2 / KVS) & 1), abort_flag, 613)) { ok = false; break; }
                 }
-                if (j < my_blk) {
-                    if (!mbar_wait(p_full(t, j & 1), (uint32_t)((j >> 1) & 1), abort_flag, 614)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_pv(j);
-                    tc_commit(pv_done(t, j & 1));
-                    if (j2 < my_blk) {
-                        issue_qk(j2);  // into the slot that P_j has just been read from (in-order execution)
-                        tc_commit(s_full(t, j & 1));
-                    }
-                    if (j + 1 == my_blk) {
-                        mbar_arrive(o_final(t));
-                        tc_commit(o_final(t));
-                    }
-                    tc_commit(v_empty(s));
-                    if (j2 < max_blk) {
-                        if (j2 < my_blk) tc_commit(k_empty(j2 % KVS));
-                        else mbar_arrive(k_empty(j2 % KVS));
-                    }
-                } else {
-                    mbar_arrive(v_empty(s));
-                    if (j2 < max_blk) mbar_arrive(k_empty(j2 % KVS));
+                if (!mbar_wait(p_full(j & 1), (uint32_t)((j >> 1) & 1), abort_flag, 614)) { ok = false; break; }
+                tc_fence_after();
+                issue_pv(j);
+                tc_commit(pv_done(j & 1));
+                if (j2 < visits) {
+                    issue_qk(j2);  // into the slot that P_j has just been read from (in-order execution)
+                    tc_commit(s_full(j & 1));
                 }
+                if (j + 1 == visits) {
+                    mbar_arrive(o_final);
+                    tc_commit(o_final);
+                }
+                tc_commit(v_empty(s));
+                if (j2 < visits) tc_commit(k_empty(j2 % KVS));
             }
         }
       } else if (Cfg::kMaskRing && warp >= W0 + 2) {
@@ -449,12 +404,12 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
         // [3, 12, 333, 64] where EDGE takes 12.0.)
         const int lt = (int)threadIdx.x - (W0 + 2) * 32;
         const int r0 = lt / 9, ch = lt % 9;
-        const int rows = lt < 63 ? min(kAttnBlock, p.M - mt[0] * kAttnBlock) : 0;
+        const int rows = lt < 63 ? min(kAttnBlock, p.M - mt * kAttnBlock) : 0;
         const int64_t step = 14 * p.mask_strides[2];
         const uint8_t* base = reinterpret_cast<const uint8_t*>(p.mask) +
-                              2 * ((int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)(mt[0] * kAttnBlock + r0) * p.mask_strides[2]);
+                              2 * ((int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)(mt * kAttnBlock + r0) * p.mask_strides[2]);
         const uint32_t dst0 = smem_u32(mask_ring) + (uint32_t)(r0 * Cfg::kMaskRowBytes + ch * 16);
-        for (int j = 0; j < n_tile[0]; ++j) {
+        for (int j = 0; j < visits; ++j) {
             if (!mbar_wait(m_empty(j & 1), (uint32_t)(((j >> 1) & 1) ^ 1), abort_flag, 640)) break;
             const uint32_t dst = dst0 + (uint32_t)((j & 1) * Cfg::kMaskSlotBytes);
             const uint8_t* first = base + j * (kBlkN * 2);
@@ -499,14 +454,14 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
     } else {
         asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Shape::kRegsHigh));
         // ------------------------------------------------------------------ softmax warps
-        const int t = warp >> 3;
         const int hf = (warp >> 2) & 1;  // which 32 key columns of every block
         const int q = warp & 3;          // TMEM lane quarter = 32 query rows
-        if (t < ntl && nblk[t] > 0) {
-            const int nb = n_tile[t];
+        // (always so; without the test the compiler arranges the key loop of MODE 1 otherwise: [2, 12, 8192, 64] 864 -> 923 us)
+        if (visits > 0) {
+            const int nb = visits;
             const int r_in_tile = q * 32 + lane;
-            const int row = mt[t] * kAttnBlock + r_in_tile;
-            const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(t * 256);
+            const int row = mt * kAttnBlock + r_in_tile;
+            const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
             const uint32_t o_own = lane_addr + (uint32_t)(128 + hf * 64);
             const float c = p.scale_log2;
             const float mlow = mask_lowest(p.mask_dtype);
@@ -527,7 +482,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 const int bf = j & 1;
                 const uint32_t ph = (uint32_t)((j >> 1) & 1);
                 const uint32_t s_addr = lane_addr + (uint32_t)(bf * kBlkN + hf * 32);
-                if (!mbar_wait(s_full(t, bf), ph, abort_flag, 630 + t)) { ok = false; break; }
+                if (!mbar_wait(s_full(bf), ph, abort_flag, 630)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t sr[32];
                 tmem_ld_32x32(s_addr, sr);
@@ -569,7 +524,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                         }
                     }
                 }
-                const bool causal_edge = p.is_causal && col0 + 31 > mt[t] * kAttnBlock;
+                const bool causal_edge = p.is_causal && col0 + 31 > mt * kAttnBlock;
                 if ((MODE != 1 && col0 + 32 > p.N) || causal_edge) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
@@ -597,7 +552,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                     // complete, the ((j-1)>>1)-th completion of the barrier of parity (j-1)&1. S_j
                     // being ready implies P·V of block j-2 (hence j-3) complete, i.e. every earlier
                     // completion of this barrier, so the parity cannot be mistaken for an older phase.
-                    if (!mbar_wait(pv_done(t, (j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1), abort_flag, 650 + t)) { ok = false; break; }
+                    if (!mbar_wait(pv_done((j - 1) & 1), (uint32_t)(((j - 1) >> 1) & 1), abort_flag, 650)) { ok = false; break; }
                     tc_fence_after();
 #pragma unroll
                     for (int dch = 0; dch < D / 16; ++dch) {
@@ -633,7 +588,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
                 tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(p_full(t, bf));
+                if (lane == 0) mbar_arrive(p_full(bf));
             }
             // The key loop is over: a dependent kernel's CTAs may take the slots that free up from
             // here on and set themselves up (they read nothing before this grid has completed). The
@@ -644,13 +599,13 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
             // (m, l) of this half to the partner warp (same rows, other half) through shared memory
             // a half that never saw a finite score (all of its columns beyond N) must not set the scale
             const float m_own = (l > 0.f) ? m_ref * unit : -INFINITY;
-            xch[(t * 2 + hf) * kAttnBlock + r_in_tile] = make_float2(m_own, l);
+            xch[hf * kAttnBlock + r_in_tile] = make_float2(m_own, l);
             __syncwarp();
-            if (lane == 0) mbar_arrive(ep_bar(t, q));
-            if (ok && mbar_wait(ep_bar(t, q), 0, abort_flag, 660 + t) && mbar_wait(o_final(t), 0, abort_flag, 670 + t)) {
+            if (lane == 0) mbar_arrive(ep_bar(q));
+            if (ok && mbar_wait(ep_bar(q), 0, abort_flag, 660) && mbar_wait(o_final, 0, abort_flag, 670)) {
                 tc_fence_after();
-                const int m_end = s_expired[t] == 0 ? p.M : 0;  // rows that may be stored
-                const float2 other = xch[(t * 2 + (hf ^ 1)) * kAttnBlock + r_in_tile];
+                const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
+                const float2 other = xch[(hf ^ 1) * kAttnBlock + r_in_tile];
                 float m_all = fmaxf(m_own, other.x);
                 if (m_all == -INFINITY) m_all = 0.f;
                 const float w_own = fast_exp2(m_own - m_all), w_oth = fast_exp2(other.x - m_all);
@@ -695,10 +650,10 @@ static bool mask_has_edges(const kb_attn_params& p) {
     return ((((uintptr_t)p.mask) | ((uintptr_t)p.mask + 2 * (uintptr_t)last)) & 15) != 0;
 }
 
-template <typename T, int MODE, int TILES, bool EDGE = false>
-static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stream) {
-    using Cfg = AttnSplitCfgT<TILES, MODE>;
-    using Shape = SplitShape<TILES>;
+template <typename T, int MODE, bool EDGE = false>
+static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t stream) {
+    using Cfg = AttnSplitCfg<MODE>;
+    using Shape = SplitShape;
     CUtensorMap tq, tk, tv;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;
@@ -736,7 +691,7 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
     }
     d.mask_lead = p.mask != nullptr ? (int)((uintptr_t)p.mask & 15) : 0;
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
-    d.num_pairs = (num_m_tiles + TILES - 1) / TILES;  // work items per (batch, head): tile pairs, or tiles
+    d.num_pairs = num_m_tiles;  // work items per (batch, head)
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
     d.kv_group = (int)kv_group;
     d.d_out = (int)p.D;
@@ -745,33 +700,23 @@ static int launch_attention_split_tmt(const kb_attn_params& p, cudaStream_t stre
         // setmaxnreg.inc blocks until the CTA's pool holds the registers: refuse to launch a build
         // whose launch allocation is smaller than the redistribution assumes.
         cudaFuncAttributes fa;
-        if (cudaFuncGetAttributes(&fa, attention_split_kernel<T, MODE, TILES, EDGE>) != cudaSuccess) return KB_ERR_LAUNCH;
+        if (cudaFuncGetAttributes(&fa, attention_split_kernel<T, MODE, EDGE>) != cudaSuccess) return KB_ERR_LAUNCH;
         regs_ok = (fa.numRegs < Shape::kRegsLaunch) ? -1 : 1;
     }
     if (regs_ok < 0) return KB_ERR_UNSUPPORTED;
     static PerDeviceOnce attr_once;
     if (!attr_once.run([] {
-            return cudaFuncSetAttribute(attention_split_kernel<T, MODE, TILES, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemMax) == cudaSuccess;
+            return cudaFuncSetAttribute(attention_split_kernel<T, MODE, EDGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemMax) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
     const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
     if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     const int num_n_blocks = (int)((p.N + kBlkN - 1) / kBlkN);
     const size_t smem_bytes = (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)num_n_blocks * kBlkN * 4 : 0);
-    if (launch_pdl(attention_split_kernel<T, MODE, TILES, EDGE>, (unsigned)grid, (unsigned)Shape::kThreads, smem_bytes, stream, tq,
+    if (launch_pdl(attention_split_kernel<T, MODE, EDGE>, (unsigned)grid, (unsigned)Shape::kThreads, smem_bytes, stream, tq,
                    tk, tv, d) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
-}
-
-// One tile per CTA, two CTAs per SM, is the shape the dispatcher uses: measured against the two-tile
-// CTA it is 2 % (B8 H12 S4096) to 20 % (B64 H12 S512) faster on launches of many waves as well, not
-// only on small ones — two independent CTAs hide each other's latencies better than two tiles inside
-// one CTA share K/V. The two-tile shape stays selectable (kb_debug_split_tiles) and tested.
-template <typename T, int MODE>
-static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t stream) {
-    if (g_split_tiles == 2) return launch_attention_split_tmt<T, MODE, 2>(p, stream);
-    return launch_attention_split_tmt<T, MODE, 1>(p, stream);
 }
 
 // The persistent form of this kernel (attention_persist.cuh) takes the launches it is made for.
@@ -782,8 +727,8 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
 template <typename T>
 static int launch_attention_split_t(const kb_attn_params& p, cudaStream_t stream) {
     const int mode = (p.mask == nullptr && p.sm_scale > 0.f) ? 0
-                     : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg::kMaskMaxN) ? 1
-                     : (g_split_tiles != 2 && p.mask_strides[2] != 0 && mask_is_staged(p)) ? 3 : 2;
+                     : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg<1>::kMaskMaxN) ? 1
+                     : (p.mask_strides[2] != 0 && mask_is_staged(p)) ? 3 : 2;
     if (g_split_tiles == 0 && attention_persist_applicable(p, mode)) {
         if (mode == 0) return launch_attention_persist_tm<T, 0>(p, stream);
         if (mode == 1) return launch_attention_persist_tm<T, 1>(p, stream);
@@ -792,7 +737,7 @@ static int launch_attention_split_t(const kb_attn_params& p, cudaStream_t stream
     if (mode == 0) return launch_attention_split_tm<T, 0>(p, stream);
     if (mode == 1) return launch_attention_split_tm<T, 1>(p, stream);
     if (mode == 2) return launch_attention_split_tm<T, 2>(p, stream);
-    return mask_has_edges(p) ? launch_attention_split_tmt<T, 3, 1, true>(p, stream) : launch_attention_split_tmt<T, 3, 1>(p, stream);
+    return mask_has_edges(p) ? launch_attention_split_tm<T, 3, true>(p, stream) : launch_attention_split_tm<T, 3>(p, stream);
 }
 
 static int launch_attention_split(const kb_attn_params& p, cudaStream_t stream) {

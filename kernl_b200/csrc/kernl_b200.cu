@@ -10,7 +10,7 @@
 #include "norm.cuh"
 #include "linear.cuh"
 #include "linear_pair.cuh"
-#include "linear_smallm.cuh"
+#include "linear_stream.cuh"
 #include "linear_cluster.cuh"
 #include "attention.cuh"
 #include "attention_split.cuh"

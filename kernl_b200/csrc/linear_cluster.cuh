@@ -18,7 +18,7 @@
 #pragma once
 #include "linear.cuh"
 #include "linear_pair.cuh"
-#include "linear_smallm.cuh"
+#include "linear_stream.cuh"
 
 namespace kb {
 
