@@ -288,9 +288,12 @@ static int launch_linear_cluster_n(const kb_linear_params& p, cudaStream_t strea
 
 // ---- which kernel a problem goes to
 //
-// Estimates in us, fitted to times of the kernels (graphs of calls with cold W) over 20 to 3000 rows and W
-// from 500 x 1000 to 12288 x 4096; off by up to a fifth, mostly by less than a tenth. An SM pulls about 118 bytes
-// per ns through its port to L2, shared by its CTAs; W comes from HBM at 6.5 bytes per ps at best.
+// Estimates in us, fitted to times of the kernels (graphs of calls with cold W) over 16 to 8192 rows and W from 500 x 1000
+// to 11008 x 4096. An SM pulls about 118 bytes per ns through its port to L2, shared by its CTAs; W comes from HBM at
+// 6.5 bytes per ps at best. Estimate over time, at 27 problems: CTA pairs 0.85 to 1.05, single CTAs 0.84 to 1.18 from 32 rows
+// on but for 2000 rows of [504, 1000] (0.75), clusters 0.93 to 1.07 where their tiles fit at once. (While the clusters' sums
+// were a constant per column and single CTAs took 118 bytes per ns at every width, [512, 3072] x [768, 3072] ran in
+// 13.2 us where single CTAs take 9.9, [300, 4096] x [1024, 4096] in 14.4 for 12.2, [48, 1000] x [1000, 1000] in 7.5 for 5.0.)
 struct ClusterPlan {
     int nb, splits;
     double us;
@@ -305,14 +308,19 @@ static ClusterPlan linear_cluster_plan(const kb_linear_params& p) {
         const int64_t tiles = ((p.M + nb - 1) / nb) * num_n;
         const int* table = nb == 32 ? linear_cluster_resident<T, 32>() : nb == 64 ? linear_cluster_resident<T, 64>() : linear_cluster_resident<T, 128>();
         if (table == nullptr) continue;
-        for (int s = 1; s <= kClMaxSplits && s <= num_k; ++s) {
+        // Powers of two: they pack the GPU's clusters of SMs and divide the sums of the epilogue, which take four partial
+        // tiles at a time, evenly. (Five CTAs per tile at 512 rows of [768, 3072]: 13.1 us, four: 10.7.)
+        for (int s = 1; s <= kClMaxSplits && s <= num_k; s *= 2) {
             const int resident = table[s];
             if (resident == 0) continue;
             const double waves = (double)((tiles + resident - 1) / resident);
-            const bool shared_sm = (tiles < resident ? tiles : resident) * s > sm_count();
-            const double load = (double)((num_k + s - 1) / s) * (16384.0 + (double)(p.M < nb ? p.M : nb) * 128.0) / (shared_sm ? 59e3 : 100e3);
+            // two CTAs meet on an SM before every SM has one: clusters do not fill all of them
+            const bool shared_sm = (tiles < resident ? tiles : resident) * s > sm_count() * 7 / 8;
+            const double rows = (double)(p.M < nb ? p.M : nb);
+            const double load = (double)((num_k + s - 1) / s) * (16384.0 + rows * 128.0) / (shared_sm ? 85e3 : 100e3);
             const double body = waves * load > hbm ? waves * load : hbm;
-            const double us = 4.1 + (w_bytes > 8e6 ? 2.0 : 0.0) + body + waves * nb * 0.012;
+            const double sums = 0.0203 * rows * (double)((s + 3) / 4 * 4) / (double)s * (shared_sm ? 2.0 : 1.0);
+            const double us = 3.9 + (w_bytes > 8e6 ? 2.0 : 0.0) + body + waves * sums;
             if (us < best.us) best = ClusterPlan{nb, s, us};
         }
     }
@@ -322,9 +330,12 @@ static double linear_single_us(const kb_linear_params& p) {
     const int bn = plan_linear_bn(p.M, p.N, p.K, 0);
     const int64_t tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + bn - 1) / bn);
     const double waves = (double)((tiles + gemm_sms() - 1) / gemm_sms());
-    // 0.012: the epilogue of a column; a tile of which most rows lie outside x arrives later (zero fill): 5.5 us at
-    // 128 rows of [3072, 768], 6.9 at 33
-    return 2.8 + (p.M < 96 ? 1.3 : 0.0) + waves * ((double)(kGemmBM + bn) * (double)p.K * 2.0 / 118e3 + 0.012 * bn);
+    // An SM's port gives 118 bytes per ns, narrow tiles pull faster (512 rows of [768, 3072], 32 columns: 9.9 us, 11.5 at that
+    // rate), rows that are no multiple of 128 bytes take longer. An epilogue stores a column of a tile in 0.012 us by whole
+    // 16-byte pieces, in 0.05 value by value. A tile of which most rows lie outside x arrives later (zero fill): 5.5 us at
+    // 128 rows of [3072, 768], 6.9 at 33.
+    const double load = (double)(kGemmBM + bn) * (double)p.K * 2.0 / (bn <= 64 ? 150e3 : 118e3) * (p.K % kGemmBK != 0 ? 1.8 : 1.0);
+    return 2.8 + (p.M < 96 ? 1.3 : 0.0) + waves * (load + (linear_stores_values(p) ? 0.05 : 0.012) * bn);
 }
 template <typename T>
 static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
@@ -347,9 +358,10 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
     }
     if (p.M <= 1024 && gemm_sms() == sm_count()) {
         const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
-        if (stream_us < single && stream_us < cl.us) return launch_linear_stream_t<T>(p, stream);
-        // (the cluster kernel has to be clearly ahead: where the two are close, its estimate is the less certain one)
-        if (cl.us < 0.94 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+        // (the streaming kernel's estimate is a tenth high for few rows: 5.5 us for 5.0 at 33 rows of [3072, 768], the cluster's 5.3 for 5.4)
+        if (stream_us < single && stream_us < 1.05 * cl.us) return launch_linear_stream_t<T>(p, stream);
+        // (ahead by more than a trifle: where the two are close, the cluster's estimate is the less certain one)
+        if (cl.us < 0.97 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
     }
     return launch_linear_single<T>(p, stream, 0);
 }

@@ -441,6 +441,9 @@ static double linear_pair_us(const kb_linear_params& p, int bn) {
     return (bn == 192 ? 4.1 : 5.4) + (double)rounds * (num_k * block + 0.7);
 }
 
+// Whether the rows of y do not allow stores of 16 bytes.
+static bool linear_stores_values(const kb_linear_params& p) { return p.y_row_stride % 8 != 0 || (((uintptr_t)p.y) & 15) != 0; }
+
 // Tile width (192 or 256 columns), and the estimate that goes with it. 192 columns want the staged epilogue (whole
 // 16-byte pieces, no gated or pre-activation output); among close estimates the wide tile, which pulls less.
 static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
@@ -448,7 +451,7 @@ static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
                         (((uintptr_t)p.y) & 15) == 0;
     const double wide = linear_pair_us(p, 256), narrow = linear_pair_us(p, 192);
     const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : staged && narrow < 0.97 * wide ? 192 : 256;
-    *us = bn == 192 ? narrow : wide;
+    *us = (bn == 192 ? narrow : wide) + (linear_stores_values(p) ? 16.0 : 0.0);  // (26.6 us at 2000 rows of [500, 768])
     return bn;
 }
 

@@ -316,7 +316,8 @@ static StreamPlan stream_plan_x(const kb_linear_params& p) {
         const int64_t ctas = (p.N + rows - 1) / rows;
         const double load = (double)p.K * 2.0 * (rows + kStreamMaxM) / 59e3;
         const double math = (double)((rows + 15) / 16 * 16) * kStreamMaxM * (double)p.K / 486e3;
-        const double us = 2.4 + 1.2 * (double)((ctas * groups + slots - 1) / slots) * (load + 0.5 * math + 0.3);
+        // (rows of W that are no multiple of 128 bytes: 6.6 us for the 5.0 this gives without at 128 rows of [500, 1000])
+        const double us = 2.4 + (p.K % kStreamK != 0 ? 1.8 : 1.2) * (double)((ctas * groups + slots - 1) / slots) * (load + 0.5 * math + 0.3);
         if (us < best.us) best = StreamPlan{ctas, 1, rows, us};
     }
     const double hbm = (double)p.N * (double)p.K * 2.0 / 5.0e6;  // (with x in every ring, W does not come faster)
