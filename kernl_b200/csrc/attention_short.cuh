@@ -294,7 +294,7 @@ static bool attention_short_layout(const kb_attn_params& p) {
 // Which kernel is faster, from times measured over 16 to 800 keys, 1 to 200 sequences of 12 and 16 heads (ns).
 // A launch takes the latency of one tile (a fixed part and one per key block) and, for every tile beyond
 // one per SM, what a tile costs when the GPU is full (the same two parts). Per tile of 64 rows, this
-// kernel: 3.5 + 4 per 64-key block (D = 64), 9.5 + 5 (80), 11 + 7 (128). Per tile of 128 rows, the kernels
+// kernel: 3.5 + 4 per 64-key block (D = 64), 7 + 8 (80), 6 + 12 (128). Per tile of 128 rows, the kernels
 // for D = 64: 8 + 4.3 per block, with a row mask 17.5 + 4.3, with a full mask 11 + 7. Per pair of tiles of
 // 128 rows, attention.cuh: 57 (one tile: 35) + 13 per 128-key block, more with masks.
 static bool attention_short_applicable(const kb_attn_params& p) {
@@ -319,12 +319,15 @@ static bool attention_short_applicable(const kb_attn_params& p) {
         return mine < other;
     }
     const bool d80 = p.D <= 80;
-    const double mine = estimate(tiles64, 2300.0 + (d80 ? 1080.0 : 1650.0) * fb * live, (d80 ? 9.5 : 11.0) + 2 * fa + (d80 ? 5.0 : 7.2) * fb * live);
+    // a causal launch takes as long as its last tile, which meets all blocks; from a tile per SM on, two share an SM
+    const double lat = 2300.0 + (d80 ? 1080.0 : 1650.0) * fb * (p.is_causal ? blocks : live);
+    const double spread = estimate(tiles64, lat, (d80 ? 7.0 : 6.0) + 2 * fa + (d80 ? 8.0 : 12.0) * fb * live);
+    const double mine = tiles64 > sms && spread < 1.45 * lat ? 1.45 * lat : spread;
     const double pairs = bh * (double)((p.M + 255) / 256), b128 = (double)((p.N + 127) / 128);
     const double live128 = p.is_causal ? (b128 + 1) / 2 : row_mask && b128 > 1 ? 0.33 + 0.67 * b128 : b128;
     const bool ragged = full_mask && (p.mask_strides[2] % 8 != 0 || p.mask_strides[3] != 1);
     const double slow = ragged ? 2.6 : full_mask ? 1.8 : row_mask ? 1.15 : 1.0;  // masks cost that kernel's softmax warps
-    const double other = estimate(pairs, (5000.0 + 2500.0 * live128) * slow, (p.M > 128 ? 57.0 : 35.0) * (full_mask ? 1.5 : 1.0) + 13.0 * live128 * slow);
+    const double other = estimate(pairs, (3000.0 + 2950.0 * live128) * slow, (p.M > 128 ? 57.0 : 35.0) * (full_mask ? 1.5 : 1.0) + 13.0 * live128 * slow);
     return mine < other;
 }
 
