@@ -143,6 +143,8 @@ int kb_rope_kv_write(const kb_rope_params* p, void* stream);
  *   mask: additive, logical shape [B|1, H|1, M|1, N]; a broadcast dimension is passed with
  *   stride 0. -inf entries are clamped to the lowest finite value of mask_dtype
  *   (attention.py:380,516). is_causal keeps col <= row, top-left aligned (attention.py:347).
+ *   Nothing ahead of the mask's first value or behind its last one is read; where its rows are
+ *   apart (a view), what lies between them may be read and has no effect on the result.
  * ------------------------------------------------------------------------------------- */
 typedef struct {
     const void* q; const void* k; const void* v; void* o;

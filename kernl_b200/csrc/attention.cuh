@@ -630,7 +630,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 const float neg_ref = -m_ref * unit;
                 const float2 unit2 = make_float2(unit, unit), neg2 = make_float2(neg_ref, neg_ref);
                 // Row sum: four scalar chains (pair i adds to chain i & 3), taken after P has been handed over. Two values
-                // per instruction would save issue slots (155 us instead of 164 at [4, 32 over 8, 2048, 128] causal) but
+                // per instruction would save issue slots (155 us instead of 164 at [4, 32 over 8, 2048, 128] causal, a few calls at
+                // full clock; kept up, the card's power cap takes the clock to 1.76 GHz and a call to 184 us) but
                 // add in another order, and a decoder's greedy tokens should not depend on that. (A quarter to a half
                 // of the exponentials on the FMA pipe was no faster: the special-function unit is half idle.)
                 float lp[4] = {0.f, 0.f, 0.f, 0.f};
