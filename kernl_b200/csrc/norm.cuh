@@ -30,6 +30,8 @@ __device__ __forceinline__ void st_stream_16B(void* p, uint4 v) {
                  : "memory");
 }
 
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
 
 // WPR warps share one row: 1 for many short rows, 4 (the whole CTA) for rows of more than 1024 columns and for
@@ -51,17 +53,28 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
                         float* __restrict__ rstd_out, int64_t rows, int cols, int64_t x_row_stride,
                         int64_t y_row_stride, float eps, const T* __restrict__ residual,
                         T* __restrict__ sum_out) {
-    pdl_wait();
-    pdl_launch_dependents();
     __shared__ float red_s[2][8];
     __shared__ float chain_s[CHAIN ? 32 : 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int wir = warp % WPR;  // this warp's position inside its row
     const int64_t row = WPR == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
+#define KB_NORM_COL(c) (((CHAIN ? wir * CHUNKS + (c) : (c) * WPR + wir) * 32 + lane) * 8)
+    if (WPR == 4 && !CHAIN && (lane & 7) == 0) {
+#pragma unroll
+        for (int c = 0; c < CHUNKS; ++c) {
+            const int col = KB_NORM_COL(c);
+            if (col < cols) {
+                prefetch_l2(gamma + col);
+                if (!RMS && beta != nullptr) prefetch_l2(beta + col);
+                if (residual != nullptr) prefetch_l2(residual + row * (int64_t)cols + col);
+            }
+        }
+    }
+    pdl_wait();
+    pdl_launch_dependents();
     if (row >= rows) return;  // (WPR > 1: the whole CTA leaves together)
     const T* xr = x + row * x_row_stride;
     T* yr = y + row * y_row_stride;
-#define KB_NORM_COL(c) (((CHAIN ? wir * CHUNKS + (c) : (c) * WPR + wir) * 32 + lane) * 8)
 
     uint4 v[CHUNKS];
 #pragma unroll
