@@ -22,7 +22,7 @@
 //   empty[s]   in each CTA: `tcgen05.commit` of the leader, multicast to both CTAs;
 //   tfull[a]   in each CTA: accumulator a complete (multicast commit);
 //   tempty[a]  in the leader: all 32 epilogue warps of the pair have read accumulator a (a warp
-//              arrives as soon as its 64 columns are in registers, before it converts and stores them).
+//              arrives as soon as its columns are in registers).
 // Accumulators are double-buffered (2 x 256 columns = all of tensor memory), the ring has six stages.
 // Every bulk copy has one destination CTA: the pair's sharing happens inside the tensor-core instruction.
 #pragma once
@@ -31,34 +31,29 @@
 namespace kb {
 
 constexpr int kPairBN = 256;          // columns of the pair's widest tile (the kernel is also built for 192)
-constexpr int kPairHalfN = 128;       // W rows staged by each CTA at that width
 #ifndef KB_PAIR_STAGES
 #define KB_PAIR_STAGES 6
 #endif
 constexpr int kPairStages = KB_PAIR_STAGES;
 constexpr int kPairABytes = kGemmBM * kGemmBK * 2;     // 16 KB: this CTA's 128 rows of x
-constexpr int kPairBBytes = kPairHalfN * kGemmBK * 2;  // 16 KB: this CTA's half of the W tile
-constexpr int kPairStageBytes = kPairABytes + kPairBBytes;
 constexpr int kPairEpilogueWarps = 16;
 constexpr int kPairThreads = (2 + kPairEpilogueWarps) * 32;
-// Output staging of the epilogue: per epilogue warp 32 rows x kPairPassCols columns of 16-bit
-// results, in 16-byte pieces; piece c of row r sits at r * row_bytes + (c ^ f(r)) * 16 with f chosen so
-// that the row-wise writes and the piece-wise reads are both free of bank conflicts (64-byte rows:
-// f = (r >> 1) & 3; 32-byte rows: f = (r >> 2) & 1). Behind it the warp's 64 bias values as fp32.
-#ifndef KB_PAIR_PASS_COLS
-#define KB_PAIR_PASS_COLS 16
-#endif
-constexpr int kPairPassCols = KB_PAIR_PASS_COLS;
-static_assert(kPairPassCols == 16 || kPairPassCols == 32, "columns per staging pass");
-constexpr int kPairRowBytes = kPairPassCols * 2;
-constexpr int kPairOutWarpBytes = 32 * kPairRowBytes;
-constexpr int kPairBiasWarpBytes = 64 * 4;
-constexpr int kPairOutBytes = kPairEpilogueWarps * (kPairOutWarpBytes + kPairBiasWarpBytes);
-constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + 256 + kPairOutBytes + 1024;
-__device__ __forceinline__ int pair_stage_offset(int r, int piece) {
-    return kPairPassCols == 32 ? r * 64 + ((piece ^ ((r >> 1) & 3)) * 16) : r * 32 + ((piece ^ ((r >> 2) & 1)) * 16);
-}
-static_assert(kPairSmemBytes <= 227 * 1024, "shared memory of the pair kernel");
+// Output staging of the epilogue: 32 rows x kStoreCols columns of 16-bit results per epilogue warp, the box of one
+// bulk tensor store. 256-column tiles: a warp's 64 columns go in two boxes of 32 (64-byte rows, 64-byte swizzle: piece c of
+// row r sits at c ^ ((r >> 1) & 3)), so that six stages still fit beside them. 192: all 48 columns in one box
+// (96-byte rows, no swizzle), and a stage needs 28 KB only.
+template <int BN>
+struct PairCfg {
+    static_assert(BN == 256 || BN == 192, "tile width of the pair kernel");
+    static constexpr int kHalfN = BN / 2;                                   // W rows staged by each CTA
+    static constexpr int kStageBytes = kPairABytes + kHalfN * kGemmBK * 2;  // bytes one CTA's copies put into a stage
+    static constexpr int kWarpCols = BN / 4;                                // accumulator columns of an epilogue warp
+    static constexpr int kStoreCols = BN == 256 ? 32 : 48;
+    static constexpr int kOutWarpBytes = 32 * kStoreCols * 2;
+    static constexpr int kSmemBytes = kPairStages * kStageBytes + kPairEpilogueWarps * kOutWarpBytes + 256 + 1024;
+    static_assert(kStageBytes % 1024 == 0 && kOutWarpBytes % 1024 == 0, "swizzled buffers begin at multiples of 1024 bytes");
+    static_assert(kSmemBytes <= 227 * 1024 - 64, "shared memory of the pair kernel");
+};
 constexpr uint32_t kPairTmemCols = 512;
 // The address, in the cluster's shared window, of the leader's (rank 0) copy of one of this CTA's own
 // shared-memory locations: both CTAs lay out their shared memory identically.
@@ -119,11 +114,21 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
+// Asynchronous store of a box from shared memory; rows and columns beyond the tensor's end are left out.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(map)),
+                 "r"(src), "r"(x), "r"(y)
+                 : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// This thread's stores have read their shared memory / have been written.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
 // Optional clock stamps for tuning (compiled in with -DKB_GEMM_TRACE only): per CTA and for its first
 // eight tiles, clock64 of: 0 issuer starts waiting for the accumulator, 1 has it, 2 has issued the
-// tile's last MMA; 3 epilogue warp 2 starts waiting for the accumulator, 4 has it, 5 is done with it;
-// 6 the same warp's first 64 columns are stored (8 / 9 / 10: its first tensor-memory load has
-// landed / values are in shared memory / the warp has synchronised). Event 7 of tile 0 is the CTA's start.
+// tile's last MMA; 3 epilogue warp 2 starts waiting for the accumulator, 4 has it, 5 is done with it; 8 its
+// columns are in registers, 9 its first box is in shared memory. Event 7 of tile 0 is the CTA's start.
 #ifdef KB_GEMM_TRACE
 __device__ long long g_gemm_trace[148 * 8 * 16];
 #define KB_GTRACE(tile, ev)                                                                   \
@@ -141,19 +146,18 @@ __device__ long long g_gemm_trace[148 * 8 * 16];
 template <typename T, int BN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
-                   const T* __restrict__ bias, T* __restrict__ y, T* __restrict__ act_inputs, int M, int N, int K,
+                   const __grid_constant__ CUtensorMap tmap_y, int staged, const T* __restrict__ bias, T* __restrict__ y, T* __restrict__ act_inputs, int M, int N, int K,
                    int64_t y_row_stride, int activation) {
     constexpr int STAGES = kPairStages;
-    static_assert(BN == 256 || BN == 192, "tile width of the pair kernel");
-    constexpr int kHalfN = BN / 2;                     // W rows this CTA stages
-    constexpr int kStageTx = kPairABytes + kHalfN * kGemmBK * 2;  // bytes one CTA's copies put into a stage
-    constexpr int CW = BN / 4;                         // columns per epilogue warp
+    using Cfg = PairCfg<BN>;
+    constexpr int kStageBytes = Cfg::kStageBytes;
+    constexpr int CW = Cfg::kWarpCols;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + STAGES * kPairStageBytes);
+    uint8_t* out_stage = smem + STAGES * kStageBytes;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(out_stage + kPairEpilogueWarps * Cfg::kOutWarpBytes);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-    uint8_t* out_stage = smem + STAGES * kPairStageBytes + 256;
 
     const uint32_t smem_base = smem_u32(smem);
     const uint32_t bar_base = smem_u32(bars);
@@ -188,6 +192,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmap_x);
         tma_prefetch_desc(&tmap_w);
+        if (staged) tma_prefetch_desc(&tmap_y);
     }
     __syncthreads();
     cluster_sync_all();  // both CTAs' barriers exist before anybody signals across the pair
@@ -227,12 +232,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 int m_idx, n_idx;
                 tile_coords(t, num_m, num_n, m_idx, n_idx);
                 const int row0 = m_idx * 2 * kGemmBM + (int)rank * kGemmBM;    // this CTA's rows of x
-                const int wrow0 = n_idx * BN + (int)rank * kHalfN;    // this CTA's rows of W
+                const int wrow0 = n_idx * BN + (int)rank * Cfg::kHalfN;    // this CTA's rows of W
                 for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag, 110)) { ok = false; break; }
                     // the leader's barrier counts the bytes of both CTAs' copies of this stage
-                    if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * kStageTx);
-                    const uint32_t a_dst = smem_base + stage * kPairStageBytes;
+                    if (rank == 0) mbar_arrive_expect_tx(full_bar(stage), 2 * kStageBytes);
+                    const uint32_t a_dst = smem_base + stage * kStageBytes;
                     const uint32_t leader_full = in_leader(full_bar(stage));
                     tma_load_2d_pair(a_dst, &tmap_x, leader_full, kb * kGemmBK, row0);
                     tma_load_2d_pair(a_dst + kPairABytes, &tmap_w, leader_full, kb * kGemmBK, wrow0);
@@ -263,7 +268,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(full_bar(stage), phase, abort_flag, 211)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t a_addr = smem_base + stage * kPairStageBytes;
+                    const uint32_t a_addr = smem_base + stage * kStageBytes;
                     const uint64_t a_desc = make_smem_desc_sw128(a_addr, 16, 1024);
                     const uint64_t b_desc = make_smem_desc_sw128(a_addr + kPairABytes, 16, 1024);
 #pragma unroll
@@ -284,111 +289,138 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         const int q = warp & 3;                 // TMEM lane quadrant this warp may access
         const int c_begin = ((warp - 2) >> 2) * CW;  // the warp's CW columns of the tile
         const uint32_t leader_tempty[2] = {in_leader(tempty_bar(0)), in_leader(tempty_bar(1))};
-        // whole 16-byte pieces of y: plain activations, no pre-activation output, aligned rows
-        const bool staged = activation != KB_ACT_SWIGLU && act_inputs == nullptr && (N & 7) == 0 && (y_row_stride & 7) == 0 &&
-                            (((uintptr_t)y) & 15) == 0;
-        uint8_t* mine = out_stage + (warp - 2) * (kPairOutWarpBytes + kPairBiasWarpBytes);
-        float* bias_s = reinterpret_cast<float*>(mine + kPairOutWarpBytes);
+        uint8_t* mine = out_stage + (warp - 2) * Cfg::kOutWarpBytes;
+        const bool gated = CW == 64 && activation == KB_ACT_SWIGLU;  // (192-column tiles are not chosen for it; forced, they store value by value)
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
         int ti = 0;
-        // the warp's bias values of a tile (lane l: columns 2l, 2l + 1 of the warp's 64)
-        auto load_bias = [&](int tile) -> float2 {
-            float2 b2 = make_float2(0.f, 0.f);
-            if (bias != nullptr && tile < num_tiles) {
-                int m_i, n_i;
-                tile_coords(tile, num_m, num_n, m_i, n_i);
-                const int c = n_i * BN + c_begin + 2 * lane;
-                if (2 * lane < CW && c < N) b2.x = Elem<T>::to_f32(bias[c]);
-                if (2 * lane < CW && c + 1 < N) b2.y = Elem<T>::to_f32(bias[c + 1]);
-            }
-            return b2;
-        };
-        if (staged) reinterpret_cast<float2*>(bias_s)[lane] = load_bias(pair);
         if (threadIdx.x == 64) s_expired = status_word();
         named_barrier(1, kPairEpilogueWarps * 32);
         const int m_end = s_expired == 0 ? M : 0;  // rows that may be stored
+        int m_idx, n_idx;
+        tile_coords(pair, num_m, num_n, m_idx, n_idx);
         for (int t = pair; t < num_tiles && ok; t += num_pairs, ++ti) {
-            int m_idx, n_idx;
-            tile_coords(t, num_m, num_n, m_idx, n_idx);
             const int n0 = n_idx * BN;
-            // the next tile's bias is requested now and put into shared memory when this tile is done
-            float2 bias_next = make_float2(0.f, 0.f);
-            if (staged) bias_next = load_bias(t + num_pairs);
+            const int row_base = m_idx * 2 * kGemmBM + (int)rank * kGemmBM + q * 32;  // the warp's first row
+            // The bias of the warp's first box, asked for ahead of the accumulator (loads between the conversions of a box stalled
+            // every 16 columns: 2300 cycles for 48 columns without an activation). Every lane reads the same 16 bytes.
+            constexpr int kPieces = Cfg::kStoreCols / 8;  // 16-byte pieces of a staged row
+            uint4 bias_w[kPieces];
+            auto load_bias = [&](int c) {
+#pragma unroll
+                for (int v = 0; v < kPieces; ++v) {
+                    const int col = n0 + c_begin + c + v * 8;
+                    bias_w[v] = staged && bias != nullptr && col < N ? __ldg(reinterpret_cast<const uint4*>(bias + col)) : make_uint4(0u, 0u, 0u, 0u);
+                }
+            };
+            load_bias(0);
             if (warp == 2 && lane == 0) KB_GTRACE(ti, 3);
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 310)) { ok = false; break; }
             if (warp == 2 && lane == 0) KB_GTRACE(ti, 4);
             tc_fence_after();
-            const int row = m_idx * 2 * kGemmBM + (int)rank * kGemmBM + q * 32 + lane;
-            T* y_row = y + (int64_t)row * y_row_stride;
-            T* a_row = act_inputs ? act_inputs + (int64_t)row * y_row_stride : nullptr;
             if (staged) {
-                // Results go through shared memory so that the warp writes whole row segments (eight
-                // rows x 64 bytes per store instruction) instead of 32 rows x 16 bytes: a
-                // thread-per-row store touches 32 cache lines per instruction.
-                const int row_base = m_idx * 2 * kGemmBM + (int)rank * kGemmBM + q * 32;
-                // all CW columns in one tensor-memory round trip; with them in registers the
-                // accumulator goes back to the issuer at once. (Fetching the second half while the
-                // first is converted and stored was slower: the accumulator came back later.)
-                uint32_t r2[CW];
+                // Whole boxes of results go through shared memory to bulk tensor stores, one per warp: what a warp's
+                // own stores cost (a thousand cycles per 16 columns with all sixteen warps at it, 6000 to 7500 per tile, where a
+                // main loop of twelve k-blocks takes 4600 to 6100) the copy engine does while the warps convert: 1500 to 2500
+                // cycles, 3500 to 4500 with a GELU. [8192, 768] x [2304, 768] 26.4 -> 24.0 us, x [3072, 768] with GELU 36.8 -> 33.6,
+                // [4000, 512] x [3000, 512] 16.3 -> 13.9 (clocks at the power cap for the first two).
+                // (256 columns: a box's 32 at a time. All 64 at once and the bias do not fit in 96 registers.)
+                constexpr int SC = Cfg::kStoreCols;
+                uint32_t r2[SC];
                 const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kPairBN + c_begin);
-                {
-                    uint32_t (&lo)[32] = *reinterpret_cast<uint32_t(*)[32]>(&r2[0]);
-                    tmem_ld_32x32(t_addr, lo);
-                    if (CW == 64) {
-                        uint32_t (&hi)[32] = *reinterpret_cast<uint32_t(*)[32]>(&r2[CW - 32]);
-                        tmem_ld_32x32(t_addr + 32, hi);
-                    } else {
-                        uint32_t (&hi)[16] = *reinterpret_cast<uint32_t(*)[16]>(&r2[CW - 16]);
-                        tmem_ld_32x16(t_addr + 32, hi);
-                    }
-                }
+                tmem_ld_32x32(t_addr, *reinterpret_cast<uint32_t(*)[32]>(&r2[0]));
+                if (SC == 48) tmem_ld_32x16(t_addr + 32, *reinterpret_cast<uint32_t(*)[16]>(&r2[SC - 16]));
                 tmem_ld_wait();
-                tc_fence_before();
-                __syncwarp();  // (also: every lane's bias values are in bias_s)
-                if (lane == 0) mbar_arrive_cluster(leader_tempty[acc]);
+                auto release = [&] {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_cluster(leader_tempty[acc]);
+                };
+                if (SC == CW) release();
                 if (warp == 2 && lane == 0) KB_GTRACE(ti, 8);
-                constexpr int kPieces = kPairPassCols / 8;     // 16-byte pieces per staged row
-                constexpr int kRowsPerStore = 32 / kPieces;  // rows one store instruction covers
+                // z = accumulator + bias of the 16 columns from c on (of a box; their bias is in bias_w[c / 8] and the one behind it)
+                auto add_bias = [&](int c, float (&z)[16]) {
 #pragma unroll
-                for (int ps = 0; ps < CW / kPairPassCols; ++ps) {
-                    const int pc0 = c_begin + ps * kPairPassCols;  // first column of the pass, inside the tile
-                    if (n0 + pc0 >= N) break;
-                    float z[kPairPassCols];
+                    for (int g = 0; g < 2; ++g) {
+                        const uint4 w = bias_w[c / 8 + g];
+                        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-                    for (int v = 0; v < kPairPassCols / 4; ++v) {
-                        const float4 b4 = reinterpret_cast<const float4*>(bias_s)[ps * (kPairPassCols / 4) + v];
-                        z[v * 4 + 0] = __uint_as_float(r2[ps * kPairPassCols + v * 4 + 0]) + b4.x;
-                        z[v * 4 + 1] = __uint_as_float(r2[ps * kPairPassCols + v * 4 + 1]) + b4.y;
-                        z[v * 4 + 2] = __uint_as_float(r2[ps * kPairPassCols + v * 4 + 2]) + b4.z;
-                        z[v * 4 + 3] = __uint_as_float(r2[ps * kPairPassCols + v * 4 + 3]) + b4.w;
+                        for (int i = 0; i < 4; ++i) {
+                            const float2 b2 = Elem<T>::unpack2(ww[i]);
+                            z[g * 8 + 2 * i] = __uint_as_float(r2[c + g * 8 + 2 * i]) + b2.x;
+                            z[g * 8 + 2 * i + 1] = __uint_as_float(r2[c + g * 8 + 2 * i + 1]) + b2.y;
+                        }
                     }
-                    apply_activation<kPairPassCols>(z, activation);
+                };
+                uint32_t o[kPieces * 4];
 #pragma unroll
-                    for (int v = 0; v < kPieces; ++v) {
-                        uint4 o;
-                        o.x = Elem<T>::pack2(z[v * 8 + 0], z[v * 8 + 1]);
-                        o.y = Elem<T>::pack2(z[v * 8 + 2], z[v * 8 + 3]);
-                        o.z = Elem<T>::pack2(z[v * 8 + 4], z[v * 8 + 5]);
-                        o.w = Elem<T>::pack2(z[v * 8 + 6], z[v * 8 + 7]);
-                        *reinterpret_cast<uint4*>(mine + pair_stage_offset(lane, v)) = o;
+                for (int bx = 0; bx < CW / SC; ++bx) {
+                    if (gated) {
+                        // blocks of eight gate and eight up columns: the 64 accumulator columns make one box of 32
+#pragma unroll
+                        for (int c = 0; c < SC; c += 16) {
+                            float z[16];
+                            add_bias(c, z);
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+                                o[(bx * SC + c) / 4 % (kPieces * 4) + i] = Elem<T>::pack2(act_silu(z[2 * i]) * z[8 + 2 * i], act_silu(z[2 * i + 1]) * z[8 + 2 * i + 1]);
+                        }
+                    } else {
+#pragma unroll
+                        for (int c = 0; c < SC; c += 16) {
+                            float z[16];
+                            add_bias(c, z);
+                            apply_activation<16>(z, activation);
+#pragma unroll
+                            for (int i = 0; i < 8; ++i) o[c / 2 + i] = Elem<T>::pack2(z[2 * i], z[2 * i + 1]);
+                        }
                     }
-                    if (warp == 2 && lane == 0 && ps == 0) KB_GTRACE(ti, 9);
+                    if (bx + 1 < CW / SC) {
+                        load_bias((bx + 1) * SC);
+                        tmem_ld_32x32(t_addr + (uint32_t)((bx + 1) * SC), *reinterpret_cast<uint32_t(*)[32]>(&r2[0]));
+                    }
+                    const int ycol = gated ? (n0 + c_begin) / 2 : n0 + c_begin + bx * SC;
+                    if (gated && bx + 1 < CW / SC) {  // (half of the box only)
+                        tmem_ld_wait();
+                        continue;
+                    }
+                    if (lane == 0) bulk_wait_read();  // the box before this one has left the buffer
                     __syncwarp();
-                    if (warp == 2 && lane == 0 && ps == 0) KB_GTRACE(ti, 10);
+                    if (SC == 32) {
 #pragma unroll
-                    for (int it = 0; it < 32 / kRowsPerStore; ++it) {
-                        const int rr = it * kRowsPerStore + lane / kPieces, pc = lane % kPieces;
-                        const uint4 o = *reinterpret_cast<const uint4*>(mine + pair_stage_offset(rr, pc));
-                        const int grow = row_base + rr, gcol = n0 + pc0 + pc * 8;
-                        if (grow < m_end && gcol < N) *reinterpret_cast<uint4*>(y + (int64_t)grow * y_row_stride + gcol) = o;
+                        for (int v = 0; v < kPieces; ++v)
+                            *reinterpret_cast<uint4*>(mine + lane * 64 + ((v ^ ((lane >> 1) & 3)) * 16)) =
+                                make_uint4(o[v * 4], o[v * 4 + 1], o[v * 4 + 2], o[v * 4 + 3]);
+                    } else {
+                        // rows of 96 bytes: lanes l and l + 4 meet in the same banks, so every other four lanes take their pieces in
+                        // pairs the other way round
+                        const bool swap = (lane & 4) != 0;
+#pragma unroll
+                        for (int v = 0; v < kPieces; ++v) {
+                            uint4 w;
+                            w.x = swap ? o[(v ^ 1) * 4 + 0] : o[v * 4 + 0];
+                            w.y = swap ? o[(v ^ 1) * 4 + 1] : o[v * 4 + 1];
+                            w.z = swap ? o[(v ^ 1) * 4 + 2] : o[v * 4 + 2];
+                            w.w = swap ? o[(v ^ 1) * 4 + 3] : o[v * 4 + 3];
+                            *reinterpret_cast<uint4*>(mine + lane * 96 + (swap ? v ^ 1 : v) * 16) = w;
+                        }
                     }
-                    if (warp == 2 && lane == 0 && ps == 0) KB_GTRACE(ti, 6);
+                    fence_proxy_async_smem();
                     __syncwarp();
+                    if (warp == 2 && lane == 0 && bx == 0) KB_GTRACE(ti, 9);
+                    if (lane == 0 && row_base < m_end && ycol < (gated ? N / 2 : N)) {
+                        tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
+                        bulk_commit();
+                    }
+                    if (bx + 1 < CW / SC) tmem_ld_wait();
                 }
-                reinterpret_cast<float2*>(bias_s)[lane] = bias_next;  // (all reads of this tile's values are behind the last __syncwarp)
+                if (SC != CW) release();
+                if (t + num_pairs < num_tiles) tile_coords(t + num_pairs, num_m, num_n, m_idx, n_idx);
             } else {
+                const int row = row_base + lane;
+                T* y_row = y + (int64_t)row * y_row_stride;
+                T* a_row = act_inputs ? act_inputs + (int64_t)row * y_row_stride : nullptr;
 #pragma unroll 1
                 // (a 32-column chunk at a time: with 48 columns per warp, warps pair up on chunks — the
                 // even warp of a pair of column groups takes the chunk that straddles them)
@@ -409,11 +441,13 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(leader_tempty[acc]);  // counted in the leader, whose issuer reuses the accumulator
+                if (t + num_pairs < num_tiles) tile_coords(t + num_pairs, num_m, num_n, m_idx, n_idx);
             }
             if (warp == 2 && lane == 0) KB_GTRACE(ti, 5);
             acc ^= 1;
             if (acc == 0) acc_phase ^= 1;
         }
+        if (staged && lane == 0) bulk_wait_all();
     }
 
     // Teardown: every role of both CTAs falls through to here, also after an abandoned wait. Neither
@@ -429,35 +463,43 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
 static int g_linear_pair = 1;  // test hook (kb_debug_linear_pair): 0 = never use the pair kernel, 192 / 256 = force that tile width
 
-// Estimated time in us of the pair kernel with tiles of 256 x `bn`: a fixed part, and rounds of tiles on the pairs of
-// (k-blocks x time of one + the part of an epilogue that the next tile does not hide). A k-block of 64 costs
-// 0.24 us (192 columns) or 0.285 us (256) while few pairs are busy, up to a quarter more when all of them pull
-// on L2. Fitted to 128 to 3000 rows, K from 768 to 11008; mostly within 8 %.
+// Estimated time in us of the pair kernel with tiles of 256 x `bn`: a fixed part (more of it when there is one round only,
+// whose first operands and epilogue nothing hides), and rounds of tiles on the pairs of (k-blocks x time of one + the part of
+// an epilogue that the next tile does not hide; the exponential of a GELU costs 0.3 more). A k-block of 64 costs 0.235 us (192 columns) or 0.268
+// (256) while few pairs are busy, up to a third more when all of them pull on L2: about 60 bytes per cycle and SM arrive
+// where the products want 75 and 64. Fitted to 1000 to 8192 rows, K from 512 to 4096.
 static double linear_pair_us(const kb_linear_params& p, int bn) {
     const int64_t pairs = gemm_sms() / 2 > 0 ? gemm_sms() / 2 : 1;
     const int64_t tiles = ((p.M + 255) / 256) * ((p.N + bn - 1) / bn), rounds = (tiles + pairs - 1) / pairs;
     const double busy = (double)tiles / (double)(rounds * pairs), num_k = (double)((p.K + kGemmBK - 1) / kGemmBK);
-    const double block = bn == 192 ? 0.24 + 0.05 * busy * busy : 0.285 + 0.09 * busy * busy;
-    return (bn == 192 ? 4.1 : 5.4) + (double)rounds * (num_k * block + 0.7);
+    const double act = p.activation == KB_ACT_GELU ? 0.3 : 0.0, b2 = busy * busy;
+    if (bn == 192) return 4.0 + (rounds == 1 ? 1.6 : 0.0) + (double)rounds * (num_k * (0.235 + 0.07 * b2 * b2 * b2) + 0.4 + act);
+    return 2.7 + act + (rounds == 1 ? 2.3 : 0.0) + (double)rounds * (num_k * (0.268 + 0.09 * b2) + 1.0 + act);
 }
 
 // Whether the rows of y do not allow stores of 16 bytes.
 static bool linear_stores_values(const kb_linear_params& p) { return p.y_row_stride % 8 != 0 || (((uintptr_t)p.y) & 15) != 0; }
 
-// Tile width (192 or 256 columns), and the estimate that goes with it. 192 columns want the staged epilogue (whole
-// 16-byte pieces, no gated or pre-activation output); among close estimates the wide tile, which pulls less.
+// Whether results leave through bulk tensor stores: rows of y at whole 16 bytes, no pre-activation output, whole pieces of eight
+// columns of y and bias; the gated form needs the 64 accumulator columns per warp of the wide tile.
+static bool linear_pair_staged(const kb_linear_params& p, int bn) {
+    if (p.act_inputs != nullptr || linear_stores_values(p) || p.y_row_stride <= 0 || (((uintptr_t)p.bias) & 15) != 0) return false;
+    return p.activation == KB_ACT_SWIGLU ? bn == 256 && p.N % 16 == 0 : p.N % 8 == 0;
+}
+
+// Tile width (192 or 256 columns), and the estimate that goes with it. 192 columns want the staged epilogue; among close estimates the wide tile, which pulls less.
 static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
-    const bool staged = p.activation != KB_ACT_SWIGLU && p.act_inputs == nullptr && (p.N & 7) == 0 && (p.y_row_stride & 7) == 0 &&
-                        (((uintptr_t)p.y) & 15) == 0;
+    const bool staged = linear_pair_staged(p, 192);
     const double wide = linear_pair_us(p, 256), narrow = linear_pair_us(p, 192);
-    const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : staged && narrow < 0.97 * wide ? 192 : 256;
+    const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : staged && narrow < 0.96 * wide ? 192 : 256;
     *us = (bn == 192 ? narrow : wide) + (linear_stores_values(p) ? 16.0 : 0.0);  // (26.6 us at 2000 rows of [500, 768])
     return bn;
 }
 
 template <typename T, int BN>
 static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream) {
-    CUtensorMap tmap_x, tmap_w;
+    using Cfg = PairCfg<BN>;
+    CUtensorMap tmap_x, tmap_w, tmap_y;
     {
         const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.M};
         const uint64_t strides[2] = {0, (uint64_t)p.x_row_stride * 2};
@@ -474,9 +516,20 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (st != KB_OK) return st;
     }
+    const int staged = linear_pair_staged(p, BN) ? 1 : 0;
+    if (staged) {
+        const uint64_t dims[2] = {(uint64_t)(p.activation == KB_ACT_SWIGLU ? p.N / 2 : p.N), (uint64_t)p.M};
+        const uint64_t strides[2] = {0, (uint64_t)p.y_row_stride * 2};
+        const uint32_t box[2] = {(uint32_t)Cfg::kStoreCols, 32};
+        const int st = encode_tmap_16bit(&tmap_y, p.y, 2, dims, strides, box, BN == 256 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                                         CU_TENSOR_MAP_L2_PROMOTION_NONE);
+        if (st != KB_OK) return st;
+    } else {
+        tmap_y = tmap_x;  // (not used)
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kPairThreads);
-    cfg.dynamicSmemBytes = kPairSmemBytes;
+    cfg.dynamicSmemBytes = Cfg::kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -493,7 +546,7 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return KB_ERR_LAUNCH;
     int resident = max_pairs[dev].load(std::memory_order_acquire);
     if (resident == 0) {
-        if (cudaFuncSetAttribute(linear_pair_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) != cudaSuccess)
+        if (cudaFuncSetAttribute(linear_pair_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
             return KB_ERR_LAUNCH;
         cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
         int n = 0;
@@ -509,7 +562,7 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     if (pairs > gemm_sms() / 2) pairs = gemm_sms() / 2;  // a caller-set limit leaves SMs to a concurrent collective
     cfg.gridDim = dim3(2 * (unsigned)pairs);
     cfg.numAttrs = g_use_pdl ? 2u : 1u;
-    if (cudaLaunchKernelEx(&cfg, linear_pair_kernel<T, BN>, tmap_x, tmap_w, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M,
+    if (cudaLaunchKernelEx(&cfg, linear_pair_kernel<T, BN>, tmap_x, tmap_w, tmap_y, staged, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M,
                            (int)p.N, (int)p.K, p.y_row_stride, p.activation) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
