@@ -11,6 +11,11 @@
 // The third warpgroup shrinks its register allowance (setmaxnreg) so that the softmax threads can
 // hold a whole 128-wide score row in registers.
 // While one group runs its exponentials, the tensor core works on the other tile (ping-pong).
+// Without a mask (MODE 0) a CTA stays for the whole launch, one per SM: further items (pairs of query tiles) come from a
+// device-side counter, the issuer starts an item's scores while the softmax warps store the one before, and every barrier's
+// phase counts on over the items. A CTA per item spent 12 000 of 45 000 to 67 000 cycles on setting itself up, its first
+// loads, its stores and its end (all of an SM's tensor memory and shared memory are one CTA's). [4, 32 over 8, 2048, 128]
+// causal 166 -> 149 us (with the hand-over of P below), [16, 16, 512, 128] 61 -> 46, [2, 32, 4096, 128] 463 -> 440; same bits.
 // TMEM columns: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+D)  O_1 [384,384+D); P_t (16-bit, two
 // per column) overwrites the first 64 columns of S_t once the thread has its row in registers.
 //
@@ -32,16 +37,48 @@ constexpr int kAttnThreads = 384;
 constexpr int kAttnBlock = 128;  // rows per query tile and keys per block
 constexpr int kBlkN = 64;        // keys per block of the head-dimension-64 kernel (attention_split.cuh)
 // Register re-balancing between the warpgroups (setmaxnreg). The CTA is launched with
-// 65536 / 384 -> 168 registers per thread; the third warpgroup shrinks to kAttnRegsLow and the two
-// softmax warpgroups grow to kAttnRegsHigh. The increase waits (without bound) until the CTA's own
+// 65536 / 384 -> 168 registers per thread; the third warpgroup shrinks to attn_regs_low() and the two
+// softmax warpgroups grow to attn_regs_high(). The increase waits (without bound) until the CTA's own
 // pool has the registers, so the totals MUST fit the launch allocation: 2*high + low <= 3*168.
 constexpr int kAttnRegsLaunch = 168;
-constexpr int kAttnRegsLow = 40;
-constexpr int kAttnRegsHigh = 232;
-static_assert(2 * kAttnRegsHigh + kAttnRegsLow <= 3 * kAttnRegsLaunch, "setmaxnreg totals exceed the CTA's register pool");
-static_assert(kAttnRegsLow % 8 == 0 && kAttnRegsHigh % 8 == 0, "setmaxnreg wants multiples of 8");
+// (The issuer and producer of the persistent form, MODE 0, keep more counters than 72 registers hold.)
+__host__ __device__ constexpr int attn_regs_low(int mode) { return mode == 0 ? 104 : 72; }
+__host__ __device__ constexpr int attn_regs_high(int mode) { return mode == 0 ? 200 : 216; }
+static_assert(2 * attn_regs_high(0) + attn_regs_low(0) <= 3 * kAttnRegsLaunch && 2 * attn_regs_high(1) + attn_regs_low(1) <= 3 * kAttnRegsLaunch,
+              "setmaxnreg totals exceed the CTA's register pool");
+static_assert(attn_regs_low(0) % 8 == 0 && attn_regs_high(0) % 8 == 0 && attn_regs_low(1) % 8 == 0 && attn_regs_high(1) % 8 == 0,
+              "setmaxnreg wants multiples of 8");
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLazyThreshold = 8.0f;
+
+// Work queues of the persistent kernels. A launch takes the next slot (host-side round robin) and its CTAs draw tile numbers
+// from slot[0]; slot[1] counts CTAs that have finished, and the last one puts both words back to
+// zero, so a slot is clean again when its launch ends — also when the launch gave up on an expired
+// wait. Two launches would have to be in flight kAttnQueueSlots launches apart to share a slot.
+constexpr int kAttnQueueSlots = 1024;
+__device__ unsigned int g_attn_queue[kAttnQueueSlots][2];
+
+// The next queue slot on the current device. g_attn_queue is a host-side handle; its device address
+// is looked up once per device (with that device current) and kept.
+static unsigned int* attention_queue_slot() {
+    static unsigned int* base[64] = {};
+    static std::mutex mu;
+    static std::atomic<unsigned> next_slot{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (base[dev] == nullptr) {
+            void* ptr = nullptr;
+            if (cudaGetSymbolAddress(&ptr, g_attn_queue) != cudaSuccess || ptr == nullptr) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            base[dev] = reinterpret_cast<unsigned int*>(ptr);
+        }
+    }
+    return base[dev] + 2 * (next_slot.fetch_add(1) % (unsigned)kAttnQueueSlots);
+}
 
 struct AttnDev {
     void* o;
@@ -55,6 +92,7 @@ struct AttnDev {
     int mask_vec;   // mask rows can be read with aligned 128-bit loads
     int mask_lead;  // the mask's address modulo 16 (head dimension 64, staged per-row masks)
     int num_pairs;  // ceil(ceil(M/128)/2)
+    int o_bulk;     // head dimensions above 64, no mask: the result can leave through bulk tensor stores
     int head_group; // heads whose CTAs are interleaved (see attn_work_item)
     int kv_group;   // query heads per K/V head (grouped-query attention), >= 1
     int d_out;      // head dimension of the caller's tensors (a multiple of 8, at most the kernel's D): the
@@ -89,16 +127,16 @@ __device__ __forceinline__ void attn_store_32(T* __restrict__ o_row, int col0, i
     }
 }
 
-// CTA -> (batch*head, query-tile pair). Heads are taken in groups of p.head_group; inside a group
+// Work item (a CTA's number, or one drawn from a queue) -> (batch*head, query-tile pair). Heads are taken in groups of p.head_group; inside a group
 // the order is pair-major with the late (causally heavier) pairs first, so the tail of a causal
 // launch is made of light tiles, and consecutive CTAs are different heads of the same group. The
 // group is sized on the host so that the K/V of all its heads (what the resident CTAs stream) stay
 // in L2: with one group over all heads, 148 resident CTAs of a long-sequence launch streamed the
 // K/V of 148 heads and DRAM read traffic was ten times the algorithmic bytes.
-__device__ __forceinline__ void attn_work_item(const AttnDev& p, int BH, int& bh, int& pair) {
+__device__ __forceinline__ void attn_work_item(const AttnDev& p, int BH, int idx, int& bh, int& pair) {
     const int per_group = p.num_pairs * p.head_group;
-    const int g = (int)(blockIdx.x / per_group);
-    const int rem = (int)(blockIdx.x % per_group);
+    const int g = idx / per_group;
+    const int rem = idx % per_group;
     const int first = g * p.head_group;
     const int gsz = min(p.head_group, BH - first);
     pair = p.num_pairs - 1 - rem / gsz;
@@ -119,6 +157,10 @@ struct AttnCfg {
     static constexpr int kSmemBase = (2 + 2 * kKvStages) * kTileBytes + 512 + 1024;
     static constexpr int kMaskMaxN = 7168;  // MODE 1: the longest mask row that fits behind the tiles
     static constexpr int kMaskRingBytes = 2 * 2 * kAttnBlock * 4;  // MODE 3
+    static constexpr int kOutWarpBytes = 32 * 64 * 2;  // MODE 0: 32 rows x 64 columns of results per softmax warp, a box of one bulk store
+    static constexpr int kOutOffset = (2 + 2 * kKvStages) * kTileBytes + 1024;
+    static constexpr int kSmemMode0 = kOutOffset + 8 * kOutWarpBytes + 1024;
+    static_assert(kSmemMode0 <= 227 * 1024 - 256, "shared memory of one CTA");
     static constexpr int kSmemMax = kSmemBase + kMaskMaxN * 4;
     static_assert(kSmemMax <= 227 * 1024 - 256, "shared memory of one CTA");
 };
@@ -240,7 +282,8 @@ __device__ __forceinline__ int bits_count_below(const uint32_t (&w)[4], int limi
 template <typename T, int D, int MODE>
 __global__ void __launch_bounds__(kAttnThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                    const __grid_constant__ CUtensorMap tmap_v, const AttnDev p) {
+                    const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const AttnDev p,
+                    const int num_items, unsigned int* const queue) {
     using Cfg = AttnCfg<D>;
     constexpr int KVS = Cfg::kKvStages;
     constexpr int TILE = Cfg::kTileBytes;
@@ -265,12 +308,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     auto o_final = [&](int t) { return bar_base + 8u * (6 + 4 * KVS + t); };
     auto m_full = [&](int t, int bf) { return bar_base + 8u * (12 + 4 * KVS + t * 2 + bf); };  // MODE 3
     auto m_empty = [&](int t, int bf) { return bar_base + 8u * (16 + 4 * KVS + t * 2 + bf); };
-    constexpr int kNumBars = 20 + 4 * KVS;
-    static_assert(kNumBars * 8 + 32 <= 512, "barrier area too small");
+    auto q_empty = [&](int t) { return bar_base + 8u * (20 + 4 * KVS + t); };    // the last product of an item has read Q_t
+    auto o_free = [&](int t) { return bar_base + 8u * (22 + 4 * KVS + t); };     // O_t is in the softmax warps' registers
+    auto item_full = [&](int s) { return bar_base + 8u * (24 + 4 * KVS + s); };  // MODE 0: drawn items
+    auto item_free = [&](int s) { return bar_base + 8u * (26 + 4 * KVS + s); };
+    constexpr int kNumBars = 28 + 4 * KVS;
+    static_assert(kNumBars * 8 + 48 <= 512, "barrier area too small");
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + kNumBars);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
     float* mask_smem = reinterpret_cast<float*>(smem + (2 + 2 * KVS) * TILE + 512);  // MODE 1: [N rounded up to 128]; MODE 3: [tile][two blocks][128]
     uint32_t* act_bits = tmem_slot + 2;  // MODE 1: key blocks with an unmasked key
+    volatile int* items = reinterpret_cast<volatile int*>(tmem_slot + 6);  // MODE 0: two slots for drawn items, -1: no more
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -278,34 +326,53 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     // the host has read (and cleared) it, so that one failure cannot cost a second per CTA. What is read here may be
     // too early (status_word()); the epilogue looks again before it stores.
     __shared__ int s_expired;
+    // MODE 0: one thread of every CTA reports in when it draws no more items; the last one leaves the queue's slot clean.
+    // (Reported by the producer, while the last item is computed: at the CTA's end it cost a microsecond.)
+    const bool draws = MODE == 0 && num_items > (int)gridDim.x;
+    auto report = [&] {
+        if (draws) {
+            __threadfence();
+            if (atomicAdd(&queue[1], 1u) == gridDim.x - 1) {
+                queue[0] = 0u;
+                queue[1] = 0u;
+                __threadfence();
+            }
+        }
+    };
     {
         __shared__ int s_skip;
         if (threadIdx.x == 0) s_skip = status_word();
         __syncthreads();
         if (s_skip != 0) {
             pdl_wait();
+            if (threadIdx.x == 0) report();
             return;
         }
     }
 
     // Work assignment: heavy (late) query tiles first so that causal work is balanced.
     const int BH = p.B * p.H;
-    int bh, pair;
-    attn_work_item(p, BH, bh, pair);
-    const int b = bh / p.H, h = bh % p.H;
     const int num_m_tiles = (p.M + kAttnBlock - 1) / kAttnBlock;
     const int num_n_blocks = (p.N + kAttnBlock - 1) / kAttnBlock;
-    int mt[2], nblk[2];
-    int ntl = 0;  // live tiles in this CTA (1 or 2)
-    for (int t = 0; t < 2; ++t) {
-        mt[t] = pair * 2 + t;
-        if (mt[t] < num_m_tiles) {
-            ntl = t + 1;
-            nblk[t] = p.is_causal ? min(num_n_blocks, mt[t] + 1) : num_n_blocks;
-        } else {
+    int b, h, mt[2], nblk[2];
+    int ntl;  // live tiles of the item (1 or 2)
+    auto locate = [&](int idx) {
+        int bh, pair;
+        attn_work_item(p, BH, idx, bh, pair);
+        b = bh / p.H;
+        h = bh % p.H;
+        ntl = 0;
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+            mt[t] = pair * 2 + t;
             nblk[t] = 0;
+            if (mt[t] < num_m_tiles) {
+                ntl = t + 1;
+                nblk[t] = p.is_causal ? min(num_n_blocks, mt[t] + 1) : num_n_blocks;
+            }
         }
-    }
+    };
+    locate((int)blockIdx.x);
     const int max_blk = max(nblk[0], nblk[1]);
 
     if (threadIdx.x == 0) {
@@ -319,6 +386,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 mbar_init(m_empty(t, bf), 4);  // the tile's softmax warps
             }
             mbar_init(o_final(t), 2);  // the last product, and the issuer itself, for s_expired
+            mbar_init(q_empty(t), 1);
+            mbar_init(o_free(t), 4);
+            mbar_init(item_full(t), 1);
+            mbar_init(item_free(t), 9);  // the softmax warps and the issuer
         }
         for (int s = 0; s < KVS; ++s) {
             mbar_init(k_full(s), 1);
@@ -338,6 +409,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tma_prefetch_desc(&tmap_q);
         tma_prefetch_desc(&tmap_k);
         tma_prefetch_desc(&tmap_v);
+        if (MODE == 0 && p.o_bulk) tma_prefetch_desc(&tmap_o);
     }
     tc_fence_before();
     __syncthreads();
@@ -376,30 +448,65 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         nblk[1] = bits_count_below(act, nblk[1]);
     }
     // from here on nblk counts the blocks that a tile visits; both tiles visit a prefix of the same list
-    const int visits = max(nblk[0], nblk[1]);
+    // The CTA's item number `u` + 1, as the producer has drawn it (MODE 0): false when there is none. `warp_wide`: called by a whole warp.
+    auto next_item = [&](int u, bool warp_wide, bool& ok) -> bool {
+        if (MODE != 0) return false;
+        if (!mbar_wait(item_full(u & 1), (uint32_t)((u >> 1) & 1), abort_flag, 500)) { ok = false; return false; }
+        const int idx = items[u & 1];
+        if (warp_wide) __syncwarp();
+        if (!warp_wide || lane == 0) mbar_arrive(item_free(u & 1));
+        if (idx < 0) return false;
+        locate(idx);
+        return true;
+    };
     auto next_blk = [&](int from) { return MODE == 1 ? bits_next(act, from) : from; };
 
     if (warp >= 8) {
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kAttnRegsLow));
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(attn_regs_low(MODE)));
       if (warp == 8) {
         // ------------------------------------------------------------------ TMA producer
         if (elect_one()) {
             bool ok = true;
-            int jb = next_blk(0);
-            for (int j = 0; j < visits && ok; ++j, jb = next_blk(jb + 1)) {
-                const int s = j % KVS;
-                const uint32_t ph = (uint32_t)((j / KVS) & 1);
-                if (!mbar_wait(k_empty(s), ph ^ 1, abort_flag, 100)) { ok = false; break; }
-                mbar_arrive_expect_tx(k_full(s), TILE);
-                for (int c = 0; c < D / 64; ++c)
-                    tma_load_4d(k_smem + s * TILE + c * CHUNK, &tmap_k, k_full(s), c * 64,
-                                jb * kAttnBlock, h / p.kv_group, b);
-                if (!mbar_wait(v_empty(s), ph ^ 1, abort_flag, 101)) { ok = false; break; }
-                mbar_arrive_expect_tx(v_full(s), TILE);
-                for (int c = 0; c < D / 64; ++c)
-                    tma_load_4d(v_smem + s * TILE + c * CHUNK, &tmap_v, v_full(s), c * 64,
-                                jb * kAttnBlock, h / p.kv_group, b);
+            int kv = 0;                 // ring position, running over the CTA's items (as every barrier's phase does)
+            int seen[2] = {ntl > 0, ntl > 1};  // items in which a tile was live: their Q has been asked for
+            for (int u = 0; ok; ++u) {
+                const int visits = max(nblk[0], nblk[1]);
+                int jb = next_blk(0);
+                for (int j = 0; j < visits && ok; ++j, ++kv, jb = next_blk(jb + 1)) {
+                    const int s = kv % KVS;
+                    const uint32_t ph = (uint32_t)((kv / KVS) & 1);
+                    if (!mbar_wait(k_empty(s), ph ^ 1, abort_flag, 100)) { ok = false; break; }
+                    mbar_arrive_expect_tx(k_full(s), TILE);
+                    for (int c = 0; c < D / 64; ++c)
+                        tma_load_4d(k_smem + s * TILE + c * CHUNK, &tmap_k, k_full(s), c * 64,
+                                    jb * kAttnBlock, h / p.kv_group, b);
+                    if (!mbar_wait(v_empty(s), ph ^ 1, abort_flag, 101)) { ok = false; break; }
+                    mbar_arrive_expect_tx(v_full(s), TILE);
+                    for (int c = 0; c < D / 64; ++c)
+                        tma_load_4d(v_smem + s * TILE + c * CHUNK, &tmap_v, v_full(s), c * 64,
+                                    jb * kAttnBlock, h / p.kv_group, b);
+                }
+                if (MODE != 0 || !ok) break;
+                // The item's last block is on its way, so the item is two blocks from its end: time to draw the next one. (A CTA
+                // that is busy with a long item should not hold back one that an idle CTA could start.)
+                if (u >= 2 && !mbar_wait(item_free(u & 1), (uint32_t)(((u >> 1) - 1) & 1), abort_flag, 102)) { ok = false; break; }
+                const int drawn = draws ? (int)gridDim.x + (int)atomicAdd(&queue[0], 1u) : num_items;
+                items[u & 1] = drawn < num_items ? drawn : -1;
+                mbar_arrive(item_full(u & 1));
+                if (drawn >= num_items) {
+                    pdl_launch_dependents();  // nothing more to draw: a dependent launch may take the SM once this item is done
+                    break;
+                }
+                locate(drawn);
+                for (int t = 0; t < ntl; ++t) {
+                    if (seen[t] > 0 && !mbar_wait(q_empty(t), (uint32_t)((seen[t] - 1) & 1), abort_flag, 103)) { ok = false; break; }
+                    ++seen[t];
+                    mbar_arrive_expect_tx(q_full(t), TILE);
+                    for (int c = 0; c < D / 64; ++c)
+                        tma_load_4d(q_smem + t * TILE + c * CHUNK, &tmap_q, q_full(t), c * 64, mt[t] * kAttnBlock, h, b);
+                }
             }
+            report();
             if (!ok) {
                 for (int i = 0; i < 64; ++i) __nanosleep(2000);
             }
@@ -441,50 +548,64 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                               (accumulate || ks > 0) ? 1u : 0u);
                 }
             };
-            for (int t = 0; t < ntl && ok; ++t)
-                if (!mbar_wait(q_full(t), 0, abort_flag, 200)) ok = false;
-            if (ok && visits > 0) {
-                if (!mbar_wait(k_full(0), 0, abort_flag, 201)) ok = false;
-                if (ok) {
+            int kv = 0;             // ring position of the item's first block
+            int cnt[2] = {0, 0};    // blocks of each tile in the items before
+            int seen[2] = {0, 0};   // items before in which the tile was live
+            for (int u = 0; ok; ++u) {
+                const int visits = max(nblk[0], nblk[1]);
+                // the first scores, while the softmax warps are still storing the item before: S_t is free, since that
+                // item's last P·V has been issued ahead of this product
+                if (!mbar_wait(k_full(kv % KVS), (uint32_t)((kv / KVS) & 1), abort_flag, 201)) { ok = false; break; }
+                for (int t = 0; t < ntl && ok; ++t) {
+                    if (!mbar_wait(q_full(t), (uint32_t)(seen[t] & 1), abort_flag, 200)) { ok = false; break; }
                     tc_fence_after();
-                    for (int t = 0; t < ntl; ++t) {
-                        if (nblk[t] > 0) {
-                            issue_qk(t, 0);
-                            tc_commit(s_full(t));
-                        }
-                    }
-                    tc_commit(k_empty(0));
-                }
-            }
-            for (int j = 0; j < visits && ok; ++j) {
-                const int s = j % KVS;
-                const uint32_t ph = (uint32_t)((j / KVS) & 1);
-                const int s1 = (j + 1) % KVS;
-                const uint32_t ph1 = (uint32_t)(((j + 1) / KVS) & 1);
-                if (!mbar_wait(v_full(s), ph, abort_flag, 202)) { ok = false; break; }
-                if (j + 1 < visits) {
-                    if (!mbar_wait(k_full(s1), ph1, abort_flag, 203)) { ok = false; break; }
-                }
-                for (int t = 0; t < ntl; ++t) {
-                    if (j >= nblk[t]) continue;
-                    // P in halves: the first product runs while the second half's exponentials are taken
-                    if (!mbar_wait(p_full(t, 0), (uint32_t)(j & 1), abort_flag, 204)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_pv(t, s, 0, j > 0);
-                    if (!mbar_wait(p_full(t, 1), (uint32_t)(j & 1), abort_flag, 205)) { ok = false; break; }
-                    tc_fence_after();
-                    issue_pv(t, s, 1, true);
-                    if (j + 1 < nblk[t]) {
-                        issue_qk(t, s1);
-                        tc_commit(s_full(t));
-                    } else {
-                        mbar_arrive(o_final(t));
-                        tc_commit(o_final(t));
-                    }
+                    issue_qk(t, kv % KVS);
+                    tc_commit(s_full(t));
+                    if (nblk[t] == 1) tc_commit(q_empty(t));
                 }
                 if (!ok) break;
-                tc_commit(v_empty(s));
-                if (j + 1 < visits) tc_commit(k_empty(s1));
+                tc_commit(k_empty(kv % KVS));
+                for (int j = 0; j < visits && ok; ++j) {
+                    const int s = (kv + j) % KVS;
+                    const uint32_t ph = (uint32_t)(((kv + j) / KVS) & 1);
+                    const int s1 = (kv + j + 1) % KVS;
+                    const uint32_t ph1 = (uint32_t)(((kv + j + 1) / KVS) & 1);
+                    if (!mbar_wait(v_full(s), ph, abort_flag, 202)) { ok = false; break; }
+                    if (j + 1 < visits) {
+                        if (!mbar_wait(k_full(s1), ph1, abort_flag, 203)) { ok = false; break; }
+                    }
+                    for (int t = 0; t < ntl; ++t) {
+                        if (j >= nblk[t]) continue;
+                        const uint32_t pp = (uint32_t)((cnt[t] + j) & 1);
+                        // P in halves: the first product runs while the second half's exponentials are taken
+                        if (!mbar_wait(p_full(t, 0), pp, abort_flag, 204)) { ok = false; break; }
+                        if (j == 0 && seen[t] > 0) {  // the item before: O_t has been read out
+                            if (!mbar_wait(o_free(t), (uint32_t)((seen[t] - 1) & 1), abort_flag, 206)) { ok = false; break; }
+                        }
+                        tc_fence_after();
+                        issue_pv(t, s, 0, j > 0);
+                        if (!mbar_wait(p_full(t, 1), pp, abort_flag, 205)) { ok = false; break; }
+                        tc_fence_after();
+                        issue_pv(t, s, 1, true);
+                        if (j + 1 < nblk[t]) {
+                            issue_qk(t, s1);
+                            tc_commit(s_full(t));
+                            if (j + 2 == nblk[t]) tc_commit(q_empty(t));
+                        } else {
+                            mbar_arrive(o_final(t));
+                            tc_commit(o_final(t));
+                        }
+                    }
+                    if (!ok) break;
+                    tc_commit(v_empty(s));
+                    if (j + 1 < visits) tc_commit(k_empty(s1));
+                }
+                kv += visits;
+                for (int t = 0; t < 2; ++t) {
+                    cnt[t] += nblk[t];
+                    seen[t] += nblk[t] > 0;
+                }
+                if (!ok || !next_item(u, false, ok)) break;
             }
         }
       } else if (MODE == 3) {
@@ -493,6 +614,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const float mlow = mask_lowest(p.mask_dtype);
         const int64_t moff = (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1];
         bool ok = true;
+        const int visits = max(nblk[0], nblk[1]);
         for (int j = 0; j < visits && ok; ++j) {
             float a[2];
 #pragma unroll
@@ -511,30 +633,33 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         }
       }
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kAttnRegsHigh));
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(attn_regs_high(MODE)));
         // ------------------------------------------------------------------ softmax groups
         const int t = warp >> 2;        // tile handled by this group
         const int q = warp & 3;         // TMEM lane quadrant of this warp
-        if (t < ntl && nblk[t] > 0) {
-            const int row = mt[t] * kAttnBlock + q * 32 + lane;
-            const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
-            const uint32_t s_addr = lane_addr + (uint32_t)(t * 128);
-            const uint32_t o_addr = lane_addr + (uint32_t)(256 + t * 128);
-            const float c = p.scale_log2;
-            const float mlow = mask_lowest(p.mask_dtype);
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+        const uint32_t s_addr = lane_addr + (uint32_t)(t * 128);
+        const uint32_t o_addr = lane_addr + (uint32_t)(256 + t * 128);
+        const float c = p.scale_log2;
+        const float mlow = mask_lowest(p.mask_dtype);
+        // In MODE 0 the running maximum is kept in raw score units and the exponent is
+        // (s - m_ref) * c; otherwise scores are first moved to the log2 domain (s*c + mask).
+        const float unit = (MODE == 0) ? c : 1.0f;
+        int cnt = 0, seen = 0;  // blocks of this tile in the items before, and items in which it was live
+        bool ok = true;
+        for (int u = 0; ok; ++u) {
+          const int m0 = t == 0 ? mt[0] : mt[1], nb = t == 0 ? nblk[0] : nblk[1];
+          if (t < ntl && nb > 0) {
+            const int row = m0 * kAttnBlock + q * 32 + lane;
             const int64_t mask_row_off =
                 (MODE == 2 && p.mask != nullptr)
                     ? (int64_t)b * p.mask_strides[0] + (int64_t)h * p.mask_strides[1] + (int64_t)min(row, p.M - 1) * p.mask_strides[2]
                     : 0;
-            // In MODE 0 the running maximum is kept in raw score units and the exponent is
-            // (s - m_ref) * c; otherwise scores are first moved to the log2 domain (s*c + mask).
-            const float unit = (MODE == 0) ? c : 1.0f;
             float m_ref = -INFINITY;
             float l = 0.f;
-            bool ok = true;
             int jb = next_blk(0);
-            for (int j = 0; j < nblk[t]; ++j, jb = next_blk(jb + 1)) {
-                if (!mbar_wait(s_full(t), (uint32_t)(j & 1), abort_flag, 300 + t)) { ok = false; break; }
+            for (int j = 0; j < nb; ++j, jb = next_blk(jb + 1)) {
+                if (!mbar_wait(s_full(t), (uint32_t)((cnt + j) & 1), abort_flag, 300 + t)) { ok = false; break; }
                 tc_fence_after();
                 uint32_t sr[4][32];
 #pragma unroll
@@ -542,7 +667,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 tmem_ld_wait();
 
                 const int col0 = jb * kAttnBlock;
-                const bool causal_edge = p.is_causal && col0 + kAttnBlock - 1 > mt[t] * kAttnBlock;
+                const bool causal_edge = p.is_causal && col0 + kAttnBlock - 1 > m0 * kAttnBlock;
                 if (MODE == 1 || MODE == 3) {
                     if (MODE == 3 && !mbar_wait(m_full(t, j & 1), (uint32_t)((j >> 1) & 1), abort_flag, 320 + t)) { ok = false; break; }
                     const float4* ms = reinterpret_cast<const float4*>(mask_smem + (MODE == 1 ? col0 : (t * 2 + (j & 1)) * kAttnBlock));
@@ -646,13 +771,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         sr[cch][2 * i + 1] = __float_as_uint(e1);
                         pk[i] = Elem<T>::pack2(e0, e1);
                     }
-                    tmem_st_32x16(s_addr + cch * 16, pk);
-                    if (cch & 1) {
+                    // (the first half is handed over once the third quarter's exponentials are under way: waiting for its store
+                    // right away leaves the special-function unit idle for the store's latency)
+                    if (cch >= 2) {
+                        if (cch == 3) tmem_st_32x16(s_addr + cch * 16, pk);
                         tmem_st_wait();
                         tc_fence_before();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(p_full(t, cch >> 1));
+                        if (lane == 0) mbar_arrive(p_full(t, cch - 2));
                     }
+                    if (cch < 3) tmem_st_32x16(s_addr + cch * 16, pk);
                 }
 #pragma unroll
                 for (int cch = 0; cch < 4; ++cch) {
@@ -661,12 +789,45 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 }
                 l += (lp[0] + lp[1]) + (lp[2] + lp[3]);
             }
-            pdl_launch_dependents();  // the key loop is over: a dependent launch may take the slots that free up
+            if (MODE != 0) pdl_launch_dependents();  // the key loop is over: a dependent launch may take the slots that free up
             // ---- epilogue: O / l -> global
-            if (ok && mbar_wait(o_final(t), 0, abort_flag, 310 + t)) {
-                tc_fence_after();
-                const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
-                const float inv_l = 1.0f / l;
+            if (!ok || !mbar_wait(o_final(t), (uint32_t)(seen & 1), abort_flag, 310 + t)) { ok = false; break; }
+            tc_fence_after();
+            const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
+            const float inv_l = 1.0f / l;
+            if (MODE == 0 && p.o_bulk) {
+                // Boxes of 32 rows x 64 columns through shared memory to bulk stores (rows of 128 bytes, 128-byte swizzle; rows
+                // beyond M and columns beyond the head dimension are left out): a thread per row stores 16 bytes to each of 32 lines
+                // at a time, 2600 cycles per item in which the tile's next scores wait.
+                uint8_t* mine = smem + Cfg::kOutOffset + warp * Cfg::kOutWarpBytes;
+                uint32_t orr[4][32];
+#pragma unroll
+                for (int dch = 0; dch < 4; ++dch) tmem_ld_32x32(o_addr + dch * 32, orr[dch]);
+                tmem_ld_wait();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(o_free(t));
+#pragma unroll
+                for (int hf = 0; hf < 2; ++hf) {
+                    if (lane == 0) bulk_wait_read();  // the box before this one has left the buffer
+                    __syncwarp();
+#pragma unroll
+                    for (int v = 0; v < 8; ++v) {
+                        const uint32_t (&w)[32] = orr[hf * 2 + v / 4];
+                        uint32_t o4[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            o4[i] = Elem<T>::pack2(__uint_as_float(w[(v & 3) * 8 + 2 * i]) * inv_l, __uint_as_float(w[(v & 3) * 8 + 2 * i + 1]) * inv_l);
+                        *reinterpret_cast<uint4*>(mine + lane * 128 + ((v ^ (lane & 7)) * 16)) = make_uint4(o4[0], o4[1], o4[2], o4[3]);
+                    }
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (lane == 0 && m0 * kAttnBlock + q * 32 < m_end) {
+                        tma_store_4d(&tmap_o, smem_u32(mine), hf * 64, m0 * kAttnBlock + q * 32, h, b);
+                        bulk_commit();
+                    }
+                }
+            } else {
                 T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                            (int64_t)row * p.o_strides[2];
                 const bool vec = p.o_strides[3] == 1 && ((((uintptr_t)o_row) & 15) == 0);
@@ -683,8 +844,16 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         else attn_store_32<T, true>(o_row, dch * 32, p.o_strides[3], vec, val, p.d_out);
                     }
                 }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(o_free(t));
             }
+            cnt += nb;
+            ++seen;
+          }
+          if (!next_item(u, true, ok)) break;
         }
+        if (MODE == 0 && p.o_bulk && lane == 0) bulk_wait_all();
     }
 
     tc_fence_before();
@@ -698,10 +867,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 template <typename T, int D, int MODE>
 static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     using Cfg = AttnCfg<D>;
-    CUtensorMap tq, tk, tv;
+    CUtensorMap tq, tk, tv, to;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;
-    auto enc = [&](CUtensorMap* out, const void* ptr, int64_t rows, const int64_t* st, int64_t heads) -> int {
+    auto enc = [&](CUtensorMap* out, const void* ptr, int64_t rows, const int64_t* st, int64_t heads, int box_rows = kAttnBlock) -> int {
         if (st[3] != 1) return KB_ERR_UNSUPPORTED;
         const uint64_t dims[4] = {(uint64_t)p.D, (uint64_t)rows, (uint64_t)heads, (uint64_t)p.B};  // boxes reach to D: zero fill
         // A dimension of extent 1 may carry any stride in the caller's tensor; TMA still wants a
@@ -710,7 +879,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
             return (extent == 1) ? 16u : (uint64_t)stride * 2u;
         };
         const uint64_t strides[4] = {0, fix(rows, st[2]), fix(heads, st[1]), fix(p.B, st[0])};
-        const uint32_t box[4] = {64, (uint32_t)kAttnBlock, 1, 1};
+        const uint32_t box[4] = {64, (uint32_t)box_rows, 1, 1};
         return encode_tmap_16bit(out, ptr, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     };
@@ -722,6 +891,19 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     if (st != KB_OK) return st;
 
     AttnDev d;
+    // Bulk stores want rows, heads and batches of the result at whole 16 bytes; anything else is stored by the threads.
+    const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
+    d.num_pairs = (num_m_tiles + 1) / 2;
+    const int64_t items = (int64_t)d.num_pairs * p.B * p.H;
+    if (items > 0x3fffffff) return KB_ERR_UNSUPPORTED;
+    d.o_bulk = 0;
+    to = tq;
+    if (MODE == 0 && p.o_strides[3] == 1 && (((uintptr_t)p.o) & 15) == 0) {
+        const int64_t extent[3] = {p.B, p.H, p.M};
+        bool whole = true;
+        for (int i = 0; i < 3; ++i) whole = whole && (extent[i] == 1 || (p.o_strides[i] > 0 && p.o_strides[i] % 8 == 0));
+        if (whole && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK) d.o_bulk = 1;
+    }
     d.o = p.o;
     d.mask = p.mask;
     for (int i = 0; i < 4; ++i) {
@@ -737,22 +919,27 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
         const int64_t per16 = (p.mask_dtype == KB_F32) ? 4 : 8;  // elements per 16 bytes
         d.mask_vec = (p.mask_strides[0] % per16 == 0 && p.mask_strides[1] % per16 == 0 && p.mask_strides[2] % per16 == 0) ? 1 : 0;
     }
-    const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
-    d.num_pairs = (num_m_tiles + 1) / 2;
     d.head_group = attn_head_group(p.B * p.H, p.N, p.D);
     d.kv_group = (int)kv_group;
     d.d_out = (int)p.D;
 
     static PerDeviceOnce attr_once;
     if (!attr_once.run([] {
-            return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase + (MODE == 3 ? Cfg::kMaskRingBytes : 0)) == cudaSuccess;
+            const int most = MODE == 0 ? Cfg::kSmemMode0 : MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase + (MODE == 3 ? Cfg::kMaskRingBytes : 0);
+            return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
-    const int64_t grid = (int64_t)d.num_pairs * p.B * p.H;
-    if (grid > 0x7fffffff) return KB_ERR_UNSUPPORTED;
-    if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads,
-                   (size_t)Cfg::kSmemBase + (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : MODE == 3 ? Cfg::kMaskRingBytes : 0), stream, tq, tk, tv, d) != cudaSuccess)
+    int64_t grid = items;
+    unsigned int* queue = nullptr;
+    if (MODE == 0) {
+        // one CTA per SM that draws its items; a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
+        grid = items < gemm_sms() ? items : gemm_sms();
+        queue = attention_queue_slot();
+        if (queue == nullptr) return KB_ERR_LAUNCH;
+    }
+    const size_t smem_bytes = MODE == 0 ? (size_t)Cfg::kSmemMode0 : (size_t)Cfg::kSmemBase +
+        (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : MODE == 3 ? Cfg::kMaskRingBytes : 0);
+    if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads, smem_bytes, stream, tq, tk, tv, to, d, (int)items, queue) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }

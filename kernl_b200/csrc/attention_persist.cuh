@@ -27,13 +27,6 @@
 
 namespace kb {
 
-// Work queues. A launch takes the next slot (host-side round robin) and its CTAs draw tile numbers
-// from slot[0]; slot[1] counts CTAs that have finished, and the last one puts both words back to
-// zero, so a slot is clean again when its launch ends — also when the launch gave up on an expired
-// wait. Two launches would have to be in flight kAttnQueueSlots launches apart to share a slot.
-constexpr int kAttnQueueSlots = 1024;
-__device__ unsigned int g_attn_queue[kAttnQueueSlots][2];
-
 // Optional time stamps for tuning (compiled in with -DKB_ATTN_TRACE only): per CTA and tile, when the
 // tile was published, when the softmax warps began it, when its first scores were ready, when its key
 // loop and its epilogue ended (%globaltimer, ns); slot 15 of a CTA holds start, end, SM id and tiles.
@@ -904,28 +897,6 @@ static bool attention_persist_applicable(const kb_attn_params& p, int mode) {
 }
 
 static int g_attn_sort_batches = 1;  // test hook (kb_debug_attention_persistent: bit 1 of the mode switches it off)
-
-// The next queue slot on the current device. g_attn_queue is a host-side handle; its device address
-// is looked up once per device (with that device current) and kept.
-static unsigned int* attention_queue_slot() {
-    static unsigned int* base[64] = {};
-    static std::mutex mu;
-    static std::atomic<unsigned> next_slot{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (base[dev] == nullptr) {
-            void* ptr = nullptr;
-            if (cudaGetSymbolAddress(&ptr, g_attn_queue) != cudaSuccess || ptr == nullptr) {
-                cudaGetLastError();
-                return nullptr;
-            }
-            base[dev] = reinterpret_cast<unsigned int*>(ptr);
-        }
-    }
-    return base[dev] + 2 * (next_slot.fetch_add(1) % (unsigned)kAttnQueueSlots);
-}
 
 template <typename T, int MODE>
 static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream) {

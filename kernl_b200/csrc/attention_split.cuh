@@ -195,7 +195,7 @@ attention_split_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_
 
     const int BH = p.B * p.H;
     int bh, mt;  // (batch, head) and query tile
-    attn_work_item(p, BH, bh, mt);
+    attn_work_item(p, BH, (int)blockIdx.x, bh, mt);
     const int b = bh / p.H, h = bh % p.H;
     const int hk = h / p.kv_group;  // K/V head of this query head
     const int num_n_blocks = (p.N + kBlkN - 1) / kBlkN;

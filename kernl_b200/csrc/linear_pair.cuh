@@ -114,17 +114,6 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                  : "memory");
 }
 
-// Asynchronous store of a box from shared memory; rows and columns beyond the tensor's end are left out.
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(reinterpret_cast<uint64_t>(map)),
-                 "r"(src), "r"(x), "r"(y)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// This thread's stores have read their shared memory / have been written.
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
 // Optional clock stamps for tuning (compiled in with -DKB_GEMM_TRACE only): per CTA and for its first
 // eight tiles, clock64 of: 0 issuer starts waiting for the accumulator, 1 has it, 2 has issued the
 // tile's last MMA; 3 epilogue warp 2 starts waiting for the accumulator, 4 has it, 5 is done with it; 8 its
