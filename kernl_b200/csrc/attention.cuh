@@ -92,7 +92,7 @@ struct AttnDev {
     int mask_vec;   // mask rows can be read with aligned 128-bit loads
     int mask_lead;  // the mask's address modulo 16 (head dimension 64, staged per-row masks)
     int num_pairs;  // ceil(ceil(M/128)/2)
-    int o_bulk;     // head dimensions above 64, no mask: the result can leave through bulk tensor stores
+    int o_bulk;     // persistent kernels: the result leaves through bulk tensor stores
     int head_group; // heads whose CTAs are interleaved (see attn_work_item)
     int kv_group;   // query heads per K/V head (grouped-query attention), >= 1
     int d_out;      // head dimension of the caller's tensors (a multiple of 8, at most the kernel's D): the
@@ -148,6 +148,14 @@ static int attn_head_group(int64_t BH, int64_t N, int64_t D) {
     if (g < 1) g = 1;
     if (g > BH) g = BH;
     return (int)g;
+}
+
+// Bulk stores want rows, heads and batches of the result at whole 16 bytes; anything else is stored by the threads.
+static bool attn_bulk_out(const kb_attn_params& p) {
+    const int64_t extent[3] = {p.B, p.H, p.M};
+    bool whole = p.o_strides[3] == 1 && (((uintptr_t)p.o) & 15) == 0;
+    for (int i = 0; i < 3; ++i) whole = whole && (extent[i] == 1 || (p.o_strides[i] > 0 && p.o_strides[i] % 8 == 0));
+    return whole;
 }
 
 template <int D>
@@ -891,19 +899,12 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     if (st != KB_OK) return st;
 
     AttnDev d;
-    // Bulk stores want rows, heads and batches of the result at whole 16 bytes; anything else is stored by the threads.
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
     d.num_pairs = (num_m_tiles + 1) / 2;
     const int64_t items = (int64_t)d.num_pairs * p.B * p.H;
     if (items > 0x3fffffff) return KB_ERR_UNSUPPORTED;
-    d.o_bulk = 0;
-    to = tq;
-    if (MODE == 0 && p.o_strides[3] == 1 && (((uintptr_t)p.o) & 15) == 0) {
-        const int64_t extent[3] = {p.B, p.H, p.M};
-        bool whole = true;
-        for (int i = 0; i < 3; ++i) whole = whole && (extent[i] == 1 || (p.o_strides[i] > 0 && p.o_strides[i] % 8 == 0));
-        if (whole && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK) d.o_bulk = 1;
-    }
+    d.o_bulk = MODE == 0 && attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK ? 1 : 0;
+    if (!d.o_bulk) to = tq;  // (not used)
     d.o = p.o;
     d.mask = p.mask;
     for (int i = 0; i < 4; ++i) {

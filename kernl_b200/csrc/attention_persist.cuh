@@ -146,7 +146,7 @@ __device__ __forceinline__ void stage_mask_row(const AttnDev& p, int b, int h, f
 template <typename T, int MODE>
 __global__ void __launch_bounds__(AttnPersistCfg::kThreads, 2)
 attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
-                         const __grid_constant__ CUtensorMap tmap_v, const AttnDev p, const int num_items,
+                         const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const AttnDev p, const int num_items,
                          const int mask_cols, unsigned int* const queue, const int sort_batches) {
     using Cfg = AttnPersistCfg;
     constexpr int D = 64;
@@ -257,6 +257,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
                 tma_prefetch_desc(&tmap_q);
                 tma_prefetch_desc(&tmap_k);
                 tma_prefetch_desc(&tmap_v);
+                if (p.o_bulk) tma_prefetch_desc(&tmap_o);
                 for (int s = 0; s < 2; ++s) {
                     mbar_init(item_full(s), 1);
                     mbar_init(slot_free(s), 9);  // eight softmax warps + the issuer's last Q·Kᵀ of the tile
@@ -677,6 +678,13 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             if (!mbar_wait(item_full(slot), (uint32_t)((it >> 1) & 1), abort_flag, 730)) { ok = false; break; }
             const int bh = items[slot].bh;
             if (bh < 0) break;
+            if (p.o_bulk && it > 0) {  // the tile before: its results have left its Q buffer
+                if (lane == 0) {
+                    bulk_wait_read();
+                    mbar_arrive(slot_free(slot ^ 1));
+                }
+                __syncwarp();
+            }
 #ifdef KB_ATTN_TRACE
             if (threadIdx.x == 0) KB_TRACE(it, 1, trace_now());
 #endif
@@ -807,7 +815,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #endif
             // the key loop is over: this warp no longer reads the slot's mask row or item
             __syncwarp();
-            if (lane == 0) mbar_arrive(slot_free(slot));
+            if (!p.o_bulk && lane == 0) mbar_arrive(slot_free(slot));
             // ---- epilogue: merge the two halves of every row, O / l -> global
             // a half that never saw a finite score (all of its columns beyond N) must not set the scale
             const float m_own = (l > 0.f) ? m_ref * unit : -INFINITY;
@@ -834,13 +842,31 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(o_free);  // the issuer may overwrite O with the next tile's first P·V
+            float val[32];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) val[i] = fmaf(__uint_as_float(oa[i]), wa, __uint_as_float(ob[i]) * wb);
             T* o_row = reinterpret_cast<T*>(p.o) + (int64_t)b * p.o_strides[0] + (int64_t)h * p.o_strides[1] +
                        (int64_t)row * p.o_strides[2];
             const bool vec = p.o_strides[3] == 1 && ((((uintptr_t)o_row) & 15) == 0);
-            if (row < m_end) {
-                float val[32];
+            if (p.o_bulk) {
+                // 32 rows x 32 columns per warp through the tile's own Q buffer (its last product is complete; the next tile's Q is in the
+                // other one) to a bulk store: a thread per row writes 16 bytes to each of 32 lines at a time, 2.1 us per tile.
+                // Rows of 64 bytes, 64-byte swizzle; rows beyond M and columns beyond the head dimension are left out.
+                uint8_t* mine = smem + slot * QTILE + warp * 2048;
 #pragma unroll
-                for (int i = 0; i < 32; ++i) val[i] = fmaf(__uint_as_float(oa[i]), wa, __uint_as_float(ob[i]) * wb);
+                for (int v = 0; v < 4; ++v) {
+                    uint32_t w[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) w[i] = Elem<T>::pack2(val[v * 8 + 2 * i], val[v * 8 + 2 * i + 1]);
+                    *reinterpret_cast<uint4*>(mine + lane * 64 + ((v ^ ((lane >> 1) & 3)) * 16)) = make_uint4(w[0], w[1], w[2], w[3]);
+                }
+                fence_proxy_async_smem();
+                __syncwarp();
+                if (lane == 0 && mt * kAttnBlock + q * 32 < m_end && hf * 32 < p.d_out) {
+                    tma_store_4d(&tmap_o, smem_u32(mine), hf * 32, mt * kAttnBlock + q * 32, h, b);
+                    bulk_commit();
+                }
+            } else if (row < m_end) {
                 if (hf * 32 + 32 <= p.d_out) attn_store_32<T, false>(o_row, hf * 32, p.o_strides[3], vec, val, p.d_out);
                 else attn_store_32<T, true>(o_row, hf * 32, p.o_strides[3], vec, val, p.d_out);
             }
@@ -848,6 +874,7 @@ attention_persist_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
             if (threadIdx.x == 0) KB_TRACE(it, 4, trace_now());
 #endif
         }
+        if (p.o_bulk && lane == 0) bulk_wait_all();
       }
     }
 
@@ -901,16 +928,16 @@ static int g_attn_sort_batches = 1;  // test hook (kb_debug_attention_persistent
 template <typename T, int MODE>
 static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream) {
     using Cfg = AttnPersistCfg;
-    CUtensorMap tq, tk, tv;
+    CUtensorMap tq, tk, tv, to;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;
-    auto enc = [&](CUtensorMap* out, const void* ptr, int64_t rows, const int64_t* st, uint32_t box_rows, int64_t heads) -> int {
+    auto enc = [&](CUtensorMap* out, const void* ptr, int64_t rows, const int64_t* st, uint32_t box_rows, int64_t heads, bool out_box = false) -> int {
         if (st[3] != 1) return KB_ERR_UNSUPPORTED;
         const uint64_t dims[4] = {(uint64_t)p.D, (uint64_t)rows, (uint64_t)heads, (uint64_t)p.B};  // the box reaches to 64: zero fill
         auto fix = [](int64_t extent, int64_t stride) -> uint64_t { return (extent == 1) ? 16u : (uint64_t)stride * 2u; };
         const uint64_t strides[4] = {0, fix(rows, st[2]), fix(heads, st[1]), fix(p.B, st[0])};
-        const uint32_t box[4] = {64, box_rows, 1, 1};
-        return encode_tmap_16bit(out, ptr, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B,
+        const uint32_t box[4] = {out_box ? 32u : 64u, box_rows, 1, 1};
+        return encode_tmap_16bit(out, ptr, 4, dims, strides, box, out_box ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
                                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B);
     };
     int st = enc(&tq, p.q, p.M, p.q_strides, kAttnBlock, p.H);
@@ -921,6 +948,8 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     if (st != KB_OK) return st;
 
     AttnDev d;
+    d.o_bulk = attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, 32, p.H, true) == KB_OK ? 1 : 0;
+    if (!d.o_bulk) to = tq;  // (not used)
     d.o = p.o;
     d.mask = p.mask;
     for (int i = 0; i < 4; ++i) {
@@ -972,7 +1001,7 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
                               (p.mask_dtype == KB_F16 || p.mask_dtype == KB_BF16) && p.mask_strides[3] == 1 && p.N % 8 == 0 &&
                               p.mask_strides[0] % 8 == 0 && (((uintptr_t)p.mask) & 15) == 0)
                                  ? 1 : 0;
-    if (launch_pdl(attention_persist_kernel<T, MODE>, (unsigned)grid, (unsigned)Cfg::kThreads, smem_bytes, stream, tq, tk, tv, d,
+    if (launch_pdl(attention_persist_kernel<T, MODE>, (unsigned)grid, (unsigned)Cfg::kThreads, smem_bytes, stream, tq, tk, tv, to, d,
                    (int)tiles, mask_cols, queue, sort_batches) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;

@@ -674,6 +674,7 @@ static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t strea
     if (st != KB_OK) return st;
 
     AttnDev d;
+    d.o_bulk = 0;
     d.o = p.o;
     d.mask = p.mask;
     for (int i = 0; i < 4; ++i) {

@@ -1,4 +1,4 @@
-"""Head dimensions above 64 without a mask: several pairs of query tiles per CTA, drawn from the device-side counter."""
+"""Persistent attention: several query tiles (head dimensions above 64: pairs of them) per CTA, drawn from a device-side counter."""
 import pytest
 import torch
 
@@ -10,7 +10,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("layout", ["heads_first", "heads_last", "odd_rows"])  # odd_rows: no bulk stores
 @pytest.mark.parametrize("B, H, HK, M, N, D, causal", [(5, 16, 16, 700, 700, 128, True), (3, 52, 13, 129, 257, 128, False), (38, 8, 2, 128, 64, 72, False),
-                                                       (7, 12, 12, 513, 300, 104, True), (75, 4, 4, 385, 640, 128, False)])
+                                                       (7, 12, 12, 513, 300, 104, True), (75, 4, 4, 385, 640, 128, False),
+                                                       (5, 16, 16, 700, 700, 64, True), (30, 12, 3, 200, 130, 64, False), (25, 12, 12, 129, 77, 40, False),
+                                                       (40, 8, 8, 127, 65, 24, False)])
 def test_items(B, H, HK, M, N, D, causal, layout, dtype):
     from kernl_b200.implementations.attention import attention_forward
 
