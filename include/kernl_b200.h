@@ -131,6 +131,11 @@ typedef struct {
 
 int kb_rope_kv_write(const kb_rope_params* p, void* stream);
 
+/* kb_linear_fwd of a stacked q/k/v projection followed by kb_rope_kv_write of its result, with the same values: in one
+ * launch where the projection's kernel can rotate and write from its accumulators, else in two. lin->y ([M, N] without gaps,
+ * M = B * S, N = 3 * H * D) is scratch: it holds the projection's result afterwards or is left as it was. rope->qkv is not read. */
+int kb_linear_rope_kv_write(const kb_linear_params* lin, const kb_rope_params* rope, void* stream);
+
 /* ---------------------------------------------------------------------------------------
  * Fused attention forward: O = softmax(sm_scale · Q·Kᵀ + mask [causal]) · V, online softmax.
  * Replaces: src/kernl/implementations/attention.py:438-529 (Attention.forward launching

@@ -26,6 +26,7 @@ EXPORTED_SYMBOLS = [
     "kb_attention_decode_scratch_bytes",
     "kb_attention_decode_fwd",
     "kb_rope_kv_write",
+    "kb_linear_rope_kv_write",
     "kb_allreduce_residual_fwd",
     "kb_peer_alloc", "kb_peer_free", "kb_peer_export", "kb_peer_open", "kb_peer_close",
     "kb_attention_decode_static_max_bytes",
@@ -122,6 +123,8 @@ def load() -> ctypes.CDLL:
     lib.kb_attention_decode_fwd_static.restype = ctypes.c_int
     lib.kb_rope_kv_write.argtypes = [POINTER(RopeParams), c_void_p]
     lib.kb_rope_kv_write.restype = ctypes.c_int
+    lib.kb_linear_rope_kv_write.argtypes = [POINTER(LinearParams), POINTER(RopeParams), c_void_p]
+    lib.kb_linear_rope_kv_write.restype = ctypes.c_int
     lib.kb_allreduce_residual_fwd.argtypes = [POINTER(AllReduceParams), c_void_p]
     lib.kb_allreduce_residual_fwd.restype = ctypes.c_int
     lib.kb_peer_alloc.argtypes = [c_int64, POINTER(c_void_p)]

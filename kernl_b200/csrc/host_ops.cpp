@@ -296,60 +296,109 @@ PyObject* decode_attention(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// rope_kv_write(qkv, k_cache, v_cache, cos, sin, pos, batch, seq) -> rotated q or None
-PyObject* rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    HANDLE_TH_ERRORS
-    if (!arity(n, 8, "rope_kv_write")) return nullptr;
-    const at::Tensor* t[5];
-    for (int i = 0; i < 5; ++i)
-        if ((t[i] = cuda_tensor(a[i])) == nullptr || t[i]->device() != t[0]->device() || !t[i]->is_contiguous()) Py_RETURN_NONE;
-    const at::Tensor &qkv = *t[0], &kc = *t[1], &vc = *t[2], &cos = *t[3], &sin = *t[4];
-    if (!is_16bit(qkv.scalar_type()) || !like(kc, qkv) || !like(vc, qkv) || cos.scalar_type() != at::kFloat || sin.scalar_type() != at::kFloat)
-        Py_RETURN_NONE;
-    const int64_t batch = PyLong_AsLongLong(a[6]), seq = PyLong_AsLongLong(a[7]);
-    if (PyErr_Occurred()) return nullptr;
-    if (kc.dim() != 4 || kc.size(0) != batch || !vc.sizes().equals(kc.sizes())) Py_RETURN_NONE;
-    const int64_t H = kc.size(1), max_seq = kc.size(2), D = kc.size(3);
-    if (qkv.dim() != 2 || qkv.size(0) != batch * seq || qkv.size(1) != 3 * H * D || !cos.sizes().equals({max_seq, D / 2}) ||
-        !sin.sizes().equals(cos.sizes()))
-        Py_RETURN_NONE;
-    kb_rope_params p{};
-    if (PyLong_Check(a[5])) {
-        p.pos_host = PyLong_AsLongLong(a[5]);
-        if (p.pos_host == -1 && PyErr_Occurred()) return nullptr;
+// The caches, tables and position of a rotary embedding with cache write: false for what the Python front-end has to look at.
+// a: k_cache, v_cache, cos, sin, pos, batch, seq
+bool rope_args(PyObject* const* a, const at::Tensor& like_this, kb_rope_params& p) {
+    const at::Tensor* t[4];
+    for (int i = 0; i < 4; ++i)
+        if ((t[i] = cuda_tensor(a[i])) == nullptr || t[i]->device() != like_this.device() || !t[i]->is_contiguous()) return false;
+    const at::Tensor &kc = *t[0], &vc = *t[1], &cos = *t[2], &sin = *t[3];
+    if (!is_16bit(like_this.scalar_type()) || !like(kc, like_this) || !like(vc, like_this) || cos.scalar_type() != at::kFloat ||
+        sin.scalar_type() != at::kFloat)
+        return false;
+    p.B = PyLong_AsLongLong(a[5]);
+    p.S = PyLong_AsLongLong(a[6]);
+    if (PyErr_Occurred()) return false;
+    if (kc.dim() != 4 || kc.size(0) != p.B || !vc.sizes().equals(kc.sizes())) return false;
+    p.H = kc.size(1);
+    p.max_seq = kc.size(2);
+    p.D = kc.size(3);
+    if (!cos.sizes().equals({p.max_seq, p.D / 2}) || !sin.sizes().equals(cos.sizes())) return false;
+    if (PyLong_Check(a[4])) {
+        p.pos_host = PyLong_AsLongLong(a[4]);
+        if (p.pos_host == -1 && PyErr_Occurred()) return false;
     } else {
-        const at::Tensor* pos = cuda_tensor(a[5]);
-        if (pos == nullptr || pos->scalar_type() != at::kLong || pos->numel() != 1 || pos->device() != qkv.device()) Py_RETURN_NONE;
+        const at::Tensor* pos = cuda_tensor(a[4]);
+        if (pos == nullptr || pos->scalar_type() != at::kLong || pos->numel() != 1 || pos->device() != like_this.device()) return false;
         p.pos_dev = pos->data_ptr<int64_t>();
     }
-    p.qkv = qkv.data_ptr();
     p.k_cache = kc.data_ptr();
     p.v_cache = vc.data_ptr();
     p.cos = cos.data_ptr<float>();
     p.sin = sin.data_ptr<float>();
-    p.B = batch;
-    p.S = seq;
-    p.H = H;
-    p.D = D;
-    p.max_seq = max_seq;
-    p.dtype = dtype_code(qkv.scalar_type());
+    p.dtype = dtype_code(like_this.scalar_type());
+    return true;
+}
+
+// rope_kv_write(qkv, k_cache, v_cache, cos, sin, pos, batch, seq) -> rotated q or None
+PyObject* rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!arity(n, 8, "rope_kv_write")) return nullptr;
+    const at::Tensor* qkv = cuda_tensor(a[0]);
+    kb_rope_params p{};
+    if (qkv == nullptr || !qkv->is_contiguous() || !rope_args(a + 1, *qkv, p)) {
+        if (PyErr_Occurred()) return nullptr;
+        Py_RETURN_NONE;
+    }
+    if (qkv->dim() != 2 || qkv->size(0) != p.B * p.S || qkv->size(1) != 3 * p.H * p.D) Py_RETURN_NONE;
+    p.qkv = qkv->data_ptr();
     at::Tensor q;
     int st;
     {
         const WithoutGil unlocked;
-        const c10::cuda::CUDAGuard guard(qkv.device());
-        q = empty({batch, seq, H, D}, qkv);
+        const c10::cuda::CUDAGuard guard(qkv->device());
+        q = empty({p.B, p.S, p.H, p.D}, *qkv);
         p.q_out = q.data_ptr();
-        st = kb_rope_kv_write(&p, stream_of(qkv));
+        st = kb_rope_kv_write(&p, stream_of(*qkv));
     }
     if (st != KB_OK) return failed("rope_kv_write", st);
     return THPVariable_Wrap(std::move(q));
     END_HANDLE_TH_ERRORS
 }
 
+// linear_rope_kv_write(x, weight, k_cache, v_cache, cos, sin, pos, batch, seq) -> rotated q or None
+PyObject* linear_rope_kv_write(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (!arity(n, 9, "linear_rope_kv_write")) return nullptr;
+    const at::Tensor *x = cuda_tensor(a[0]), *w = cuda_tensor(a[1]);
+    kb_rope_params p{};
+    if (x == nullptr || w == nullptr || autocast_on() || !rope_args(a + 2, *x, p)) {
+        if (PyErr_Occurred()) return nullptr;
+        Py_RETURN_NONE;
+    }
+    if (!like(*w, *x) || w->dim() != 2 || x->dim() != 2) Py_RETURN_NONE;
+    const int64_t M = x->size(0), K = x->size(1), N = w->size(0);
+    if (M == 0 || K % 8 != 0 || x->stride(0) % 8 != 0 || x->stride(1) != 1 || w->size(1) != K || !w->is_contiguous() || !aligned16(*x) ||
+        !aligned16(*w) || M != p.B * p.S || N != 3 * p.H * p.D)
+        Py_RETURN_NONE;
+    kb_linear_params l{};
+    l.x = x->data_ptr();
+    l.w = w->data_ptr();
+    l.M = M;
+    l.N = N;
+    l.K = K;
+    l.x_row_stride = x->stride(0);
+    l.y_row_stride = N;
+    l.dtype = p.dtype;
+    at::Tensor q;
+    int st;
+    {
+        const WithoutGil unlocked;
+        const c10::cuda::CUDAGuard guard(x->device());
+        q = empty({p.B, p.S, p.H, p.D}, *x);
+        const at::Tensor qkv = empty({M, N}, *x);  // (on this stream: given back to it when the launches are queued)
+        p.q_out = q.data_ptr();
+        l.y = qkv.data_ptr();
+        st = kb_linear_rope_kv_write(&l, &p, stream_of(*x));
+    }
+    if (st != KB_OK) return failed("linear_rope_kv_write", st);
+    return THPVariable_Wrap(std::move(q));
+    END_HANDLE_TH_ERRORS
+}
+
 #define KB_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {KB_METHOD(linear), KB_METHOD(layer_norm), KB_METHOD(attention),
-                         KB_METHOD(decode_attention), KB_METHOD(rope_kv_write), {nullptr, nullptr, 0, nullptr}};
+                         KB_METHOD(decode_attention), KB_METHOD(rope_kv_write), KB_METHOD(linear_rope_kv_write), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host_ops", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace

@@ -210,7 +210,7 @@ int kb_debug_wait_limit(int64_t in_kernel_cycles, int64_t peer_cycles) {
     return cudaDeviceSynchronize() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
 
-int kb_linear_fwd(const kb_linear_params* p, void* stream) {
+static int check_linear(const kb_linear_params* p) {
     if (p == nullptr || p->x == nullptr || p->w == nullptr || p->y == nullptr) return KB_ERR_BAD_ARG;
     if (p->M < 0 || p->N <= 0 || p->K <= 0) return KB_ERR_BAD_ARG;
     if (p->activation < KB_ACT_NONE || p->activation > KB_ACT_SWIGLU) return KB_ERR_BAD_ARG;
@@ -219,7 +219,13 @@ int kb_linear_fwd(const kb_linear_params* p, void* stream) {
     if (p->K % 8 != 0 || p->x_row_stride % 8 != 0) return KB_ERR_UNSUPPORTED;
     if (((uintptr_t)p->x & 15) || ((uintptr_t)p->w & 15)) return KB_ERR_UNSUPPORTED;
     if (p->M > 0x7fffffff || p->N > 0x7fffffff || p->K > 0x7fffffff) return KB_ERR_UNSUPPORTED;
-    int st = check_device();
+    return KB_OK;
+}
+
+int kb_linear_fwd(const kb_linear_params* p, void* stream) {
+    int st = check_linear(p);
+    if (st != KB_OK || p->M == 0) return st;
+    st = check_device();
     if (st != KB_OK) return st;
     return launch_linear(*p, (cudaStream_t)stream, g_forced_bn, g_forced_splits);
 }
@@ -284,27 +290,59 @@ int kb_attention_decode_fwd(const kb_attn_params* p, void* scratch, int64_t scra
     return launch_attention_decode(*p, scratch, scratch_bytes, (cudaStream_t)stream);
 }
 
-int kb_rope_kv_write(const kb_rope_params* p, void* stream) {
-    if (p == nullptr || p->qkv == nullptr || p->q_out == nullptr || p->k_cache == nullptr || p->v_cache == nullptr ||
-        p->cos == nullptr || p->sin == nullptr)
+static int check_rope(const kb_rope_params* p) {
+    if (p == nullptr || p->q_out == nullptr || p->k_cache == nullptr || p->v_cache == nullptr || p->cos == nullptr || p->sin == nullptr)
         return KB_ERR_BAD_ARG;
     if (p->B < 0 || p->S < 0 || p->H <= 0 || p->D <= 0 || p->max_seq <= 0) return KB_ERR_BAD_ARG;
     if (p->D % 8 != 0) return KB_ERR_UNSUPPORTED;
-    if ((((uintptr_t)p->qkv) | ((uintptr_t)p->q_out) | ((uintptr_t)p->k_cache) | ((uintptr_t)p->v_cache) |
-         ((uintptr_t)p->cos) | ((uintptr_t)p->sin)) & 15)
+    if ((((uintptr_t)p->q_out) | ((uintptr_t)p->k_cache) | ((uintptr_t)p->v_cache) | ((uintptr_t)p->cos) | ((uintptr_t)p->sin)) & 15)
         return KB_ERR_UNSUPPORTED;
-    if (p->B == 0 || p->S == 0) return KB_OK;
-    int st = check_device();
-    if (st != KB_OK) return st;
+    return KB_OK;
+}
+
+static RopeDev rope_dev(const kb_rope_params* p) {
     RopeDev d;
     d.qkv = p->qkv; d.q_out = p->q_out; d.k_cache = p->k_cache; d.v_cache = p->v_cache;
     d.cos_t = p->cos; d.sin_t = p->sin;
     d.pos_dev = reinterpret_cast<const long long*>(p->pos_dev);
     d.pos_host = p->pos_host;
     d.B = (int)p->B; d.S = (int)p->S; d.H = (int)p->H; d.D = (int)p->D; d.max_seq = (int)p->max_seq;
+    return d;
+}
+
+int kb_rope_kv_write(const kb_rope_params* p, void* stream) {
+    int st = check_rope(p);
+    if (st != KB_OK) return st;
+    if (p->qkv == nullptr) return KB_ERR_BAD_ARG;
+    if (((uintptr_t)p->qkv) & 15) return KB_ERR_UNSUPPORTED;
+    if (p->B == 0 || p->S == 0) return KB_OK;
+    st = check_device();
+    if (st != KB_OK) return st;
+    const RopeDev d = rope_dev(p);
     if (p->dtype == KB_F16) return launch_rope_t<__half>(d, (cudaStream_t)stream);
     if (p->dtype == KB_BF16) return launch_rope_t<__nv_bfloat16>(d, (cudaStream_t)stream);
     return KB_ERR_UNSUPPORTED;
+}
+
+int kb_linear_rope_kv_write(const kb_linear_params* lin, const kb_rope_params* rope, void* stream) {
+    int st = check_linear(lin);
+    if (st != KB_OK) return st;
+    st = check_rope(rope);
+    if (st != KB_OK) return st;
+    // the projection's result has to be what kb_rope_kv_write reads: [B * S, 3, H, D] without gaps
+    if (lin->M != rope->B * rope->S || lin->N != 3 * rope->H * rope->D || lin->y_row_stride != lin->N || lin->dtype != rope->dtype ||
+        lin->activation == KB_ACT_SWIGLU)
+        return KB_ERR_BAD_ARG;
+    if (lin->M == 0) return KB_OK;
+    st = check_device();
+    if (st != KB_OK) return st;
+    const RopeDev d = rope_dev(rope);
+    bool roped = false;
+    st = launch_linear(*lin, (cudaStream_t)stream, g_forced_bn, g_forced_splits, &d, &roped);
+    if (st != KB_OK || roped) return st;
+    kb_rope_params after = *rope;
+    after.qkv = lin->y;
+    return kb_rope_kv_write(&after, stream);
 }
 
 int kb_allreduce_residual_fwd(const kb_allreduce_params* p, void* stream) {

@@ -338,7 +338,9 @@ static double linear_single_us(const kb_linear_params& p) {
     return 2.8 + (p.M < 96 ? 1.3 : 0.0) + waves * (load + (linear_stores_values(p) ? 0.05 : 0.012) * bn);
 }
 template <typename T>
-static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
+static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits, const RopeDev* rope, bool* roped) {
+    // `rope`: the rotary embedding and cache write that follow; *roped says that the projection's kernel has done them
+    const RopeDev* in_pair = rope != nullptr && linear_pair_rope(p, *rope) ? rope : nullptr;
     if (forced_splits > 1) {
         const int num_k = (int)((p.K + kGemmBK - 1) / kGemmBK), most = num_k < kClMaxSplits ? num_k : kClMaxSplits;
         const int nb = forced_bn == 32 || forced_bn == 64 ? forced_bn : p.M <= 64 ? 32 : 128;
@@ -353,7 +355,10 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
         const int bn = linear_pair_tile_width(p, &pair);
         // (at thousands of rows the estimates no longer matter: the pair kernel pulls half as much W through each SM's port)
         if (g_linear_pair != 1 || pair < 0.93 * single || (p.M > 4096 && p.N >= 256)) {
-            if (pair <= cl.us) return launch_linear_pair_t<T>(p, stream, bn);
+            if (pair <= cl.us) {
+                if (in_pair != nullptr) *roped = true;
+                return launch_linear_pair_t<T>(p, stream, bn, in_pair);
+            }
         }
     }
     if (p.M <= 1024 && gemm_sms() == sm_count()) {
@@ -366,9 +371,10 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
     return launch_linear_single<T>(p, stream, 0);
 }
 
-static int launch_linear(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits) {
-    if (p.dtype == KB_F16) return launch_linear_t<__half>(p, stream, forced_bn, forced_splits);
-    if (p.dtype == KB_BF16) return launch_linear_t<__nv_bfloat16>(p, stream, forced_bn, forced_splits);
+static int launch_linear(const kb_linear_params& p, cudaStream_t stream, int forced_bn, int forced_splits, const RopeDev* rope = nullptr,
+                         bool* roped = nullptr) {
+    if (p.dtype == KB_F16) return launch_linear_t<__half>(p, stream, forced_bn, forced_splits, rope, roped);
+    if (p.dtype == KB_BF16) return launch_linear_t<__nv_bfloat16>(p, stream, forced_bn, forced_splits, rope, roped);
     return KB_ERR_UNSUPPORTED;
 }
 

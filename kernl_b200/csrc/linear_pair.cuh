@@ -26,7 +26,10 @@
 // Accumulators are double-buffered (2 x 256 columns = all of tensor memory), the ring has six stages.
 // Every bulk copy has one destination CTA: the pair's sharing happens inside the tensor-core instruction.
 #pragma once
+#include <type_traits>
+
 #include "linear.cuh"
+#include "rope.cuh"
 
 namespace kb {
 
@@ -132,13 +135,21 @@ __device__ long long g_gemm_trace[148 * 8 * 16];
 // keeps its 32 KB stride), the accumulators sit at tensor-memory columns 0 and 256 whatever BN, and an
 // epilogue warp owns BN / 4 columns. The narrower tile exists for problems of a few rounds: 384 tiles
 // of 256 columns on 74 pairs run 5.2 rounds as 6, 512 tiles of 192 columns run 6.9 rounds as 7.
-template <typename T, int BN>
+// ROPE: a stacked q/k/v projection whose results are rotated (q, k) on their way out and whose k and v go to the cache, [B, H, max_seq, D].
+// Saves the kernel behind it its pass over the projection's result (402 MB per layer at 8192 rows of [12288, 4096], 74 us).
+struct PairRope {
+    CUtensorMap k, v;  // the caches; q goes by tmap_y
+    RopeDev r;
+};
+struct NoRope {};
+template <typename T, int BN, bool ROPE = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                    const __grid_constant__ CUtensorMap tmap_y, int staged, const T* __restrict__ bias, T* __restrict__ y, T* __restrict__ act_inputs, int M, int N, int K,
-                   int64_t y_row_stride, int activation) {
+                   int64_t y_row_stride, int activation, const __grid_constant__ std::conditional_t<ROPE, PairRope, NoRope> rope) {
     constexpr int STAGES = kPairStages;
     using Cfg = PairCfg<BN>;
+    static_assert(!ROPE || BN == 256, "the rotary epilogue takes boxes of 32 columns, inside a head");
     constexpr int kStageBytes = Cfg::kStageBytes;
     constexpr int CW = Cfg::kWarpCols;
     extern __shared__ uint8_t smem_raw[];
@@ -355,6 +366,9 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                             for (int i = 0; i < 4; ++i)
                                 o[(bx * SC + c) / 4 % (kPieces * 4) + i] = Elem<T>::pack2(act_silu(z[2 * i]) * z[8 + 2 * i], act_silu(z[2 * i + 1]) * z[8 + 2 * i + 1]);
                         }
+                    } else if constexpr (ROPE) {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) o[i] = Elem<T>::pack2(__uint_as_float(r2[2 * i]), __uint_as_float(r2[2 * i + 1]));
                     } else {
 #pragma unroll
                         for (int c = 0; c < SC; c += 16) {
@@ -373,6 +387,42 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     if (gated && bx + 1 < CW / SC) {  // (half of the box only)
                         tmem_ld_wait();
                         continue;
+                    }
+                    int part = 0, b0 = 0, head = 0, d0 = 0;  // ROPE: q, k or v; the first row's sequence; head and its first column
+                    long long pos0 = 0;                      // the first row's position
+                    bool box = true;                         // the rows go out as one box
+                    if constexpr (ROPE) {
+                        const RopeDev& rp = rope.r;
+                        const int hd = rp.H * rp.D;
+                        part = ycol / hd;
+                        head = (ycol % hd) / rp.D;
+                        d0 = (ycol % hd) % rp.D;
+                        b0 = row_base / rp.S;
+                        const long long first = rp.pos_dev ? *rp.pos_dev : rp.pos_host;
+                        pos0 = first + (row_base - b0 * rp.S);
+                        const int row = row_base + lane, b = row / rp.S;
+                        const long long pos = first + (row - b * rp.S);
+                        const bool inside = pos >= 0 && pos < rp.max_seq;
+                        if (part < 2) {
+                            const int64_t at = (inside ? pos : 0) * (rp.D / 2) + d0 / 2;
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) {
+                                const float4 c4 = __ldg(reinterpret_cast<const float4*>(rp.cos_t + at) + v), s4 = __ldg(reinterpret_cast<const float4*>(rp.sin_t + at) + v);
+                                const float cs[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+#pragma unroll
+                                for (int i = 0; i < 4; ++i) {
+                                    const float2 t2 = rope_pair(Elem<T>::unpack2(o[v * 4 + i]), cs[i], ss[i]);
+                                    o[v * 4 + i] = Elem<T>::pack2(t2.x, t2.y);
+                                }
+                            }
+                        }
+                        // rows of k and v that lie in two sequences, or beyond the last one, are stored one by one
+                        box = part == 0 || (row_base + 31 < M && (row_base + 31) / rp.S == b0 && pos0 >= 0);
+                        if (!box && row < m_end && inside && ycol < N) {
+                            T* dst = reinterpret_cast<T*>(part == 1 ? rp.k_cache : rp.v_cache) + (((int64_t)b * rp.H + head) * rp.max_seq + pos) * rp.D + d0;
+#pragma unroll
+                            for (int v = 0; v < 4; ++v) reinterpret_cast<uint4*>(dst)[v] = make_uint4(o[v * 4], o[v * 4 + 1], o[v * 4 + 2], o[v * 4 + 3]);
+                        }
                     }
                     if (lane == 0) bulk_wait_read();  // the box before this one has left the buffer
                     __syncwarp();
@@ -399,7 +449,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     __syncwarp();
                     if (warp == 2 && lane == 0 && bx == 0) KB_GTRACE(ti, 9);
                     if (lane == 0 && row_base < m_end && ycol < (gated ? N / 2 : N)) {
-                        tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
+                        if constexpr (ROPE) {
+                            if (part == 0) tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
+                            else if (box) tma_store_4d(part == 1 ? &rope.k : &rope.v, smem_u32(mine), d0, (int)pos0, head, b0);
+                        } else {
+                            tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
+                        }
                         bulk_commit();
                     }
                     if (bx + 1 < CW / SC) tmem_ld_wait();
@@ -485,9 +540,20 @@ static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
     return bn;
 }
 
-template <typename T, int BN>
-static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream) {
+template <typename T, int BN, bool ROPE = false>
+static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream, const RopeDev* rope = nullptr) {
     using Cfg = PairCfg<BN>;
+    auto kernel = linear_pair_kernel<T, BN, ROPE>;
+    std::conditional_t<ROPE, PairRope, NoRope> rp;
+    if constexpr (ROPE) {
+        rp.r = *rope;
+        const uint64_t dims[4] = {(uint64_t)rope->D, (uint64_t)rope->max_seq, (uint64_t)rope->H, (uint64_t)rope->B};
+        const uint64_t row = (uint64_t)rope->D * 2, strides[4] = {0, row, row * rope->max_seq, row * rope->max_seq * rope->H};
+        const uint32_t box[4] = {32, 32, 1, 1};
+        int st = encode_tmap_16bit(&rp.k, rope->k_cache, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+        if (st == KB_OK) st = encode_tmap_16bit(&rp.v, rope->v_cache, 4, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE);
+        if (st != KB_OK) return st;
+    }
     CUtensorMap tmap_x, tmap_w, tmap_y;
     {
         const uint64_t dims[2] = {(uint64_t)p.K, (uint64_t)p.M};
@@ -505,12 +571,13 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (st != KB_OK) return st;
     }
-    const int staged = linear_pair_staged(p, BN) ? 1 : 0;
+    const int staged = ROPE || linear_pair_staged(p, BN) ? 1 : 0;
     if (staged) {
-        const uint64_t dims[2] = {(uint64_t)(p.activation == KB_ACT_SWIGLU ? p.N / 2 : p.N), (uint64_t)p.M};
-        const uint64_t strides[2] = {0, (uint64_t)p.y_row_stride * 2};
+        const int64_t cols = p.activation == KB_ACT_SWIGLU ? p.N / 2 : ROPE ? p.N / 3 : p.N;  // (ROPE: q alone)
+        const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)p.M};
+        const uint64_t strides[2] = {0, (uint64_t)(ROPE ? cols : p.y_row_stride) * 2};
         const uint32_t box[2] = {(uint32_t)Cfg::kStoreCols, 32};
-        const int st = encode_tmap_16bit(&tmap_y, p.y, 2, dims, strides, box, BN == 256 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
+        const int st = encode_tmap_16bit(&tmap_y, ROPE ? rope->q_out : p.y, 2, dims, strides, box, BN == 256 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                                          CU_TENSOR_MAP_L2_PROMOTION_NONE);
         if (st != KB_OK) return st;
     } else {
@@ -535,11 +602,11 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return KB_ERR_LAUNCH;
     int resident = max_pairs[dev].load(std::memory_order_acquire);
     if (resident == 0) {
-        if (cudaFuncSetAttribute(linear_pair_kernel<T, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
             return KB_ERR_LAUNCH;
         cfg.gridDim = dim3(2 * (unsigned)(sm_count() / 2));
         int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, linear_pair_kernel<T, BN>, &cfg) != cudaSuccess || n <= 0) {
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
             cudaGetLastError();
             return KB_ERR_LAUNCH;
         }
@@ -551,14 +618,23 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream)
     if (pairs > gemm_sms() / 2) pairs = gemm_sms() / 2;  // a caller-set limit leaves SMs to a concurrent collective
     cfg.gridDim = dim3(2 * (unsigned)pairs);
     cfg.numAttrs = g_use_pdl ? 2u : 1u;
-    if (cudaLaunchKernelEx(&cfg, linear_pair_kernel<T, BN>, tmap_x, tmap_w, tmap_y, staged, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M,
-                           (int)p.N, (int)p.K, p.y_row_stride, p.activation) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, kernel, tmap_x, tmap_w, tmap_y, staged, (const T*)p.bias, (T*)p.y, (T*)p.act_inputs, (int)p.M,
+                           (int)p.N, (int)p.K, p.y_row_stride, p.activation, rp) != cudaSuccess)
         return KB_ERR_LAUNCH;
     return cudaGetLastError() == cudaSuccess ? KB_OK : KB_ERR_LAUNCH;
 }
 
+// Whether this kernel's rotary epilogue can take the place of the launch behind the projection: heads of whole boxes of 32 columns, stored
+// at whole 16 bytes. (The streaming kernel of a decode step keeps the launch behind it: with pairs of rows as its unit and the rotation in
+// its epilogue a step of eight layers took 1031 us, 1019 without, since decode attention's first K and V arrive behind that launch.)
+static bool linear_pair_rope(const kb_linear_params& p, const RopeDev& r) {
+    return p.activation == KB_ACT_NONE && p.bias == nullptr && p.act_inputs == nullptr && p.N == 3 * (int64_t)r.H * r.D &&
+           p.M == (int64_t)r.B * r.S && r.D % 32 == 0 && ((((uintptr_t)r.q_out) | ((uintptr_t)r.k_cache) | ((uintptr_t)r.v_cache)) & 15) == 0;
+}
+
 template <typename T>
-static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream, int bn) {
+static int launch_linear_pair_t(const kb_linear_params& p, cudaStream_t stream, int bn, const RopeDev* rope = nullptr) {
+    if (rope != nullptr) return launch_linear_pair_tb<T, 256, true>(p, stream, rope);
     return bn == 192 ? launch_linear_pair_tb<T, 192>(p, stream) : launch_linear_pair_tb<T, 256>(p, stream);
 }
 

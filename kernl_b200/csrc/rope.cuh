@@ -5,6 +5,8 @@
 // caches [B, heads, max_seq, D] at that position — one launch instead of the dozen elementwise
 // kernels and two index-copies of an eager implementation. The start position comes from device
 // memory when given (so that a captured decode step stays valid as the position advances).
+// The projection of a long prompt rotates and writes from its accumulators instead (linear_pair.cuh, kb_linear_rope_kv_write); this
+// kernel follows the others.
 // Semantics: experimental/llama-v2/kernel/pytorch_reference.py:37-80 of the reference (interleaved
 // pairs, theta = 10000); its Triton counterpart is the RoPE epilogue of fused_kernel_proj_qkv.py.
 #pragma once
@@ -23,6 +25,13 @@ struct RopeDev {
     long long pos_host;
     int B, S, H, D, max_seq;
 };
+
+// A pair of neighbouring elements by the angle of its position. Every kernel that rotates gives the same bits: the elements come
+// rounded to 16 bits, as a separate projection stores them, and which product is rounded is written out (left to the compiler, it is
+// not the same one everywhere, and a deep decoder's hidden states and near-ties of its tokens change with it).
+__device__ __forceinline__ float2 rope_pair(float2 x, float c, float s) {
+    return make_float2(__fmaf_rn(x.x, c, -__fmul_rn(x.y, s)), __fmaf_rn(x.x, s, __fmul_rn(x.y, c)));
+}
 
 // One thread per (token, head, 8 consecutive elements = 4 rotation pairs).
 template <typename T>
@@ -52,10 +61,10 @@ rope_kv_write_kernel(const RopeDev p) {
         uint32_t qo[4], ko[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const float2 qf = Elem<T>::unpack2(qi[j]);
-            const float2 kf = Elem<T>::unpack2(ki[j]);
-            qo[j] = Elem<T>::pack2(qf.x * cs[j] - qf.y * ss[j], qf.x * ss[j] + qf.y * cs[j]);
-            ko[j] = Elem<T>::pack2(kf.x * cs[j] - kf.y * ss[j], kf.x * ss[j] + kf.y * cs[j]);
+            const float2 qf = rope_pair(Elem<T>::unpack2(qi[j]), cs[j], ss[j]);
+            const float2 kf = rope_pair(Elem<T>::unpack2(ki[j]), cs[j], ss[j]);
+            qo[j] = Elem<T>::pack2(qf.x, qf.y);
+            ko[j] = Elem<T>::pack2(kf.x, kf.y);
         }
         T* qdst = reinterpret_cast<T*>(p.q_out) + (tok * p.H + h) * (long long)p.D + v * 8;
         *reinterpret_cast<uint4*>(qdst) = make_uint4(qo[0], qo[1], qo[2], qo[3]);

@@ -1,4 +1,4 @@
-"""Rotary embedding + KV-cache write front-end (kb_rope_kv_write)."""
+"""Rotary embedding + KV-cache write front-ends (kb_rope_kv_write, kb_linear_rope_kv_write)."""
 from typing import Optional, Union
 
 import torch
@@ -32,3 +32,15 @@ def rope_kv_write(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tenso
     with torch.cuda.device(qkv.device):
         _lib.check(_lib.load().kb_rope_kv_write(p, _lib.current_stream(qkv.device)), "rope_kv_write")
     return q_out
+
+
+def linear_rope_kv_write(x: torch.Tensor, weight: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, cos: torch.Tensor,
+                         sin: torch.Tensor, pos: Union[int, torch.Tensor], batch: int, seq: int) -> torch.Tensor:
+    """`rope_kv_write(linear_layer(x, weight, None), ...)` for a stacked q/k/v projection, weight [3*H*D, K], with the same values:
+    in one launch where the projection's kernel can rotate and write from its accumulators, else in two."""
+    done = _lib.native().linear_rope_kv_write(x, weight, k_cache, v_cache, cos, sin, pos, batch, seq)
+    if done is not None:
+        return done
+    from kernl_b200.implementations.linear_layer import linear_layer
+
+    return rope_kv_write(linear_layer(x, weight, None), k_cache, v_cache, cos, sin, pos, batch, seq)

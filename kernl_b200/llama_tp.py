@@ -82,6 +82,13 @@ class CudaOps:
         return rope_kv_write(qkv, k_cache, v_cache, cos, sin, pos, batch, seq)
 
     @staticmethod
+    def linear_rope_kv_write(x, w, k_cache, v_cache, cos, sin, pos, batch, seq):
+        """The q/k/v projection with rotation and cache write in its epilogue, where its kernel has one."""
+        from kernl_b200.implementations.rope import linear_rope_kv_write
+
+        return linear_rope_kv_write(x, w, k_cache, v_cache, cos, sin, pos, batch, seq)
+
+    @staticmethod
     def attention_prefill(q, k, v, sm_scale):
         from kernl_b200.implementations.attention import attention_forward
 
@@ -187,6 +194,14 @@ class LlamaTP:
         self._host_pos = 0  # host-side copy of the position, for the length checks
 
     # ------------------------------------------------------------------ blocks
+    def _qkv(self, h, layer, k_cache, v_cache, pos, batch, seq):
+        """Projects h, rotates q and k, writes k and v into the cache at `pos` and behind; returns q [batch, seq, heads, D].
+        (Ops without the fused call get the two steps.)"""
+        fused = getattr(self.ops, "linear_rope_kv_write", None)
+        if fused is not None:
+            return fused(h, layer["wqkv"], k_cache, v_cache, self.cos, self.sin, pos, batch, seq)
+        return self.ops.rope_kv_write(self.ops.linear(h, layer["wqkv"]), k_cache, v_cache, self.cos, self.sin, pos, batch, seq)
+
     def _row_parallel(self, x2d, w, residual, next_norm):
         """x = residual + all_reduce(x2d · wᵀ) and h = rms_norm(x) · next_norm, the input of the next
         sub-block. The GEMM writes its partial into the communicator's buffer when it has one
@@ -275,9 +290,7 @@ class LlamaTP:
         x = self.embed.index_select(0, ids.reshape(-1)).reshape(B * S, cfg.hidden)
         h = self.ops.rms_norm(x, self.layers[0]["norm1"], cfg.eps)
         for li, layer in enumerate(self.layers):
-            qkv = self.ops.linear(h, layer["wqkv"])
-            # rotate q and k, write k and v into the cache at positions 0..S-1: one kernel
-            q = self.ops.rope_kv_write(qkv, self.kcache[li, rows], self.vcache[li, rows], self.cos, self.sin, 0, B, S)
+            q = self._qkv(h, layer, self.kcache[li, rows], self.vcache[li, rows], 0, B, S)
             attn = self.ops.attention_prefill(q.transpose(1, 2), self.kcache[li, rows, :, :S], self.vcache[li, rows, :, :S],
                                               self.sm_scale)  # [B, hl, S, D]
             attn2d = attn.transpose(1, 2).reshape(B * S, hl * D)
@@ -304,8 +317,7 @@ class LlamaTP:
             self.len_mask.masked_fill_(self._slots == self.pos, 0.0)
         h = self.ops.rms_norm(x, self.layers[0]["norm1"], cfg.eps)
         for li, layer in enumerate(self.layers):
-            qkv = self.ops.linear(h, layer["wqkv"])
-            q = self.ops.rope_kv_write(qkv, self.kcache[li], self.vcache[li], self.cos, self.sin, self.pos, B, 1)
+            q = self._qkv(h, layer, self.kcache[li], self.vcache[li], self.pos, B, 1)
             attn = self.ops.attention_decode(q.transpose(1, 2), self.kcache[li], self.vcache[li],
                                              self.sm_scale, self.len_mask, self.kv_len)  # [B, hl, 1, D]
             x, h = self._row_parallel(attn.reshape(B, hl * D), layer["wo"], x, layer["norm2"])
