@@ -296,7 +296,8 @@ static bool attention_short_layout(const kb_attn_params& p) {
 // one per SM, what a tile costs when the GPU is full (the same two parts). Per tile of 64 rows, this
 // kernel: 3.5 + 4 per 64-key block (D = 64), 7 + 8 (80), 6 + 12 (128). Per tile of 128 rows, the kernels
 // for D = 64: 8 + 4.3 per block, with a row mask 17.5 + 4.3, with a full mask 11 + 7. Per pair of tiles of
-// 128 rows, attention.cuh: 57 (one tile: 35) + 13 per 128-key block, more with masks.
+// 128 rows, attention.cuh: 57 (one tile: 35) + 13 per 128-key block, more with masks, 28 (12) + 13 without a mask, where
+// its CTAs stay ([64, 32, 130, 80] causal 97 us, 117 here).
 static bool attention_short_applicable(const kb_attn_params& p) {
     if (g_attn_short == 0 || !attention_short_layout(p)) return false;
     if (g_attn_short == 1) return true;
@@ -327,7 +328,9 @@ static bool attention_short_applicable(const kb_attn_params& p) {
     const double live128 = p.is_causal ? (b128 + 1) / 2 : row_mask && b128 > 1 ? 0.33 + 0.67 * b128 : b128;
     const bool ragged = full_mask && (p.mask_strides[2] % 8 != 0 || p.mask_strides[3] != 1);
     const double slow = ragged ? 2.6 : full_mask ? 1.8 : row_mask ? 1.15 : 1.0;  // masks cost that kernel's softmax warps
-    const double other = estimate(pairs, (3000.0 + 2950.0 * live128) * slow, (p.M > 128 ? 57.0 : 35.0) * (full_mask ? 1.5 : 1.0) + 13.0 * live128 * slow);
+    const bool stays = p.mask == nullptr && p.sm_scale > 0.f;  // its CTAs take several pairs each
+    const double per_pair = stays ? (p.M > 128 ? 28.0 : 12.0) : (p.M > 128 ? 57.0 : 35.0) * (full_mask ? 1.5 : 1.0);
+    const double other = estimate(pairs, (3000.0 + 2950.0 * live128) * slow, per_pair + 13.0 * live128 * slow);
     return mine < other;
 }
 
