@@ -259,6 +259,57 @@ __device__ __forceinline__ void epilogue_chunk_swiglu(const float (&accv)[32], c
     }
 }
 
+// Epilogue of 16 columns of one output row, for the 32-column tiles of latency-bound problems. `bias_w`: the columns' bias if
+// `bias_ready`, asked for before the accumulator was complete (loaded behind it, it held the warp up for some 800 of the
+// 1600 cycles between accumulator and store). All eight warps take part; four of them storing 32 columns each took 1600 cycles,
+// 2400 with a GELU, of the 8000 to 8800 that a launch of 128 rows of [2304, 768] or [3072, 768] lasts behind its wait for the kernel
+// ahead (2000 until the first operands are there, 3200 for the others at 70 bytes per cycle). In the encoder of 1 x 128 tokens such a
+// launch went from 5.7 to 4.7 us.
+template <typename T>
+__device__ __forceinline__ void epilogue_16(const uint32_t (&acc)[16], const uint4 (&bias_w)[2], bool bias_ready, const T* __restrict__ bias,
+                                            T* __restrict__ y_row, T* __restrict__ a_row, int col0, int N, bool row_ok, int activation) {
+    float z[16];
+#pragma unroll
+    for (int v = 0; v < 2; ++v) {
+        const uint32_t w[4] = {bias_w[v].x, bias_w[v].y, bias_w[v].z, bias_w[v].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 b2 = bias_ready ? Elem<T>::unpack2(w[i]) : make_float2(0.f, 0.f);
+            z[v * 8 + 2 * i] = __uint_as_float(acc[v * 8 + 2 * i]) + b2.x;
+            z[v * 8 + 2 * i + 1] = __uint_as_float(acc[v * 8 + 2 * i + 1]) + b2.y;
+        }
+    }
+    if (bias != nullptr && !bias_ready) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+            if (col0 + j < N) z[j] += Elem<T>::to_f32(bias[col0 + j]);
+    }
+    if (!row_ok) return;
+    auto store = [&](T* dst, int first, int n, int left) {  // z[first ... first + n) of which `left` exist
+        if (left >= n && (((uintptr_t)dst) & 15) == 0) {
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {
+                if (v * 8 >= n) break;
+                reinterpret_cast<uint4*>(dst)[v] = make_uint4(Elem<T>::pack2(z[first + v * 8 + 0], z[first + v * 8 + 1]), Elem<T>::pack2(z[first + v * 8 + 2], z[first + v * 8 + 3]),
+                                                              Elem<T>::pack2(z[first + v * 8 + 4], z[first + v * 8 + 5]), Elem<T>::pack2(z[first + v * 8 + 6], z[first + v * 8 + 7]));
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (j < n && j < left) dst[j] = Elem<T>::from_f32(z[first + j]);
+        }
+    };
+    if (activation == KB_ACT_SWIGLU) {  // eight gate and eight up columns
+#pragma unroll
+        for (int i = 0; i < 8; ++i) z[i] = act_silu(z[i]) * z[8 + i];
+        if (col0 < N) store(y_row + col0 / 2, 0, 8, 8);
+        return;
+    }
+    if (a_row != nullptr) store(a_row + col0, 0, 16, N - col0);
+    apply_activation<16>(z, activation);
+    store(y_row + col0, 0, 16, N - col0);
+}
+
 template <typename T, int BN>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
@@ -280,6 +331,12 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     auto tempty_bar = [&](int a) { return bar_base + 8u * (2 * STAGES + 2 + a); };
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int num_m = (M + kGemmBM - 1) / kGemmBM;
+    const int num_n = (N + BN - 1) / BN;
+    const int num_tiles = num_m * num_n;
+    const int num_k = (K + kGemmBK - 1) / kGemmBK;
+    int m_idx, n_idx;  // the role's tile
+    tile_coords((int)blockIdx.x, num_m, num_n, m_idx, n_idx);
 
     // Launched with programmatic dependent launch: barriers, tensor memory and descriptors are set up, and the
     // first tile's W is asked for in L2 (not read: it may be the output of the kernel ahead), while the
@@ -304,9 +361,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmap_x);
         tma_prefetch_desc(&tmap_w);
-        int m_idx, n_idx;
-        tile_coords((int)blockIdx.x, (M + kGemmBM - 1) / kGemmBM, (N + BN - 1) / BN, m_idx, n_idx);
-        for (int kb = 0; kb < min(2 * STAGES, (K + kGemmBK - 1) / kGemmBK); ++kb) tma_prefetch_l2_2d(&tmap_w, kb * kGemmBK, n_idx * BN);
+        for (int kb = 0; kb < min(2 * STAGES, num_k); ++kb) tma_prefetch_l2_2d(&tmap_w, kb * kGemmBK, n_idx * BN);
     }
     if (warp == 1) {
         tmem_alloc(smem_u32(tmem_slot), Cfg::kTmemCols);
@@ -318,11 +373,6 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const uint32_t tmem_base = *tmem_slot;
     pdl_wait();
     const bool skip = s_skip != 0;
-
-    const int num_m = (M + kGemmBM - 1) / kGemmBM;
-    const int num_n = (N + BN - 1) / BN;
-    const int num_tiles = num_m * num_n;
-    const int num_k = (K + kGemmBK - 1) / kGemmBK;
     if (skip) {
         // (falls through to the teardown)
     } else if (warp == 0) {
@@ -331,8 +381,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
             uint32_t phase = 0;
             bool ok = true;
             for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
-                int m_idx, n_idx;
-                tile_coords(w, num_m, num_n, m_idx, n_idx);
+                if (w != (int)blockIdx.x) tile_coords(w, num_m, num_n, m_idx, n_idx);
                 for (int kb = 0; kb < num_k; ++kb) {
                     if (!mbar_wait(empty_bar(stage), phase ^ 1, abort_flag, 100)) { ok = false; break; }
                     mbar_arrive_expect_tx(full_bar(stage), Cfg::kStageBytes);
@@ -385,9 +434,9 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     } else {
         const int q = warp & 3;  // TMEM lane quadrant this warp may access
         const int col_half = (warp - 2) >> 2;  // which half of the tile's columns this warp handles
-        constexpr int kHalfCols = BN / 2 >= 32 ? BN / 2 : 32;
+        constexpr int kHalfCols = BN / 2;
         const int c_begin = col_half * kHalfCols;
-        const int c_end = (BN >= 64) ? c_begin + kHalfCols : (col_half == 0 ? BN : 0);
+        const int c_end = c_begin + kHalfCols;
         int acc = 0;
         uint32_t acc_phase = 0;
         bool ok = true;
@@ -395,15 +444,28 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         named_barrier(1, kGemmEpilogueWarps * 32);
         const int m_end = s_expired == 0 ? M : 0;  // rows that may be stored
         for (int w = blockIdx.x; w < num_tiles && ok; w += gridDim.x) {
-            int m_idx, n_idx;
-            tile_coords(w, num_m, num_n, m_idx, n_idx);
+            if (w != (int)blockIdx.x) tile_coords(w, num_m, num_n, m_idx, n_idx);
+            const int n0 = n_idx * BN;
+            uint4 bias_w[2];
+            bool bias_ready = false;
+            if constexpr (BN == 32) {
+                const T* mine = bias + n0 + col_half * 16;
+                bias_ready = bias != nullptr && n0 + col_half * 16 + 16 <= N && (((uintptr_t)mine) & 15) == 0;
+#pragma unroll
+                for (int v = 0; v < 2; ++v) bias_w[v] = bias_ready ? __ldg(reinterpret_cast<const uint4*>(mine) + v) : make_uint4(0u, 0u, 0u, 0u);
+            }
             if (!mbar_wait(tfull_bar(acc), acc_phase, abort_flag, 300)) { ok = false; break; }
             tc_fence_after();
             const int row = m_idx * kGemmBM + q * 32 + lane;
             const bool row_ok = row < m_end;
-            const int n0 = n_idx * BN;
             T* y_row = y + (int64_t)row * y_row_stride;
             T* a_row = act_inputs ? act_inputs + (int64_t)row * y_row_stride : nullptr;
+            if constexpr (BN == 32) {  // all eight warps, 16 columns each
+                uint32_t r[16];
+                tmem_ld_32x16(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN + col_half * 16), r);
+                tmem_ld_wait();
+                epilogue_16<T>(r, bias_w, bias_ready, bias, y_row, a_row, n0 + col_half * 16, N, row_ok, activation);
+            } else {
 #pragma unroll 1
             for (int c0 = c_begin; c0 < c_end; c0 += 32) {
                 if (n0 + c0 >= N) break;
@@ -416,6 +478,7 @@ linear_tc_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                 for (int j = 0; j < 32; ++j) accv[j] = __uint_as_float(r[j]);
                 if (activation == KB_ACT_SWIGLU) epilogue_chunk_swiglu<T>(accv, bias, y_row, col0, N, row_ok);
                 else epilogue_chunk<T>(accv, bias, y_row, a_row, col0, N, row_ok, activation);
+            }
             }
             tc_fence_before();
             __syncwarp();
