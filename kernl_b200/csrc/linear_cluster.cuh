@@ -8,8 +8,10 @@
 //   * W is the M = 128 operand of tcgen05.mma, x the N = 32, 64 or 128 one: a few rows waste no tensor
 //     memory or shared memory on absent ones, and a tile of 128 x 128 reads the least per product;
 //   * the K range of a tile goes to `splits` CTAs (one cluster, up to sixteen), so that every SM takes part
-//     and each pulls little. The fp32 partial tiles meet in distributed shared memory: every CTA adds up
-//     its share of the tile over the cluster, applies bias and activation and stores it. No workspace, no
+//     and each pulls little. The fp32 partial tiles meet in distributed shared memory: every CTA writes each
+//     row of its part to the CTA that adds that row up, which applies bias and activation and stores it. (Reading
+//     the others' parts instead waits for the cluster's memory twice per four values: 3700 to 6100 cycles, and a third barrier
+//     before anybody may leave: [128, 3072] x [768, 3072] 6.9 us, 6.4 this way, [512, 3072] x [768, 3072] 10.2 and 9.5.) No workspace, no
 //     atomics, no second launch (the split-K this replaces took 2.6 us for its finishing kernel alone and
 //     added in no fixed order);
 //   * two CTAs share an SM; barriers, tensor memory and descriptors are set up, and the first W tiles asked
@@ -31,16 +33,15 @@ struct ClCfg {  // NB: rows of x per tile
     static constexpr int kStageBytes = kWBytes + NB * kGemmBK * 2;
     static constexpr int kStages = NB == 128 ? 3 : NB == 64 ? 4 : 5;
     static constexpr int kSmemBytes = kStages * kStageBytes + 256 + 1024;
-    static_assert(NB * 128 * 4 <= kStages * kStageBytes, "the partial tile reuses the stages");
+    static_assert((NB + kClMaxSplits - 1) * 128 * 4 <= kStages * kStageBytes, "the parts to be added up reuse the stages");
     static_assert(2 * (kSmemBytes + 1024) <= 227 * 1024, "two CTAs per SM");
 };
 
-__device__ __forceinline__ float4 ld_cluster_f32x4(uint32_t own_addr, uint32_t rank) {
+// Into the shared memory of the cluster's CTA `rank`, at the place that has the address `own_addr` here.
+__device__ __forceinline__ void st_cluster_f32(uint32_t own_addr, uint32_t rank, uint32_t v) {
     uint32_t a;
-    float4 v;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(own_addr), "r"(rank));
-    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
-    return v;
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
 }
 
 template <typename T, int NB>
@@ -93,6 +94,22 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
     // CTAs of a cluster, which may read it at different times, take the same way through its barriers)
     const int skip = status_word();
 
+    // A thread adds up the same four columns in every row (its step is a multiple of a row's groups): their bias is asked for here.
+    const bool gated = activation == KB_ACT_SWIGLU;
+    const int quads = gated ? 16 : 32;  // groups of four output columns of a tile row
+    static_assert(kClThreads % 32 == 0, "whole rows of groups");
+    float bias_lo[4] = {0.f, 0.f, 0.f, 0.f}, bias_up[4] = {0.f, 0.f, 0.f, 0.f};
+    if (bias != nullptr) {
+        const int g = (int)threadIdx.x % quads, nl = gated ? (g >> 1) * 16 + (g & 1) * 4 : g * 4;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            if (n0 + nl + e < N) bias_lo[e] = Elem<T>::to_f32(__ldg(bias + n0 + nl + e));
+            if (gated && n0 + nl + 8 + e < N) bias_up[e] = Elem<T>::to_f32(__ldg(bias + n0 + nl + 8 + e));
+        }
+    }
+    const int rows = min(NB, M - m0);            // rows of x in this tile: row m is added up by rank m % splits
+    const int own = (NB + splits - 1) / splits;  // most rows of a rank
+    bool complete = false;                       // an epilogue warp: this CTA's products are
     if (warp == 0) {
         if (elect_one()) {
             bool ok = true;
@@ -125,57 +142,72 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
             }
             if (ok) tc_commit(done_bar);
         }
-    } else if (mbar_wait(done_bar, 0, abort_flag, 330)) {
-        // every product of this CTA is complete, so the stages are free: the partial tile goes there, [x row][W row]
+    } else {
+        complete = __all_sync(0xffffffffu, mbar_wait(done_bar, 0, abort_flag, 330));
+    }
+    // Once every CTA's products are complete the stages are free in all of them: the rows' parts go there, [rank][row / splits][W row].
+    __syncwarp();
+    cluster_arrive();
+    const int q = warp & 3;  // tensor-memory quadrant: 32 rows of W
+    const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    uint32_t r[32];
+    if (complete) {
         tc_fence_after();
-        const int q = warp & 3;  // tensor-memory quadrant: 32 rows of W
-        float* part = reinterpret_cast<float*>(smem) + q * 32 + lane;
+        tmem_ld_32x32(t_addr, r);
+        tmem_ld_wait();
+    }
+    __syncwarp();
+    cluster_wait();
+    if (complete) {
+        const uint32_t to = smem_base + (uint32_t)((rank * own * 128 + q * 32 + lane) * 4);
+        int owner = 0, at = 0;
 #pragma unroll 1
-        for (int c0 = 0; c0 < NB && m0 + c0 < M; c0 += 32) {
-            uint32_t r[32];
-            tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-            tmem_ld_wait();
+        for (int c0 = 0; c0 < rows; c0 += 32) {
+            if (c0 > 0) {
+                tmem_ld_32x32(t_addr + (uint32_t)c0, r);
+                tmem_ld_wait();
+            }
 #pragma unroll
-            for (int j = 0; j < 32; ++j) part[(c0 + j) * 128] = __uint_as_float(r[j]);
+            for (int j = 0; j < 32; ++j) {
+                if (c0 + j < rows) st_cluster_f32(to + (uint32_t)(at * 512), (uint32_t)owner, r[j]);
+                if (++owner == splits) { owner = 0; ++at; }
+            }
         }
         tc_fence_before();
     }
     __syncwarp();
-    cluster_sync_all();  // (a cluster of one: a CTA barrier)
+    cluster_sync_all();  // (nobody reads or writes another CTA's memory behind this)
 
-    // ---- this CTA's share of the tile: four outputs per thread, summed over the cluster in rank order
-    const bool gated = activation == KB_ACT_SWIGLU;
-    const int quads = gated ? 16 : 32;  // groups of four output columns of a tile row
-    const int total = min(NB, M - m0) * quads;
-    for (int i = rank * kClThreads + (int)threadIdx.x; i < total; i += splits * kClThreads) {
-        const int m = i / quads, q = i % quads;
+    // ---- this CTA's rows of the tile: four outputs per thread, summed in rank order
+    const int total = rows > rank ? (rows - rank + splits - 1) / splits * quads : 0;
+    for (int i = (int)threadIdx.x; i < total; i += kClThreads) {
+        const int at = i / quads, m = at * splits + rank, q = i % quads;
         // gated: W rows in blocks of eight gate and eight up rows; outputs 8 j .. from gate rows 16 j .., up rows 16 j + 8 ..
         const int nl = gated ? (q >> 1) * 16 + (q & 1) * 4 : q * 4;
-        auto sum4 = [&](int n_local, float (&z)[4]) {
-            const uint32_t addr = smem_base + (uint32_t)((m * 128 + n_local) * 4);
+        auto sum4 = [&](int n_local, const float (&b4)[4], float (&z)[4]) {
+            const float* part = reinterpret_cast<const float*>(smem) + at * 128 + n_local;
             z[0] = z[1] = z[2] = z[3] = 0.f;
             for (int s = 0; s < splits; s += 4) {  // four loads on their way before the first is added
                 float4 f[4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) f[e] = ld_cluster_f32x4(addr, (uint32_t)min(s + e, splits - 1));
+                for (int e = 0; e < 4; ++e) f[e] = *reinterpret_cast<const float4*>(part + min(s + e, splits - 1) * own * 128);
 #pragma unroll
                 for (int e = 0; e < 4; ++e)
                     if (s + e < splits) { z[0] += f[e].x; z[1] += f[e].y; z[2] += f[e].z; z[3] += f[e].w; }
             }
             if (bias != nullptr) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (n0 + n_local + e < N) z[e] += Elem<T>::to_f32(__ldg(bias + n0 + n_local + e));
+                for (int e = 0; e < 4; ++e) z[e] += b4[e];
             }
         };
         if (n0 + nl >= N) continue;
         float z[4];
-        sum4(nl, z);
+        sum4(nl, bias_lo, z);
         const int64_t row = (int64_t)(m0 + m) * y_row_stride;
         int n_out = n0 + nl, left = N - n_out;
         if (gated) {
             float up[4];
-            sum4(nl + 8, up);
+            sum4(nl + 8, bias_up, up);
 #pragma unroll
             for (int e = 0; e < 4; ++e) z[e] = act_silu(z[e]) * up[e];
             n_out = (n0 >> 1) + (q >> 1) * 8 + (q & 1) * 4;
@@ -196,7 +228,6 @@ linear_cluster_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         }
     }
     __syncwarp();
-    cluster_sync_all();  // nobody leaves while its shared memory may still be read
     if (warp == 1) tmem_dealloc(tmem_base, NB);
 }
 
