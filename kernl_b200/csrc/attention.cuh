@@ -54,16 +54,18 @@ constexpr float kLazyThreshold = 8.0f;
 // Work queues of the persistent kernels. A launch takes the next slot (host-side round robin) and its CTAs draw tile numbers
 // from slot[0]; slot[1] counts CTAs that have finished, and the last one puts both words back to
 // zero, so a slot is clean again when its launch ends — also when the launch gave up on an expired
-// wait. Two launches would have to be in flight kAttnQueueSlots launches apart to share a slot.
-constexpr int kAttnQueueSlots = 1024;
-__device__ unsigned int g_attn_queue[kAttnQueueSlots][2];
+// wait. Two launches would have to be in flight kAttnQueueSlots launches apart to share a slot. Captured launches, which come
+// again whenever their graph is replayed, have slots of their own (half a megabyte): a replay shares none with the calls of another
+// stream, and two graphs would have to be kAttnGraphSlots captured launches apart.
+constexpr int kAttnQueueSlots = 1024, kAttnGraphSlots = 65536;
+__device__ unsigned int g_attn_queue[kAttnQueueSlots + kAttnGraphSlots][2];
 
 // The next queue slot on the current device. g_attn_queue is a host-side handle; its device address
 // is looked up once per device (with that device current) and kept.
-static unsigned int* attention_queue_slot() {
+static unsigned int* attention_queue_slot(cudaStream_t stream) {
     static unsigned int* base[64] = {};
     static std::mutex mu;
-    static std::atomic<unsigned> next_slot{0};
+    static std::atomic<unsigned> next_slot{0}, next_graph_slot{0};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     {
@@ -77,6 +79,13 @@ static unsigned int* attention_queue_slot() {
             base[dev] = reinterpret_cast<unsigned int*>(ptr);
         }
     }
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {  // (the legacy stream while another one is captured: the launch will say so)
+        cudaGetLastError();
+        capture = cudaStreamCaptureStatusNone;
+    }
+    if (capture != cudaStreamCaptureStatusNone)
+        return base[dev] + 2 * (kAttnQueueSlots + next_graph_slot.fetch_add(1) % (unsigned)kAttnGraphSlots);
     return base[dev] + 2 * (next_slot.fetch_add(1) % (unsigned)kAttnQueueSlots);
 }
 
@@ -763,8 +772,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 const float neg_ref = -m_ref * unit;
                 const float2 unit2 = make_float2(unit, unit), neg2 = make_float2(neg_ref, neg_ref);
                 // Row sum: four scalar chains (pair i adds to chain i & 3), taken after P has been handed over. Two values
-                // per instruction would save issue slots (155 us instead of 164 at [4, 32 over 8, 2048, 128] causal, a few calls at
-                // full clock; kept up, the card's power cap takes the clock to 1.76 GHz and a call to 184 us) but
+                // per instruction would save issue slots (155 us instead of 164 at [4, 32 over 8, 2048, 128] causal with a CTA per item) but
                 // add in another order, and a decoder's greedy tokens should not depend on that. (A quarter to a half
                 // of the exponentials on the FMA pipe was no faster: the special-function unit is half idle.)
                 float lp[4] = {0.f, 0.f, 0.f, 0.f};
@@ -935,7 +943,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     if (MODE == 0) {
         // one CTA per SM that draws its items; a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
         grid = items < gemm_sms() ? items : gemm_sms();
-        queue = attention_queue_slot();
+        queue = attention_queue_slot(stream);
         if (queue == nullptr) return KB_ERR_LAUNCH;
     }
     const size_t smem_bytes = MODE == 0 ? (size_t)Cfg::kSmemMode0 : (size_t)Cfg::kSmemBase +

@@ -991,7 +991,7 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     if (smem_bytes > (size_t)Cfg::kSmemLimit) return KB_ERR_UNSUPPORTED;
     const int64_t tiles = (int64_t)d.num_pairs * p.B * p.H;
     const int64_t grid = tiles < 2 * (int64_t)sm_count() ? tiles : 2 * (int64_t)sm_count();
-    unsigned int* queue = attention_queue_slot();
+    unsigned int* queue = attention_queue_slot(stream);
     if (queue == nullptr) return KB_ERR_LAUNCH;
     // Longest-first order of the batches: for padding masks (one row per batch, shared by heads and
     // query rows) of a size that every CTA can scan during its set-up.

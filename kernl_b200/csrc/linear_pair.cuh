@@ -573,7 +573,7 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream,
                                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B);
         if (st != KB_OK) return st;
     }
-    const int staged = ROPE || linear_pair_staged(p, BN) ? 1 : 0;
+    int staged = ROPE || linear_pair_staged(p, BN) ? 1 : 0;
     if (staged) {
         const int64_t cols = p.activation == KB_ACT_SWIGLU ? p.N / 2 : ROPE ? p.N / 3 : p.N;  // (ROPE: q alone)
         const uint64_t dims[2] = {(uint64_t)cols, (uint64_t)p.M};
@@ -581,10 +581,12 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream,
         const uint32_t box[2] = {(uint32_t)Cfg::kStoreCols, 32};
         const int st = encode_tmap_16bit(&tmap_y, ROPE ? rope->q_out : p.y, 2, dims, strides, box, BN == 256 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_NONE,
                                          CU_TENSOR_MAP_L2_PROMOTION_NONE);
-        if (st != KB_OK) return st;
-    } else {
-        tmap_y = tmap_x;  // (not used)
+        if (st != KB_OK) {
+            if (ROPE) return st;
+            staged = 0;  // (rows of y further apart than a tensor map takes)
+        }
     }
+    if (!staged) tmap_y = tmap_x;  // (not used)
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = Cfg::kSmemBytes;
@@ -631,7 +633,7 @@ static int launch_linear_pair_tb(const kb_linear_params& p, cudaStream_t stream,
 // its epilogue a step of eight layers took 1031 us, 1019 without, since decode attention's first K and V arrive behind that launch.)
 static bool linear_pair_rope(const kb_linear_params& p, const RopeDev& r) {
     return p.activation == KB_ACT_NONE && p.bias == nullptr && p.act_inputs == nullptr && p.N == 3 * (int64_t)r.H * r.D &&
-           p.M == (int64_t)r.B * r.S && r.D % 32 == 0 && ((((uintptr_t)r.q_out) | ((uintptr_t)r.k_cache) | ((uintptr_t)r.v_cache)) & 15) == 0;
+           p.M == (int64_t)r.B * r.S && r.D % 32 == 0 && (int64_t)r.H * r.max_seq * r.D < ((int64_t)1 << 38) && ((((uintptr_t)r.q_out) | ((uintptr_t)r.k_cache) | ((uintptr_t)r.v_cache)) & 15) == 0;
 }
 
 template <typename T>
