@@ -46,7 +46,11 @@ constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
 // its greedy tokens with them. Nothing more is promised: the same row in a launch of up to 1024 rows, longer rows
 // (eight warps) and LayerNorm add up their warps' sums pairwise. The hand-over is
 // hidden behind the other CTAs of the SM.
-template <typename T, int CHUNKS, bool RMS, int WPR = 1, bool CHAIN = false>
+// EARLY (up to 64 rows of more than 1024 columns: the norms of a decode step): gamma, beta and the residual are asked for in L2 ahead of the
+// wait; behind it they would queue behind the weights that the next GEMM asks for (8 rows of 4096: 5.2 -> 3.8 us between the ends of the
+// two kernels, a step of eight layers 1034 -> 1019). With more rows it is a second pass over the residual: LayerNorm of [500, 3000]
+// 4.0 us without, 4.4 with it, of [2430, 2368] 9.9 and 12.0.
+template <typename T, int CHUNKS, bool RMS, int WPR = 1, bool CHAIN = false, bool EARLY = false>
 __global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
 norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ gamma,
                         const T* __restrict__ beta, float* __restrict__ mean_out,
@@ -59,7 +63,7 @@ norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __r
     const int wir = warp % WPR;  // this warp's position inside its row
     const int64_t row = WPR == 1 ? (int64_t)blockIdx.x * 4 + warp : (int64_t)blockIdx.x;
 #define KB_NORM_COL(c) (((CHAIN ? wir * CHUNKS + (c) : (c) * WPR + wir) * 32 + lane) * 8)
-    if (WPR == 4 && !CHAIN && (lane & 7) == 0) {
+    if (EARLY && (lane & 7) == 0) {
 #pragma unroll
         for (int c = 0; c < CHUNKS; ++c) {
             const int col = KB_NORM_COL(c);
@@ -317,6 +321,11 @@ static int launch_norm_t(const kb_norm_params& p, cudaStream_t stream) {
         if (p.cols <= 3 * 2048) KB_NORM_LAUNCH(3, 8);
         if (p.cols <= 4 * 2048) KB_NORM_LAUNCH(4, 8);
         KB_NORM_LAUNCH(8, 8);
+    }
+    if (vec_ok && p.rows <= 64 && p.cols > 1024) {
+        if (p.cols <= 2 * 1024) KB_NORM_LAUNCH(2, 4, false, true);
+        if (p.cols <= 3 * 1024) KB_NORM_LAUNCH(3, 4, false, true);
+        KB_NORM_LAUNCH(4, 4, false, true);
     }
     if (vec_ok && p.rows <= 1024) {
         if (p.cols <= 1024) KB_NORM_LAUNCH(1, 4);
