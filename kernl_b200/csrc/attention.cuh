@@ -787,8 +787,19 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                         sr[cch][2 * i + 1] = __float_as_uint(e1);
                         pk[i] = Elem<T>::pack2(e0, e1);
                     }
-                    // (the first half is handed over once the third quarter's exponentials are under way: waiting for its store
-                    // right away leaves the special-function unit idle for the store's latency)
+                    // Without a mask the first half is handed over once the third quarter's exponentials are under way: waiting for its
+                    // store right away leaves the special-function unit idle for the store's latency (4 % there). With one the
+                    // values held meanwhile cost more than that ([2, 32, 3916, 128] padded 297 us as here, 309 handed over late).
+                    if (MODE != 0) {
+                        tmem_st_32x16(s_addr + cch * 16, pk);
+                        if (cch & 1) {
+                            tmem_st_wait();
+                            tc_fence_before();
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(p_full(t, cch >> 1));
+                        }
+                        continue;
+                    }
                     if (cch >= 2) {
                         if (cch == 3) tmem_st_32x16(s_addr + cch * 16, pk);
                         tmem_st_wait();
