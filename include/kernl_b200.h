@@ -120,7 +120,8 @@ int kb_silu_mul(const void* gu, void* y, int64_t M, int64_t N, int32_t dtype, vo
  * pos_dev (device int64) when it is not NULL, else pos_host. cos/sin: fp32 [max_seq, D/2].
  * Rotation on interleaved pairs as in the reference's experimental Llama kernels
  * (experimental/llama-v2/kernel/pytorch_reference.py:37-80, fused_kernel_proj_qkv.py:116-347);
- * nothing in the reference's dispatched path corresponds to it. D must be a multiple of 8. */
+ * nothing in the reference's dispatched path corresponds to it. D must be a multiple of 8. Rows whose
+ * position lies outside [0, max_seq) are left out: their q_out and every cache slot stay as they were. */
 typedef struct {
     const void* qkv; void* q_out; void* k_cache; void* v_cache;
     const float* cos; const float* sin;

@@ -418,10 +418,13 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                                 }
                             }
                         }
-                        // rows of k and v that lie in two sequences, or beyond the last one, are stored one by one
-                        box = part == 0 || (row_base + 31 < M && (row_base + 31) / rp.S == b0 && pos0 >= 0);
+                        // Stored one by one: rows of k and v that lie in two sequences, or beyond the last one, and boxes with a position
+                        // outside the cache, whose rows (those of q too) stay as they are, as in rope_kv_write_kernel. Positions are compared
+                        // in 64 bits; those of a whole box fit the copy's 32-bit coordinate.
+                        box = __all_sync(0xffffffffu, inside || row >= M) && (part == 0 || (row_base + 31 < M && (row_base + 31) / rp.S == b0));
                         if (!box && row < m_end && inside && ycol < N) {
-                            T* dst = reinterpret_cast<T*>(part == 1 ? rp.k_cache : rp.v_cache) + (((int64_t)b * rp.H + head) * rp.max_seq + pos) * rp.D + d0;
+                            T* dst = part == 0 ? reinterpret_cast<T*>(rp.q_out) + (int64_t)row * hd + ycol
+                                               : reinterpret_cast<T*>(part == 1 ? rp.k_cache : rp.v_cache) + (((int64_t)b * rp.H + head) * rp.max_seq + pos) * rp.D + d0;
 #pragma unroll
                             for (int v = 0; v < 4; ++v) reinterpret_cast<uint4*>(dst)[v] = make_uint4(o[v * 4], o[v * 4 + 1], o[v * 4 + 2], o[v * 4 + 3]);
                         }
@@ -452,7 +455,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     if (warp == 2 && lane == 0 && bx == 0) KB_GTRACE(ti, 9);
                     if (lane == 0 && row_base < m_end && ycol < (gated ? N / 2 : N)) {
                         if constexpr (ROPE) {
-                            if (part == 0) tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
+                            if (part == 0 && box) tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
                             else if (box) tma_store_4d(part == 1 ? &rope.k : &rope.v, smem_u32(mine), d0, (int)pos0, head, b0);
                         } else {
                             tma_store_2d(&tmap_y, smem_u32(mine), ycol, row_base);
