@@ -103,6 +103,9 @@ class CudaOps:
         return skinny_attention_forward(q, k, v, torch.empty_like(q), sm_scale, False, None, kv_len=kv_len)
 
 
+_FUSED_QKV = (CudaOps.linear_rope_kv_write, CudaOps.linear, CudaOps.rope_kv_write)  # the fused call and what it stands for
+
+
 def _seeded(shape, std, seed, device, dtype):
     """N(0, std) tensor that is identical on every rank (same seed, same generator device)."""
     g = torch.Generator(device=device).manual_seed(seed)
@@ -196,11 +199,15 @@ class LlamaTP:
     # ------------------------------------------------------------------ blocks
     def _qkv(self, h, layer, k_cache, v_cache, pos, batch, seq):
         """Projects h, rotates q and k, writes k and v into the cache at `pos` and behind; returns q [batch, seq, heads, D].
-        (Ops without the fused call get the two steps.)"""
-        fused = getattr(self.ops, "linear_rope_kv_write", None)
+        (Ops without the fused call get the two steps, and so do ops with a projection or rotation other than CudaOps' own
+        behind CudaOps' fused call, which would pass them by.)"""
+        ops = self.ops
+        fused = getattr(ops, "linear_rope_kv_write", None)
+        if fused is _FUSED_QKV[0] and (ops.linear, ops.rope_kv_write) != _FUSED_QKV[1:]:
+            fused = None
         if fused is not None:
             return fused(h, layer["wqkv"], k_cache, v_cache, self.cos, self.sin, pos, batch, seq)
-        return self.ops.rope_kv_write(self.ops.linear(h, layer["wqkv"]), k_cache, v_cache, self.cos, self.sin, pos, batch, seq)
+        return ops.rope_kv_write(ops.linear(h, layer["wqkv"]), k_cache, v_cache, self.cos, self.sin, pos, batch, seq)
 
     def _row_parallel(self, x2d, w, residual, next_norm):
         """x = residual + all_reduce(x2d · wᵀ) and h = rms_norm(x) · next_norm, the input of the next

@@ -62,6 +62,52 @@ def _cpu_model(world=1, rank=0, cfg=SMALL):
     return LlamaTP(cfg, rank=rank, world=world, device="cpu", dtype=torch.float32, ops=OracleOps(), seed=0)
 
 
+@pytest.mark.parametrize("how", ["subclass", "instance"])
+@pytest.mark.parametrize("own", [("linear", "rope_kv_write"), ("linear",), ("rope_kv_write",)])
+def test_own_projection_or_rotation_is_not_passed_by(own, how, monkeypatch):
+    """Ops that replace CudaOps' `linear` or `rope_kv_write` are called for the q/k/v projection too, not the fused call behind them."""
+    import kernl_b200.llama_tp as llama
+
+    steps = {name: staticmethod(getattr(OracleOps, name)) for name in dir(OracleOps) if not name.startswith("_")}
+    fused_calls = []
+
+    def fused(x, w, *rest):
+        fused_calls.append(1)
+        return OracleOps.rope_kv_write(OracleOps.linear(x, w), *rest)
+
+    base = type("Base", (), dict(steps, linear_rope_kv_write=staticmethod(fused)))  # in the place of CudaOps, on the CPU
+    monkeypatch.setattr(llama, "_FUSED_QKV", (base.linear_rope_kv_write, base.linear, base.rope_kv_write), raising=False)
+    calls = []
+
+    def counted(name):
+        def call(*args, **kwargs):
+            calls.append(name)
+            return getattr(OracleOps, name)(*args, **kwargs)
+
+        return call
+
+    if how == "subclass":
+        ops = type("Own", (base,), {name: staticmethod(counted(name)) for name in own})()
+    else:
+        ops = base()
+        for name in own:
+            setattr(ops, name, counted(name))
+    ids = torch.arange(6).reshape(1, 6)
+    model = LlamaTP(SMALL, device="cpu", dtype=torch.float32, ops=ops, seed=0)
+    logits = model.prefill(ids)
+    assert not fused_calls and set(calls) == set(own)
+    assert torch.equal(logits, _cpu_model().prefill(ids))
+    plain = LlamaTP(SMALL, device="cpu", dtype=torch.float32, ops=base(), seed=0)
+    assert torch.equal(plain.prefill(ids), logits) and len(fused_calls) == SMALL.n_layers
+
+
+def test_cuda_ops_fused_call_stands_for_its_own_steps():
+    from kernl_b200.llama_tp import _FUSED_QKV, CudaOps
+
+    ops = CudaOps()
+    assert (ops.linear_rope_kv_write, ops.linear, ops.rope_kv_write) == _FUSED_QKV
+
+
 def test_gate_up_interleave_layout():
     from kernl_b200.implementations.linear_layer import interleave_gate_up
 
