@@ -326,12 +326,12 @@ static int launch_linear_cluster_n(const kb_linear_params& p, cudaStream_t strea
 
 // ---- which kernel a problem goes to
 //
-// Estimates in us, fitted to times of the kernels (graphs of calls with cold W) over 16 to 8192 rows and W from 500 x 1000
-// to 11008 x 4096. An SM pulls about 118 bytes per ns through its port to L2, shared by its CTAs; W comes from HBM at
-// 6.5 bytes per ps at best. Estimate over time, at 27 problems: CTA pairs 0.85 to 1.05, single CTAs 0.84 to 1.18 from 32 rows
-// on but for 2000 rows of [504, 1000] (0.75), clusters 0.93 to 1.07 where their tiles fit at once. (While the clusters' sums
-// were a constant per column and single CTAs took 118 bytes per ns at every width, [512, 3072] x [768, 3072] ran in
-// 13.2 us where single CTAs take 9.9, [300, 4096] x [1024, 4096] in 14.4 for 12.2, [48, 1000] x [1000, 1000] in 7.5 for 5.0.)
+// Estimates in us, fitted to times of the kernels (graphs of calls with cold W). Above 128 rows, at 1170 problems that the fit has not
+// seen (129 to 8192 rows, K and N from 256 to 11008, every activation): the chosen kernel is 0.5 % slower than the fastest one on
+// average, at 6 % of them by more than 3 %, at 1.5 % by more than 10. (Estimates fitted to some thirty problems, before the kernels' epilogues
+// changed, and bent towards the new ones since: 1.6 % on average, 13 % and 7 %; 3 % of the problems were slower than with the earlier kernels
+// and their own estimates, [129, 256] x [11008, 256] by 32 %, [2000, 8192] x [1024, 8192] by 22.) Up to 128 rows an SM pulls about
+// 118 bytes per ns through its port to L2, shared by its CTAs; W comes from HBM at 6.5 bytes per ps at best.
 struct ClusterPlan {
     int nb, splits;
     double us;
@@ -368,6 +368,11 @@ static double linear_single_us(const kb_linear_params& p) {
     const int bn = plan_linear_bn(p.M, p.N, p.K, 0);
     const int64_t tiles = ((p.M + kGemmBM - 1) / kGemmBM) * ((p.N + bn - 1) / bn);
     const double waves = (double)((tiles + gemm_sms() - 1) / gemm_sms());
+    if (p.M > 128) {
+        static constexpr GemmCost kTile[4] = {{2.7, 0.0, 0.146, 0.020, 0.25, 0.15, -0.2, 0.25, 0.35, 0.1, 3.5}, {2.6, 0.1, 0.159, 0.018, 1.1, 0.36, -0.75, 0.40, 0.70, 0.5, 8.3},
+                                              {3.4, 0.55, 0.220, 0.025, 0.62, 0.74, -1.2, 0.38, 1.05, 1.0, 17.0}, {2.7, 1.1, 0.357, 0.090, 2.4, 1.2, -1.7, 0.26, 0.80, 2.7, 32.0}};
+        return gemm_us(kTile[bn == 32 ? 0 : bn == 64 ? 1 : bn == 128 ? 2 : 3], p, tiles, gemm_sms(), p.act_inputs != nullptr);
+    }
     // An SM's port gives 118 bytes per ns, narrow tiles pull faster (512 rows of [768, 3072], 32 columns: 9.9 us, 11.5 at that
     // rate), rows that are no multiple of 128 bytes take longer. An epilogue stores a column of a tile in 0.012 us by whole
     // 16-byte pieces, in 0.05 value by value. A tile of which most rows lie outside x arrives later (zero fill): 5.5 us at
@@ -390,12 +395,19 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
     const ClusterPlan cl = p.M <= 1024 && g_linear_pair == 1 && gemm_sms() == sm_count() ? linear_cluster_plan<T>(p) : ClusterPlan{0, 0, 1e300};
     if (p.M > 128 && p.N >= 128 && p.K >= 256 && g_linear_pair != 0) {
         double pair;
-        const int bn = linear_pair_tile_width(p, &pair);
-        // (at thousands of rows the estimates no longer matter: the pair kernel pulls half as much W through each SM's port)
-        if (g_linear_pair != 1 || pair < 0.93 * single || (p.M > 4096 && p.N >= 256)) {
+        int bn = linear_pair_tile_width(p, &pair);
+        if (in_pair != nullptr && g_linear_pair == 1) {
+            // The rotary epilogue has the wide tile only, and saves a launch that reads and writes the result (402 MB in 74 us at 8192 rows of
+            // [12288, 4096]) for some work of its own. Where the narrow tile is faster by more than that, the launch stays: prompts of 141 and 198
+            // tokens, four and three layers, 673 us for 694 and 524 for 538.
+            const double wide = linear_pair_us(p, 256) + 2.0 - (double)p.M * (double)p.N * 4.0 / 5.5e6;
+            if (bn == 256 || wide < pair) {
+                bn = 256;
+                pair = wide;
+            }
+        }
+        if (g_linear_pair != 1 || pair < single) {
             if (pair <= cl.us) {
-                // (the rotary epilogue has the wide tile only: where the narrow one is the faster, a launch behind it costs less than the wide
-                // tile would: a prompt of 141 tokens, four layers, 673 us for 694)
                 const RopeDev* fused = bn == 256 ? in_pair : nullptr;
                 if (fused != nullptr) *roped = true;
                 return launch_linear_pair_t<T>(p, stream, bn, fused);
@@ -404,10 +416,18 @@ static int launch_linear_t(const kb_linear_params& p, cudaStream_t stream, int f
     }
     if (p.M <= 1024 && gemm_sms() == sm_count()) {
         const double stream_us = stream_layout(p) && p.M <= 512 ? stream_plan_x(p).us : 1e300;
-        // (the streaming kernel's estimate is a tenth high for few rows: 5.5 us for 5.0 at 33 rows of [3072, 768], the cluster's 5.3 for 5.4)
-        if (stream_us < single && stream_us < 1.05 * cl.us) return launch_linear_stream_t<T>(p, stream);
-        // (ahead by more than a trifle: where the two are close, the cluster's estimate is the less certain one)
-        if (cl.us < 0.97 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+        if (p.M <= 128) {
+            // (the streaming kernel's estimate is a tenth high for few rows: 5.5 us for 5.0 at 33 rows of [3072, 768], the cluster's 5.3 for 5.4)
+            if (stream_us < single && stream_us < 1.05 * cl.us) return launch_linear_stream_t<T>(p, stream);
+            // (ahead by more than a trifle: where the two are close, the cluster's estimate is the less certain one)
+            if (cl.us < 0.97 * single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+        } else {
+            // (here the streaming kernel's is a little low, for gated calls high, 4.3 us for 2.8 at 150 rows of [256, 360], and does not know
+            // what values stored one by one cost it: 30 us at 200 rows of [8192, 512], 22 with single CTAs)
+            const double likely = stream_us * (p.activation == KB_ACT_SWIGLU ? 0.9 : 1.05) + (linear_stores_values(p) ? 8e-6 * (double)p.M * (double)p.N : 0.0);
+            if (likely < single && likely < 1.1 * cl.us) return launch_linear_stream_t<T>(p, stream);
+            if (cl.us < single) return launch_linear_cluster_n<T>(p, stream, cl.nb, cl.splits);
+        }
     }
     return launch_linear_single<T>(p, stream, 0);
 }

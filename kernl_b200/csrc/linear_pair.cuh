@@ -524,20 +524,6 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
 
 static int g_linear_pair = 1;  // test hook (kb_debug_linear_pair): 0 = never use the pair kernel, 192 / 256 = force that tile width
 
-// Estimated time in us of the pair kernel with tiles of 256 x `bn`: a fixed part (more of it when there is one round only,
-// whose first operands and epilogue nothing hides), and rounds of tiles on the pairs of (k-blocks x time of one + the part of
-// an epilogue that the next tile does not hide; the exponential of a GELU costs 0.3 more). A k-block of 64 costs 0.235 us (192 columns) or 0.268
-// (256) while few pairs are busy, up to a third more when all of them pull on L2: about 60 bytes per cycle and SM arrive
-// where the products want 75 and 64. Fitted to 1000 to 8192 rows, K from 512 to 4096.
-static double linear_pair_us(const kb_linear_params& p, int bn) {
-    const int64_t pairs = gemm_sms() / 2 > 0 ? gemm_sms() / 2 : 1;
-    const int64_t tiles = ((p.M + 255) / 256) * ((p.N + bn - 1) / bn), rounds = (tiles + pairs - 1) / pairs;
-    const double busy = (double)tiles / (double)(rounds * pairs), num_k = (double)((p.K + kGemmBK - 1) / kGemmBK);
-    const double act = p.activation == KB_ACT_GELU ? 0.3 : 0.0, b2 = busy * busy;
-    if (bn == 192) return 4.0 + (rounds == 1 ? 1.6 : 0.0) + (double)rounds * (num_k * (0.235 + 0.07 * b2 * b2 * b2) + 0.4 + act);
-    return 2.7 + act + (rounds == 1 ? 2.3 : 0.0) + (double)rounds * (num_k * (0.268 + 0.09 * b2) + 1.0 + act);
-}
-
 // Whether the rows of y do not allow stores of 16 bytes.
 static bool linear_stores_values(const kb_linear_params& p) { return p.y_row_stride % 8 != 0 || (((uintptr_t)p.y) & 15) != 0; }
 
@@ -548,12 +534,39 @@ static bool linear_pair_staged(const kb_linear_params& p, int bn) {
     return p.activation == KB_ACT_SWIGLU ? bn == 256 && p.N % 16 == 0 : p.N % 8 == 0;
 }
 
-// Tile width (192 or 256 columns), and the estimate that goes with it. 192 columns want the staged epilogue; among close estimates the wide tile, which pulls less.
+// What a GEMM kernel whose CTAs stay for several tiles costs, in us: a fixed part, more of it when there is one round of tiles only,
+// whose first operands and epilogue nothing hides; per round the k-blocks of 64, each the dearer the more SMs pull on L2 at once, and
+// the part of an epilogue that the next tile does not hide, with what a GELU's exponential adds to it, what a gated epilogue, which
+// stores half, takes off, and what threads that store for themselves add, by 16 bytes a row or value by value; more of it for rows of x
+// and W that are no multiple of 128 bytes. Fitted to 12 400 problems of 129 to 8192 rows (ratios of the kernels' times inside each problem).
+struct GemmCost {
+    double fixed, one_round, block, busy_block, epilogue, gelu, gated, ragged, ragged_epilogue, rows, values;
+};
+static double gemm_us(const GemmCost& c, const kb_linear_params& p, int64_t tiles, int64_t slots, bool by_rows) {
+    const int64_t rounds = (tiles + slots - 1) / slots;
+    const double busy = (double)tiles / (double)(rounds * slots), num_k = (double)((p.K + kGemmBK - 1) / kGemmBK);
+    const bool ragged = p.K % kGemmBK != 0;
+    const double block = (c.block + c.busy_block * busy * busy * busy) * (ragged ? 1.0 + c.ragged : 1.0);
+    const double act = p.activation == KB_ACT_GELU ? c.gelu : p.activation == KB_ACT_SWIGLU ? c.gated : 0.0;
+    const double stores = linear_stores_values(p) ? c.values : by_rows ? c.rows : 0.0;
+    const double us = c.fixed + (rounds == 1 ? c.one_round : 0.0) + (double)rounds * (num_k * block + c.epilogue + act + (ragged ? c.ragged_epilogue : 0.0) + stores);
+    const double hbm = c.fixed + (double)p.N * (double)p.K * 2.0 / 6.8e6;  // W once from memory
+    return us > hbm ? us : hbm;
+}
+
+// Estimated time in us of the pair kernel with tiles of 256 x `bn`.
+static double linear_pair_us(const kb_linear_params& p, int bn) {
+    static constexpr GemmCost kNarrow{3.3, 1.04, 0.244, 0.068, 0.60, 0.70, 0.0, 0.10, 0.45, 3.5, 23.0};
+    static constexpr GemmCost kWide{3.3, 1.25, 0.311, 0.100, 0.64, 0.70, 0.0, 0.05, 0.40, 5.5, 31.0};
+    const int64_t pairs = gemm_sms() / 2 > 0 ? gemm_sms() / 2 : 1;
+    return gemm_us(bn == 192 ? kNarrow : kWide, p, ((p.M + 255) / 256) * ((p.N + bn - 1) / bn), pairs, !linear_pair_staged(p, bn));
+}
+
+// Tile width (192 or 256 columns), and the estimate that goes with it.
 static int linear_pair_tile_width(const kb_linear_params& p, double* us) {
-    const bool staged = linear_pair_staged(p, 192);
     const double wide = linear_pair_us(p, 256), narrow = linear_pair_us(p, 192);
-    const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : staged && narrow < 0.96 * wide ? 192 : 256;
-    *us = (bn == 192 ? narrow : wide) + (linear_stores_values(p) ? 16.0 : 0.0);  // (26.6 us at 2000 rows of [500, 768])
+    const int bn = g_linear_pair == 192 || g_linear_pair == 256 ? g_linear_pair : p.activation != KB_ACT_SWIGLU && narrow < wide ? 192 : 256;
+    *us = bn == 192 ? narrow : wide;
     return bn;
 }
 

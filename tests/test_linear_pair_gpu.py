@@ -79,3 +79,36 @@ def test_bias_that_begins_anywhere(lib, width, M, K, N, act, off):
             end.synchronize()
             best[i] = min(best[i], start.elapsed_time(end))
     assert best[1] < 1.25 * best[0], best  # (stores by the threads: 1.5 to 1.6 times)
+
+
+@pytest.mark.parametrize("width", [192, 256])
+@pytest.mark.parametrize("M, K, N, act, pre, gap", [(129, 256, 136, "gelu", True, 0), (300, 264, 1000, "relu", True, 0), (257, 256, 200, "", True, 3),
+                                                    (300, 264, 1000, "gelu", False, 3), (513, 256, 131, "", False, 0), (520, 320, 4000, "tanh", True, 1)])
+def test_linear_pair_stored_by_threads(lib, M, K, N, act, pre, gap, width):
+    """Results that bulk stores cannot take, which the narrow tile now serves too: pre-activation output, rows of y at odd places, ragged columns."""
+    from kernl_b200.implementations.linear_layer import linear_layer
+
+    g = torch.Generator().manual_seed(M + N)
+    x, w = torch.randn((M, K), generator=g).half().cuda(), (torch.randn((N, K), generator=g) * K ** -0.5).half().cuda()
+    b = torch.randn((N,), generator=g).half().cuda()
+
+    def call():
+        around = torch.full((M + 2, N + gap), 7.0, dtype=torch.float16, device="cuda")
+        before = torch.full((M + 2, N), 7.0, dtype=torch.float16, device="cuda")
+        if pre and gap:
+            pytest.skip("the pre-activation output has the rows of y")
+        linear_layer(x, w, b, act, act_inputs=before[1:M + 1] if pre else None, out=around[1:M + 1, :N])
+        return around, before
+
+    try:
+        lib.kb_debug_linear_pair(0)
+        lib.kb_debug_force_bn(128)
+        expected = call()
+        lib.kb_debug_force_bn(0)
+        lib.kb_debug_linear_pair(width)
+        got = call()
+    finally:
+        lib.kb_debug_force_bn(0)
+        lib.kb_debug_linear_pair(1)
+    for a, e in zip(got, expected):
+        assert torch.equal(a, e)
