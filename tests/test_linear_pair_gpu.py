@@ -82,8 +82,8 @@ def test_bias_that_begins_anywhere(lib, width, M, K, N, act, off):
 
 
 @pytest.mark.parametrize("width", [192, 256])
-@pytest.mark.parametrize("M, K, N, act, pre, gap", [(129, 256, 136, "gelu", True, 0), (300, 264, 1000, "relu", True, 0), (257, 256, 200, "", True, 3),
-                                                    (300, 264, 1000, "gelu", False, 3), (513, 256, 131, "", False, 0), (520, 320, 4000, "tanh", True, 1)])
+@pytest.mark.parametrize("M, K, N, act, pre, gap", [(129, 256, 136, "gelu", True, 0), (300, 264, 1000, "relu", True, 0), (513, 256, 4000, "tanh", True, 0),
+                                                    (300, 264, 1000, "gelu", False, 3), (513, 256, 131, "", False, 0), (520, 320, 4000, "relu", False, 1)])
 def test_linear_pair_stored_by_threads(lib, M, K, N, act, pre, gap, width):
     """Results that bulk stores cannot take, which the narrow tile now serves too: pre-activation output, rows of y at odd places, ragged columns."""
     from kernl_b200.implementations.linear_layer import linear_layer
@@ -95,8 +95,6 @@ def test_linear_pair_stored_by_threads(lib, M, K, N, act, pre, gap, width):
     def call():
         around = torch.full((M + 2, N + gap), 7.0, dtype=torch.float16, device="cuda")
         before = torch.full((M + 2, N), 7.0, dtype=torch.float16, device="cuda")
-        if pre and gap:
-            pytest.skip("the pre-activation output has the rows of y")
         linear_layer(x, w, b, act, act_inputs=before[1:M + 1] if pre else None, out=around[1:M + 1, :N])
         return around, before
 
