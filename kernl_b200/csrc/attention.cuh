@@ -11,11 +11,12 @@
 // The third warpgroup shrinks its register allowance (setmaxnreg) so that the softmax threads can
 // hold a whole 128-wide score row in registers.
 // While one group runs its exponentials, the tensor core works on the other tile (ping-pong).
-// Without a mask (MODE 0) a CTA stays for the whole launch, one per SM: further items (pairs of query tiles) come from a
+// Without a mask, in launches of more pairs of query tiles than SMs (MODE 0), a CTA stays for the whole launch, one per SM: further items (pairs of query tiles) come from a
 // device-side counter, the issuer starts an item's scores while the softmax warps store the one before, and every barrier's
 // phase counts on over the items. A CTA per item spent 12 000 of 45 000 to 67 000 cycles on setting itself up, its first
 // loads, its stores and its end (all of an SM's tensor memory and shared memory are one CTA's). [4, 32 over 8, 2048, 128]
-// causal 166 -> 149 us (with the hand-over of P below), [16, 16, 512, 128] 61 -> 46, [2, 32, 4096, 128] 463 -> 440; same bits.
+// causal 174 -> 149 us (with the hand-over of P below), [16, 16, 512, 128] 61 -> 46, [2, 32, 4096, 128] 463 -> 440; same bits.
+// A launch without a second item per SM (MODE 4) has one CTA per item and none of that.
 // TMEM columns: S_0 [0,128)  S_1 [128,256)  O_0 [256,256+D)  O_1 [384,384+D); P_t (16-bit, two
 // per column) overwrites the first 64 columns of S_t once the thread has its row in registers.
 //
@@ -174,10 +175,10 @@ struct AttnCfg {
     static constexpr int kSmemBase = (2 + 2 * kKvStages) * kTileBytes + 512 + 1024;
     static constexpr int kMaskMaxN = 7168;  // MODE 1: the longest mask row that fits behind the tiles
     static constexpr int kMaskRingBytes = 2 * 2 * kAttnBlock * 4;  // MODE 3
-    static constexpr int kOutWarpBytes = 32 * 64 * 2;  // MODE 0: 32 rows x 64 columns of results per softmax warp, a box of one bulk store
+    static constexpr int kOutWarpBytes = 32 * 64 * 2;  // MODE 0 and 4: 32 rows x 64 columns of results per softmax warp, a box of one bulk store
     static constexpr int kOutOffset = (2 + 2 * kKvStages) * kTileBytes + 1024;
-    static constexpr int kSmemMode0 = kOutOffset + 8 * kOutWarpBytes + 1024;
-    static_assert(kSmemMode0 <= 227 * 1024 - 256, "shared memory of one CTA");
+    static constexpr int kSmemNoMask = kOutOffset + 8 * kOutWarpBytes + 1024;
+    static_assert(kSmemNoMask <= 227 * 1024 - 256, "shared memory of one CTA");
     static constexpr int kSmemMax = kSmemBase + kMaskMaxN * 4;
     static_assert(kSmemMax <= 227 * 1024 - 256, "shared memory of one CTA");
 };
@@ -289,7 +290,8 @@ __device__ __forceinline__ int bits_count_below(const uint32_t (&w)[4], int limi
     }
     return n;
 }
-// MODE 0: no mask and positive scale (maximum taken on raw scores, one FFMA + EX2 per element);
+// MODE 0: no mask and positive scale (maximum taken on raw scores, one FFMA + EX2 per element), CTAs that stay; MODE 4: the same, a CTA
+//         per item;
 // MODE 1: additive mask that is the same for every query row (padding masks): all threads stage it in
 //         shared memory during set-up, already clamped, scaled by log2(e) and with -inf for columns
 //         beyond N, and key blocks that are masked throughout are not visited; MODE 2: anything else (per-row masks read from global memory with
@@ -302,6 +304,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_o, const AttnDev p,
                     const int num_items, unsigned int* const queue) {
     using Cfg = AttnCfg<D>;
+    constexpr bool kNoMask = MODE == 0 || MODE == 4;
     constexpr int KVS = Cfg::kKvStages;
     constexpr int TILE = Cfg::kTileBytes;
     constexpr int CHUNK = kAttnBlock * 64 * 2;  // one 64-column (128-byte swizzled) slab of a tile
@@ -345,9 +348,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
     __shared__ int s_expired;
     // MODE 0: one thread of every CTA reports in when it draws no more items; the last one leaves the queue's slot clean.
     // (Reported by the producer, while the last item is computed: at the CTA's end it cost a microsecond.)
-    const bool draws = MODE == 0 && num_items > (int)gridDim.x;
     auto report = [&] {
-        if (draws) {
+        if (MODE == 0) {
             __threadfence();
             if (atomicAdd(&queue[1], 1u) == gridDim.x - 1) {
                 queue[0] = 0u;
@@ -426,7 +428,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         tma_prefetch_desc(&tmap_q);
         tma_prefetch_desc(&tmap_k);
         tma_prefetch_desc(&tmap_v);
-        if (MODE == 0 && p.o_bulk) tma_prefetch_desc(&tmap_o);
+        if (kNoMask && p.o_bulk) tma_prefetch_desc(&tmap_o);
     }
     tc_fence_before();
     __syncthreads();
@@ -507,7 +509,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 // The item's last block is on its way, so the item is two blocks from its end: time to draw the next one. (A CTA
                 // that is busy with a long item should not hold back one that an idle CTA could start.)
                 if (u >= 2 && !mbar_wait(item_free(u & 1), (uint32_t)(((u >> 1) - 1) & 1), abort_flag, 102)) { ok = false; break; }
-                const int drawn = draws ? (int)gridDim.x + (int)atomicAdd(&queue[0], 1u) : num_items;
+                const int drawn = (int)gridDim.x + (int)atomicAdd(&queue[0], 1u);
                 items[u & 1] = drawn < num_items ? drawn : -1;
                 mbar_arrive(item_full(u & 1));
                 if (drawn >= num_items) {
@@ -659,9 +661,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         const uint32_t o_addr = lane_addr + (uint32_t)(256 + t * 128);
         const float c = p.scale_log2;
         const float mlow = mask_lowest(p.mask_dtype);
-        // In MODE 0 the running maximum is kept in raw score units and the exponent is
+        // Without a mask the running maximum is kept in raw score units and the exponent is
         // (s - m_ref) * c; otherwise scores are first moved to the log2 domain (s*c + mask).
-        const float unit = (MODE == 0) ? c : 1.0f;
+        const float unit = kNoMask ? c : 1.0f;
         int cnt = 0, seen = 0;  // blocks of this tile in the items before, and items in which it was live
         bool ok = true;
         for (int u = 0; ok; ++u) {
@@ -790,7 +792,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                     // Without a mask the first half is handed over once the third quarter's exponentials are under way: waiting for its
                     // store right away leaves the special-function unit idle for the store's latency (4 % there). With one the
                     // values held meanwhile cost more than that ([2, 32, 3916, 128] padded 297 us as here, 309 handed over late).
-                    if (MODE != 0) {
+                    if (!kNoMask) {
                         tmem_st_32x16(s_addr + cch * 16, pk);
                         if (cch & 1) {
                             tmem_st_wait();
@@ -822,7 +824,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
             tc_fence_after();
             const int m_end = s_expired == 0 ? p.M : 0;  // rows that may be stored
             const float inv_l = 1.0f / l;
-            if (MODE == 0 && p.o_bulk) {
+            if (kNoMask && p.o_bulk) {
                 // Boxes of 32 rows x 64 columns through shared memory to bulk stores (rows of 128 bytes, 128-byte swizzle; rows
                 // beyond M and columns beyond the head dimension are left out): a thread per row stores 16 bytes to each of 32 lines
                 // at a time, 2600 cycles per item in which the tile's next scores wait.
@@ -880,7 +882,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
           }
           if (!next_item(u, true, ok)) break;
         }
-        if (MODE == 0 && p.o_bulk && lane == 0) bulk_wait_all();
+        if (kNoMask && p.o_bulk && lane == 0) bulk_wait_all();
     }
 
     tc_fence_before();
@@ -894,6 +896,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 template <typename T, int D, int MODE>
 static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     using Cfg = AttnCfg<D>;
+    constexpr bool kNoMask = MODE == 0 || MODE == 4;
     CUtensorMap tq, tk, tv, to;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
     if (p.H % kv_group != 0) return KB_ERR_BAD_ARG;
@@ -922,7 +925,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     d.num_pairs = (num_m_tiles + 1) / 2;
     const int64_t items = (int64_t)d.num_pairs * p.B * p.H;
     if (items > 0x3fffffff) return KB_ERR_UNSUPPORTED;
-    d.o_bulk = MODE == 0 && attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK ? 1 : 0;
+    d.o_bulk = kNoMask && attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK ? 1 : 0;
     if (!d.o_bulk) to = tq;  // (not used)
     d.o = p.o;
     d.mask = p.mask;
@@ -945,19 +948,18 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
 
     static PerDeviceOnce attr_once;
     if (!attr_once.run([] {
-            const int most = MODE == 0 ? Cfg::kSmemMode0 : MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase + (MODE == 3 ? Cfg::kMaskRingBytes : 0);
+            const int most = kNoMask ? Cfg::kSmemNoMask : MODE == 1 ? Cfg::kSmemMax : Cfg::kSmemBase + (MODE == 3 ? Cfg::kMaskRingBytes : 0);
             return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
     int64_t grid = items;
     unsigned int* queue = nullptr;
     if (MODE == 0) {
-        // one CTA per SM that draws its items; a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
-        grid = items < gemm_sms() ? items : gemm_sms();
+        grid = gemm_sms();  // a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
         queue = attention_queue_slot(stream);
         if (queue == nullptr) return KB_ERR_LAUNCH;
     }
-    const size_t smem_bytes = MODE == 0 ? (size_t)Cfg::kSmemMode0 : (size_t)Cfg::kSmemBase +
+    const size_t smem_bytes = kNoMask ? (size_t)Cfg::kSmemNoMask : (size_t)Cfg::kSmemBase +
         (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : MODE == 3 ? Cfg::kMaskRingBytes : 0);
     if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads, smem_bytes, stream, tq, tk, tv, to, d, (int)items, queue) != cudaSuccess)
         return KB_ERR_LAUNCH;
@@ -966,7 +968,12 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
 
 template <typename T, int D>
 static int launch_attention_td(const kb_attn_params& p, cudaStream_t stream) {
-    if (p.mask == nullptr && p.sm_scale > 0.f) return launch_attention_tdm<T, D, 0>(p, stream);
+    if (p.mask == nullptr && p.sm_scale > 0.f) {
+        // As many CTAs as pairs of query tiles where an SM holds them at once. (Drawing, counters and registers for several items cost a launch
+        // that has no second item 0.1 to 0.5 us: [4, 32, 200, 128] 9.9 -> 9.5, causal 9.75 -> 9.45, [4, 32 over 8, 130, 128] causal 9.5 -> 9.1.)
+        const int64_t items = (p.M + 2 * kAttnBlock - 1) / (2 * kAttnBlock) * p.B * p.H;
+        return items <= gemm_sms() ? launch_attention_tdm<T, D, 4>(p, stream) : launch_attention_tdm<T, D, 0>(p, stream);
+    }
     if (p.mask != nullptr && p.mask_strides[2] == 0)
         return p.N <= AttnCfg<D>::kMaskMaxN ? launch_attention_tdm<T, D, 1>(p, stream) : launch_attention_tdm<T, D, 3>(p, stream);
     return launch_attention_tdm<T, D, 2>(p, stream);

@@ -31,3 +31,27 @@ def test_items(B, H, HK, M, N, D, causal, layout, dtype):
     O.assert_parity(o, expected, max_abs=1e-2 if dtype == torch.float16 else 4e-2, what="attention")
     o.fill_(7.0)
     assert torch.equal(around, torch.full_like(around, 7.0))
+
+
+@pytest.mark.parametrize("layout", ["bulk", "odd_rows"])
+@pytest.mark.parametrize("causal", [False, True])
+@pytest.mark.parametrize("D", [72, 128])
+@pytest.mark.parametrize("more", [-1, 0, 1])
+def test_as_many_items_as_sms(lib, more, D, causal, layout):
+    """One item per CTA up to as many as there are SMs, CTAs that stay above: the same bits for the heads that both launches have."""
+    from kernl_b200.implementations.attention import attention_forward
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H = sms // 2 + more  # two pairs of tiles per head
+    g = torch.Generator(device="cuda").manual_seed(D + more)
+    q, k, v = (torch.randn((1, H + 40, 300, D), generator=g, device="cuda").half() for _ in range(3))
+
+    def call(heads):
+        o = torch.full((1, heads, 301, D + (3 if layout == "odd_rows" else 8)), 7.0, dtype=torch.float16, device="cuda")
+        attention_forward(q[:, :heads], k[:, :heads], v[:, :heads], o[:, :, :300, :D], D ** -0.5, causal, None)
+        return o
+
+    few, many = call(H), call(H + 40)
+    assert torch.equal(few, many[:, :H])
+    assert bool((few[:, :, 300] == 7.0).all()) and bool((few[:, :, :, D:] == 7.0).all())
+    O.assert_parity(few[:, :3, :300, :D], O.attention(q[:, :3].cpu(), k[:, :3].cpu(), v[:, :3].cpu(), D ** -0.5, causal, None), what="attention")
