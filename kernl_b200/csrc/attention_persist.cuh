@@ -948,7 +948,10 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     if (st != KB_OK) return st;
 
     AttnDev d;
-    d.o_bulk = attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, 32, p.H, true) == KB_OK ? 1 : 0;
+    // Without a mask and with heads below 64 the threads store for themselves: a box that ends inside a row's sectors costs more than it saves where
+    // nothing else of a tile takes long ([30, 12, 200, 40] 16.5 us, 17.5 with boxes; [64, 12, 130, 16 to 56] 26.4 to 27.8, 27.2 to 28.4). With a
+    // row mask boxes are the faster way there too ([64, 12, 130, 56] 31.7 -> 30.1).
+    d.o_bulk = (p.D == 64 || MODE != 0) && attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, 32, p.H, true) == KB_OK ? 1 : 0;
     if (!d.o_bulk) to = tq;  // (not used)
     d.o = p.o;
     d.mask = p.mask;
