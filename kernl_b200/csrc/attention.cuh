@@ -509,14 +509,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
                 // The item's last block is on its way, so the item is two blocks from its end: time to draw the next one. (A CTA
                 // that is busy with a long item should not hold back one that an idle CTA could start.)
                 if (u >= 2 && !mbar_wait(item_free(u & 1), (uint32_t)(((u >> 1) - 1) & 1), abort_flag, 102)) { ok = false; break; }
-                const int drawn = (int)gridDim.x + (int)atomicAdd(&queue[0], 1u);
-                items[u & 1] = drawn < num_items ? drawn : -1;
+                const unsigned int drawn = gridDim.x + atomicAdd(&queue[0], 1u);  // (up to num_items + 2 x gridDim.x: beyond 31 bits)
+                const bool more = drawn < (unsigned int)num_items;
+                items[u & 1] = more ? (int)drawn : -1;
                 mbar_arrive(item_full(u & 1));
-                if (drawn >= num_items) {
+                if (!more) {
                     pdl_launch_dependents();  // nothing more to draw: a dependent launch may take the SM once this item is done
                     break;
                 }
-                locate(drawn);
+                locate((int)drawn);
                 for (int t = 0; t < ntl; ++t) {
                     if (seen[t] > 0 && !mbar_wait(q_empty(t), (uint32_t)((seen[t] - 1) & 1), abort_flag, 103)) { ok = false; break; }
                     ++seen[t];
@@ -924,7 +925,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
     const int num_m_tiles = (int)((p.M + kAttnBlock - 1) / kAttnBlock);
     d.num_pairs = (num_m_tiles + 1) / 2;
     const int64_t items = (int64_t)d.num_pairs * p.B * p.H;
-    if (items > 0x3fffffff) return KB_ERR_UNSUPPORTED;
+    if (items > 0x7fffffff) return KB_ERR_UNSUPPORTED;
     d.o_bulk = kNoMask && attn_bulk_out(p) && enc(&to, p.o, p.M, p.o_strides, p.H, 32) == KB_OK ? 1 : 0;
     if (!d.o_bulk) to = tq;  // (not used)
     d.o = p.o;
