@@ -30,6 +30,10 @@ void kb_debug_attention_short(int mode);
 /* 0 = large GEMMs stay on the one-CTA-per-tile kernel instead of CTA pairs on 256-row tiles;
  * 192 / 256 = CTA pairs with that tile width whatever the cost model says; 1 = dispatcher's choice. */
 void kb_debug_linear_pair(int mode);
+/* Work queues of the persistent attention kernels on the current device. what = 0: the slot that the last launch of the process took (eager
+ * launches 0 ... 1023, captured ones 1024 and above), -1 before any; 1: how many slots graphs own at present; 2: at most `limit` slots for
+ * graphs (a limit outside 0 ... 65536 restores the default). */
+int kb_debug_attention_slots(int what, int limit);
 /* 0 = launch every kernel with plain stream ordering instead of programmatic dependent launch. */
 void kb_debug_pdl(int on);
 /* Limits (SM clock cycles) of the bounded device-side waits on the CURRENT device: waits inside one

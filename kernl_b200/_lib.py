@@ -146,6 +146,9 @@ def load() -> ctypes.CDLL:
         if hasattr(lib, hook):
             getattr(lib, hook).argtypes = [ctypes.c_int]
             getattr(lib, hook).restype = None
+    if hasattr(lib, "kb_debug_attention_slots"):
+        lib.kb_debug_attention_slots.argtypes = [ctypes.c_int, ctypes.c_int]
+        lib.kb_debug_attention_slots.restype = ctypes.c_int
     if hasattr(lib, "kb_debug_wait_limit"):
         lib.kb_debug_wait_limit.argtypes = [c_int64, c_int64]
         lib.kb_debug_wait_limit.restype = ctypes.c_int

@@ -52,42 +52,99 @@ static_assert(attn_regs_low(0) % 8 == 0 && attn_regs_high(0) % 8 == 0 && attn_re
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLazyThreshold = 8.0f;
 
-// Work queues of the persistent kernels. A launch takes the next slot (host-side round robin) and its CTAs draw tile numbers
+// Work queues of the persistent kernels. A launch has a slot and its CTAs draw tile numbers
 // from slot[0]; slot[1] counts CTAs that have finished, and the last one puts both words back to
 // zero, so a slot is clean again when its launch ends — also when the launch gave up on an expired
-// wait. Two launches would have to be in flight kAttnQueueSlots launches apart to share a slot. Captured launches, which come
-// again whenever their graph is replayed, have slots of their own (half a megabyte): a replay shares none with the calls of another
-// stream, and two graphs would have to be kAttnGraphSlots captured launches apart.
+// wait. Eager launches take theirs from a ring: two would have to be in flight kAttnQueueSlots launches apart to share one.
+// A captured launch comes again whenever its graph is replayed, beside the calls of other streams, so it owns its slot for as long as
+// the graph, or one instantiated or cloned from it, exists.
 constexpr int kAttnQueueSlots = 1024, kAttnGraphSlots = 65536;
 __device__ unsigned int g_attn_queue[kAttnQueueSlots + kAttnGraphSlots][2];
 
-// The next queue slot on the current device. g_attn_queue is a host-side handle; its device address
-// is looked up once per device (with that device current) and kept.
-static unsigned int* attention_queue_slot(cudaStream_t stream) {
-    static unsigned int* base[64] = {};
-    static std::mutex mu;
-    static std::atomic<unsigned> next_slot{0}, next_graph_slot{0};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-    {
-        std::lock_guard<std::mutex> lock(mu);
-        if (base[dev] == nullptr) {
-            void* ptr = nullptr;
-            if (cudaGetSymbolAddress(&ptr, g_attn_queue) != cudaSuccess || ptr == nullptr) {
-                cudaGetLastError();
-                return nullptr;
+struct AttnSlots {  // of one device
+    std::atomic<unsigned int*> base{nullptr};  // g_attn_queue there (the symbol is a host-side handle)
+    std::atomic<unsigned> next{0};             // the eager ring
+    std::atomic<unsigned> from{0};             // where the next search begins
+    std::atomic<int> held{0};                  // slots that graphs own
+    std::atomic<uint64_t> owned[kAttnGraphSlots / 64] = {};
+};
+static AttnSlots g_attn_slots[64];
+static int g_attn_graph_slots = kAttnGraphSlots;  // test hook (kb_debug_attention_slots)
+static std::atomic<int> g_attn_last_slot{-1};     // likewise
+
+// A free slot of the captured launches' pool, now owned; -1: none.
+static int attention_own_slot(AttnSlots& d) {
+    const unsigned words = (unsigned)(g_attn_graph_slots + 63) / 64, first = words > 0 ? d.from.load() % words : 0;
+    for (unsigned n = 0; n < words; ++n) {
+        const unsigned w = (first + n) % words;
+        uint64_t seen = d.owned[w].load();
+        while (~seen != 0) {
+            const int bit = __builtin_ctzll(~seen);
+            if ((int)(w * 64) + bit >= g_attn_graph_slots) break;
+            if (d.owned[w].compare_exchange_weak(seen, seen | (1ull << bit))) {
+                d.from.store(w);
+                d.held.fetch_add(1);
+                return (int)(w * 64) + bit;
             }
-            base[dev] = reinterpret_cast<unsigned int*>(ptr);
         }
     }
+    return -1;
+}
+// The last graph that owned a slot is gone (called by CUDA on a thread of its own, after the last replay has ended).
+static void CUDART_CB attention_free_slot(void* which) {
+    const uintptr_t id = (uintptr_t)which - 1;
+    AttnSlots& d = g_attn_slots[id / kAttnGraphSlots];
+    const unsigned slot = (unsigned)(id % kAttnGraphSlots);
+    d.owned[slot / 64].fetch_and(~(1ull << (slot % 64)));
+    d.held.fetch_sub(1);
+}
+
+// A queue slot on the current device for a launch into `stream`. nullptr: none (as many captured launches as there are slots; the caller
+// has a form that does not draw), or no device.
+static unsigned int* attention_queue_slot(cudaStream_t stream) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    AttnSlots& d = g_attn_slots[dev];
+    unsigned int* base = d.base.load(std::memory_order_acquire);
+    if (base == nullptr) {
+        void* ptr = nullptr;
+        if (cudaGetSymbolAddress(&ptr, g_attn_queue) != cudaSuccess || ptr == nullptr) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        base = reinterpret_cast<unsigned int*>(ptr);
+        d.base.store(base, std::memory_order_release);
+    }
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(stream, &capture) != cudaSuccess) {  // (the legacy stream while another one is captured: the launch will say so)
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo_v2(stream, &capture, nullptr, &graph) != cudaSuccess) {  // (the legacy stream while another one is captured: the launch will say so)
         cudaGetLastError();
         capture = cudaStreamCaptureStatusNone;
     }
-    if (capture != cudaStreamCaptureStatusNone)
-        return base[dev] + 2 * (kAttnQueueSlots + next_graph_slot.fetch_add(1) % (unsigned)kAttnGraphSlots);
-    return base[dev] + 2 * (next_slot.fetch_add(1) % (unsigned)kAttnQueueSlots);
+    if (capture == cudaStreamCaptureStatusNone) {
+        const int slot = (int)(d.next.fetch_add(1) % (unsigned)kAttnQueueSlots);
+        g_attn_last_slot.store(slot, std::memory_order_relaxed);
+        return base + 2 * slot;
+    }
+    const int slot = attention_own_slot(d);
+    if (slot < 0) return nullptr;
+    const uintptr_t id = (uintptr_t)dev * kAttnGraphSlots + (uintptr_t)slot;
+    cudaUserObject_t owner = nullptr;
+    if (cudaUserObjectCreate(&owner, reinterpret_cast<void*>(id + 1), attention_free_slot, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        attention_free_slot(reinterpret_cast<void*>(id + 1));
+        return nullptr;
+    }
+    if (graph == nullptr || cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(owner, 1);  // (gives the slot back)
+        return nullptr;
+    }
+    g_attn_last_slot.store(kAttnQueueSlots + slot, std::memory_order_relaxed);
+    return base + 2 * (kAttnQueueSlots + slot);
 }
 
 struct AttnDev {
@@ -895,7 +952,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
 }
 
 template <typename T, int D, int MODE>
-static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
+static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream, unsigned int* queue = nullptr) {
     using Cfg = AttnCfg<D>;
     constexpr bool kNoMask = MODE == 0 || MODE == 4;
     CUtensorMap tq, tk, tv, to;
@@ -953,13 +1010,7 @@ static int launch_attention_tdm(const kb_attn_params& p, cudaStream_t stream) {
             return cudaFuncSetAttribute(attention_tc_kernel<T, D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, most) == cudaSuccess;
         }))
         return KB_ERR_LAUNCH;
-    int64_t grid = items;
-    unsigned int* queue = nullptr;
-    if (MODE == 0) {
-        grid = gemm_sms();  // a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
-        queue = attention_queue_slot(stream);
-        if (queue == nullptr) return KB_ERR_LAUNCH;
-    }
+    const int64_t grid = MODE == 0 ? gemm_sms() : items;  // a caller-set limit leaves SMs to a concurrent collective, as for the GEMMs
     const size_t smem_bytes = kNoMask ? (size_t)Cfg::kSmemNoMask : (size_t)Cfg::kSmemBase +
         (MODE == 1 ? (size_t)((p.N + kAttnBlock - 1) / kAttnBlock) * kAttnBlock * 4 : MODE == 3 ? Cfg::kMaskRingBytes : 0);
     if (launch_pdl(attention_tc_kernel<T, D, MODE>, (unsigned)grid, kAttnThreads, smem_bytes, stream, tq, tk, tv, to, d, (int)items, queue) != cudaSuccess)
@@ -973,7 +1024,8 @@ static int launch_attention_td(const kb_attn_params& p, cudaStream_t stream) {
         // As many CTAs as pairs of query tiles where an SM holds them at once. (Drawing, counters and registers for several items cost a launch
         // that has no second item 0.1 to 0.5 us: [4, 32, 200, 128] 9.9 -> 9.5, causal 9.75 -> 9.45, [4, 32 over 8, 130, 128] causal 9.5 -> 9.1.)
         const int64_t items = (p.M + 2 * kAttnBlock - 1) / (2 * kAttnBlock) * p.B * p.H;
-        return items <= gemm_sms() ? launch_attention_tdm<T, D, 4>(p, stream) : launch_attention_tdm<T, D, 0>(p, stream);
+        unsigned int* queue = items > gemm_sms() ? attention_queue_slot(stream) : nullptr;
+        return queue == nullptr ? launch_attention_tdm<T, D, 4>(p, stream) : launch_attention_tdm<T, D, 0>(p, stream, queue);
     }
     if (p.mask != nullptr && p.mask_strides[2] == 0)
         return p.N <= AttnCfg<D>::kMaskMaxN ? launch_attention_tdm<T, D, 1>(p, stream) : launch_attention_tdm<T, D, 3>(p, stream);

@@ -926,7 +926,7 @@ static bool attention_persist_applicable(const kb_attn_params& p, int mode) {
 static int g_attn_sort_batches = 1;  // test hook (kb_debug_attention_persistent: bit 1 of the mode switches it off)
 
 template <typename T, int MODE>
-static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream) {
+static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream, unsigned int* queue) {
     using Cfg = AttnPersistCfg;
     CUtensorMap tq, tk, tv, to;
     const int64_t kv_group = p.kv_group > 1 ? p.kv_group : 1;
@@ -994,8 +994,6 @@ static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t str
     if (smem_bytes > (size_t)Cfg::kSmemLimit) return KB_ERR_UNSUPPORTED;
     const int64_t tiles = (int64_t)d.num_pairs * p.B * p.H;
     const int64_t grid = tiles < 2 * (int64_t)sm_count() ? tiles : 2 * (int64_t)sm_count();
-    unsigned int* queue = attention_queue_slot(stream);
-    if (queue == nullptr) return KB_ERR_LAUNCH;
     // Longest-first order of the batches: for padding masks (one row per batch, shared by heads and
     // query rows) of a size that every CTA can scan during its set-up.
     const int sort_batches = (MODE == 1 && g_attn_sort_batches && !p.is_causal && p.mask_strides[1] == 0 && p.mask_strides[0] != 0 &&

@@ -723,17 +723,18 @@ static int launch_attention_split_tm(const kb_attn_params& p, cudaStream_t strea
 // The persistent form of this kernel (attention_persist.cuh) takes the launches it is made for.
 static bool attention_persist_applicable(const kb_attn_params& p, int mode);
 template <typename T, int MODE>
-static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream);
+static int launch_attention_persist_tm(const kb_attn_params& p, cudaStream_t stream, unsigned int* queue);
 
 template <typename T>
 static int launch_attention_split_t(const kb_attn_params& p, cudaStream_t stream) {
     const int mode = (p.mask == nullptr && p.sm_scale > 0.f) ? 0
                      : (p.mask != nullptr && p.mask_strides[2] == 0 && p.N <= AttnSplitCfg<1>::kMaskMaxN) ? 1
                      : (p.mask_strides[2] != 0 && mask_is_staged(p)) ? 3 : 2;
-    if (g_split_tiles == 0 && attention_persist_applicable(p, mode)) {
-        if (mode == 0) return launch_attention_persist_tm<T, 0>(p, stream);
-        if (mode == 1) return launch_attention_persist_tm<T, 1>(p, stream);
-        return launch_attention_persist_tm<T, 2>(p, stream);
+    unsigned int* queue = g_split_tiles == 0 && attention_persist_applicable(p, mode) ? attention_queue_slot(stream) : nullptr;
+    if (queue != nullptr) {
+        if (mode == 0) return launch_attention_persist_tm<T, 0>(p, stream, queue);
+        if (mode == 1) return launch_attention_persist_tm<T, 1>(p, stream, queue);
+        return launch_attention_persist_tm<T, 2>(p, stream, queue);
     }
     if (mode == 0) return launch_attention_split_tm<T, 0>(p, stream);
     if (mode == 1) return launch_attention_split_tm<T, 1>(p, stream);

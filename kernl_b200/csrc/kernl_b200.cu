@@ -178,6 +178,16 @@ void kb_debug_attention_persistent(int mode) {
     g_attn_sort_batches = mode == 2 ? 0 : 1;
 }
 void kb_debug_attention_short(int mode) { g_attn_short = mode; }
+int kb_debug_attention_slots(int what, int limit) {
+    if (what == 0) return g_attn_last_slot.load();
+    if (what == 2) g_attn_graph_slots = limit >= 0 && limit <= kAttnGraphSlots ? limit : kAttnGraphSlots;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        cudaGetLastError();
+        return -1;
+    }
+    return g_attn_slots[dev].held.load();
+}
 void kb_debug_pdl(int on) { g_use_pdl = on ? 1 : 0; }
 void kb_debug_linear_pair(int mode) { g_linear_pair = (mode == 192 || mode == 256) ? mode : (mode ? 1 : 0); }
 void kb_debug_force_splits(int splits) { g_forced_splits = splits; }
