@@ -109,3 +109,39 @@ def test_kernels_with_waits_store_nothing_after_an_expiry(lib, kernel):
         assert lib.kb_debug_wait_limit(0, 0) == 0
         for hook, _, off in hooks:
             hook(off)
+
+
+@pytest.mark.parametrize("D, shape", [(128, (10, 16, 300)), (64, (6, 16, 700))])
+def test_queues_are_clean_after_an_expiry(lib, D, shape):
+    """Launches that draw their tiles from a counter put it back also when they skip their work: every slot of the ring serves a full
+    launch afterwards."""
+    from kernl_b200 import _lib
+    from kernl_b200.implementations.attention import attention_forward
+
+    dev = torch.device("cuda", 0)
+    bufs = [torch.zeros(4096, dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    flags = [torch.zeros(64, dtype=torch.int32, device=dev) for _ in range(2)]
+    out = torch.zeros(4096, dtype=torch.bfloat16, device=dev)
+    g = torch.Generator(device="cuda").manual_seed(D)
+    B, H, S = shape
+    q = torch.randn((B, H, S, D), generator=g, device=dev).half()
+    expected = attention_forward(q, q, q, torch.empty_like(q), D ** -0.5, True, None)
+    skipped = torch.full_like(q, 7.0)
+    _lib.device_status()
+    try:
+        assert lib.kb_debug_wait_limit(0, 20000) == 0
+        assert lib.kb_allreduce_residual_fwd(_params(bufs, flags, out, out), _lib.current_stream(dev)) == 0
+        for _ in range(3):
+            attention_forward(q, q, q, skipped, D ** -0.5, True, None)
+        slot = lib.kb_debug_attention_slots(0, 0)
+        with pytest.raises(RuntimeError, match="wait expired"):
+            _lib.device_status()
+    finally:
+        assert lib.kb_debug_wait_limit(0, 0) == 0
+    assert bool((skipped == 7.0).all())
+    slots = set()
+    for _ in range(1030):
+        got = attention_forward(q, q, q, torch.zeros_like(q), D ** -0.5, True, None)
+        slots.add(lib.kb_debug_attention_slots(0, 0))
+        assert torch.equal(got, expected)
+    assert slot in slots and len(slots) == 1024
