@@ -22,7 +22,8 @@
 //   empty[s]   in each CTA: `tcgen05.commit` of the leader, multicast to both CTAs;
 //   tfull[a]   in each CTA: accumulator a complete (multicast commit);
 //   tempty[a]  in the leader: all 32 epilogue warps of the pair have read accumulator a (a warp
-//              arrives as soon as its columns are in registers).
+//              arrives as soon as the last of its columns are in registers: ahead of the conversion and store of its only box of 48,
+//              or of the second of its two boxes of 32; behind the second one's store [4096, 256] x [8192, 256] took 23.4 us, 22.3 so).
 // Accumulators are double-buffered (2 x 256 columns = all of tensor memory), the ring has six stages.
 // Every bulk copy has one destination CTA: the pair's sharing happens inside the tensor-core instruction.
 #pragma once
@@ -400,6 +401,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                     const int ycol = gated ? (n0 + c_begin) / 2 : n0 + c_begin + bx * SC;
                     if (gated && bx + 1 < CW / SC) {  // (half of the box only)
                         tmem_ld_wait();
+                        if (bx + 2 == CW / SC) release();
                         continue;
                     }
                     int part = 0, b0 = 0, head = 0, d0 = 0;  // ROPE: q, k or v; the first row's sequence; head and its first column
@@ -474,9 +476,11 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
                         }
                         bulk_commit();
                     }
-                    if (bx + 1 < CW / SC) tmem_ld_wait();
+                    if (bx + 1 < CW / SC) {
+                        tmem_ld_wait();
+                        if (bx + 2 == CW / SC) release();  // the last box is in registers
+                    }
                 }
-                if (SC != CW) release();
                 if (t + num_pairs < num_tiles) tile_coords(t + num_pairs, num_m, num_n, m_idx, n_idx);
             } else {
                 const int row = row_base + lane;
