@@ -258,12 +258,14 @@ int kb_attention_decode_fwd_static(const kb_attn_params* p, void* stream);
  * kb_device_status_read synchronises the current device, returns the word and clears it. */
 int kb_device_status_read(int32_t* status_out);
 
-/* ---- SMs for the persistent GEMM kernels ------------------------------------------------
- * The fused-linear kernels for large problems are persistent: one CTA (or CTA pair) per SM for the
- * whole launch, so a collective that should run AT THE SAME TIME (the all-reduce of one half of a
- * batch while the other half computes) finds no SM until the GEMM ends. kb_gemm_sm_limit(n) makes
- * later launches use at most n SMs (0 = all, the default); the setting is process-wide and read
- * when a launch is enqueued. Nothing in the reference corresponds to it (it has no multi-GPU path). */
+/* ---- SMs for the persistent kernels -------------------------------------------------------
+ * Some kernels hold every SM they get for the whole launch: the fused-linear kernels for large problems (one CTA, or
+ * CTA pair, per SM) and attention above head dimension 64 without a mask in launches of more pairs of 128-row query tiles than SMs
+ * (one CTA per SM). A collective that should run AT THE SAME TIME (the all-reduce of one half of a
+ * batch while the other half computes) finds no SM until such a launch ends. kb_gemm_sm_limit(n) makes
+ * later launches of these use at most n SMs (0 = all, the default); the setting is process-wide and read
+ * when a launch is enqueued. It does not reach attention up to head dimension 64, whose CTAs stay as well in launches of more
+ * than two query tiles per SM and take two CTA slots of every SM. Nothing in the reference corresponds to it (it has no multi-GPU path). */
 int kb_gemm_sm_limit(int sms);
 
 const char* kb_status_str(int status);

@@ -11,7 +11,7 @@
 //
 // Roles per CTA (576 threads): warp 0 TMA producer, warp 1 tcgen05 issuer (only the pair's leader —
 // cluster rank 0 — issues; the other CTA's warp 1 only allocates tensor memory), warps 2..17
-// epilogue: warp w reads the tensor-memory lanes of quadrant w % 4 (its 32 rows) and the 64 columns
+// epilogue: warp w reads the tensor-memory lanes of quadrant w % 4 (its 32 rows) and the 64 (narrow tile: 48) columns
 // (w - 2) / 4 of the CTA's 128 x 256 accumulator. Sixteen warps, because with a short K loop the
 // epilogue is the longer of the two pipelines: clock stamps at K = 768 showed eight warps needing
 // 7500-9000 cycles per tile (tensor-memory reads, conversion and stores each saturate their unit in
@@ -134,10 +134,11 @@ __device__ long long g_gemm_trace[148 * 8 * 16];
 #define KB_GTRACE(tile, ev) do { } while (0)
 #endif
 
-// BN: columns of the pair's tile, 256 or 192. Each CTA stages BN / 2 rows of W per stage (the stage
-// keeps its 32 KB stride), the accumulators sit at tensor-memory columns 0 and 256 whatever BN, and an
-// epilogue warp owns BN / 4 columns. The narrower tile exists for problems of a few rounds: 384 tiles
-// of 256 columns on 74 pairs run 5.2 rounds as 6, 512 tiles of 192 columns run 6.9 rounds as 7.
+// BN: columns of the pair's tile, 256 or 192. Each CTA stages BN / 2 rows of W per stage (32 or 28 KB a stage),
+// the accumulators sit at tensor-memory columns 0 and 256 whatever BN, and an epilogue warp owns BN / 4 columns. The narrower
+// tile leaves less undone where the wide one does not fill its rounds: [1800, 768] x [3072, 768] is 96 wide tiles on 74 pairs, two rounds
+// and 13.5 us, or 128 narrow ones, two cheaper rounds and 12.5; one-round problems have the cheaper round, too. (Where both take several rounds
+// there is little between them: [8192, 768] x [3072, 768], 6 or 7 rounds, 34.9 us both.)
 // ROPE: a stacked q/k/v projection whose results are rotated (q, k) on their way out and whose k and v go to the cache, [B, H, max_seq, D].
 // Saves the kernel behind it its pass over the projection's result (402 MB per layer at 8192 rows of [12288, 4096], 74 us).
 struct PairRope {

@@ -173,9 +173,9 @@ class LlamaTP:
         self.vcache = None
         self.sm_scale = D ** -0.5
         self.overlap_prefill = True  # two half-batches on two streams when tensor parallel (see prefill)
-        # SMs left free for the collective while the two halves overlap: the GEMMs of the prefill are
+        # SMs left free for the collective while the two halves overlap: the GEMMs of the prefill and its attention are
         # persistent (one CTA per SM for the whole launch), so without this an all-reduce that is ready
-        # to run finds no SM until the other half's GEMM has ended. 24 goes with a collective limited to
+        # to run finds no SM until the other half's launch has ended. 24 goes with a collective limited to
         # 24 CTAs (NCCL_MAX_CTAS=24, set by the caller before the process group exists); measured at
         # TP = 4, prefill 8 x 2048: 66.7 ms with nothing reserved, 61.5 ms with 24 / 24. Two ranks exchange
         # less; there the setting did not move the result (101.7-106.0 ms with 16 or 24 SMs)
