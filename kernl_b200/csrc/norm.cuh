@@ -46,10 +46,11 @@ constexpr int kNormMaxCols = 16384;  // longest row that is held in registers
 // its greedy tokens with them. Nothing more is promised: the same row in a launch of up to 1024 rows, longer rows
 // (eight warps) and LayerNorm add up their warps' sums pairwise. The hand-over is
 // hidden behind the other CTAs of the SM.
-// EARLY (up to 64 rows of more than 1024 columns: the norms of a decode step): gamma, beta and the residual are asked for in L2 ahead of the
+// EARLY (up to 64 rows of 1025 to 4096 columns: the norms of a decode step): gamma, beta and the residual are asked for in L2 ahead of the
 // wait; behind it they would queue behind the weights that the next GEMM asks for (8 rows of 4096: 5.2 -> 3.8 us between the ends of the
-// two kernels, a step of eight layers 1034 -> 1019). With more rows it is a second pass over the residual: LayerNorm of [500, 3000]
-// 4.0 us without, 4.4 with it, of [2430, 2368] 9.9 and 12.0.
+// two kernels, a step of eight layers 1034 -> 1019). A decode step of four layers without and with it: 16 rows 475 and 467 us, 32 548 and 538,
+// 64 649 and 642, 96 760 and 753, 128 852 and 847, 192 and 256 rows no difference. With hundreds of rows it is a second pass over the residual:
+// LayerNorm of [500, 3000] 4.0 us without, 4.4 with it, of [2430, 2368] 9.9 and 12.0. Rows of 8192 (eight warps): no difference at 8 and 64 rows.
 template <typename T, int CHUNKS, bool RMS, int WPR = 1, bool CHAIN = false, bool EARLY = false>
 __global__ void __launch_bounds__(WPR == 8 ? 256 : 128)
 norm_fwd_rowwarp_kernel(const T* __restrict__ x, T* __restrict__ y, const T* __restrict__ gamma,
