@@ -57,7 +57,7 @@ constexpr float kLazyThreshold = 8.0f;
 // zero, so a slot is clean again when its launch ends — also when the launch gave up on an expired
 // wait. Eager launches take theirs from a ring: two would have to be in flight kAttnQueueSlots launches apart to share one.
 // A captured launch comes again whenever its graph is replayed, beside the calls of other streams, so it owns its slot for as long as
-// the graph, or one instantiated or cloned from it, exists.
+// the graph, or one instantiated or cloned from it, exists. (A graph that is only used to update another's instantiation has to outlive that.)
 constexpr int kAttnQueueSlots = 1024, kAttnGraphSlots = 65536;
 __device__ unsigned int g_attn_queue[kAttnQueueSlots + kAttnGraphSlots][2];
 
